@@ -1617,7 +1617,15 @@ int autotune_trials(gbh_engine *e)
         for (Save &s : saves) cudaFree(s.dst);
         return GBH_ERR_CUDA;
     }
-    for (Save &s : saves) CK(cudaMemcpy(s.dst, s.src, s.bytes, cudaMemcpyDeviceToDevice));
+    // save and restore on the engine's own stream: device-to-device copies on
+    // the default stream return before they are done, and the trials' kernels
+    // (a non-blocking stream) would overtake them
+    for (Save &s : saves) CK(cudaMemcpyAsync(s.dst, s.src, s.bytes, cudaMemcpyDeviceToDevice, e->stream));
+    auto restore = [&]() {
+        for (Save &s : saves)
+            CK(cudaMemcpyAsync((void *)s.src, s.dst, s.bytes, cudaMemcpyDeviceToDevice, e->stream));
+        return GBH_OK;
+    };
     double best = 1e300;
     int best_v = 0, best_s = spls[0];
     for (int vi = 0; vi < nvar; ++vi) {
@@ -1641,7 +1649,7 @@ int autotune_trials(gbh_engine *e)
                         e->jit_warps[vi], e->jit_minb[vi], e->jit_compact[vi] ? 1 : e->jit_smemrows[vi] ? 2 : 0, spl,
                         per * 1e3);
             if (per < best) { best = per; best_v = vi; best_s = spl; }
-            for (Save &s : saves) CK(cudaMemcpy((void *)s.src, s.dst, s.bytes, cudaMemcpyDeviceToDevice));
+            if (restore()) return GBH_ERR_CUDA;
         }
     }
     // networks: the cooperative multi-step launch against the best per-step plan
@@ -1671,7 +1679,7 @@ int autotune_trials(gbh_engine *e)
                 cudaGetLastError();   // e.g. too many tiles to be resident at once: keep per-step launches
             }
             e->net_coop = false;
-            for (Save &s : saves) CK(cudaMemcpy((void *)s.src, s.dst, s.bytes, cudaMemcpyDeviceToDevice));
+            if (restore()) return GBH_ERR_CUDA;
         }
         int status = 0;
         CK(cudaMemcpy(&status, e->d_status.p, sizeof(int), cudaMemcpyDeviceToHost));
@@ -1685,9 +1693,11 @@ int autotune_trials(gbh_engine *e)
             e->net_spl = coop_k;
         }
     }
+    CK(cudaStreamSynchronize(e->stream));
     for (Save &s : saves) cudaFree(s.dst);
-    if (e->d_spiked.p) CK(cudaMemset(e->d_spiked.p, 0, e->d_spiked.n * sizeof(unsigned)));   // trial spikes
-    if (e->rows_itot) CK(cudaMemset(e->d_IT.p, 0, e->d_IT.n * sizeof(double)));   // trial itotal sums
+    if (e->d_spiked.p)   // trial spikes
+        CK(cudaMemsetAsync(e->d_spiked.p, 0, e->d_spiked.n * sizeof(unsigned), e->stream));
+    if (e->rows_itot) CK(cudaMemsetAsync(e->d_IT.p, 0, e->d_IT.n * sizeof(double), e->stream));   // trial itotal sums
     for (size_t k = 0; k < e->jits.size(); ++k) e->jits[k] = e->jit_var[k][best_v];
     e->jit_choice = best_v;
     e->steps_per_launch = best_s;
