@@ -84,6 +84,7 @@ struct Launch {
     bool wide = false;    // one neuron per block (wide tiles)
     bool stack = false;   // stack elimination (smax = shared doubles per lane)
     bool split = false;   // stack: some tile's rows above its static ones go to a second warp
+    int level = -1;       // level elimination: kernel index (tile0..tile1 are groups, smax the shared bytes)
 };
 
 // Element idx of a block of rows starting at row `base`: lane-interleaved
@@ -166,6 +167,15 @@ struct gbh_engine {
     int64_t rows_fld = 0, rows_int = 0, rows_pool = 0, rows_giv = 0, rows_vm = 0, rows_topo = 0,
             rows_syn = 0, rows_scr = 0, rows_rav = 0, rows_itot = 0;
     std::vector<Launch> launches;
+    std::vector<Launch> giv_launches;   // the plan of a step that records givals, where it differs
+    // level elimination (gbh_level.cuh)
+    std::vector<JitKernel> lv_kern;
+    DBuf<LevelGroup> d_lgroups;
+    DBuf<int2> d_lchunks;
+    DBuf<int> d_lmap, d_lkid, d_lpar, d_ltopkid;
+    DBuf<double2> d_lkt, d_lcy;
+    DBuf<double> d_ld, d_lpd;
+    DBuf<unsigned> d_lgen;
     int steps_per_launch = 1;
     bool has_network = false;
     bool givals_enabled = false;
@@ -331,6 +341,38 @@ std::vector<int> slot_field_ranges(const std::vector<int> &prog, const TileType 
     return out;
 }
 
+// Rows below the first compartment with channels (TileType::nstatic), from
+// slot_field_ranges.
+int static_rows(const std::vector<int> &pf, int nslots)
+{
+    int n = 0;
+    while (n < nslots && pf[6 * n + 2] >= 0) ++n;
+    return n;
+}
+
+// A neuron's tile type but for the offsets of its programs.
+TileType tile_type_of(const Neuron &N)
+{
+    TileType tt{};
+    tt.nslots = N.nrows;
+    tt.nfields = (int)N.fsrc.size();
+    tt.nints = (int)N.iops.size();
+    tt.npools = (int)N.pool_conc.size();
+    tt.ngiv = (int)N.giv_ref.size();
+    tt.table_set = N.table_set;
+    tt.crank = N.crank;
+    tt.chanmode5 = N.c5;
+    tt.interp = N.interp;
+    tt.has_spike = N.spike_op >= 0;
+    tt.nsyn = (int)N.syn_op.size();
+    tt.has_cd = N.has_cd;
+    tt.nscratch = N.nscratch;
+    tt.sym = !N.sym.empty();
+    tt.nrav = (int)N.rav.size();
+    tt.nitot = N.nitot;
+    return tt;
+}
+
 // Slot and rows of the spike detector in a type's program (M_SPIKE operands:
 // threshold field, counter and refractory int rows).
 bool spike_rows(const std::vector<int> &prog, const TileType &tt, int &slot, int &fth, int &icnt, int &iref)
@@ -405,6 +447,15 @@ constexpr int kSmemPerBlock = 96 * 1024;
 constexpr int kStackMin = 8;
 // Shared memory a stack-elimination warp may take (doubles per lane).
 constexpr int kStackCapMax = 200 * 1024 / (LANES * (int)sizeof(double)) - 2 * kSplitRows;
+
+// Level elimination: shared memory of a block, groups wanted (two a SM of
+// the 152) and distinct programs compiled.
+constexpr int kLevelSmemMax = 224 * 1024, kLevelGroups = 304;
+constexpr size_t kLevelKernels = 8;
+
+// Largest types specialised whole: the looped forms keep 2 x nslots x 32 rows
+// per warp in shared memory, 4-warp blocks of more would not fit.
+constexpr int kJitMaxSlots = 96;
 
 // Composite tables on the device: FP64 copy (plus one padding row), axis
 // value pools and their geometry.
@@ -642,6 +693,217 @@ void wide_schedule(const std::vector<int> &parent, std::vector<int> &out)
     out.insert(out.end(), br.begin(), br.end());
 }
 
+// ---- level elimination (gbh_level.cuh) ----
+// Is a type of neurons with passive dendrites swept level by level? Not when
+// its neurons share one tree of little branching (fewer than two rows a
+// level, as in a cable): the specialised kernel then keeps the rows in
+// registers and needs neither barriers nor indices. parent: any neuron's.
+bool level_type(const TileType &tt, const std::vector<int> &prog, const std::vector<int> &parent, bool uniform,
+                LevelProg &lp)
+{
+    if (!tt.stack) return false;
+    if (uniform && tt.nslots <= kJitMaxSlots) {
+        std::vector<int> depth(tt.nslots, 0);
+        int levels = 0;
+        for (int s = tt.nstatic - 1; s >= 0; --s) {   // children have lower rows than their parents
+            depth[s] = parent[s] < tt.nstatic ? depth[parent[s]] + 1 : 1;
+            levels = std::max(levels, depth[s]);
+        }
+        if (tt.nstatic < 2 * levels) return false;
+    }
+    if (level_smem(kSplitRows, tt.nstatic, tt.nstatic + 1, tt.crank != 0) > (size_t)kLevelSmemMax) return false;
+    if (tt.nstatic * LANES >= 1 << LV_KID_BITS) return false;
+    lp = level_prog(tt, prog);
+    return lp.ok;
+}
+
+struct LevelPlan {
+    std::vector<LevelGroup> groups;
+    std::vector<Launch> launches;
+};
+
+// One group's level order: appends its rows, chunks (of `nt` rows at most)
+// and the top rows' static children to the pools.
+struct LevelPools {
+    std::vector<int2> chunks;
+    std::vector<int> map, kid, par, topkid;
+    std::vector<double2> cy;
+};
+
+// Level order of the static rows of a group: order[] = row * 32 + group lane,
+// level starts; kid / par as LevelView holds them. Rows of a level are
+// sorted by their parent's place, then ascending, so a row's children are
+// consecutive and in the order the sequential sweep subtracts them.
+void level_order(const std::vector<const Neuron *> &cells, int nst, int ntop, std::vector<int> &order,
+                 std::vector<int> &start, std::vector<int> &kid, std::vector<int> &par, std::vector<int> &topkid)
+{
+    const int nl = (int)cells.size();
+    std::vector<std::vector<int>> kids((size_t)(nst + ntop) * nl);   // static children of row * nl + lane, ascending
+    for (int l = 0; l < nl; ++l)
+        for (int s = 0; s < nst; ++s) kids[(size_t)cells[l]->parent[s] * nl + l].push_back(s);
+    order.clear();
+    kid.assign((size_t)nst * nl, 0);
+    par.assign((size_t)nst * nl, 0);
+    topkid.assign((size_t)ntop * LANES, 0);
+    start.assign(1, 0);
+    auto put = [&](int row, int l, int p) {   // the children of a row whose solution is at p
+        const std::vector<int> &c = kids[(size_t)row * nl + l];
+        const int word = (int)order.size() | (int)((unsigned)c.size() << LV_KID_BITS);
+        for (int k : c) {
+            par[order.size()] = p;
+            order.push_back(k * LANES + l);
+        }
+        return word;
+    };
+    for (int s = 0; s < ntop; ++s)
+        for (int l = 0; l < nl; ++l) topkid[s * LANES + l] = put(nst + s, l, s * LANES + l);
+    while ((int)order.size() > start.back()) {
+        const int e0 = start.back(), e1 = (int)order.size();
+        start.push_back(e1);
+        for (int e = e0; e < e1; ++e) kid[e] = put(order[e] / LANES, order[e] % LANES, ntop * LANES + e);
+    }
+}
+
+int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const std::vector<int> &prog_pool,
+               const std::vector<TableGeom> &tg, LevelPlan &out)
+{
+    const Decoded &dec = e->dec;
+    const bool mixed = e->opt.precision == GBH_PREC_MIXED;
+    // ---- eligible types and their kernels ----
+    std::map<std::string, int> kern;
+    std::vector<std::string> srcs;
+    std::vector<int> ntop(e->types.size(), 0);
+    int64_t cells = 0;
+    for (size_t ti = 0; ti < e->types.size(); ++ti) {
+        TileType &tt = e->types[ti];
+        bool uni = true;
+        for (int i : members[ti]) uni = uni && dec.neurons[i].parent == dec.neurons[members[ti][0]].parent;
+        LevelProg lp;
+        if (!level_type(tt, prog_pool, dec.neurons[members[ti][0]].parent, uni, lp)) continue;
+        auto it = kern.find(lp.key);
+        if (it == kern.end()) {
+            if (kern.size() >= kLevelKernels) continue;
+            const std::string src = jit_level_source(lp, tt, tg[tt.table_set], mixed);
+            if (src.empty()) continue;
+            it = kern.emplace(lp.key, (int)srcs.size()).first;
+            srcs.push_back(src);
+        }
+        tt.level = 1 + it->second;
+        tt.lv_f0 = lp.f0;
+        ntop[ti] = lp.ntop;
+        cells += (int64_t)members[ti].size();
+    }
+    if (srcs.empty()) return GBH_OK;
+    int major = 10, minor = 3;
+    cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, e->opt.device);
+    cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, e->opt.device);
+    e->lv_kern.resize(srcs.size());
+    std::vector<int> ok(srcs.size(), 0);
+    std::vector<std::string> logs(srcs.size());
+    std::vector<std::thread> th;
+    for (size_t c = 0; c < srcs.size(); ++c)
+        th.emplace_back([&, c]() {
+            cudaSetDevice(e->opt.device);
+            ok[c] = jit_compile(srcs[c], !mixed, major, minor, &e->lv_kern[c], &logs[c]) == 0 &&
+                    jit_allow_smem(e->lv_kern[c], kLevelSmemMax);
+        });
+    for (auto &x : th) x.join();
+    for (size_t c = 0; c < srcs.size(); ++c)
+        if (!ok[c]) {   // these types keep the stack elimination
+            if (e->jit_log.size() < 4000) e->jit_log += logs[c];
+            for (TileType &tt : e->types)
+                if (tt.level == 1 + (int)c) tt.level = 0;
+        }
+    // ---- groups: enough of them for two blocks a SM, as many neurons each as
+    // that leaves (the top rows' warp issues for 32 neurons what it issues for one) ----
+    const int per_cells = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + kLevelGroups - 1) / kLevelGroups));
+    struct Cand { LevelGroup g; int warps, bucket; size_t smem; };
+    std::vector<Cand> cand;
+    LevelPools P;
+    std::vector<std::vector<int>> cells_of(e->tiles.size());
+    for (size_t i = 0; i < dec.neurons.size(); ++i) {
+        const int t = e->neuron_tile[i];
+        if (!e->types[e->tiles[t].type].level) continue;
+        cells_of[t].resize(e->tiles[t].nlanes, -1);
+        cells_of[t][e->neuron_lane[i]] = (int)i;
+    }
+    for (size_t t = 0; t < e->tiles.size(); ++t) {
+        const Tile &tl = e->tiles[t];
+        const TileType &tt = e->types[tl.type];
+        if (!tt.level) continue;
+        const int nst = tt.nstatic, nt_top = ntop[tl.type];
+        int fit = LANES;   // neurons whose rows fit the shared memory (a chunk has at least 32 rows or ends a level)
+        while (fit > 1 && level_smem(nt_top, fit * nst, fit * nst / LANES + nst + 1, tt.crank != 0) > (size_t)kLevelSmemMax)
+            --fit;
+        const int most = std::min(per_cells, fit);
+        const int ng = (tl.nlanes + most - 1) / most;
+        for (int q = 0, l0 = 0; q < ng; ++q) {
+            const int nl = (tl.nlanes - l0 + (ng - q) - 1) / (ng - q);
+            std::vector<const Neuron *> cl;
+            for (int l = l0; l < l0 + nl; ++l) cl.push_back(&dec.neurons[cells_of[t][l]]);
+            std::vector<int> order, start, kid, par, topkid;
+            level_order(cl, nst, nt_top, order, start, kid, par, topkid);
+            LevelGroup g{};
+            g.tile = (int)t;
+            g.lane0 = l0;
+            g.nlanes = nl;
+            g.n = (int)order.size();
+            g.eoff = (int64_t)P.map.size();
+            g.kidoff = (int)P.topkid.size();
+            g.choff = (int)P.chunks.size();
+            const int nlev = (int)start.size() - 1;
+            int warps = 1;   // as many sweeping warps as a level has rows for, on average
+            while (warps < 8 && warps * LANES * nlev < g.n) warps *= 2;
+            const int nt = warps * LANES;
+            for (int d = 0; d < nlev; ++d)
+                for (int a = start[d]; a < start[d + 1]; a += nt) {
+                    const int n = std::min(nt, start[d + 1] - a);
+                    P.chunks.push_back(make_int2(a, n | (a == start[d] ? LV_FIRST : 0) |
+                                                        (a + n == start[d + 1] ? LV_LAST : 0)));
+                }
+            g.nch = (int)P.chunks.size() - g.choff;
+            for (int x : order) {
+                const int row = x / LANES, l = x % LANES;
+                P.map.push_back(row * LANES + l0 + l);
+                P.cy.push_back(make_double2(cl[l]->C[row], 0.0));
+            }
+            P.kid.insert(P.kid.end(), kid.begin(), kid.end());
+            P.par.insert(P.par.end(), par.begin(), par.end());
+            P.topkid.insert(P.topkid.end(), topkid.begin(), topkid.end());
+            Cand c;
+            c.g = g;
+            c.warps = warps;
+            c.smem = level_smem(nt_top, g.n, g.nch, tt.crank != 0);
+            // launches of similar blocks: by kernel, warps and shared memory class
+            int cls = 0;
+            while (cls < 3 && c.smem > ((size_t)kLevelSmemMax / 8 << cls)) ++cls;
+            c.bucket = (tt.level - 1) * 64 + warps * 4 + cls;
+            cand.push_back(c);
+            l0 += nl;
+        }
+    }
+    if (cand.empty()) return GBH_OK;
+    std::stable_sort(cand.begin(), cand.end(), [](const Cand &a, const Cand &b) {
+        return a.bucket != b.bucket ? a.bucket > b.bucket : a.g.n > b.g.n;
+    });
+    for (size_t a = 0; a < cand.size();) {
+        size_t b = a, smem = 0;
+        for (; b < cand.size() && cand[b].bucket == cand[a].bucket; ++b) smem = std::max(smem, cand[b].smem);
+        Launch L{(int)a, (int)b, (int)smem, cand[a].warps};
+        L.level = cand[a].bucket / 64;
+        out.launches.push_back(L);
+        a = b;
+    }
+    for (const Cand &c : cand) out.groups.push_back(c.g);
+    const size_t n = P.map.size();
+    if (e->d_lgroups.upload(out.groups) || e->d_lchunks.upload(P.chunks) || e->d_lmap.upload(P.map) ||
+        e->d_lkid.upload(P.kid) || e->d_lpar.upload(P.par) || e->d_ltopkid.upload(P.topkid) || e->d_lcy.upload(P.cy) ||
+        e->d_lkt.alloc(n) || e->d_ld.alloc(n) || e->d_lpd.alloc(n) ||
+        e->d_lgen.upload(std::vector<unsigned>(out.groups.size(), 0u)))
+        return GBH_ERR_CUDA;
+    return GBH_OK;
+}
+
 int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn, const gbh_remote_synapses *remote,
                  gbh_error *err)
 {
@@ -655,31 +917,15 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         auto it = type_of_key.find(dec.neurons[i].key);
         if (it == type_of_key.end()) {
             const Neuron &N = dec.neurons[i];
-            TileType tt{};
-            tt.nslots = N.nrows;
-            tt.nfields = (int)N.fsrc.size();
-            tt.nints = (int)N.iops.size();
-            tt.npools = (int)N.pool_conc.size();
-            tt.ngiv = (int)N.giv_ref.size();
+            TileType tt = tile_type_of(N);
             tt.prog_off = (int)prog_pool.size();
             prog_pool.insert(prog_pool.end(), N.prog.begin(), N.prog.end());
             tt.pool_off = (int)prog_pool.size();
             prog_pool.insert(prog_pool.end(), N.pool_prog.begin(), N.pool_prog.end());
-            tt.table_set = N.table_set;
-            tt.crank = N.crank;
-            tt.chanmode5 = N.c5;
-            tt.interp = N.interp;
-            tt.has_spike = N.spike_op >= 0;
-            tt.nsyn = (int)N.syn_op.size();
-            tt.has_cd = N.has_cd;
-            tt.nscratch = N.nscratch;
-            if (!N.sym.empty()) {
-                tt.sym = 1;
+            if (tt.sym) {
                 tt.sym_off = (int)prog_pool.size();
                 prog_pool.insert(prog_pool.end(), N.sym.begin(), N.sym.end());
-                tt.nrav = (int)N.rav.size();
             }
-            tt.nitot = N.nitot;
             type_of_key[N.key] = (int)e->types.size();
             e->types.push_back(tt);
             members.emplace_back();
@@ -730,8 +976,7 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
             tt.np1 = np1;
             tt.slots = np1 && slots;
             const std::vector<int> pf = slot_field_ranges(prog_pool, tt);
-            tt.nstatic = 0;
-            while (tt.nstatic < tt.nslots && pf[6 * tt.nstatic + 2] >= 0) ++tt.nstatic;
+            tt.nstatic = static_rows(pf, tt.nslots);
             e->stack_dfield.resize(e->types.size());
             e->stack_kfield.resize(e->types.size());
             e->stack_dfield[ti].assign(tt.nfields, 0);
@@ -1134,6 +1379,17 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
     rc |= e->d_status.upload(std::vector<int>(1, 0));
     if (rc) return fail_err(err, GBH_ERR_CUDA, "%s", g_last_error);
 
+    // ---- level elimination of the trees with passive dendrites ----
+    LevelPlan lplan;
+    if (!e->has_network && e->opt.jit == 0 && jit_available(nullptr)) {
+        const int rcl = level_plan(e, members, prog_pool, tg, lplan);
+        if (rcl) return fail_err(err, rcl, "%s", g_last_error);
+        // the types' level flags
+        if (!lplan.groups.empty() && cudaMemcpy(e->d_types.p, e->types.data(), e->types.size() * sizeof(TileType),
+                                                cudaMemcpyHostToDevice) != cudaSuccess)
+            return fail_err(err, GBH_ERR_CUDA, "upload of the tile types failed");
+    }
+
     // ---- specialised kernels (one per tile type with enough tiles) ----
     std::vector<int> type_t0(e->types.size(), -1), type_t1(e->types.size(), -1);
     for (size_t ti = 0; ti < e->tiles.size(); ++ti) {
@@ -1149,11 +1405,9 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
     if (jit_on) {
         // types in tile order, largest first
         std::vector<int> cand;
-        // the looped forms keep 2 x nslots x 32 rows per warp in shared memory:
-        // 4-warp blocks of more than 96 compartments would not fit
         for (int ti : torder)
             if (type_t0[ti] >= 0 && !e->types[ti].wide && !e->types[ti].sym && !e->types[ti].nitot &&
-                e->types[ti].nslots <= 96)
+                !e->types[ti].level && e->types[ti].nslots <= kJitMaxSlots)
                 cand.push_back(ti);
         std::stable_sort(cand.begin(), cand.end(), [&](int a, int b) {
             return (type_t1[a] - type_t0[a]) > (type_t1[b] - type_t0[b]);
@@ -1237,62 +1491,75 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         }
     }
     // ---- launch plan: specialised types alone, the rest bucketed by slot count ----
-    size_t t0 = 0;
-    while (t0 < e->tiles.size()) {
-        const int ty0 = e->tiles[t0].type;
-        if (type_jit[ty0] >= 0) {
-            const int S = e->types[ty0].nslots;
-            Launch L{(int)t0, type_t1[ty0], S, 4};
-            L.jit = type_jit[ty0];
-            L.uniform = type_uniform[ty0] != 0;
-            e->launches.push_back(L);
-            t0 = type_t1[ty0];
-            continue;
-        }
-        const int smax = e->types[ty0].nslots;
-        size_t t1 = t0;
-        if (e->types[ty0].stack) {   // one warp per tile, every size in one launch
-            int cap = 1;
-            while (t1 < e->tiles.size() && type_jit[e->tiles[t1].type] < 0 && e->types[e->tiles[t1].type].stack) {
-                cap = std::max(cap, e->types[e->tiles[t1].type].scap);
-                ++t1;
+    // (skip_level: the level-eliminated tiles are launched by groups, below)
+    auto plan = [&](std::vector<Launch> &out, bool skip_level) {
+        auto typ = [&](size_t t) -> const TileType & { return e->types[e->tiles[t].type]; };
+        auto lev = [&](size_t t) { return skip_level && typ(t).level; };
+        size_t t0 = 0;
+        while (t0 < e->tiles.size()) {
+            const int ty0 = e->tiles[t0].type;
+            if (lev(t0)) {
+                ++t0;
+                continue;
             }
-            Launch L{(int)t0, (int)t1, cap, 1};
-            L.stack = true;
-            for (size_t u = t0; u < t1; ++u) {
-                const TileType &tt = e->types[e->tiles[u].type];
-                L.split = L.split || (tt.nstatic > 0 && tt.nslots - tt.nstatic <= kSplitRows);
+            if (type_jit[ty0] >= 0) {
+                const int S = e->types[ty0].nslots;
+                Launch L{(int)t0, type_t1[ty0], S, 4};
+                L.jit = type_jit[ty0];
+                L.uniform = type_uniform[ty0] != 0;
+                out.push_back(L);
+                t0 = type_t1[ty0];
+                continue;
             }
-            e->launches.push_back(L);
-            t0 = t1;
-            continue;
-        }
-        if (e->types[ty0].wide) {   // one block per neuron
-            while (t1 < e->tiles.size() && e->types[e->tiles[t1].type].wide &&
-                   e->types[e->tiles[t1].type].nslots * 2 > smax)
+            const int smax = e->types[ty0].nslots;
+            size_t t1 = t0;
+            if (e->types[ty0].stack) {   // one warp per tile, every size in one launch
+                int cap = 1;
+                while (t1 < e->tiles.size() && type_jit[e->tiles[t1].type] < 0 && typ(t1).stack && !lev(t1)) {
+                    cap = std::max(cap, typ(t1).scap);
+                    ++t1;
+                }
+                Launch L{(int)t0, (int)t1, cap, 1};
+                L.stack = true;
+                for (size_t u = t0; u < t1; ++u) {
+                    const TileType &tt = typ(u);
+                    L.split = L.split || (tt.nstatic > 0 && tt.nslots - tt.nstatic <= kSplitRows);
+                }
+                out.push_back(L);
+                t0 = t1;
+                continue;
+            }
+            if (e->types[ty0].wide) {   // one block per neuron
+                while (t1 < e->tiles.size() && typ(t1).wide && typ(t1).nslots * 2 > smax) ++t1;
+                if (smax * (2 * sizeof(double) + 4 * sizeof(int)) > 200 * 1024)
+                    return fail_err(err, GBH_ERR_UNSUPPORTED, "neuron with %d compartments exceeds the shared memory",
+                                    smax);
+                Launch L{(int)t0, (int)t1, smax, 1};
+                L.wide = true;
+                out.push_back(L);
+                t0 = t1;
+                continue;
+            }
+            while (t1 < e->tiles.size() && type_jit[e->tiles[t1].type] < 0 && !typ(t1).wide && !lev(t1) &&
+                   typ(t1).nslots * 2 > smax)
                 ++t1;
-            if (smax * (2 * sizeof(double) + 4 * sizeof(int)) > 200 * 1024)
-                return fail_err(err, GBH_ERR_UNSUPPORTED, "neuron with %d compartments exceeds the shared memory",
-                                smax);
-            Launch L{(int)t0, (int)t1, smax, 1};
-            L.wide = true;
-            e->launches.push_back(L);
+            const int per_warp = 2 * smax * LANES * (int)sizeof(double);
+            int warps = e->opt.warps_per_block > 0 ? std::min(e->opt.warps_per_block, 4) : 4;
+            warps = std::max(1, std::min(warps, kSmemPerBlock / per_warp));
+            if (per_warp > 200 * 1024)
+                return fail_err(err, GBH_ERR_UNSUPPORTED,
+                                "neuron with %d compartments exceeds the shared-memory sweep", smax);
+            out.push_back({(int)t0, (int)t1, smax, warps});
             t0 = t1;
-            continue;
         }
-        while (t1 < e->tiles.size() && type_jit[e->tiles[t1].type] < 0 && !e->types[e->tiles[t1].type].wide &&
-               e->types[e->tiles[t1].type].nslots * 2 > smax)
-            ++t1;
-        const int per_warp = 2 * smax * LANES * (int)sizeof(double);
-        int warps = e->opt.warps_per_block > 0 ? std::min(e->opt.warps_per_block, 4) : 4;
-        warps = std::max(1, std::min(warps, kSmemPerBlock / per_warp));
-        if (per_warp > 200 * 1024)
-            return fail_err(err, GBH_ERR_UNSUPPORTED, "neuron with %d compartments exceeds the shared-memory sweep",
-                            smax);
-        e->launches.push_back({(int)t0, (int)t1, smax, warps});
-        t0 = t1;
+        return (int)GBH_OK;
+    };
+    if (!lplan.groups.empty()) {
+        const int rcg = plan(e->giv_launches, false);
+        if (rcg) return rcg;
+        e->launches = lplan.launches;
     }
-    return GBH_OK;
+    return plan(e->launches, !lplan.groups.empty());
 }
 
 DevView view_of(gbh_engine *e)
@@ -1359,6 +1626,28 @@ int launch_one(gbh_engine *e, const DevView &v, const Launch &L, int k, long lon
         const cudaError_t je = jit_launch(e->jits[L.jit], v, L.tile0, L.tile1, L.smax, warps, k, step, smem, st);
         if (je != cudaSuccess) {
             set_last("specialised kernel launch failed: %s", cudaGetErrorString(je));
+            return GBH_ERR_CUDA;
+        }
+        e->stats.launches++;
+        return GBH_OK;
+    }
+    if (L.level >= 0) {
+        LevelView lv{};
+        lv.groups = e->d_lgroups.p;
+        lv.chunks = e->d_lchunks.p;
+        lv.map = e->d_lmap.p;
+        lv.kid = e->d_lkid.p;
+        lv.par = e->d_lpar.p;
+        lv.topkid = e->d_ltopkid.p;
+        lv.kt = e->d_lkt.p;
+        lv.cy = e->d_lcy.p;
+        lv.d = e->d_ld.p;
+        lv.pd = e->d_lpd.p;
+        lv.gen = e->d_lgen.p;
+        const cudaError_t je = jit_level_launch(e->lv_kern[L.level], v, lv, L.tile0, L.tile1 - L.tile0, L.warps, k,
+                                                step, (size_t)L.smax, st);
+        if (je != cudaSuccess) {
+            set_last("level elimination launch failed: %s", cudaGetErrorString(je));
             return GBH_ERR_CUDA;
         }
         e->stats.launches++;
@@ -1438,7 +1727,7 @@ int issue_steps(gbh_engine *e, const DevView &v, int nsteps, long long step0, bo
     }
     if (giv_last && nsteps > 0) {
         if (spikes(step0 + nsteps - 1, st)) return GBH_ERR_CUDA;
-        for (const Launch &L : e->launches) {
+        for (const Launch &L : e->giv_launches.empty() ? e->launches : e->giv_launches) {
             const int rc = launch_one(e, v, L, 1, step0 + nsteps - 1, mixed, true, st);
             if (rc) return rc;
             if (kernels) ++*kernels;
@@ -2295,24 +2584,11 @@ int64_t gbh_jit_source(const gbh_batch_desc *desc, int precision, int type_index
     for (const Neuron &N : dec.neurons) {
         auto it = keys.find(N.key);
         if (it == keys.end()) {
-            TileType tt{};
-            tt.nslots = N.nrows;
-            tt.nfields = (int)N.fsrc.size();
-            tt.nints = (int)N.iops.size();
-            tt.npools = (int)N.pool_conc.size();
-            tt.ngiv = (int)N.giv_ref.size();
+            TileType tt = tile_type_of(N);
             tt.prog_off = (int)prog_pool.size();
             prog_pool.insert(prog_pool.end(), N.prog.begin(), N.prog.end());
             tt.pool_off = (int)prog_pool.size();
             prog_pool.insert(prog_pool.end(), N.pool_prog.begin(), N.pool_prog.end());
-            tt.table_set = N.table_set;
-            tt.crank = N.crank;
-            tt.chanmode5 = N.c5;
-            tt.interp = N.interp;
-            tt.has_cd = N.has_cd;
-            tt.nscratch = N.nscratch;
-            tt.sym = !N.sym.empty();
-            tt.nitot = N.nitot;
             keys[N.key] = (int)types.size();
             types.push_back(tt);
             parents.push_back(N.parent);
@@ -2328,16 +2604,21 @@ int64_t gbh_jit_source(const gbh_batch_desc *desc, int precision, int type_index
         int cap = 0;
         if (!tt.sym && tt.nslots >= kStackMin && stack_plan(parents[type_index], fl, cap) && cap <= kStackCapMax) {
             const std::vector<int> pf = slot_field_ranges(prog_pool, tt);
-            while (tt.nstatic < tt.nslots && pf[6 * tt.nstatic + 2] >= 0) ++tt.nstatic;
+            tt.nstatic = static_rows(pf, tt.nslots);
         }
     }
     std::vector<TableGeom> tg;
     std::vector<double> tab64, xy;
     build_tables(desc, tg, tab64, xy);
-    const std::string src = jit_source(types[type_index], prog_pool, tg[types[type_index].table_set],
-                                       precision == GBH_PREC_MIXED, false,
-                                       uniform[type_index] ? &parents[type_index] : nullptr, 6, compact == 1,
-                                       compact == 2);
+    std::string src;
+    if (compact == 3) {
+        const LevelProg lp = level_prog(types[type_index], prog_pool);
+        if (lp.ok) src = jit_level_source(lp, types[type_index], tg[types[type_index].table_set],
+                                          precision == GBH_PREC_MIXED);
+    } else {
+        src = jit_source(types[type_index], prog_pool, tg[types[type_index].table_set], precision == GBH_PREC_MIXED,
+                         false, uniform[type_index] ? &parents[type_index] : nullptr, 6, compact == 1, compact == 2);
+    }
     if (buf && buflen > 0) {
         const int64_t n = std::min<int64_t>(buflen - 1, (int64_t)src.size());
         memcpy(buf, src.data(), (size_t)n);
@@ -2375,6 +2656,35 @@ namespace {
 gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, const gbh_remote_synapses *remote,
                         const gbh_options *opt, gbh_error *err, gbh_engine *&made, const Decoded *pre = nullptr);
 
+// Do all neurons that could run wide (32 compartments and more) run the
+// level elimination when lane-mapped (level_type)?
+bool level_everywhere(const gbh_engine *e)
+{
+    if (e->has_network || e->opt.jit != 0 || !jit_available(nullptr)) return false;
+    struct Seen { const Neuron *first; bool uniform; };
+    std::map<std::string, Seen> types;
+    std::vector<int> fl;
+    for (const Neuron &N : e->dec.neurons) {
+        if (N.nrows < 32) continue;
+        int cap = 0;
+        if (!stack_plan(N.parent, fl, cap) || cap > kStackCapMax) return false;
+        auto it = types.emplace(N.key, Seen{&N, true}).first;
+        it->second.uniform = it->second.uniform && N.parent == it->second.first->parent;
+    }
+    for (const auto &kv : types) {
+        const Neuron &N = *kv.second.first;
+        TileType tt = tile_type_of(N);
+        std::vector<int> prog = N.prog;
+        tt.pool_off = (int)prog.size();
+        prog.insert(prog.end(), N.pool_prog.begin(), N.pool_prog.end());
+        tt.stack = !tt.sym;
+        tt.nstatic = static_rows(slot_field_ranges(prog, tt), tt.nslots);
+        LevelProg lp;
+        if (!level_type(tt, prog, N.parent, kv.second.uniform, lp)) return false;
+    }
+    return true;
+}
+
 // The neuron-to-warp mapping, chosen by trial (gbh_options.wide_min 0): for
 // each candidate -- neurons of at least 32, 64 or 128 compartments one per
 // warp (wide tiles), or none (every large neuron lane-mapped, 32 per warp,
@@ -2397,6 +2707,7 @@ int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses
     for (int w : {32, 64, 128})
         if (w <= maxrows) cand.push_back(w);
     if (cand.empty()) return -1;   // nothing large enough to run wide
+    if (level_everywhere(e)) return -1;   // no trial: the level elimination beats every mapping it tries
     cand.push_back(-1);
     int best = cand[0];
     double best_ms = 1e300;
@@ -2527,13 +2838,14 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
         if (L.wide) e->stats.wide_tiles += L.tile1 - L.tile0;
         if (L.stack) e->stats.stack_tiles += L.tile1 - L.tile0;
     }
+    for (const Tile &t : e->tiles) e->stats.stack_tiles += e->types[t.type].level ? 1 : 0;
     e->stats.precision = e->opt.precision;
     e->stats.steps_per_launch = e->net_coop ? e->net_spl : e->steps_per_launch;
     e->stats.cooperative = e->net_coop ? 1 : 0;
     e->stats.warps_per_block = e->launches.empty() ? 0 : e->launches[0].warps;
     if (!e->launches.empty() && e->launches[0].jit >= 0 && !e->jit_warps.empty())
         e->stats.warps_per_block = e->jit_warps[e->jit_choice];
-    e->stats.jit_kernels = e->jit_compiled;
+    e->stats.jit_kernels = e->jit_compiled + (int)e->lv_kern.size();
     e->stats.jit_min_blocks = e->jit_minb.empty() ? 0 : e->jit_minb[e->jit_choice];
     e->stats.jit_compact = e->jit_compact.empty() ? 0
                            : e->jit_compact[e->jit_choice] ? 1
@@ -3234,6 +3546,10 @@ void gbh_destroy(gbh_engine *e)
     e->d_step.release();
     for (auto &vars : e->jit_var)
         for (JitKernel &k : vars) jit_release(k);
+    for (JitKernel &k : e->lv_kern) jit_release(k);
+    e->d_lgroups.release(); e->d_lchunks.release(); e->d_lmap.release(); e->d_lkid.release(); e->d_lpar.release();
+    e->d_ltopkid.release(); e->d_lkt.release(); e->d_lcy.release(); e->d_ld.release(); e->d_lpd.release();
+    e->d_lgen.release();
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
     if (e->stream) cudaStreamDestroy(e->stream);

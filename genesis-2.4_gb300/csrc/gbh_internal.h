@@ -133,6 +133,8 @@ struct TileType {
                      // trees): the forward sweep pops at most one entry per row, without a loop
     int slots;       // stack, np1: every row's stack entries are below 32 and packed in its flags
                      // (FL_SLOT_*), so the sweeps index the stack without a running top
+    int level;       // stack: 1 + index of the level-elimination kernel its tiles run (gbh_level.cuh), 0 none
+    int lv_f0;       // level: the first field row of the rows above the static ones
 };
 
 // Per-row flags of the stack elimination (DevView::ltop, topo rows, one word

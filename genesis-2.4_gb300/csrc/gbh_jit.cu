@@ -19,6 +19,8 @@
 #include <dlfcn.h>
 #include <nvrtc.h>
 
+#include <algorithm>
+#include <climits>
 #include <cstdio>
 #include <array>
 #include <cstring>
@@ -497,6 +499,23 @@ int loop_run(const std::vector<int> &prog, const std::vector<int> &sstart, int s
     return run;
 }
 
+// The Ca_concen pools of one neuron; false on another pool op.
+bool emit_ca_pools(std::ostream &t, const int *pp)
+{
+    for (; pp[0] != 0; pp += 5) {
+        if (pp[0] != PO_CACONC) return false;
+        t << "    { double *cx = &Cw[" << pp[1] * LANES << "]; const double base = Pw[" << pp[2] * LANES
+          << "]; const double itau = Pw[" << pp[3] * LANES << "];\n"
+          << "      *cx = base + ((*cx - base) * (2.0 - itau) + (Fw[" << pp[1] * LANES << "] * Pw[" << pp[4] * LANES
+          << "])) / itau; }\n";
+    }
+    return true;
+}
+
+// Level-elimination blocks: at most 8 sweeping warps and the one of the top
+// rows; the residency sets the register budget (see jit_level_source).
+constexpr int kLevelThreads = 9 * LANES, kLevelBlocks = 2;
+
 }  // namespace
 
 std::string jit_source(const TileType &tt, const std::vector<int> &prog, const TableGeom &tg, bool mixed, bool giv,
@@ -759,15 +778,7 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
     std::ostringstream t;
     t << body;
     // pools
-    const int *pp = prog.data() + tt.pool_off;
-    while (pp[0] != 0) {
-        if (pp[0] != PO_CACONC) return std::string();
-        t << "    { double *cx = &Cw[" << pp[1] * LANES << "]; const double base = Pw[" << pp[2] * LANES
-          << "]; const double itau = Pw[" << pp[3] * LANES << "];\n"
-          << "      *cx = base + ((*cx - base) * (2.0 - itau) + (Fw[" << pp[1] * LANES << "] * Pw[" << pp[4] * LANES
-          << "])) / itau; }\n";
-        pp += 5;
-    }
+    if (!emit_ca_pools(t, prog.data() + tt.pool_off)) return std::string();
     // elimination
     auto Dx = [&](int s) { return !cols ? "D[" + std::to_string(s) + "]" : "Dc[" + std::to_string(s * LANES) + "]"; };
     auto Rx = [&](int s) { return !cols ? "R[" + std::to_string(s) + "]" : "Rc[" + std::to_string(s * LANES) + "]"; };
@@ -824,6 +835,158 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
     return t.str();
 }
 
+LevelProg level_prog(const TileType &tt, const std::vector<int> &prog)
+{
+    LevelProg lp;
+    lp.ntop = tt.nslots - tt.nstatic;
+    if (tt.nstatic <= 0 || lp.ntop <= 0 || lp.ntop > kSplitRows || tt.has_cd || tt.nscratch || tt.sym || tt.nitot)
+        return lp;
+    // operands that are field rows (bit i: operand i) and the givals row (-1
+    // none) of the ops a step without givals may hold
+    auto roles = [](int code, int &fields, int &giv) {
+        fields = 0;
+        giv = -1;
+        switch (code) {
+        case M_BEGIN: fields = 0x7; giv = 3; return true;
+        case M_NEWVOLT: case M_NEWCONC1: case M_FLUX: case M_DO_TABGHK: case M_CONCVAL: case M_NEWCONC2: return true;
+        case M_DOMAIN: case M_SCALE_FLUX: case M_SAME_GHK: case M_CHAN_G: case M_SPIKE: fields = 0x1; return true;
+        case M_ELMMPUMP: fields = 0x7; giv = 3; return true;
+        case M_GHK: fields = 0x7; return true;
+        case M_NERNST: case M_CHAN: fields = 0x3; return true;
+        case M_END: fields = 0x3; giv = 2; return true;
+        case M_GATE: fields = 0x8; return true;
+        case M_SYN: fields = 0x39; return true;
+        case M_MGBLOCK: fields = 0x7; giv = 3; return true;
+        case M_ADDCURR: giv = 0; return true;
+        default: return false;
+        }
+    };
+    std::vector<size_t> fpos;
+    size_t pc = (size_t)tt.prog_off + 9 * (size_t)tt.nstatic;   // a passive row's program is 9 ints
+    for (int s = 0; s < lp.ntop;) {
+        const int code = prog[pc], n = nops_of(code);
+        int fields, giv;
+        if (n < 0 || !roles(code, fields, giv)) return lp;
+        if (code == M_SYN && prog[pc + 1] >= 0) return lp;   // SYN3 draws are keyed by the field row
+        const size_t base = lp.prog.size();
+        for (int i = 0; i <= n; ++i) lp.prog.push_back(prog[pc + i]);
+        for (int i = 0; i < n; ++i)
+            if ((fields >> i & 1) && prog[pc + 1 + i] >= 0) fpos.push_back(base + 1 + i);
+        if (giv >= 0) lp.prog[base + 1 + giv] = 0;
+        pc += 1 + n;
+        if (code == M_END) ++s;
+    }
+    lp.pool_off = (int)lp.prog.size();
+    for (const int *pp = prog.data() + tt.pool_off; pp[0] != 0; pp += 5) {
+        if (pp[0] != PO_CACONC) return lp;
+        for (int i = 0; i < 5; ++i) lp.prog.push_back(pp[i]);
+        for (int i = 2; i < 5; ++i) fpos.push_back(lp.prog.size() - 5 + i);
+    }
+    lp.prog.push_back(0);
+    lp.f0 = INT32_MAX;
+    for (size_t p : fpos) lp.f0 = std::min(lp.f0, lp.prog[p]);
+    for (size_t p : fpos) lp.prog[p] -= lp.f0;
+    std::ostringstream k;
+    k << lp.ntop << ' ' << tt.crank << ' ' << tt.chanmode5 << ' ' << tt.interp << ' ' << tt.table_set;
+    for (int x : lp.prog) k << ' ' << x;
+    lp.key = k.str();
+    lp.ok = true;
+    return lp;
+}
+
+std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed)
+{
+    Emit E;
+    E.mixed = mixed;
+    E.giv = false;
+    std::ostringstream &o = E.o;
+    const int N = lp.ntop;
+    const char *form = mixed ? "true" : "false", *crank = tt.crank ? "true" : "false";
+    o << "#include \"gbh_devfn.cuh\"\n#include \"gbh_level.cuh\"\nusing namespace gbh;\n"
+      << "extern \"C\" __global__ void __launch_bounds__(" << kLevelThreads << ", " << kLevelBlocks
+      << ") gbh_jit(DevView v, LevelView L, int g0, int nsteps, long long step0)\n{\n"
+      << "  extern __shared__ double sm[];\n"
+      << "  const LevelGroup g = L.groups[g0 + blockIdx.x];\n"
+      << "  { unsigned dsz; asm(\"mov.u32 %0, %%dynamic_smem_size;\" : \"=r\"(dsz));\n"
+      << "    if (dsz < level_smem(" << N << ", g.n, g.nch, " << crank
+      << ")) { if (v.status && threadIdx.x == 0) atomicOr(v.status, ST_SMEM); return; } }\n"
+      << "  const Tile tl = v.tiles[g.tile]; const TileType ty = v.types[tl.type];\n"
+      << "  const unsigned sgen = v.sgen ? *v.sgen : 0u;\n"
+      << "  if (threadIdx.x < blockDim.x - 32) {\n"
+      << "    const bool full = !v.sgen || L.gen[g0 + blockIdx.x] != sgen, refresh = *v.kref != 0;\n"
+      << "    level_sweep<" << form << ", " << crank << ", " << N << ">(v, L, g, tl, ty, sm, nsteps, full, refresh);\n"
+      << "    if (full && v.sgen && threadIdx.x == 0) L.gen[g0 + blockIdx.x] = sgen;\n    return;\n  }\n"
+      << "  const int lid = threadIdx.x & 31; const bool active = lid < g.nlanes; const int lane = g.lane0 + (active ? lid : 0);\n"
+      << "  const long long sbase = v.step_dev ? *v.step_dev : 0;\n"
+      << "  const bool c5 = " << (tt.chanmode5 ? "true" : "false") << "; (void)c5;\n"
+      << "  const bool interp = " << (tt.interp ? "true" : "false") << "; (void)interp;\n"
+      << "  double *Pw = v.P + (tl.fld + ty.lv_f0) * 32 + lane; int *Iw = v.I + tl.ints * 32 + lane; (void)Iw;\n"
+      << "  double *Vw = v.V + (tl.vm + ty.nstatic) * 32 + lane; double *Cw = v.C + tl.pools * 32 + lane; (void)Cw;\n"
+      << "  double *Fw = v.F + tl.pools * 32 + lane; (void)Fw;\n"
+      << "  const int64_t neuron = tl.first_neuron + lane; (void)neuron;\n"
+      << "  const int64_t trow = (tl.topo + ty.nstatic) * 32 + lane;\n"
+      << "  const RoRow<double> Aw{v.A + trow}, Bw{v.B + trow}, Cbw{v.Cb + trow}; (void)Aw; (void)Bw; (void)Cbw;\n"
+      << "  int tp[" << N << "];\n";
+    for (int s = 0; s < N; ++s)
+        o << "  { const int p = v.parent[trow + " << s * LANES << "]; tp[" << s << "] = p < 0 ? -1 : p - ty.nstatic; }\n";
+    if (mixed) {
+        o << "  const float4 *tab = v.tabdf + " << tg.tab_off << "; (void)tab;\n"
+          << "  const df xnmin = df_make(" << litf(-tg.xmin_hi) << ", " << litf(-tg.xmin_lo) << "), xinv = df_make("
+          << litf(tg.invdx_hi) << ", " << litf(tg.invdx_lo) << "); (void)xnmin; (void)xinv;\n"
+          << "  const df ynmin = df_make(" << litf(-tg.ymin_hi) << ", " << litf(-tg.ymin_lo) << "), yinv = df_make("
+          << litf(tg.invdy_hi) << ", " << litf(tg.invdy_lo) << "); (void)ynmin; (void)yinv;\n";
+    } else {
+        o << "  const double *tab = v.tab64 + " << tg.tab_off << "; (void)tab;\n"
+          << "  const double *xvals = v.xyvals + " << tg.xv_off << "; (void)xvals;\n"
+          << "  const double *yvals = v.xyvals + " << (tg.yv_off >= 0 ? tg.yv_off : tg.xv_off) << "; (void)yvals;\n";
+    }
+    o << "  double *U = sm + lid; const double *PR = sm + " << N * LANES << " + g.n;\n"
+      << "  for (int it = 0; it < nsteps; ++it) {\n"
+      << "    const long long step = sbase + step0 + it; (void)step;\n"
+      << "    double D[" << N << "], R[" << N << "], T[" << N << "], PD[" << N << "]; (void)T; (void)PD;\n"
+      << "    if (active) {\n";
+    if (mixed) {
+        o << "    DCursor vc, cc, c1; vc.row = vc.base = 0; vc.frac = df_make(0.f, 0.f); cc = vc; c1 = vc;\n"
+          << "    df Ek = df_make(0.f, 0.f), Gk = Ek, gmax = Ek; (void)gmax;\n";
+    } else {
+        o << "    VCursor vc, cc;\n"
+          << (tg.ncols ? "    vc.lo = vc.hi = 0.0;\n" : "    vc.lo = -1e20; vc.hi = 1e20;\n")
+          << "    vc.row = vc.base = 0; vc.frac = 0.0; cc.lo = cc.hi = 0.0; cc.row = cc.base = 0; cc.frac = 0.0;\n"
+          << "    double save_frac = 0.0; int tab_base = 0, ctab_base = 0; (void)save_frac; (void)tab_base; (void)ctab_base;\n"
+          << "    double Ek = 0.0, Gk = 0.0, gmax = 0.0; (void)gmax;\n";
+    }
+    o << "    double GHK = 0.0, Ik = 0.0; int doGHK = 0, sel = 0; (void)GHK; (void)doGHK; (void)sel; (void)Ik;\n";
+    const int *pc = lp.prog.data();
+    for (int s = 0; s < N; ++s)
+        if (!emit_slot(E, s, pc, tg)) return std::string();
+    emit_ca_pools(o, lp.prog.data() + lp.pool_off);
+    o << "    }\n    __syncwarp();\n    bar_named(LB_FORWARD, blockDim.x);\n    if (active) {\n";
+    for (int s = 0; s < N; ++s) {
+        const std::string S = "[" + std::to_string(s) + "]", r = std::to_string(s * LANES);
+        o << "      level_top_kids(L, g, PR, " << s << ", lid, R" << S << ", D" << S << ");\n";
+        for (int j = 0; j < s; ++j)   // top rows below this one, after the static rows: ascending row order
+            o << "      if (tp[" << j << "] == " << s << ") { D" << S << " -= PD[" << j << "]; R" << S << " -= T[" << j << "]; }\n";
+        if (mixed) o << "      D" << S << " = rcp_newton(D" << S << ");\n";
+        if (s < N - 1)   // T holds R T
+            o << "      { const double temp = Aw[" << r << (mixed ? "] * D" : "] / D") << S << "; PD" << S << " = Bw[" << r
+              << "] * temp; T" << S << " = R" << S << " * temp; }\n";
+    }
+    for (int s = N - 1; s >= 0; --s) {
+        const std::string S = "[" + std::to_string(s) + "]", r = std::to_string(s * LANES);
+        o << "      { double r = R" << S << ";";
+        if (s < N - 1)
+            o << " if (tp" << S << " >= 0) "
+              << (mixed ? "r = fma(-Cbw[" + r + "], U[tp" + S + " * 32], r);" : "r -= Cbw[" + r + "] * U[tp" + S + " * 32];");
+        o << (mixed ? " r = r * D" : " r = r / D") << S << "; U[" << r << "] = r;";
+        if (tt.crank) o << " Vw[" << r << "] = " << (mixed ? "fma(2.0, r, -Vw[" + r + "]);" : "r + r - Vw[" + r + "];");
+        else o << " Vw[" << r << "] = r;";
+        if (s == N - 1) o << " finite_check(v, r, active);";   // the root: a NaN anywhere below it reaches it
+        o << " }\n";
+    }
+    o << "    }\n    __syncwarp();\n    bar_named(LB_TOP, blockDim.x);\n  }\n}\n";
+    return o.str();
+}
+
 bool jit_available(std::string *why)
 {
     std::call_once(g_api_once, init_api);
@@ -836,9 +999,11 @@ int jit_compile(const std::string &src, bool fp64_exact, int device_major, int d
 {
     if (!jit_available(log)) return -1;
     nvrtcProgram prog;
-    const char *hdr_src[] = {kSrc_gbh_internal_h, kSrc_gbh_df_cuh, kSrc_gbh_devfn_cuh, "", kStdintStub};
-    const char *hdr_name[] = {"gbh_internal.h", "gbh_df.cuh", "gbh_devfn.cuh", "cuda_runtime.h", "stdint.h"};
-    if (g_api.create(&prog, src.c_str(), "gbh_jit.cu", 5, hdr_src, hdr_name) != NVRTC_SUCCESS) {
+    const char *hdr_src[] = {kSrc_gbh_internal_h, kSrc_gbh_df_cuh, kSrc_gbh_devfn_cuh, kSrc_gbh_level_cuh, "",
+                             kStdintStub};
+    const char *hdr_name[] = {"gbh_internal.h", "gbh_df.cuh", "gbh_devfn.cuh", "gbh_level.cuh", "cuda_runtime.h",
+                              "stdint.h"};
+    if (g_api.create(&prog, src.c_str(), "gbh_jit.cu", 6, hdr_src, hdr_name) != NVRTC_SUCCESS) {
         if (log) *log = "nvrtcCreateProgram failed";
         return -1;
     }
@@ -896,6 +1061,24 @@ cudaError_t jit_launch(const JitKernel &k, const DevView &v, int tile0, int tile
     // refuses (resources, shared memory) is a configuration error
     return r == CUDA_ERROR_LAUNCH_FAILED || r == CUDA_ERROR_ILLEGAL_ADDRESS ? cudaErrorLaunchFailure
                                                                           : cudaErrorInvalidConfiguration;
+}
+
+cudaError_t jit_level_launch(const JitKernel &k, const DevView &v, const LevelView &lv, int g0, int ngroups, int warps,
+                             int nsteps, long long step, size_t smem, cudaStream_t st)
+{
+    DevView vv = v;
+    LevelView ll = lv;
+    void *args[] = {&vv, &ll, &g0, &nsteps, &step};
+    const CUresult r = g_api.launch((CUfunction)k.fn, ngroups, 1, 1, (warps + 1) * LANES, 1, 1, (unsigned)smem,
+                                    (CUstream)st, args, nullptr);
+    if (r == CUDA_SUCCESS) return cudaSuccess;
+    return r == CUDA_ERROR_LAUNCH_FAILED || r == CUDA_ERROR_ILLEGAL_ADDRESS ? cudaErrorLaunchFailure
+                                                                          : cudaErrorInvalidConfiguration;
+}
+
+bool jit_allow_smem(const JitKernel &k, size_t smem)
+{
+    return g_api.setattr((CUfunction)k.fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem) == CUDA_SUCCESS;
 }
 
 void jit_release(JitKernel &k)

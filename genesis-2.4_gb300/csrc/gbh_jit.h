@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "gbh_devfn.cuh"
+#include "gbh_level.cuh"
 
 namespace gbh {
 
@@ -26,6 +27,25 @@ struct JitKernel {
 std::string jit_source(const TileType &tt, const std::vector<int> &prog, const TableGeom &tg, bool mixed, bool giv,
                        const std::vector<int> *uniform_parent, int min_blocks = 4, bool compact = false,
                        bool smem_rows = false, int warps = 4);
+
+// The rows above a type's static ones as the level-elimination kernel runs
+// them (gbh_level.cuh): their programs and the pool program with field rows
+// relative to `f0`, so that types which differ only in their dendrites share
+// one kernel (equal `key`). ok: the generator emits every op of them.
+struct LevelProg {
+    bool ok = false;
+    int ntop = 0, f0 = 0;
+    std::vector<int> prog;   // ntop slot programs, then the 0-terminated pool program
+    int pool_off = 0;
+    std::string key;
+};
+LevelProg level_prog(const TileType &tt, const std::vector<int> &prog);
+// Source of the level-elimination kernel (entry gbh_jit) for one such program.
+std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed);
+cudaError_t jit_level_launch(const JitKernel &k, const DevView &v, const LevelView &lv, int g0, int ngroups, int warps,
+                             int nsteps, long long step, size_t smem, cudaStream_t st);
+// Largest dynamic shared memory the kernel may be launched with.
+bool jit_allow_smem(const JitKernel &k, size_t smem);
 
 bool jit_available(std::string *why);
 int jit_compile(const std::string &src, bool fp64_exact, int device_major, int device_minor, JitKernel *out,
