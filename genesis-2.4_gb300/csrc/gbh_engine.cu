@@ -711,7 +711,9 @@ bool level_type(const TileType &tt, const std::vector<int> &prog, const std::vec
         }
         if (tt.nstatic < 2 * levels) return false;
     }
-    if (level_smem(kSplitRows, tt.nstatic, tt.nstatic + 1, tt.crank != 0) > (size_t)kLevelSmemMax) return false;
+    // one neuron's rows must fit a block (streamed constants, 8 sweeping warps)
+    if (level_smem(kSplitRows, tt.nstatic, tt.nstatic + 1, tt.crank != 0, false, false, 256) > (size_t)kLevelSmemMax)
+        return false;
     if (tt.nstatic * LANES >= 1 << LV_KID_BITS) return false;
     lp = level_prog(tt, prog);
     return lp.ok;
@@ -783,10 +785,11 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
         auto it = kern.find(lp.key);
         if (it == kern.end()) {
             if (kern.size() >= kLevelKernels) continue;
-            const std::string src = jit_level_source(lp, tt, tg[tt.table_set], mixed);
+            const std::string src = jit_level_source(lp, tt, tg[tt.table_set], mixed, true);
             if (src.empty()) continue;
-            it = kern.emplace(lp.key, (int)srcs.size()).first;
-            srcs.push_back(src);
+            it = kern.emplace(lp.key, (int)kern.size()).first;
+            srcs.push_back(src);   // kernel 2k: constants resident in shared memory, 2k + 1: streamed
+            srcs.push_back(jit_level_source(lp, tt, tg[tt.table_set], mixed, false));
         }
         tt.level = 1 + it->second;
         tt.lv_f0 = lp.f0;
@@ -812,11 +815,14 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
         if (!ok[c]) {   // these types keep the stack elimination
             if (e->jit_log.size() < 4000) e->jit_log += logs[c];
             for (TileType &tt : e->types)
-                if (tt.level == 1 + (int)c) tt.level = 0;
+                if (tt.level == 1 + (int)c / 2) tt.level = 0;
         }
     // ---- groups: enough of them for two blocks a SM, as many neurons each as
     // that leaves (the top rows' warp issues for 32 neurons what it issues for one) ----
     const int per_cells = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + kLevelGroups - 1) / kLevelGroups));
+    const char *lvenv = getenv("GBH_LV");
+    const int lvmode = lvenv ? atoi(lvenv) : 1;
+    const size_t lvmax = getenv("GBH_LVMAX") ? (size_t)atoi(getenv("GBH_LVMAX")) * 1024 : (size_t)kLevelSmemMax;
     struct Cand { LevelGroup g; int warps, bucket; size_t smem; };
     std::vector<Cand> cand;
     LevelPools P;
@@ -832,9 +838,13 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
         const TileType &tt = e->types[tl.type];
         if (!tt.level) continue;
         const int nst = tt.nstatic, nt_top = ntop[tl.type];
-        int fit = LANES;   // neurons whose rows fit the shared memory (a chunk has at least 32 rows or ends a level)
-        while (fit > 1 && level_smem(nt_top, fit * nst, fit * nst / LANES + nst + 1, tt.crank != 0) > (size_t)kLevelSmemMax)
-            --fit;
+        // neurons whose rows fit the shared memory (a chunk has at least 32 rows or ends a level)
+        auto need = [&](int cellsn, bool res) {
+            return level_smem(nt_top, cellsn * nst, cellsn * nst / LANES + nst + 1, tt.crank != 0, mixed, res, 256);
+        };
+        const bool res = lvmode == 1 && need(1, true) <= (size_t)kLevelSmemMax;
+        int fit = LANES;
+        while (fit > 1 && need(fit, res) > lvmax) --fit;
         const int most = std::min(per_cells, fit);
         const int ng = (tl.nlanes + most - 1) / most;
         for (int q = 0, l0 = 0; q < ng; ++q) {
@@ -873,11 +883,11 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
             Cand c;
             c.g = g;
             c.warps = warps;
-            c.smem = level_smem(nt_top, g.n, g.nch, tt.crank != 0);
+            c.smem = level_smem(nt_top, g.n, g.nch, tt.crank != 0, mixed, res, nt);
             // launches of similar blocks: by kernel, warps and shared memory class
             int cls = 0;
             while (cls < 3 && c.smem > ((size_t)kLevelSmemMax / 8 << cls)) ++cls;
-            c.bucket = (tt.level - 1) * 64 + warps * 4 + cls;
+            c.bucket = ((tt.level - 1) * 2 + (res ? 0 : 1)) * 64 + warps * 4 + cls;
             cand.push_back(c);
             l0 += nl;
         }
@@ -2611,10 +2621,10 @@ int64_t gbh_jit_source(const gbh_batch_desc *desc, int precision, int type_index
     std::vector<double> tab64, xy;
     build_tables(desc, tg, tab64, xy);
     std::string src;
-    if (compact == 3) {
+    if (compact == 3 || compact == 4) {
         const LevelProg lp = level_prog(types[type_index], prog_pool);
         if (lp.ok) src = jit_level_source(lp, types[type_index], tg[types[type_index].table_set],
-                                          precision == GBH_PREC_MIXED);
+                                          precision == GBH_PREC_MIXED, compact == 3);
     } else {
         src = jit_source(types[type_index], prog_pool, tg[types[type_index].table_set], precision == GBH_PREC_MIXED,
                          false, uniform[type_index] ? &parents[type_index] : nullptr, 6, compact == 1, compact == 2);

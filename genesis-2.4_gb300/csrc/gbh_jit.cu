@@ -894,27 +894,28 @@ LevelProg level_prog(const TileType &tt, const std::vector<int> &prog)
     return lp;
 }
 
-std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed)
+std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed, bool resident)
 {
     Emit E;
     E.mixed = mixed;
     E.giv = false;
     std::ostringstream &o = E.o;
     const int N = lp.ntop;
-    const char *form = mixed ? "true" : "false", *crank = tt.crank ? "true" : "false";
+    const char *form = mixed ? "true" : "false", *crank = tt.crank ? "true" : "false",
+               *res = resident ? "true" : "false";
     o << "#include \"gbh_devfn.cuh\"\n#include \"gbh_level.cuh\"\nusing namespace gbh;\n"
       << "extern \"C\" __global__ void __launch_bounds__(" << kLevelThreads << ", " << kLevelBlocks
       << ") gbh_jit(DevView v, LevelView L, int g0, int nsteps, long long step0)\n{\n"
       << "  extern __shared__ double sm[];\n"
       << "  const LevelGroup g = L.groups[g0 + blockIdx.x];\n"
       << "  { unsigned dsz; asm(\"mov.u32 %0, %%dynamic_smem_size;\" : \"=r\"(dsz));\n"
-      << "    if (dsz < level_smem(" << N << ", g.n, g.nch, " << crank
-      << ")) { if (v.status && threadIdx.x == 0) atomicOr(v.status, ST_SMEM); return; } }\n"
+      << "    if (dsz < level_smem(" << N << ", g.n, g.nch, " << crank << ", " << form << ", " << res
+      << ", blockDim.x - 32)) { if (v.status && threadIdx.x == 0) atomicOr(v.status, ST_SMEM); return; } }\n"
       << "  const Tile tl = v.tiles[g.tile]; const TileType ty = v.types[tl.type];\n"
       << "  const unsigned sgen = v.sgen ? *v.sgen : 0u;\n"
       << "  if (threadIdx.x < blockDim.x - 32) {\n"
       << "    const bool full = !v.sgen || L.gen[g0 + blockIdx.x] != sgen, refresh = *v.kref != 0;\n"
-      << "    level_sweep<" << form << ", " << crank << ", " << N << ">(v, L, g, tl, ty, sm, nsteps, full, refresh);\n"
+      << "    level_sweep<" << form << ", " << crank << ", " << N << ", " << res << ">(v, L, g, tl, ty, sm, nsteps, full, refresh);\n"
       << "    if (full && v.sgen && threadIdx.x == 0) L.gen[g0 + blockIdx.x] = sgen;\n    return;\n  }\n"
       << "  const int lid = threadIdx.x & 31; const bool active = lid < g.nlanes; const int lane = g.lane0 + (active ? lid : 0);\n"
       << "  const long long sbase = v.step_dev ? *v.step_dev : 0;\n"
@@ -940,7 +941,8 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
           << "  const double *xvals = v.xyvals + " << tg.xv_off << "; (void)xvals;\n"
           << "  const double *yvals = v.xyvals + " << (tg.yv_off >= 0 ? tg.yv_off : tg.xv_off) << "; (void)yvals;\n";
     }
-    o << "  double *U = sm + lid; const double *PR = sm + " << N * LANES << " + g.n;\n"
+    o << "  const LevelSm q = level_smem_of<" << form << ", " << crank << ", " << N << ", " << res
+      << ">(sm, g, blockDim.x - 32);\n  double *U = q.U + lid; const double *PR = q.PR;\n"
       << "  for (int it = 0; it < nsteps; ++it) {\n"
       << "    const long long step = sbase + step0 + it; (void)step;\n"
       << "    double D[" << N << "], R[" << N << "], T[" << N << "], PD[" << N << "]; (void)T; (void)PD;\n"

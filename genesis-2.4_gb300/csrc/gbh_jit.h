@@ -41,7 +41,8 @@ struct LevelProg {
 };
 LevelProg level_prog(const TileType &tt, const std::vector<int> &prog);
 // Source of the level-elimination kernel (entry gbh_jit) for one such program.
-std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed);
+// resident: the block keeps its rows' constants in shared memory.
+std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed, bool resident);
 cudaError_t jit_level_launch(const JitKernel &k, const DevView &v, const LevelView &lv, int g0, int ngroups, int warps,
                              int nsteps, long long step, size_t smem, cudaStream_t st);
 // Largest dynamic shared memory the kernel may be launched with.

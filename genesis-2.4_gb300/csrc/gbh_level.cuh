@@ -59,11 +59,20 @@ struct LevelView {
     unsigned *gen;       // per group: the fields' generation its factors were kept at (DevView::sgen)
 };
 
-// Shared doubles of a group: the top rows' solutions, R / solutions, the
-// contributions R T and, under Crank-Nicolson, Vm; then its chunks.
-__host__ __device__ inline size_t level_smem(int ntop, int n, int nch, bool crank)
+// Where a block keeps its rows' constants between steps: in shared memory,
+// read from L2 once per launch (resident), or streamed from L2 through a ring
+// of LV_RING chunks on every sweep.
+constexpr int LV_RING = 6;
+
+// Shared memory of a group's block of nt sweeping threads, in the order
+// level_smem_of lays it out: the constants (or the ring), the top rows'
+// solutions, R / solutions, the contributions R T and, under Crank-Nicolson,
+// Vm; D' (FP64), the chunks and the indices.
+__host__ __device__ inline size_t level_smem(int ntop, int n, int nch, bool crank, bool mixed, bool resident, int nt)
 {
-    return sizeof(double) * ((size_t)ntop * LANES + (size_t)n * (crank ? 3 : 2)) + sizeof(int2) * (size_t)nch;
+    const size_t row = 16 + 8 + 4;   // two constants, D' or nothing, an index
+    const size_t state = 8 * ((size_t)ntop * LANES + (size_t)n * (crank ? 3 : 2)) + 8 * (size_t)nch;
+    return state + (resident ? (size_t)n * (2 * row - (mixed ? 16 : 8)) : LV_RING * row * (size_t)nt);
 }
 
 // Named barriers of a block: 1 the sweeping warps, 2 the static rows are
@@ -71,23 +80,78 @@ __host__ __device__ inline size_t level_smem(int ntop, int n, int nch, bool cran
 enum LevelBar { LB_SWEEP = 1, LB_FORWARD = 2, LB_TOP = 3 };
 
 #ifdef __CUDACC__
-// What the sweeping warps of a block do in a launch. sm: level_smem bytes.
-template <bool MIXED, bool CRANK, int NTOP>
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// One block's arrays in shared memory.
+struct LevelSm {
+    double2 *kt, *cy;    // resident: the constants; else kt is the ring's pairs
+    double *U, *X, *PR, *O, *d;
+    int2 *ch;
+    int *kid, *par;
+};
+template <bool MIXED, bool CRANK, int NTOP, bool RES>
+__device__ __forceinline__ LevelSm level_smem_of(double *sm, const LevelGroup &g, int nt)
+{
+    LevelSm q;
+    q.kt = reinterpret_cast<double2 *>(sm);
+    q.cy = q.kt + g.n;
+    double *p = sm + (RES ? 4 * g.n : 2 * LV_RING * nt);
+    q.U = p;
+    q.X = p + NTOP * LANES;
+    q.PR = q.X + g.n;
+    q.O = CRANK ? q.PR + g.n : q.X;
+    p = q.PR + g.n * (CRANK ? 2 : 1);
+    q.d = p;
+    p += RES ? (MIXED ? 0 : g.n) : LV_RING * nt;
+    q.ch = reinterpret_cast<int2 *>(p);
+    q.kid = reinterpret_cast<int *>(q.ch + g.nch);
+    q.par = q.kid + g.n;
+    return q;
+}
+
+// A row's constants in registers: (K, T) and its children forward, (C, 1/D'),
+// D' and its parent backward.
+struct LevelRow {
+    double2 a;
+    double d;
+    int k;
+};
+
+// What the sweeping warps of a block do in a launch (sm: level_smem bytes).
+template <bool MIXED, bool CRANK, int NTOP, bool RES>
 __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L, const LevelGroup &g, const Tile &tl,
                                             const TileType &ty, double *sm, int nsteps, bool full, bool refresh)
 {
     const int tid = threadIdx.x, nt = blockDim.x - LANES, nth = blockDim.x;
-    double *U = sm;                       // top rows' solutions, then the static rows' R / solution
-    double *X = U + NTOP * LANES;
-    double *PR = X + g.n;
-    double *O = CRANK ? PR + g.n : X;     // Vm
-    int2 *ch = reinterpret_cast<int2 *>(PR + g.n * (CRANK ? 2 : 1));
+    const LevelSm q = level_smem_of<MIXED, CRANK, NTOP, RES>(sm, g, nt);
+    double *const U = q.U, *const X = q.X, *const PR = q.PR, *const O = q.O;
+    const int2 *const ch = q.ch;
     const int nch = g.nch;
     const int *map = L.map + g.eoff, *kid = L.kid + g.eoff, *par = L.par + g.eoff;
     double2 *kt = L.kt + g.eoff, *cy = L.cy + g.eoff;
     double *dd = L.d + g.eoff, *pd = L.pd + g.eoff;
     double *V = v.V + tl.vm * LANES;
-    for (int c = tid; c < nch; c += nt) ch[c] = L.chunks[g.choff + c];
+    for (int c = tid; c < nch; c += nt) q.ch[c] = L.chunks[g.choff + c];
     for (int e = tid; e < g.n; e += nt) O[e] = V[map[e]];
     bar_named(LB_SWEEP, nt);
     // a row's rhs term from its fields, as its channel program forms it
@@ -129,86 +193,146 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
     } else if (refresh) {   // inputs on the rhs fields: their terms once per launch
         for (int e = tid; e < g.n; e += nt) kt[e].x = kterm(map[e]);
     }
-    __threadfence_block();
-    bar_named(LB_SWEEP, nt);
-    // Row data is loaded PF chunks ahead, across the barriers between levels:
-    // the loads (L2: some 300 clocks) would otherwise follow each barrier.
-    constexpr int PF = 4;
-    struct Fw { double2 kt; int kid; } fw[PF];
-    struct Bw { double2 cy; double d; int par; } bw[PF];
-    auto ldf = [&](Fw &q, int c) {
-        if (c < 0) return;
-        const int2 m = ch[c];
+    if (full || refresh) {
+        __threadfence_block();
+        bar_named(LB_SWEEP, nt);
+    }
+    if (RES) {
+        for (int e = tid; e < g.n; e += nt) {
+            cp_async16(&q.kt[e], &kt[e]);
+            cp_async16(&q.cy[e], &cy[e]);
+            if (!MIXED) cp_async8(&q.d[e], &dd[e]);
+            cp_async4(&q.kid[e], &kid[e]);
+            cp_async4(&q.par[e], &par[e]);
+        }
+        cp_commit();
+        cp_wait<0>();
+        bar_named(LB_SWEEP, nt);
+    }
+    // Streamed: the chunks of a step in the order they are used -- forward
+    // from the last, backward from the first -- are fetched LV_RING - 1 uses
+    // ahead, across levels, sweeps and steps (the loads would otherwise follow
+    // each level's barrier: some 600 clocks). Each thread fetches the rows it
+    // takes itself, so only its own copies have to be waited for.
+    int fpos = 0, fslot = 0, slot = 0;   // next use to fetch, its ring slot, the slot in use
+    int *const ring_i = q.kid;
+    auto fetch = [&]() {
+        if (RES) return;
+        const bool fwd = fpos < nch;
+        const int2 m = ch[fwd ? nch - 1 - fpos : fpos - nch];
         if (tid < (m.y & LV_COUNT)) {
-            q.kt = kt[m.x + tid];
-            q.kid = __ldg(&kid[m.x + tid]);
+            const int e = m.x + tid, s = fslot * nt + tid;
+            cp_async16(&q.kt[s], fwd ? &kt[e] : &cy[e]);
+            cp_async4(&ring_i[s], fwd ? &kid[e] : &par[e]);
+            if (!MIXED && !fwd) cp_async8(&q.d[s], &dd[e]);
+        }
+        cp_commit();
+        fpos = fpos + 1 == 2 * nch ? 0 : fpos + 1;
+        fslot = fslot + 1 == LV_RING ? 0 : fslot + 1;
+    };
+    auto take = [&](int e, bool fwd, LevelRow &r) {   // (every use takes one ring slot, rows or none)
+        if (RES) {
+            r.a = fwd ? q.kt[e] : q.cy[e];
+            r.k = fwd ? q.kid[e] : q.par[e];
+            if (!MIXED && !fwd) r.d = q.d[e];
+        } else {
+            const int s = slot * nt + tid;
+            r.a = q.kt[s];
+            r.k = ring_i[s];
+            if (!MIXED && !fwd) r.d = q.d[s];
         }
     };
-    auto ldb = [&](Bw &q, int c) {
-        if (c >= nch) return;
-        const int2 m = ch[c];
-        if (tid < (m.y & LV_COUNT)) {
-            q.cy = cy[m.x + tid];
-            if (!MIXED) q.d = dd[m.x + tid];
-            q.par = __ldg(&par[m.x + tid]);
-        }
+    auto next_slot = [&]() {
+        if (RES) return;
+        slot = slot + 1 == LV_RING ? 0 : slot + 1;
     };
-#pragma unroll
-    for (int u = 0; u < PF; ++u) ldf(fw[u], nch - 1 - u);
+    if (!RES)
+        for (int u = 0; u < LV_RING - 1; ++u) fetch();
     for (int it = 0; it < nsteps; ++it) {
-        for (int c0 = nch - 1; c0 >= 0; c0 -= PF) {
-#pragma unroll
-            for (int u = 0; u < PF; ++u) {
-                const int c = c0 - u;
-                if (c < 0) break;
-                const int2 m = ch[c];
-                if (tid < (m.y & LV_COUNT)) {
-                    const int e = m.x + tid;
-                    const int k0 = fw[u].kid & ((1 << LV_KID_BITS) - 1), nk = (unsigned)fw[u].kid >> LV_KID_BITS;
-                    double R = O[e] + fw[u].kt.x;
-                    for (int k = 0; k < nk; ++k) R -= PR[k0 + k];
-                    X[e] = R;
-                    PR[e] = R * fw[u].kt.y;
-                }
-                ldf(fw[u], c - PF);
-                if ((m.y & LV_FIRST) && c > 0) bar_named(LB_SWEEP, nt);
-            }
+        LevelRow row;
+        double o = 0.0;
+        int2 m = ch[nch - 1];
+        if (!RES) cp_wait<LV_RING - 2>();
+        if (tid < (m.y & LV_COUNT)) {
+            take(m.x + tid, true, row);
+            o = O[m.x + tid];
         }
-#pragma unroll
-        for (int u = 0; u < PF; ++u) ldb(bw[u], u);
+        next_slot();
+        for (int c = nch - 1; c >= 0; --c) {
+            const int2 mn = ch[c > 0 ? c - 1 : 0];
+            fetch();
+            if (tid < (m.y & LV_COUNT)) {
+                const int e = m.x + tid;
+                const int k0 = row.k & ((1 << LV_KID_BITS) - 1), nk = (unsigned)row.k >> LV_KID_BITS;
+                // the first two children's loads together (their elements
+                // exist wherever they are subtracted)
+                const double c0 = nk > 0 ? PR[k0] : 0.0, c1 = nk > 1 ? PR[k0 + 1] : 0.0;
+                double R = o + row.a.x;
+                R = nk > 0 ? R - c0 : R;
+                R = nk > 1 ? R - c1 : R;
+                for (int k = 2; k < nk; ++k) R -= PR[k0 + k];
+                X[e] = R;
+                PR[e] = R * row.a.y;
+            }
+            if (c > 0) {   // the next rows' own data, before the barrier
+                if (!RES) cp_wait<LV_RING - 2>();
+                if (tid < (mn.y & LV_COUNT)) {
+                    take(mn.x + tid, true, row);
+                    o = O[mn.x + tid];
+                }
+                next_slot();
+                if (m.y & LV_FIRST) bar_named(LB_SWEEP, nt);
+            }
+            m = mn;
+        }
+        m = ch[0];
+        double r0 = 0.0;
+        if (!RES) cp_wait<LV_RING - 2>();
+        if (tid < (m.y & LV_COUNT)) {
+            take(m.x + tid, false, row);
+            r0 = X[m.x + tid];
+            if (CRANK) o = O[m.x + tid];
+        }
+        next_slot();
         bar_named(LB_FORWARD, nth);
         bar_named(LB_TOP, nth);
-        for (int c0 = 0; c0 < nch; c0 += PF) {
-#pragma unroll
-            for (int u = 0; u < PF; ++u) {
-                const int c = c0 + u;
-                if (c >= nch) break;
-                const int2 m = ch[c];
-                if (tid < (m.y & LV_COUNT)) {
-                    const int e = m.x + tid;
-                    const double xp = U[bw[u].par], y = bw[u].cy.y;
-                    double r;
-                    if (MIXED) {
-                        r = fma(-bw[u].cy.x, xp, X[e]) * y;
-                    } else {
-                        // RN(r / D') from the correctly rounded y = 1/D' by
-                        // Markstein's correction, the division's bits
-                        r = X[e] - bw[u].cy.x * xp;
-                        const double q = r * y;
-                        r = fma(fma(-bw[u].d, q, r), y, q);
-                    }
-                    X[e] = r;
-                    if (CRANK) O[e] = MIXED ? fma(2.0, r, -O[e]) : r + r - O[e];
+        for (int c = 0; c < nch; ++c) {
+            const int2 mn = ch[c + 1 < nch ? c + 1 : c];
+            fetch();
+            if (tid < (m.y & LV_COUNT)) {
+                const int e = m.x + tid;
+                const double xp = U[row.k], y = row.a.y;
+                double r;
+                if (MIXED) {
+                    r = fma(-row.a.x, xp, r0) * y;
+                } else {
+                    // RN(r / D') from the correctly rounded y = 1/D' by
+                    // Markstein's correction, the division's bits
+                    r = r0 - row.a.x * xp;
+                    const double t = r * y;
+                    r = fma(fma(-row.d, t, r), y, t);
                 }
-                ldb(bw[u], c + PF);
+                X[e] = r;
+                if (CRANK) O[e] = MIXED ? fma(2.0, r, -o) : r + r - o;
+            }
+            if (c + 1 < nch) {
+                if (!RES) cp_wait<LV_RING - 2>();
+                if (tid < (mn.y & LV_COUNT)) {
+                    take(mn.x + tid, false, row);
+                    r0 = X[mn.x + tid];
+                    if (CRANK) o = O[mn.x + tid];
+                }
+                next_slot();
                 if (m.y & LV_LAST) bar_named(LB_SWEEP, nt);
             }
+            m = mn;
         }
-        if (it + 1 < nsteps) {
-#pragma unroll
-            for (int u = 0; u < PF; ++u) ldf(fw[u], nch - 1 - u);
-        }
+        // (no barrier here: the next forward sweep starts with the deepest
+        // level, whose solutions no other row reads, and passes one before it
+        // rewrites any row above)
     }
+    if (!RES) cp_wait<0>();
+    bar_named(LB_SWEEP, nt);
     for (int e = tid; e < g.n; e += nt) V[map[e]] = O[e];
 }
 

@@ -257,8 +257,9 @@ int gbh_validate(const gbh_batch_desc *desc, gbh_error *err, int64_t *n_neurons,
  * type_index (neurons sharing one program) into buf (NUL-terminated,
  * truncated to buflen). Returns the full source length, or a negative error.
  * compact: 0 unrolled form, 1 compact (looped) form, 2 unrolled form with its
- * rows in shared memory, 3 the level-elimination kernel of a tree with
- * passive dendrites (length 0 where the type has none). Needs no GPU.
+ * rows in shared memory, 3 and 4 the level-elimination kernel of a tree
+ * with passive dendrites, its constants resident or streamed (length 0 where
+ * the type has none). Needs no GPU.
  */
 int64_t gbh_jit_source(const gbh_batch_desc *desc, int precision, int type_index, int compact, char *buf,
                        int64_t buflen);

@@ -143,10 +143,11 @@ def test_level_reports_a_lost_vm(gpu_engine):
 
 @pytest.mark.parametrize("prec", [engine.PREC_FP64, engine.PREC_MIXED])
 @pytest.mark.parametrize("tops", [1, 4])
-def test_level_source_compiles(tmp_path, prec, tops):
+@pytest.mark.parametrize("form", [3, 4])
+def test_level_source_compiles(tmp_path, prec, tops, form):
     h = _trees(1, 40, 5, tops=tops)[0]
-    src = engine.jit_source([h], prec, 0, 3)
-    assert "level_sweep<%s, false, %d>" % ("true" if prec else "false", tops) in src
+    src = engine.jit_source([h], prec, 0, form)
+    assert "level_sweep<%s, false, %d, %s>" % ("true" if prec else "false", tops, "true" if form == 3 else "false") in src
     f = tmp_path / "level.cu"
     f.write_text(src)
     subprocess.run([build.nvcc()] + build.ARCH + ["-std=c++17", "-I" + build.CSRC, "-cubin", "-o",
