@@ -174,7 +174,7 @@ struct gbh_engine {
     DBuf<int2> d_lchunks;
     DBuf<int> d_lmap, d_lkid, d_lpar, d_ltopkid;
     DBuf<double2> d_lkt, d_lcy;
-    DBuf<double> d_ld, d_lpd;
+    DBuf<double> d_lc, d_ld, d_lpd;
     DBuf<unsigned> d_lgen;
     int steps_per_launch = 1;
     bool has_network = false;
@@ -729,7 +729,7 @@ struct LevelPlan {
 struct LevelPools {
     std::vector<int2> chunks;
     std::vector<int> map, kid, par, topkid;
-    std::vector<double2> cy;
+    std::vector<double> c;
 };
 
 // Level order of the static rows of a group: order[] = row * 32 + group lane,
@@ -875,7 +875,7 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
             for (int x : order) {
                 const int row = x / LANES, l = x % LANES;
                 P.map.push_back(row * LANES + l0 + l);
-                P.cy.push_back(make_double2(cl[l]->C[row], 0.0));
+                P.c.push_back(cl[l]->C[row]);
             }
             P.kid.insert(P.kid.end(), kid.begin(), kid.end());
             P.par.insert(P.par.end(), par.begin(), par.end());
@@ -907,8 +907,8 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
     for (const Cand &c : cand) out.groups.push_back(c.g);
     const size_t n = P.map.size();
     if (e->d_lgroups.upload(out.groups) || e->d_lchunks.upload(P.chunks) || e->d_lmap.upload(P.map) ||
-        e->d_lkid.upload(P.kid) || e->d_lpar.upload(P.par) || e->d_ltopkid.upload(P.topkid) || e->d_lcy.upload(P.cy) ||
-        e->d_lkt.alloc(n) || e->d_ld.alloc(n) || e->d_lpd.alloc(n) ||
+        e->d_lkid.upload(P.kid) || e->d_lpar.upload(P.par) || e->d_ltopkid.upload(P.topkid) || e->d_lc.upload(P.c) ||
+        e->d_lcy.alloc(n) || e->d_lkt.alloc(n) || e->d_ld.alloc(n) || e->d_lpd.alloc(n) ||
         e->d_lgen.upload(std::vector<unsigned>(out.groups.size(), 0u)))
         return GBH_ERR_CUDA;
     return GBH_OK;
@@ -1651,6 +1651,7 @@ int launch_one(gbh_engine *e, const DevView &v, const Launch &L, int k, long lon
         lv.topkid = e->d_ltopkid.p;
         lv.kt = e->d_lkt.p;
         lv.cy = e->d_lcy.p;
+        lv.c = e->d_lc.p;
         lv.d = e->d_ld.p;
         lv.pd = e->d_lpd.p;
         lv.gen = e->d_lgen.p;
@@ -3558,7 +3559,7 @@ void gbh_destroy(gbh_engine *e)
         for (JitKernel &k : vars) jit_release(k);
     for (JitKernel &k : e->lv_kern) jit_release(k);
     e->d_lgroups.release(); e->d_lchunks.release(); e->d_lmap.release(); e->d_lkid.release(); e->d_lpar.release();
-    e->d_ltopkid.release(); e->d_lkt.release(); e->d_lcy.release(); e->d_ld.release(); e->d_lpd.release();
+    e->d_ltopkid.release(); e->d_lkt.release(); e->d_lcy.release(); e->d_lc.release(); e->d_ld.release(); e->d_lpd.release();
     e->d_lgen.release();
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);

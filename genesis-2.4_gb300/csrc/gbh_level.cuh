@@ -53,7 +53,8 @@ struct LevelView {
     const int *par;      // parent's solution: top row * 32 + lane of the group, or ntop * 32 + its element
     const int *topkid;
     double2 *kt;         // rhs term K, coupling factor T = A / D'
-    double2 *cy;         // backward coefficient C, 1 / D'
+    double2 *cy;         // backward coefficient C (mixed: C / D'), 1 / D'
+    const double *c;     // C
     double *d;           // D' (FP64 form)
     double *pd;          // B T: what the row takes from its parent's diagonal
     unsigned *gen;       // per group: the fields' generation its factors were kept at (DevView::sgen)
@@ -129,8 +130,8 @@ __device__ __forceinline__ LevelSm level_smem_of(double *sm, const LevelGroup &g
     return q;
 }
 
-// A row's constants in registers: (K, T) and its children forward, (C, 1/D'),
-// D' and its parent backward.
+// A row's constants in registers: (K, T) and its children forward, (C, 1/D')
+// -- mixed (C/D', 1/D') -- D' and its parent backward.
 struct LevelRow {
     double2 a;
     double d;
@@ -185,7 +186,7 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
                 PR[e] = b;
                 pd[e] = b;
                 kt[e] = make_double2(kterm(r), T);
-                cy[e].y = y;
+                cy[e] = make_double2(MIXED ? L.c[g.eoff + e] * y : L.c[g.eoff + e], y);
                 if (!MIXED) dd[e] = D;
             }
             if (m.y & LV_FIRST) bar_named(LB_SWEEP, nt);
@@ -216,6 +217,10 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
     // takes itself, so only its own copies have to be waited for.
     int fpos = 0, fslot = 0, slot = 0;   // next use to fetch, its ring slot, the slot in use
     int *const ring_i = q.kid;
+    // mixed, resident: a parent subtracts R T in one multiply-add, T from its
+    // child's constants; else the child leaves R T in PR
+    constexpr bool FMA = MIXED && RES;
+    const double *const pulled = FMA ? X : PR;
     auto fetch = [&]() {
         if (RES) return;
         const bool fwd = fpos < nch;
@@ -248,84 +253,113 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
     };
     if (!RES)
         for (int u = 0; u < LV_RING - 1; ++u) fetch();
+    // The FP64 unit takes an instruction from a warp every 64 clocks, whatever
+    // depends on it, so a level lasts as long as its instructions in a row:
+    // whatever does not wait for the level before is formed ahead of the
+    // barrier -- the constants, Vm + K forward and, mixed, R / D' backward.
     for (int it = 0; it < nsteps; ++it) {
         LevelRow row;
-        double o = 0.0;
+        double own = 0.0, old = 0.0;
         int2 m = ch[nch - 1];
+        bool mine = tid < (m.y & LV_COUNT);
         if (!RES) cp_wait<LV_RING - 2>();
-        if (tid < (m.y & LV_COUNT)) {
+        if (mine) {
             take(m.x + tid, true, row);
-            o = O[m.x + tid];
+            own = O[m.x + tid] + row.a.x;
         }
         next_slot();
         for (int c = nch - 1; c >= 0; --c) {
             const int2 mn = ch[c > 0 ? c - 1 : 0];
+            const bool minen = c > 0 && tid < (mn.y & LV_COUNT);
+            const int k0 = row.k & ((1 << LV_KID_BITS) - 1), nk = mine ? (unsigned)row.k >> LV_KID_BITS : 0;
+            // the first two children's loads together
+            double c0 = 0.0, c1 = 0.0, t0 = 0.0, t1 = 0.0;
+            if (nk > 0) {
+                c0 = pulled[k0];
+                if (FMA) t0 = q.kt[k0].y;
+            }
+            if (nk > 1) {
+                c1 = pulled[k0 + 1];
+                if (FMA) t1 = q.kt[k0 + 1].y;
+            }
+            LevelRow rn;
+            double on = 0.0;
             fetch();
-            if (tid < (m.y & LV_COUNT)) {
+            if (!RES) cp_wait<LV_RING - 2>();
+            if (minen) {
+                take(mn.x + tid, true, rn);
+                on = O[mn.x + tid];
+            }
+            if (c > 0) next_slot();
+            if (mine) {
                 const int e = m.x + tid;
-                const int k0 = row.k & ((1 << LV_KID_BITS) - 1), nk = (unsigned)row.k >> LV_KID_BITS;
-                // the first two children's loads together (their elements
-                // exist wherever they are subtracted)
-                const double c0 = nk > 0 ? PR[k0] : 0.0, c1 = nk > 1 ? PR[k0 + 1] : 0.0;
-                double R = o + row.a.x;
-                R = nk > 0 ? R - c0 : R;
-                R = nk > 1 ? R - c1 : R;
-                for (int k = 2; k < nk; ++k) R -= PR[k0 + k];
-                X[e] = R;
-                PR[e] = R * row.a.y;
-            }
-            if (c > 0) {   // the next rows' own data, before the barrier
-                if (!RES) cp_wait<LV_RING - 2>();
-                if (tid < (mn.y & LV_COUNT)) {
-                    take(mn.x + tid, true, row);
-                    o = O[mn.x + tid];
+                double R = own;
+                if (FMA) {
+                    if (nk > 0) R = fma(-c0, t0, R);
+                    if (nk > 1) R = fma(-c1, t1, R);
+                    for (int k = 2; k < nk; ++k) R = fma(-X[k0 + k], q.kt[k0 + k].y, R);
+                } else {
+                    if (nk > 0) R -= c0;
+                    if (nk > 1) R -= c1;
+                    for (int k = 2; k < nk; ++k) R -= PR[k0 + k];
+                    PR[e] = R * row.a.y;
                 }
-                next_slot();
-                if (m.y & LV_FIRST) bar_named(LB_SWEEP, nt);
+                X[e] = R;
             }
+            if (c > 0 && (m.y & LV_FIRST)) bar_named(LB_SWEEP, nt);
+            own = on + rn.a.x;
+            row = rn;
             m = mn;
+            mine = minen;
         }
         m = ch[0];
-        double r0 = 0.0;
+        mine = tid < (m.y & LV_COUNT);
         if (!RES) cp_wait<LV_RING - 2>();
-        if (tid < (m.y & LV_COUNT)) {
+        if (mine) {
             take(m.x + tid, false, row);
-            r0 = X[m.x + tid];
-            if (CRANK) o = O[m.x + tid];
+            own = X[m.x + tid];
+            if (MIXED) own *= row.a.y;
+            if (CRANK) old = O[m.x + tid];
         }
         next_slot();
         bar_named(LB_FORWARD, nth);
         bar_named(LB_TOP, nth);
         for (int c = 0; c < nch; ++c) {
             const int2 mn = ch[c + 1 < nch ? c + 1 : c];
+            const bool minen = c + 1 < nch && tid < (mn.y & LV_COUNT);
+            double xp = 0.0;
+            if (mine) xp = U[row.k];
+            LevelRow rn;
+            double on = 0.0, oldn = 0.0;
             fetch();
-            if (tid < (m.y & LV_COUNT)) {
+            if (!RES) cp_wait<LV_RING - 2>();
+            if (minen) {
+                take(mn.x + tid, false, rn);
+                on = X[mn.x + tid];
+                if (CRANK) oldn = O[mn.x + tid];
+            }
+            if (c + 1 < nch) next_slot();
+            if (mine) {
                 const int e = m.x + tid;
-                const double xp = U[row.k], y = row.a.y;
                 double r;
                 if (MIXED) {
-                    r = fma(-row.a.x, xp, r0) * y;
+                    r = fma(-row.a.x, xp, own);   // R / D' - (C / D') x
                 } else {
                     // RN(r / D') from the correctly rounded y = 1/D' by
                     // Markstein's correction, the division's bits
-                    r = r0 - row.a.x * xp;
-                    const double t = r * y;
-                    r = fma(fma(-row.d, t, r), y, t);
+                    r = own - row.a.x * xp;
+                    const double t = r * row.a.y;
+                    r = fma(fma(-row.d, t, r), row.a.y, t);
                 }
                 X[e] = r;
-                if (CRANK) O[e] = MIXED ? fma(2.0, r, -o) : r + r - o;
+                if (CRANK) O[e] = MIXED ? fma(2.0, r, -old) : r + r - old;
             }
-            if (c + 1 < nch) {
-                if (!RES) cp_wait<LV_RING - 2>();
-                if (tid < (mn.y & LV_COUNT)) {
-                    take(mn.x + tid, false, row);
-                    r0 = X[mn.x + tid];
-                    if (CRANK) o = O[mn.x + tid];
-                }
-                next_slot();
-                if (m.y & LV_LAST) bar_named(LB_SWEEP, nt);
-            }
+            if (c + 1 < nch && (m.y & LV_LAST)) bar_named(LB_SWEEP, nt);
+            own = MIXED ? on * rn.a.y : on;
+            old = oldn;
+            row = rn;
             m = mn;
+            mine = minen;
         }
         // (no barrier here: the next forward sweep starts with the deepest
         // level, whose solutions no other row reads, and passes one before it
@@ -338,14 +372,16 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
 
 // The static children of top row s of this lane: their contributions off
 // (R, D), in ascending row order.
-__device__ __forceinline__ void level_top_kids(const LevelView &L, const LevelGroup &g, const double *PR, int s,
+template <bool FMA>
+__device__ __forceinline__ void level_top_kids(const LevelView &L, const LevelGroup &g, const LevelSm &q, int s,
                                                int lane, double &R, double &D)
 {
     const int kk = L.topkid[g.kidoff + s * LANES + lane];
     const int k0 = kk & ((1 << LV_KID_BITS) - 1), nk = (unsigned)kk >> LV_KID_BITS;
     for (int k = 0; k < nk; ++k) {
         D -= L.pd[g.eoff + k0 + k];
-        R -= PR[k0 + k];
+        if (FMA) R = fma(-q.X[k0 + k], q.kt[k0 + k].y, R);
+        else R -= q.PR[k0 + k];
     }
 }
 #endif
