@@ -172,7 +172,7 @@ struct gbh_engine {
     std::vector<JitKernel> lv_kern;
     DBuf<LevelGroup> d_lgroups;
     DBuf<int2> d_lchunks;
-    DBuf<int> d_lmap, d_lkid, d_lpar, d_ltopkid;
+    DBuf<int> d_lmap, d_lkid, d_lnkid, d_lpar, d_ltopkid;
     DBuf<double2> d_lkt, d_lcy;
     DBuf<double> d_lc, d_ld, d_lpd;
     DBuf<unsigned> d_lgen;
@@ -711,10 +711,10 @@ bool level_type(const TileType &tt, const std::vector<int> &prog, const std::vec
         }
         if (tt.nstatic < 2 * levels) return false;
     }
-    // one neuron's rows must fit a block (streamed constants, 8 sweeping warps)
-    if (level_smem(kSplitRows, tt.nstatic, tt.nstatic + 1, tt.crank != 0, false, false, 256) > (size_t)kLevelSmemMax)
+    // one neuron's rows must fit a block (constants in global memory)
+    if (level_smem(kSplitRows, tt.nstatic, tt.nstatic + 1, tt.crank != 0, false, false) > (size_t)kLevelSmemMax)
         return false;
-    if (tt.nstatic * LANES >= 1 << LV_KID_BITS) return false;
+    if (tt.nstatic > LV_MAX_ROWS) return false;
     lp = level_prog(tt, prog);
     return lp.ok;
 }
@@ -724,45 +724,53 @@ struct LevelPlan {
     std::vector<Launch> launches;
 };
 
-// One group's level order: appends its rows, chunks (of `nt` rows at most)
-// and the top rows' static children to the pools.
+// The level-ordered arrays of all groups (LevelView).
 struct LevelPools {
     std::vector<int2> chunks;
-    std::vector<int> map, kid, par, topkid;
+    std::vector<int> map, kid, nkid, par, topkid;
     std::vector<double> c;
 };
 
 // Level order of the static rows of a group: order[] = row * 32 + group lane,
-// level starts; kid / par as LevelView holds them. Rows of a level are
-// sorted by their parent's place, then ascending, so a row's children are
-// consecutive and in the order the sequential sweep subtracts them.
+// level starts; kid, nkid, par and topkid as LevelView holds them. Rows of a
+// level are sorted by their parent's place, then ascending, so a row's
+// children are consecutive and in the order the sequential sweep subtracts
+// them.
 void level_order(const std::vector<const Neuron *> &cells, int nst, int ntop, std::vector<int> &order,
-                 std::vector<int> &start, std::vector<int> &kid, std::vector<int> &par, std::vector<int> &topkid)
+                 std::vector<int> &start, std::vector<int> &kid, std::vector<int> &nkid, std::vector<int> &par,
+                 std::vector<int> &topkid)
 {
-    const int nl = (int)cells.size();
+    const int nl = (int)cells.size(), zero = nst * nl;
     std::vector<std::vector<int>> kids((size_t)(nst + ntop) * nl);   // static children of row * nl + lane, ascending
     for (int l = 0; l < nl; ++l)
         for (int s = 0; s < nst; ++s) kids[(size_t)cells[l]->parent[s] * nl + l].push_back(s);
     order.clear();
-    kid.assign((size_t)nst * nl, 0);
-    par.assign((size_t)nst * nl, 0);
+    kid.assign((size_t)zero + LV_SPARE, zero | zero << 16);
+    nkid.assign((size_t)zero + LV_SPARE, 0);
+    par.assign((size_t)zero + LV_SPARE, 0);
     topkid.assign((size_t)ntop * LANES, 0);
     start.assign(1, 0);
     auto put = [&](int row, int l, int p) {   // the children of a row whose solution is at p
         const std::vector<int> &c = kids[(size_t)row * nl + l];
-        const int word = (int)order.size() | (int)((unsigned)c.size() << LV_KID_BITS);
         for (int k : c) {
             par[order.size()] = p;
             order.push_back(k * LANES + l);
         }
-        return word;
+        return (int)c.size();
     };
     for (int s = 0; s < ntop; ++s)
-        for (int l = 0; l < nl; ++l) topkid[s * LANES + l] = put(nst + s, l, s * LANES + l);
+        for (int l = 0; l < nl; ++l) {
+            const int k0 = (int)order.size(), n = put(nst + s, l, s * LANES + l);
+            topkid[s * LANES + l] = k0 | n << LV_KID_BITS;
+        }
     while ((int)order.size() > start.back()) {
         const int e0 = start.back(), e1 = (int)order.size();
         start.push_back(e1);
-        for (int e = e0; e < e1; ++e) kid[e] = put(order[e] / LANES, order[e] % LANES, ntop * LANES + e);
+        for (int e = e0; e < e1; ++e) {
+            const int k0 = (int)order.size(), n = put(order[e] / LANES, order[e] % LANES, ntop * LANES + e);
+            kid[e] = (n > 0 ? k0 : zero) | (n > 1 ? k0 + 1 : zero) << 16;
+            nkid[e] = n;
+        }
     }
 }
 
@@ -820,8 +828,6 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
     // ---- groups: enough of them for two blocks a SM, as many neurons each as
     // that leaves (the top rows' warp issues for 32 neurons what it issues for one) ----
     const int per_cells = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + kLevelGroups - 1) / kLevelGroups));
-    const char *lvenv = getenv("GBH_LV");
-    const int lvmode = lvenv ? atoi(lvenv) : 1;
     const size_t lvmax = getenv("GBH_LVMAX") ? (size_t)atoi(getenv("GBH_LVMAX")) * 1024 : (size_t)kLevelSmemMax;
     struct Cand { LevelGroup g; int warps, bucket; size_t smem; };
     std::vector<Cand> cand;
@@ -840,9 +846,9 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
         const int nst = tt.nstatic, nt_top = ntop[tl.type];
         // neurons whose rows fit the shared memory (a chunk has at least 32 rows or ends a level)
         auto need = [&](int cellsn, bool res) {
-            return level_smem(nt_top, cellsn * nst, cellsn * nst / LANES + nst + 1, tt.crank != 0, mixed, res, 256);
+            return level_smem(nt_top, cellsn * nst, cellsn * nst / LANES + nst + 1, tt.crank != 0, mixed, res);
         };
-        const bool res = lvmode == 1 && need(1, true) <= (size_t)kLevelSmemMax;
+        const bool res = need(1, true) <= (size_t)kLevelSmemMax;
         int fit = LANES;
         while (fit > 1 && need(fit, res) > lvmax) --fit;
         const int most = std::min(per_cells, fit);
@@ -851,8 +857,8 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
             const int nl = (tl.nlanes - l0 + (ng - q) - 1) / (ng - q);
             std::vector<const Neuron *> cl;
             for (int l = l0; l < l0 + nl; ++l) cl.push_back(&dec.neurons[cells_of[t][l]]);
-            std::vector<int> order, start, kid, par, topkid;
-            level_order(cl, nst, nt_top, order, start, kid, par, topkid);
+            std::vector<int> order, start, kid, nkid, par, topkid;
+            level_order(cl, nst, nt_top, order, start, kid, nkid, par, topkid);
             LevelGroup g{};
             g.tile = (int)t;
             g.lane0 = l0;
@@ -861,6 +867,7 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
             g.eoff = (int64_t)P.map.size();
             g.kidoff = (int)P.topkid.size();
             g.choff = (int)P.chunks.size();
+            for (int x : nkid) g.many |= x > 2;
             const int nlev = (int)start.size() - 1;
             int warps = 1;   // as many sweeping warps as a level has rows for, on average
             while (warps < 8 && warps * LANES * nlev < g.n) warps *= 2;
@@ -877,13 +884,16 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
                 P.map.push_back(row * LANES + l0 + l);
                 P.c.push_back(cl[l]->C[row]);
             }
+            P.map.resize(P.map.size() + LV_SPARE, 0);
+            P.c.resize(P.c.size() + LV_SPARE, 0.0);
             P.kid.insert(P.kid.end(), kid.begin(), kid.end());
+            P.nkid.insert(P.nkid.end(), nkid.begin(), nkid.end());
             P.par.insert(P.par.end(), par.begin(), par.end());
             P.topkid.insert(P.topkid.end(), topkid.begin(), topkid.end());
             Cand c;
             c.g = g;
             c.warps = warps;
-            c.smem = level_smem(nt_top, g.n, g.nch, tt.crank != 0, mixed, res, nt);
+            c.smem = level_smem(nt_top, g.n, g.nch, tt.crank != 0, mixed, res);
             // launches of similar blocks: by kernel, warps and shared memory class
             int cls = 0;
             while (cls < 3 && c.smem > ((size_t)kLevelSmemMax / 8 << cls)) ++cls;
@@ -907,10 +917,13 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
     for (const Cand &c : cand) out.groups.push_back(c.g);
     const size_t n = P.map.size();
     if (e->d_lgroups.upload(out.groups) || e->d_lchunks.upload(P.chunks) || e->d_lmap.upload(P.map) ||
-        e->d_lkid.upload(P.kid) || e->d_lpar.upload(P.par) || e->d_ltopkid.upload(P.topkid) || e->d_lc.upload(P.c) ||
+        e->d_lkid.upload(P.kid) || e->d_lnkid.upload(P.nkid) || e->d_lpar.upload(P.par) || e->d_ltopkid.upload(P.topkid) || e->d_lc.upload(P.c) ||
         e->d_lcy.alloc(n) || e->d_lkt.alloc(n) || e->d_ld.alloc(n) || e->d_lpd.alloc(n) ||
         e->d_lgen.upload(std::vector<unsigned>(out.groups.size(), 0u)))
         return GBH_ERR_CUDA;
+    CK(cudaMemset(e->d_lkt.p, 0, n * sizeof(double2)));   // (the spare elements' constants)
+    CK(cudaMemset(e->d_lcy.p, 0, n * sizeof(double2)));
+    CK(cudaMemset(e->d_ld.p, 0, n * sizeof(double)));
     return GBH_OK;
 }
 
@@ -1647,6 +1660,7 @@ int launch_one(gbh_engine *e, const DevView &v, const Launch &L, int k, long lon
         lv.chunks = e->d_lchunks.p;
         lv.map = e->d_lmap.p;
         lv.kid = e->d_lkid.p;
+        lv.nkid = e->d_lnkid.p;
         lv.par = e->d_lpar.p;
         lv.topkid = e->d_ltopkid.p;
         lv.kt = e->d_lkt.p;
@@ -3558,7 +3572,7 @@ void gbh_destroy(gbh_engine *e)
     for (auto &vars : e->jit_var)
         for (JitKernel &k : vars) jit_release(k);
     for (JitKernel &k : e->lv_kern) jit_release(k);
-    e->d_lgroups.release(); e->d_lchunks.release(); e->d_lmap.release(); e->d_lkid.release(); e->d_lpar.release();
+    e->d_lgroups.release(); e->d_lchunks.release(); e->d_lmap.release(); e->d_lkid.release(); e->d_lnkid.release(); e->d_lpar.release();
     e->d_ltopkid.release(); e->d_lkt.release(); e->d_lcy.release(); e->d_lc.release(); e->d_ld.release(); e->d_lpd.release();
     e->d_lgen.release();
     if (e->ev0) cudaEventDestroy(e->ev0);

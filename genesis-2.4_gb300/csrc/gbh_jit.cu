@@ -910,7 +910,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
       << "  const LevelGroup g = L.groups[g0 + blockIdx.x];\n"
       << "  { unsigned dsz; asm(\"mov.u32 %0, %%dynamic_smem_size;\" : \"=r\"(dsz));\n"
       << "    if (dsz < level_smem(" << N << ", g.n, g.nch, " << crank << ", " << form << ", " << res
-      << ", blockDim.x - 32)) { if (v.status && threadIdx.x == 0) atomicOr(v.status, ST_SMEM); return; } }\n"
+      << ")) { if (v.status && threadIdx.x == 0) atomicOr(v.status, ST_SMEM); return; } }\n"
       << "  const Tile tl = v.tiles[g.tile]; const TileType ty = v.types[tl.type];\n"
       << "  const unsigned sgen = v.sgen ? *v.sgen : 0u;\n"
       << "  if (threadIdx.x < blockDim.x - 32) {\n"
@@ -942,7 +942,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
           << "  const double *yvals = v.xyvals + " << (tg.yv_off >= 0 ? tg.yv_off : tg.xv_off) << "; (void)yvals;\n";
     }
     o << "  const LevelSm q = level_smem_of<" << form << ", " << crank << ", " << N << ", " << res
-      << ">(sm, g, blockDim.x - 32);\n  double *U = q.U + lid;\n"
+      << ">(sm, g);\n  double *U = q.U + lid;\n"
       << "  for (int it = 0; it < nsteps; ++it) {\n"
       << "    const long long step = sbase + step0 + it; (void)step;\n"
       << "    double D[" << N << "], R[" << N << "], T[" << N << "], PD[" << N << "]; (void)T; (void)PD;\n"
@@ -965,7 +965,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
     o << "    }\n    __syncwarp();\n    bar_named(LB_FORWARD, blockDim.x);\n    if (active) {\n";
     for (int s = 0; s < N; ++s) {
         const std::string S = "[" + std::to_string(s) + "]", r = std::to_string(s * LANES);
-        o << "      level_top_kids<" << (mixed && resident ? "true" : "false") << ">(L, g, q, " << s << ", lid, R" << S << ", D" << S << ");\n";
+        o << "      level_top_kids<" << form << ", " << res << ">(L, g, q, " << s << ", lid, R" << S << ", D" << S << ");\n";
         for (int j = 0; j < s; ++j)   // top rows below this one, after the static rows: ascending row order
             o << "      if (tp[" << j << "] == " << s << ") { D" << S << " -= PD[" << j << "]; R" << S << " -= T[" << j << "]; }\n";
         if (mixed) o << "      D" << S << " = rcp_newton(D" << S << ");\n";
