@@ -448,9 +448,12 @@ constexpr int kStackMin = 8;
 // Shared memory a stack-elimination warp may take (doubles per lane).
 constexpr int kStackCapMax = 200 * 1024 / (LANES * (int)sizeof(double)) - 2 * kSplitRows;
 
-// Level elimination: shared memory of a block, groups wanted (two a SM of
-// the 152) and distinct programs compiled.
-constexpr int kLevelSmemMax = 224 * 1024, kLevelGroups = 304;
+// Level elimination: most shared memory a block may take, and what groups of
+// several neurons are kept to (three blocks an SM: 16,384 random trees of
+// 8-256 compartments, mixed, 23.4 us a step; 110 KB 24.0, 224 KB 26.1, 40 KB
+// 25.4); groups wanted (one an SM; 2,000 trees, FP64: 12.1 us a step, 14.0
+// with two); distinct programs compiled.
+constexpr int kLevelSmemMax = 224 * 1024, kLevelSmemGroup = 72 * 1024, kLevelGroups = 152;
 constexpr size_t kLevelKernels = 8;
 
 // Largest types specialised whole: the looped forms keep 2 x nslots x 32 rows
@@ -825,10 +828,37 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
             for (TileType &tt : e->types)
                 if (tt.level == 1 + (int)c / 2) tt.level = 0;
         }
-    // ---- groups: enough of them for two blocks a SM, as many neurons each as
-    // that leaves (the top rows' warp issues for 32 neurons what it issues for one) ----
+    // ---- groups: enough of them for every SM, as many neurons each as that
+    // leaves (the top rows' warp issues for 32 neurons what it issues for one) ----
     const int per_cells = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + kLevelGroups - 1) / kLevelGroups));
-    const size_t lvmax = getenv("GBH_LVMAX") ? (size_t)atoi(getenv("GBH_LVMAX")) * 1024 : (size_t)kLevelSmemMax;
+    // neurons of a type that go into one group: their rows fit the shared
+    // memory (a chunk has at least 32 rows or ends a level); resident: so do
+    // their constants
+    auto most_cells = [&](const TileType &tt, int nt_top, bool &res) {
+        auto need = [&](int n) {
+            return level_smem(nt_top, n * tt.nstatic, n * tt.nstatic / LANES + tt.nstatic + 1, tt.crank != 0, mixed,
+                              res);
+        };
+        res = true;
+        res = need(1) <= (size_t)kLevelSmemMax;
+        int fit = per_cells;
+        while (fit > 1 && need(fit) > (size_t)kLevelSmemGroup) --fit;
+        return fit;
+    };
+    // sweeping warps: as many as a level has rows for, on average; twice that
+    // while the SMs have two blocks at most, so that wide levels are one chunk
+    // (2,000 trees 13.6 -> 12.1 us a step, 24 of 700-900 compartments 14.5 ->
+    // 12.3; 16,384 trees 23.4 -> 27.8, where the idle warps' slots are wanted)
+    int64_t ngroups = 0;
+    for (const Tile &tl : e->tiles) {
+        const TileType &tt = e->types[tl.type];
+        bool res;
+        if (tt.level) {
+            const int most = most_cells(tt, ntop[tl.type], res);
+            ngroups += (tl.nlanes + most - 1) / most;
+        }
+    }
+    const int spread = ngroups <= 2 * kLevelGroups ? 2 : 1;
     struct Cand { LevelGroup g; int warps, bucket; size_t smem; };
     std::vector<Cand> cand;
     LevelPools P;
@@ -844,14 +874,8 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
         const TileType &tt = e->types[tl.type];
         if (!tt.level) continue;
         const int nst = tt.nstatic, nt_top = ntop[tl.type];
-        // neurons whose rows fit the shared memory (a chunk has at least 32 rows or ends a level)
-        auto need = [&](int cellsn, bool res) {
-            return level_smem(nt_top, cellsn * nst, cellsn * nst / LANES + nst + 1, tt.crank != 0, mixed, res);
-        };
-        const bool res = need(1, true) <= (size_t)kLevelSmemMax;
-        int fit = LANES;
-        while (fit > 1 && need(fit, res) > lvmax) --fit;
-        const int most = std::min(per_cells, fit);
+        bool res;
+        const int most = most_cells(tt, nt_top, res);
         const int ng = (tl.nlanes + most - 1) / most;
         for (int q = 0, l0 = 0; q < ng; ++q) {
             const int nl = (tl.nlanes - l0 + (ng - q) - 1) / (ng - q);
@@ -869,8 +893,8 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
             g.choff = (int)P.chunks.size();
             for (int x : nkid) g.many |= x > 2;
             const int nlev = (int)start.size() - 1;
-            int warps = 1;   // as many sweeping warps as a level has rows for, on average
-            while (warps < 8 && warps * LANES * nlev < g.n) warps *= 2;
+            int warps = 1;
+            while (warps < 8 && warps * LANES * nlev < g.n * spread) warps *= 2;
             const int nt = warps * LANES;
             for (int d = 0; d < nlev; ++d)
                 for (int a = start[d]; a < start[d + 1]; a += nt) {
