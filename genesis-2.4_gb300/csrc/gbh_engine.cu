@@ -228,6 +228,9 @@ struct gbh_engine {
     double *io_pend_host = nullptr;
     int io_pend_buf = 0;
     cudaStream_t io_pend_stream = nullptr;
+    // gbh_get_state: Vm gathered into the descriptor's order
+    DBuf<int64_t> d_vm_at;
+    DBuf<double> d_vm_out;
     // per-step I/O (h_in_msgs / h_out_msgs)
     int n_in = 0, n_out = 0, n_tgt = 0;   // input values, distinct input targets, outputs
     DBuf<double> d_in_vals, d_out_vals, d_in_sa, d_in_sb;
@@ -2168,6 +2171,12 @@ int launch_spikes(gbh_engine *e, const DevView &v, long long step, cudaStream_t 
     return GBH_OK;
 }
 
+__global__ void k_gather_vm(const double *V, const int64_t *at, int64_t n, double *out)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = V[at[i]];
+}
+
 __global__ void k_gather_outputs(const double *V, const int64_t *addr, int n, double *out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2847,6 +2856,20 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
         gbh_destroy(e);
         return nullptr;
     }
+    {   // where every entry of vm[] is (without the memory for it the host gathers)
+        std::vector<int64_t> src(std::max<int64_t>(e->vm_start.back(), 1), 0);
+        for (size_t i = 0; i < e->dec.neurons.size(); ++i) {
+            const Neuron &N = e->dec.neurons[i];
+            const Tile &t = e->tiles[e->neuron_tile[i]];
+            for (int s = 0; s < N.nrows; ++s)
+                src[e->vm_start[N.solver] + N.row0 + s] = at(t.vm, s, e->neuron_lane[i], e->types[t.type].wide != 0);
+        }
+        if (e->d_vm_out.alloc(src.size()) || e->d_vm_at.upload(src)) {
+            cudaGetLastError();
+            e->d_vm_out.release();
+            e->d_vm_at.release();
+        }
+    }
     if (e->launches.size() > 1) {
         const int ns = (int)std::min<size_t>(e->launches.size(), 8);
         e->side.resize(ns);
@@ -2961,14 +2984,45 @@ int gbh_run(gbh_engine *e, int nsteps)
     return GBH_OK;
 }
 
+// Vm in the order of the batch descriptor: gathered on the device (the tiles
+// keep it lane-interleaved), one copy to the caller's array. 100,000 neurons
+// of 16 compartments: copying every state block and walking the neurons on
+// the host took 8 ms, more than 200 steps. On the default stream, as the
+// other copies of gbh_get_state: it waits for the caller's blocking streams.
+static int get_vm(gbh_engine *e, double *vm)
+{
+    const int64_t n = e->vm_start.back();
+    if (n == 0) return GBH_OK;
+    if (e->d_vm_at.p) {
+        k_gather_vm<<<(unsigned)((n + 255) / 256), 256>>>(e->d_V.p, e->d_vm_at.p, n, e->d_vm_out.p);
+        CK(cudaGetLastError());
+        CK(cudaMemcpy(vm, e->d_vm_out.p, n * sizeof(double), cudaMemcpyDeviceToHost));
+        return GBH_OK;
+    }
+    std::vector<double> V(e->rows_vm * LANES);
+    CK(cudaMemcpy(V.data(), e->d_V.p, V.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    for (size_t i = 0; i < e->dec.neurons.size(); ++i) {
+        const Neuron &N = e->dec.neurons[i];
+        const Tile &t = e->tiles[e->neuron_tile[i]];
+        const bool w = e->types[t.type].wide != 0;
+        for (int s = 0; s < N.nrows; ++s)
+            vm[e->vm_start[N.solver] + N.row0 + s] = V[at(t.vm, s, e->neuron_lane[i], w)];
+    }
+    return GBH_OK;
+}
+
 int gbh_get_state(gbh_engine *e, double *vm, double *chip, double *conc, int *ops)
 {
     if (!e) return GBH_ERR_ARG;
     const size_t L = LANES;
     CK(cudaStreamSynchronize(e->stream));
-    std::vector<double> V(e->rows_vm * L), P(e->rows_fld * L), C(e->rows_pool * L);
-    std::vector<int> I(e->rows_int * L);
-    if (!V.empty()) CK(cudaMemcpy(V.data(), e->d_V.p, V.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    if (vm) {
+        const int rc = get_vm(e, vm);
+        if (rc) return rc;
+    }
+    if (!chip && !conc && !ops) return GBH_OK;
+    std::vector<double> P(chip ? e->rows_fld * L : 0), C(conc ? e->rows_pool * L : 0);
+    std::vector<int> I(ops ? e->rows_int * L : 0);
     if (!P.empty()) CK(cudaMemcpy(P.data(), e->d_P.p, P.size() * sizeof(double), cudaMemcpyDeviceToHost));
     if (!C.empty()) CK(cudaMemcpy(C.data(), e->d_C.p, C.size() * sizeof(double), cudaMemcpyDeviceToHost));
     if (!I.empty()) CK(cudaMemcpy(I.data(), e->d_I.p, I.size() * sizeof(int), cudaMemcpyDeviceToHost));
@@ -2979,8 +3033,6 @@ int gbh_get_state(gbh_engine *e, double *vm, double *chip, double *conc, int *op
         const Tile &t = e->tiles[e->neuron_tile[i]];
         const int l = e->neuron_lane[i];
         const bool w = e->types[t.type].wide != 0;
-        if (vm)
-            for (int s = 0; s < N.nrows; ++s) vm[e->vm_start[N.solver] + N.row0 + s] = V[at(t.vm, s, l, w)];
         const std::vector<char> &dfm = e->type_df[t.type];
         if (chip)
             for (size_t f = 0; f < N.fsrc.size(); ++f) {
@@ -3570,6 +3622,7 @@ void gbh_destroy(gbh_engine *e)
     e->d_tin_start.release(); e->d_tin_off.release(); e->d_tin_idx.release();
     e->d_tout_start.release(); e->d_tout_off.release(); e->d_tout_idx.release();
     e->d_out_vals.release(); e->d_out_addr.release();
+    e->d_vm_at.release(); e->d_vm_out.release();
     drop_graphs(e);
     if (e->cap_stream) cudaStreamDestroy(e->cap_stream);
     for (cudaStream_t x : {e->io_stream, e->io_out_stream})
