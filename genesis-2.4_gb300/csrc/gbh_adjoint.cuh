@@ -168,7 +168,7 @@ k_adj_linearize(AdjView v, int smax)
                 if (interp) {
                     dfdv = locate_lin(vc, Vm, tg, xvals) ? tg.invdx : 0.0;
                 } else {
-                    locate(vc, Vm, tg.xmin, tg.invdx, tg.xdivs, xvals, ncols, false);
+                    locate(vc, Vm, tg.xmin, tg.invdx, tg.xdivs, tg.xtop, xvals, ncols, false);
                     dfdv = 0.0;
                 }
                 pc += 1;

@@ -25,6 +25,7 @@ struct DevView {
     const int *prog;
     const TableGeom *tgeom;
     const double *tab64;
+    const double2 *tabd;     // per entry: table value and next-row difference
     const float *tab32;
     const float4 *tabdf;     // per entry: table value and next-row difference, double-float
     const double *xyvals;
@@ -290,30 +291,56 @@ __device__ __forceinline__ bool grid_sync(unsigned *bar, unsigned nblocks, int *
 struct VCursor {
     double lo, hi;
     int row, base;
+    double rowd;   // (double)row
     double frac;
 };
 
-__device__ __forceinline__ void locate(VCursor &c, double v, double vmin, double inv, int divs,
+// a < b for doubles other than NaN, on the integer pipe (a comparison takes
+// an FP64 slot like any other FP64 instruction); -0 equals 0 where `a` or `b`
+// has been through dkey.
+__device__ __forceinline__ long long dkey(double x)
+{
+    const long long k = __double_as_longlong(x);
+    return k < 0 ? (long long)(0x8000000000000000ull - (unsigned long long)k) : k;
+}
+
+// Row of a fresh lookup at table position f, clamped to [0, divs]; f may be
+// clamped too. top: high word of (double)divs, or 0 where divs >= 2^20. The
+// conversions and comparisons run on the integer pipe inside the table.
+__device__ __forceinline__ void locate_row(VCursor &c, double &f, int divs, unsigned top)
+{
+    const unsigned h = (unsigned)__double2hiint(f);
+    if (h < top) {   // 0 <= f < divs: the integer part is in the high word
+        const int e = (int)(h >> 20) - 1023;
+        const unsigned drop = e < 0 ? 0u : (1u << (20 - e)) - 1u;
+        c.row = e < 0 ? 0 : (int)(((h & 0xfffffu) | 0x100000u) >> (20 - e));
+        c.rowd = e < 0 ? 0.0 : __hiloint2double((int)(h & ~drop), 0);
+    } else {
+        if (f < 0.0)
+            f = 0.0;
+        else if (f > divs)
+            f = divs;
+        c.row = f >= 0.0 ? (int)f : 0;   // (NaN: row 0, the fraction stays NaN)
+        c.rowd = (double)c.row;
+    }
+}
+
+__device__ __forceinline__ void locate(VCursor &c, double v, double vmin, double inv, int divs, unsigned top,
                                        const double *vals, int ncols, bool interp)
 {
+    const long long kv = dkey(v);
+    const bool out = dkey(c.lo) > kv || kv >= dkey(c.hi);
     if (interp) {
         double f = (v - vmin) * inv;
-        if ((c.lo > v) || (v >= c.hi)) {
-            if (f < 0.0)
-                f = 0.0;
-            else if (f > divs)
-                f = divs;
-            c.row = (int)f;
-            f = f - (double)c.row;
+        if (out) {
+            locate_row(c, f, divs, top);
             c.lo = vals[c.row];
             c.hi = vals[c.row + 1];
             c.base = c.row * ncols;
-        } else {
-            f = f - (double)c.row;
         }
-        c.frac = f;
+        c.frac = f - c.rowd;
     } else {
-        if ((c.lo > v) || (v >= c.hi)) {
+        if (out) {
             int k = (int)((v - vmin) * inv);
             if (k < 0)
                 k = 0;
@@ -456,7 +483,7 @@ __device__ __forceinline__ void st_df(double *p, df x)
 __device__ __forceinline__ df interp_df(const float4 *tab, int e, df fr)
 {
     const float4 t = __ldg(tab + e);
-    return df_add(df_make(t.x, t.y), df_mul(df_make(t.z, t.w), fr));
+    return df_add(df_make(t.x, t.y), df_mul_un(df_make(t.z, t.w), fr));
 }
 
 __device__ __forceinline__ df val_df(const float4 *tab, int e)
@@ -701,7 +728,7 @@ __device__ __forceinline__ bool pool_phase(const int *pp, const PoolLane &L)
             double *cx = &L.C[pp[1] * W];
             const double base = L.P[pp[2] * W];
             const double itau = L.P[pp[3] * W];
-            *cx = base + ((*cx - base) * (2.0 - itau) + (L.F[pp[1] * W] * L.P[pp[4] * W])) / itau;
+            *cx = base + div_rn((*cx - base) * (2.0 - itau) + (L.F[pp[1] * W] * L.P[pp[4] * W]), itau);
             pp += 5;
             break;
         }

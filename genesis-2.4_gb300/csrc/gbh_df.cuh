@@ -7,10 +7,11 @@
 // 4.2.2): TwoSum, FastTwoSum and TwoProd via fused multiply-add, composed as
 // in the double-double literature (Hida, Li, Bailey 2001, "sloppy" add).
 //
-// On GB300 the FP64 pipe runs about 1.6 DFMA per SM per clock while FP32 runs
-// ~113 FFMA, and the F2F conversions between float and double cost as much
-// as two DFMAs, so the mixed-precision step keeps gate and table arithmetic
-// in df and converts with integer bit manipulation instead of F2F.
+// On GB300 the FP64 pipe takes one warp instruction (an addition as much as a
+// multiply-add) per 19 clocks of an SM, 1.7 lanes a clock, while FP32 runs
+// ~113 FFMA lanes, and the F2F conversions between float and double cost as
+// much as two DFMAs, so the mixed-precision step keeps gate and table
+// arithmetic in df and converts with integer bit manipulation instead of F2F.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -65,6 +66,16 @@ __device__ __forceinline__ df df_mul(df x, df y)
     p.lo = __fmaf_rn(x.hi, y.lo, p.lo);
     p.lo = __fmaf_rn(x.lo, y.hi, p.lo);
     return fast_two_sum(p.hi, p.lo);
+}
+
+// A product left as it comes, |lo| up to some 2^-22 |hi|: for an operand of
+// df_add, whose first step takes any pair of leading parts.
+__device__ __forceinline__ df df_mul_un(df x, df y)
+{
+    df p = two_prod(x.hi, y.hi);
+    p.lo = __fmaf_rn(x.hi, y.lo, p.lo);
+    p.lo = __fmaf_rn(x.lo, y.hi, p.lo);
+    return p;
 }
 
 __device__ __forceinline__ df df_mul_f(df x, float y)
@@ -140,23 +151,124 @@ __device__ __forceinline__ df d2df(double d)
     return df_make(fh, __uint_as_float(lo));
 }
 
-// df -> double: exact conversions, one FP64 add
-__device__ __forceinline__ double df2d(df x) { return f2d_bits(x.hi) + f2d_bits(x.lo); }
-
-// reciprocal of a normal double to ~46 bits: the mantissa m in [1,2) gets a
-// float seed (MUFU), the seed is rescaled by the exponent on the integer
-// pipe, then one Newton step in FP64 (two DFMA). Valid for any finite d with
-// 2^-1021 < |d| < 2^1021.
-__device__ __forceinline__ double rcp_newton(double d)
+// The same for a voltage: |d| is taken into [2^-126, 2^128), so that a zero
+// costs 1e-38 V and a NaN or infinity shows as a voltage beyond 1e38 V; the
+// low 29 bits through one integer-to-float conversion. A third fewer
+// instructions than d2df.
+__device__ __forceinline__ df d2df_volt(double d)
 {
-    const int hi = __double2hiint(d), lo = __double2loint(d);
-    const int e = (hi >> 20) & 0x7ff;
-    const double m = __hiloint2double((hi & 0x800fffff) | 0x3ff00000, lo);
-    const double s = f2d_bits(rcp_approx(d2f_trunc_bits(m)));
-    const double r = __hiloint2double(__double2hiint(s) + ((1023 - e) << 20), __double2loint(s));
-    const double err = fma(-d, r, 1.0);
-    return fma(r, err, r);
+    const uint32_t h = (uint32_t)__double2hiint(d), l = (uint32_t)__double2loint(d);
+    const uint32_t a = min(max(h & 0x7fffffffu, 0x38100000u), 0x47efffffu), sign = h & 0x80000000u;
+    const uint32_t hi = __funnelshift_l(l, a - 0x38000000u, 3) | sign;
+    const uint32_t unit = (uint32_t)max((int)(a >> 20) - 948, 0) << 23 | sign;   // the last place of d
+    return df_make(__uint_as_float(hi), (float)(l & 0x1fffffffu) * __uint_as_float(unit));
 }
 
+// df -> double on the integer pipe: lo's significand, shifted to hi's unit in
+// the last place (truncated there, below 2^-52 of hi), is added to or taken
+// from hi's bits. No FP64 instruction: the FP64 unit takes one warp
+// instruction per 19 clocks of an SM, an addition as much as a multiply-add.
+// Needs |lo| < 2^-22 |hi| (any normalised df); hi zero or below the float
+// normal range gives a signed zero.
+__device__ __forceinline__ double df2d(df x)
+{
+    const uint32_t uh = __float_as_uint(x.hi), ul = __float_as_uint(x.lo);
+    const uint32_t eh = (uh >> 23) & 0xffu, el = (ul >> 23) & 0xffu;
+    const uint32_t sign = uh & 0x80000000u;
+    const uint32_t h = ((uh & 0x7fffffffu) >> 3) + 0x38000000u, l = uh << 29;
+    // lo in units of 2^-52 of hi's binade: its 24 bits, 29 places up and eh - el down
+    const uint32_t sh = eh - max(el, 1u) - 22u;
+    uint32_t m = sh > 31u ? 0u : (((ul & 0x7fffffu) | (el ? 0x800000u : 0u)) << 7) >> sh;
+    const bool minus = (int)(uh ^ ul) < 0;
+    // just below a power of two the unit is half as large
+    if (minus && (uh & 0x7fffffu) == 0u) m <<= 1;
+    const uint64_t mag = ((uint64_t)h << 32) | l;
+    const uint64_t r = minus ? mag - m : mag + m;
+    return __hiloint2double(eh == 0u ? (int)sign : (int)((uint32_t)(r >> 32) | sign), eh == 0u ? 0 : (int)(uint32_t)r);
+}
+
+// df -> double for values whose error of 2^-126 does not matter (a row's
+// right-hand side in volts, its diagonal above 1): exact conversions that
+// take a zero for 2^-127, one FP64 addition; half the instructions of df2d.
+__device__ __forceinline__ double f2d_raw(float f)
+{
+    const uint32_t u = __float_as_uint(f);
+    return __hiloint2double((int)((((u & 0x7fffffffu) >> 3) + 0x38000000u) | (u & 0x80000000u)), (int)(u << 29));
+}
+__device__ __forceinline__ double df2d_row(df x) { return f2d_raw(x.hi) + f2d_raw(x.lo); }
+
+// Reciprocal of a normal double to about 2^-44, one Newton step without FP64
+// instructions: the significand m in [1,2) as a float pair, a float seed r
+// (MUFU), its residual e = 1 - m r on FP32 multiply-adds (below 2^-22, so it
+// and r e are off by 2^-46), and r + r e assembled on the integer pipe, r e in
+// units of 2^-53. Valid for 2^-1021 < |b| < 2^1021. (With the e^2 term, good
+// to 2^-45.5, the mixed form's error on 100,000 16-compartment cables over 500
+// steps is 2.6e-10 instead of 3.0e-10 relative: no more than the rest of it.)
+__device__ __forceinline__ double rcp_seed(double b)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(b), lo = (uint32_t)__double2loint(b);
+    const float mh = __uint_as_float(0x3f800000u | (__funnelshift_l(lo, hi, 3) & 0x7fffffu));
+    const float ml = (float)(lo & 0x1fffffffu) * 0x1p-52f;
+    const float r = rcp_approx(mh);
+    const float e = __fmaf_rn(-ml, r, __fmaf_rn(-mh, r, 1.0f));
+    const int c = __float2int_rn(r * e * 0x1p53f);
+    const uint32_t ru = __float_as_uint(r);
+    const uint64_t y = (((uint64_t)((ru >> 3) + 0x38000000u) << 32) | (ru << 29)) + (uint64_t)(int64_t)c;
+    const uint32_t yh = ((uint32_t)(y >> 32) + 0x3ff00000u - (hi & 0x7ff00000u)) | (hi & 0x80000000u);
+    return __hiloint2double((int)yh, (int)(uint32_t)y);
+}
+
+// Are the exponents of all operands within 2^+-450? Quotients, reciprocals
+// and the residuals of the corrections below are then normal numbers.
+__device__ __forceinline__ bool mid_range(double a)
+{
+    return ((uint32_t)__double2hiint(a) & 0x7ff00000u) - ((1023u - 450u) << 20) <= (900u << 20);
+}
+
+// May b be divided by through rcp_seed: mid_range, and its first 20 fraction
+// bits not all ones. Just below a power of two, 1 / b lies next to the middle
+// between two doubles (1 / (2 - k 2^-52) = 1/2 + k 2^-54 + k^2 2^-107 ...),
+// closer than the seed's Newton step can tell.
+__device__ __forceinline__ bool divisor_ok(double b)
+{
+    return mid_range(b) && ((uint32_t)__double2hiint(b) & 0xfffffu) != 0xfffffu;
+}
+
+// IEEE division, out of line: operands the corrected quotients do not cover
+// (zeros, infinities, NaN, far exponents, divisors just below a power of two).
+__device__ __noinline__ static double div_ieee(double a, double b) { return a / b; }
+
+// 1 / b, correctly rounded: one Newton step y + y (1 - b y) in two FMAs from a
+// seed good to 2^-44. Before its rounding the step is off by 2^-88, so the
+// result is the correctly rounded one unless 1/b lies within 2^-88 of the
+// middle between two doubles (of the other divisors one in 2^34; there it may
+// be the neighbour). 2 FP64 instructions against the division's 5.5.
+__device__ __forceinline__ double rcp_rn(double b)
+{
+    if (!divisor_ok(b)) return div_ieee(1.0, b);
+    const double y = rcp_seed(b);
+    return fma(y, fma(-b, y, 1.0), y);
+}
+
+// RN(a / b) from y = rcp_rn(b) by Markstein's correction (P. Markstein, IBM
+// Journal of Research and Development 34, 1990): q = RN(a y) is within an ulp
+// of a / b, its residual a - b q is exact in one FMA, and RN(q + residual y)
+// is the correctly rounded quotient for a correctly rounded y. (Where y is
+// its neighbour the correction is off by 2^-52 ulp of q, which shows only if
+// a / b is that close to the middle between two doubles besides.) Needs a
+// and b in mid_range.
+__device__ __forceinline__ double div_by(double a, double b, double y)
+{
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
+// RN(a / b): 5 FP64 instructions against the division's 9.
+__device__ __forceinline__ double div_rn(double a, double b)
+{
+    if (!(mid_range(a) && divisor_ok(b))) return div_ieee(a, b);
+    const double y = rcp_seed(b);
+    return div_by(a, b, fma(y, fma(-b, y, 1.0), y));
+}
 
 }  // namespace gbh

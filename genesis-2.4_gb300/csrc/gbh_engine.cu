@@ -121,6 +121,7 @@ struct gbh_engine {
     DBuf<double> d_tab64, d_xy;
     DBuf<float> d_tab32;
     DBuf<float4> d_tabdf;
+    DBuf<double2> d_tabd;
     std::vector<std::vector<char>> type_df;     // mixed: field rows stored as packed double-float
     DBuf<double> d_P, d_V, d_C, d_F, d_A, d_B, d_Cb, d_giv, d_stab;
     DBuf<double> d_CR, d_CD, d_S;   // coresult / codiag rows, diffusion scratch
@@ -479,6 +480,14 @@ void build_tables(const gbh_batch_desc *d, std::vector<TableGeom> &tg, std::vect
         g.invdx = T.invdx;
         g.ymin = T.ymin;
         g.invdy = T.invdy;
+        auto top = [](int divs) {   // locate_row
+            const double d = divs;
+            uint64_t b;
+            memcpy(&b, &d, sizeof(b));
+            return divs > 0 && divs < 1 << 20 ? (unsigned)(b >> 32) : 0u;
+        };
+        g.xtop = top(T.xdivs);
+        g.ytop = top(T.ydivs);
         g.tab_off = (int64_t)tab64.size();
         const int64_t rows = T.ncols ? (int64_t)T.xdivs + 1 : 0;
         for (int64_t r = 0; r < rows; ++r)
@@ -1373,6 +1382,14 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
                 tabdf[i] = make_float4(th, (float)(t0 - (double)th), dh, (float)(dlt - (double)dh));
             }
     }
+    // the same in FP64: the difference rounded as the interpolation forms it
+    std::vector<double2> tabd(tab64.size());
+    for (int k = 0; k < d->ntables; ++k) {
+        const int nc = tg[k].ncols;
+        const int64_t n = nc ? ((int64_t)tg[k].xdivs + 2) * nc : 0;
+        for (int64_t i = tg[k].tab_off; i < tg[k].tab_off + n; ++i)
+            tabd[i] = make_double2(tab64[i], i + nc < tg[k].tab_off + n ? tab64[i + nc] - tab64[i] : 0.0);
+    }
     std::vector<double> stab = dec.stablist;
 
     // ---- upload ----
@@ -1382,6 +1399,7 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
     rc |= e->d_prog.upload(prog_pool);
     rc |= e->d_tgeom.upload(tg);
     rc |= e->d_tab64.upload(tab64);
+    if (!mixed) rc |= e->d_tabd.upload(tabd);
     rc |= e->d_tab32.upload(tab32);
     rc |= e->d_tabdf.upload(tabdf);
     rc |= e->d_xy.upload(xy);
@@ -1620,6 +1638,7 @@ DevView view_of(gbh_engine *e)
     v.prog = e->d_prog.p;
     v.tgeom = e->d_tgeom.p;
     v.tab64 = e->d_tab64.p;
+    v.tabd = e->d_tabd.p;
     v.tab32 = e->d_tab32.p;
     v.tabdf = e->d_tabdf.p;
     v.xyvals = e->d_xy.p;
@@ -3611,7 +3630,7 @@ void gbh_destroy(gbh_engine *e)
     if (!e) return;
     if (e->stream) cudaStreamSynchronize(e->stream);
     e->d_tiles.release(); e->d_types.release(); e->d_prog.release(); e->d_tgeom.release();
-    e->d_tab64.release(); e->d_tab32.release(); e->d_tabdf.release(); e->d_xy.release(); e->d_P.release();
+    e->d_tab64.release(); e->d_tab32.release(); e->d_tabdf.release(); e->d_tabd.release(); e->d_xy.release(); e->d_P.release();
     e->d_V.release(); e->d_C.release(); e->d_F.release(); e->d_CR.release(); e->d_CD.release(); e->d_S.release(); e->d_wtop.release(); e->d_RV.release(); e->d_IT.release(); e->d_A.release(); e->d_B.release(); e->d_ltop.release(); e->d_col.release(); e->d_kst.release(); e->d_kri.release(); e->d_sgen.release(); e->d_tgen.release(); e->d_kref.release(); e->d_out_mword.release(); e->d_rmword.release(); e->d_out_mbit.release(); e->d_rmbit.release(); e->d_synw.release(); e->d_wval.release(); e->d_wmask.release(); e->d_spike_src.release();
     e->d_Cb.release(); e->d_giv.release(); e->d_stab.release(); e->d_I.release();
     e->d_par.release(); e->d_ring.release(); e->d_out_start.release(); e->d_out_base.release();

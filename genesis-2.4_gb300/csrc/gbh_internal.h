@@ -89,7 +89,8 @@ enum SymOp { SY_ELIM = 0, SY_SET = 1, SY_SKIP = 2, SY_FASTSIB = 3, SY_COPY = 4, 
 constexpr int LANES = 32;
 
 struct TableGeom {
-    int ncols, xdivs, ydivs, pad;
+    int ncols, xdivs, ydivs;
+    unsigned xtop, ytop;   // high words of (double)xdivs, ydivs; 0 from 2^20 divisions (locate_row)
     double xmin, invdx, ymin, invdy;
     int64_t tab_off;   // offset into the table pool (doubles / floats)
     int64_t xv_off;    // offset into the value pool (xvals)

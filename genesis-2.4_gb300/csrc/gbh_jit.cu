@@ -167,10 +167,10 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
     const int ncols = tg.ncols;
     o << "    { // slot " << E.S(s) << "\n";
     o << "      const double Vm = Vw[" << E.Vrow(s) << "];\n";
-    if (mx) o << "      const df vmd = d2df(Vm);\n      df sumg = df_make(0.f, 0.f), ichan = sumg;\n";
+    if (mx) o << "      const df vmd = d2df_volt(Vm);\n      df sumg = df_make(0.f, 0.f), ichan = sumg;\n";
     else o << "      double sumg = 0.0, ichan = 0.0;\n";
     o << "      double Im = 0.0; (void)Im;\n";
-    // state carried inside the compartment
+    bool summed = false;   // sumg holds a conductance
     for (;;) {
         const int code = pc[0];
         const int n = nops_of(code);
@@ -195,8 +195,8 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
             if (mx)
                 o << "      locate_df(vc, vmd, xnmin, xinv, " << tg.xdivs << ", " << ncols << ");\n";
             else
-                o << "      locate(vc, Vm, " << lit(tg.xmin) << ", " << lit(tg.invdx) << ", " << tg.xdivs
-                  << ", xvals, " << ncols << ", interp);\n";
+                o << "      locate(vc, Vm, " << lit(tg.xmin) << ", " << lit(tg.invdx) << ", " << tg.xdivs << ", "
+                  << tg.xtop << "u, xvals, " << ncols << ", interp);\n";
             break;
         case M_CONCVAL:
             o << "      sel = " << a[0] << "; " << E.F(a[0]) << " = 0.0;\n";
@@ -207,7 +207,7 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                   << ");\n";
             else
                 o << "      locate(cc, " << E.P(a[0]) << " * Ik, " << lit(tg.ymin) << ", " << lit(tg.invdy) << ", "
-                  << tg.ydivs << ", yvals, " << ncols << ", interp); ctab_base = cc.base;\n";
+                  << tg.ydivs << ", " << tg.ytop << "u, yvals, " << ncols << ", interp); ctab_base = cc.base;\n";
             break;
         case M_NEWCONC2:
             if (mx)
@@ -215,7 +215,7 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                   << ncols << ");\n";
             else
                 o << "      tab_base = ctab_base; save_frac = cc.frac; locate(cc, " << E.C(a[0]) << ", "
-                  << lit(tg.ymin) << ", " << lit(tg.invdy) << ", " << tg.ydivs << ", yvals, " << ncols
+                  << lit(tg.ymin) << ", " << lit(tg.invdy) << ", " << tg.ydivs << ", " << tg.ytop << "u, yvals, " << ncols
                   << ", interp); ctab_base = cc.base;\n";
             break;
         case M_NEWCONC1:
@@ -223,7 +223,7 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                 o << "      locate_df(cc, d2df(Cw[sel * 32]), ynmin, yinv, " << tg.ydivs << ", " << ncols << ");\n";
             else
                 o << "      locate(cc, Cw[sel * 32], " << lit(tg.ymin) << ", " << lit(tg.invdy) << ", " << tg.ydivs
-                  << ", yvals, " << ncols << ", interp); ctab_base = cc.base;\n";
+                  << ", " << tg.ytop << "u, yvals, " << ncols << ", interp); ctab_base = cc.base;\n";
             break;
         case M_SPIKE:
             o << "      if (!v.spike_pre) " << E.I(a[1]) << " = spike_op(v, Vm, " << E.P(a[0]) << ", " << E.I(a[1])
@@ -247,9 +247,9 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
             break;
         case M_END:
             if (mx) {
-                o << "      { const df tbyc = " << E.ldr(a[0]) << "; const df dv = df_mul(ichan, tbyc);\n"
-                  << "        R[" << E.S(s) << "] = df2d(df_add(vmd, dv));\n"
-                  << "        D[" << E.S(s) << "] = df2d(df_add(df_mul(sumg, tbyc), " << E.ldr(a[1]) << ")); }\n";
+                o << "      { const df tbyc = " << E.ldr(a[0]) << "; const df dv = df_mul_un(ichan, tbyc);\n"
+                  << "        R[" << E.S(s) << "] = df2d_row(df_add(vmd, dv));\n"
+                  << "        D[" << E.S(s) << "] = df2d_row(df_add(" << E.ldr(a[1]) << ", df_mul_un(sumg, tbyc))); }\n";
             } else {
                 o << "      { const double tbyc = " << E.Pr(a[0]) << "; R[" << E.S(s) << "] = Vm + ichan * tbyc; D[" << E.S(s)
                   << "] = sumg * tbyc + " << E.Pr(a[1]) << "; }\n";
@@ -331,17 +331,17 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                         }
                         o << "        double *st = " << E.pP(fs) << ";\n";
                         if (p > 0)
-                            o << "        const df x = df_div(df_add(df_mul(ld_df(st), df_add_f(df_neg(X), 2.0f)), Y), X);\n";
+                            o << "        const df x = df_div(df_add(df_mul_un(ld_df(st), df_add_f(df_neg(X), 2.0f)), Y), X);\n";
                         else
                             o << "        const df x = df_div(Y, X);\n";
                         o << "        st_df(st, x); Gk = dpow(Gk, x, " << (p > 0 ? p : -p) << ");\n      }\n";
                     } else {
                         if (kind == GK_1V || kind == GK_1C) {
                             o << "        const int bb = " << (kind == GK_1V ? "vc.base" : "ctab_base") << " + " << col
-                              << ";\n        double X, Y;\n"
+                              << ";\n        const double2 tx = __ldg(&tabd[bb]), ty = __ldg(&tabd[bb + 1]);\n"
+                              << "        double X = tx.x, Y = ty.x;\n"
                               << "        if (interp) { const double fr = " << (kind == GK_1V ? "vc" : "cc")
-                              << ".frac; X = tab[bb]; X = X + fr * (tab[bb + " << ncols << "] - X); Y = tab[bb + 1]; Y = Y + fr * (tab[bb + 1 + "
-                              << ncols << "] - Y); }\n        else { X = tab[bb]; Y = tab[bb + 1]; }\n";
+                              << ".frac; X = X + fr * tx.y; Y = Y + fr * ty.y; }\n";
                         } else {
                             o << "        const double rf = " << (kind == GK_2V ? "vc.frac" : "save_frac")
                               << ", cf = cc.frac;\n        const int bb = " << (kind == GK_2V ? "vc.base" : "tab_base")
@@ -363,8 +363,8 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                             continue;
                         }
                         o << "        double *st = " << E.pP(fs) << ";\n";
-                        if (p > 0) o << "        const double x = (*st * (2.0 - X) + Y) / X;\n";
-                        else o << "        const double x = Y / X;\n";
+                        if (p > 0) o << "        const double x = div_rn(*st * (2.0 - X) + Y, X);\n";
+                        else o << "        const double x = div_rn(Y, X);\n";
                         o << "        *st = x; Gk = gpow<double>(Gk, x, " << (p > 0 ? p : -p) << ");\n      }\n";
                     }
                     pc += 1 + m;
@@ -406,14 +406,16 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                     continue;
                 } else if (k == M_ADDCURR) {
                     const int g = b[0];
+                    const bool first = !summed;   // (0 + Gk is Gk)
+                    summed = true;
                     if (mx) {
-                        o << "      { sumg = df_add(sumg, Gk); ichan = df_add(ichan, df_mul(Ek, Gk)); const double gk = df2d(Gk), ek = df2d(Ek); Ik = gk * (ek - Vm);";
+                        o << "      { sumg = " << (first ? "Gk" : "df_add(sumg, Gk)") << "; ichan = df_add(ichan, df_mul_un(Ek, Gk)); const double gk = df2d(Gk), ek = df2d(Ek); Ik = gk * (ek - Vm);";
                         if (giv)
                             o << " { const double gm = c5 ? df2d(gmax) : 1.0; " << E.G(g) << " = gk / gm; " << E.G(g + 1)
                               << " = Ik / gm; " << E.G(g + 2) << " = ek; }";
                         o << " Im += Ik; }\n";
                     } else {
-                        o << "      { sumg += Gk; ichan += Ek * Gk; Ik = Gk * (Ek - Vm);";
+                        o << "      { sumg " << (first ? "=" : "+=") << " Gk; ichan += Ek * Gk; Ik = Gk * (Ek - Vm);";
                         if (giv)
                             o << " if (c5) { " << E.G(g) << " = Gk / gmax; " << E.G(g + 1) << " = Ik / gmax; } else { "
                               << E.G(g) << " = Gk; " << E.G(g + 1) << " = Ik; } " << E.G(g + 2) << " = Ek;";
@@ -506,8 +508,8 @@ bool emit_ca_pools(std::ostream &t, const int *pp)
         if (pp[0] != PO_CACONC) return false;
         t << "    { double *cx = &Cw[" << pp[1] * LANES << "]; const double base = Pw[" << pp[2] * LANES
           << "]; const double itau = Pw[" << pp[3] * LANES << "];\n"
-          << "      *cx = base + ((*cx - base) * (2.0 - itau) + (Fw[" << pp[1] * LANES << "] * Pw[" << pp[4] * LANES
-          << "])) / itau; }\n";
+          << "      *cx = base + div_rn((*cx - base) * (2.0 - itau) + (Fw[" << pp[1] * LANES << "] * Pw[" << pp[4] * LANES
+          << "]), itau); }\n";
     }
     return true;
 }
@@ -555,6 +557,7 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
           << litf(tg.invdy_hi) << ", " << litf(tg.invdy_lo) << "); (void)ynmin; (void)yinv;\n";
     } else {
         o << "  const double *tab = v.tab64 + " << tg.tab_off << "; (void)tab;\n"
+          << "  const double2 *tabd = v.tabd + " << tg.tab_off << "; (void)tabd;\n"
           << "  const double *xvals = v.xyvals + " << tg.xv_off << "; (void)xvals;\n"
           << "  const double *yvals = v.xyvals + " << (tg.yv_off >= 0 ? tg.yv_off : tg.xv_off) << "; (void)yvals;\n";
     }
@@ -585,7 +588,7 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
         o << "    VCursor vc, cc;\n";
         if (tg.ncols) o << "    vc.lo = vc.hi = 0.0;\n";
         else o << "    vc.lo = -1e20; vc.hi = 1e20;\n";
-        o << "    vc.row = vc.base = 0; vc.frac = 0.0; cc.lo = cc.hi = 0.0; cc.row = cc.base = 0; cc.frac = 0.0;\n"
+        o << "    vc.row = vc.base = 0; vc.rowd = vc.frac = 0.0; cc.lo = cc.hi = 0.0; cc.row = cc.base = 0; cc.rowd = cc.frac = 0.0;\n"
           << "    double save_frac = 0.0; int tab_base = 0, ctab_base = 0; (void)save_frac; (void)tab_base; (void)ctab_base;\n"
           << "    double Ek = 0.0, Gk = 0.0, gmax = 0.0; (void)gmax;\n";
     }
@@ -708,12 +711,12 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
                 }
                 if (fast && kept) {
                 } else if (mixed) {
-                    el << " const double ri = rcp_newton(D[" << s << "]); D[" << s << "] = ri;";
+                    el << " const double ri = rcp_seed(D[" << s << "]); D[" << s << "] = ri;";
                     if (par[s] >= 0) el << " T[" << s << "] = Aw[" << s * LANES << "] * ri;";
                 } else {
                     // FP64: one correctly rounded y = 1/D' per row; T = A/D' and the back
                     // substitution's quotient by Markstein's correction (the divisions' bits)
-                    el << " Y[" << s << "] = 1.0 / D[" << s << "];";
+                    el << " Y[" << s << "] = rcp_rn(D[" << s << "]);";
                     if (par[s] >= 0)
                         el << " { const double a = Aw[" << s * LANES << "], qa = a * Y[" << s << "]; T[" << s
                            << "] = fma(fma(-D[" << s << "], qa, a), Y[" << s << "], qa); }";
@@ -810,7 +813,7 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
     } else {
         t << "    for (int s = 0; s < " << S << "; ++s) { const int p = par[s * 32];\n";
         if (mixed)
-            t << "      const double ri = rcp_newton(Dc[s * 32]); Dc[s * 32] = ri;\n"
+            t << "      const double ri = rcp_seed(Dc[s * 32]); Dc[s * 32] = ri;\n"
               << "      if (p >= 0) { const double temp = Aw[s * 32] * ri; Dc[p * 32] = fma(-Bw[s * 32], temp, Dc[p * 32]); Rc[p * 32] = fma(-Rc[s * 32], temp, Rc[p * 32]); } }\n";
         else
             t << "      if (p >= 0) { const double d = Dc[s * 32]; const double temp = Aw[s * 32] / d; Dc[p * 32] -= Bw[s * 32] * temp; Rc[p * 32] -= Rc[s * 32] * temp; } }\n";
@@ -938,6 +941,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
           << litf(tg.invdy_hi) << ", " << litf(tg.invdy_lo) << "); (void)ynmin; (void)yinv;\n";
     } else {
         o << "  const double *tab = v.tab64 + " << tg.tab_off << "; (void)tab;\n"
+          << "  const double2 *tabd = v.tabd + " << tg.tab_off << "; (void)tabd;\n"
           << "  const double *xvals = v.xyvals + " << tg.xv_off << "; (void)xvals;\n"
           << "  const double *yvals = v.xyvals + " << (tg.yv_off >= 0 ? tg.yv_off : tg.xv_off) << "; (void)yvals;\n";
     }
@@ -953,7 +957,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
     } else {
         o << "    VCursor vc, cc;\n"
           << (tg.ncols ? "    vc.lo = vc.hi = 0.0;\n" : "    vc.lo = -1e20; vc.hi = 1e20;\n")
-          << "    vc.row = vc.base = 0; vc.frac = 0.0; cc.lo = cc.hi = 0.0; cc.row = cc.base = 0; cc.frac = 0.0;\n"
+          << "    vc.row = vc.base = 0; vc.rowd = vc.frac = 0.0; cc.lo = cc.hi = 0.0; cc.row = cc.base = 0; cc.rowd = cc.frac = 0.0;\n"
           << "    double save_frac = 0.0; int tab_base = 0, ctab_base = 0; (void)save_frac; (void)tab_base; (void)ctab_base;\n"
           << "    double Ek = 0.0, Gk = 0.0, gmax = 0.0; (void)gmax;\n";
     }
@@ -968,10 +972,10 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
         o << "      level_top_kids<" << form << ", " << res << ">(L, g, q, " << s << ", lid, R" << S << ", D" << S << ");\n";
         for (int j = 0; j < s; ++j)   // top rows below this one, after the static rows: ascending row order
             o << "      if (tp[" << j << "] == " << s << ") { D" << S << " -= PD[" << j << "]; R" << S << " -= T[" << j << "]; }\n";
-        if (mixed) o << "      D" << S << " = rcp_newton(D" << S << ");\n";
+        if (mixed) o << "      D" << S << " = rcp_seed(D" << S << ");\n";
         if (s < N - 1)   // T holds R T
-            o << "      { const double temp = Aw[" << r << (mixed ? "] * D" : "] / D") << S << "; PD" << S << " = Bw[" << r
-              << "] * temp; T" << S << " = R" << S << " * temp; }\n";
+            o << "      { const double temp = " << (mixed ? "Aw[" + r + "] * D" + S : "div_rn(Aw[" + r + "], D" + S + ")")
+              << "; PD" << S << " = Bw[" << r << "] * temp; T" << S << " = R" << S << " * temp; }\n";
     }
     for (int s = N - 1; s >= 0; --s) {
         const std::string S = "[" + std::to_string(s) + "]", r = std::to_string(s * LANES);
@@ -979,7 +983,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
         if (s < N - 1)
             o << " if (tp" << S << " >= 0) "
               << (mixed ? "r = fma(-Cbw[" + r + "], U[tp" + S + " * 32], r);" : "r -= Cbw[" + r + "] * U[tp" + S + " * 32];");
-        o << (mixed ? " r = r * D" : " r = r / D") << S << "; U[" << r << "] = r;";
+        o << (mixed ? " r = r * D" + S : " r = div_rn(r, D" + S + ")") << "; U[" << r << "] = r;";
         if (tt.crank) o << " Vw[" << r << "] = " << (mixed ? "fma(2.0, r, -Vw[" + r + "]);" : "r + r - Vw[" + r + "];");
         else o << " Vw[" << r << "] = r;";
         if (s == N - 1) o << " finite_check(v, r, active);";   // the root: a NaN anywhere below it reaches it

@@ -50,10 +50,10 @@ __device__ __forceinline__ void chan_state_reset(ChanState &cs, int ncols)
 {
     if (ncols) { cs.vc.lo = cs.vc.hi = 0.0; } else { cs.vc.lo = -1e20; cs.vc.hi = 1e20; }
     cs.vc.row = cs.vc.base = 0;
-    cs.vc.frac = 0.0;
+    cs.vc.rowd = cs.vc.frac = 0.0;
     cs.cc.lo = cs.cc.hi = 0.0;
     cs.cc.row = cs.cc.base = 0;
-    cs.cc.frac = 0.0;
+    cs.cc.rowd = cs.cc.frac = 0.0;
     cs.save_frac = 0.0;
     cs.tab_base = cs.ctab_base = cs.sel = 0;
     cs.Ek = cs.Gk = cs.gmax = cs.Ik = cs.GHK = 0.0;
@@ -108,7 +108,7 @@ __device__ __forceinline__ bool chan_compartment(const DevView &v, const ChanEnv
             }
             pc += 5;
         } else if (code == M_NEWVOLT) {
-            locate(vc, Vm, tg.xmin, tg.invdx, tg.xdivs, xvals, ncols, interp);
+            locate(vc, Vm, tg.xmin, tg.invdx, tg.xdivs, tg.xtop, xvals, ncols, interp);
             pc += 1;
         } else if (code == M_CONCVAL) {
             sel = pc[1];
@@ -116,19 +116,19 @@ __device__ __forceinline__ bool chan_compartment(const DevView &v, const ChanEnv
             pc += 2;
         } else if (code == M_DOMAIN) {
             const double concen = N.P[(pc[1]) * STR] * Ik;
-            locate(cc, concen, tg.ymin, tg.invdy, tg.ydivs, yvals, ncols, interp);
+            locate(cc, concen, tg.ymin, tg.invdy, tg.ydivs, tg.ytop, yvals, ncols, interp);
             ctab_base = cc.base;
             pc += 2;
         } else if (code == M_NEWCONC2) {
             const double concen = N.C[(pc[1]) * STR];
             tab_base = ctab_base;
             save_frac = cc.frac;
-            locate(cc, concen, tg.ymin, tg.invdy, tg.ydivs, yvals, ncols, interp);
+            locate(cc, concen, tg.ymin, tg.invdy, tg.ydivs, tg.ytop, yvals, ncols, interp);
             ctab_base = cc.base;
             pc += 2;
         } else if (code == M_NEWCONC1) {
             const double concen = N.C[(sel) * STR];
-            locate(cc, concen, tg.ymin, tg.invdy, tg.ydivs, yvals, ncols, interp);
+            locate(cc, concen, tg.ymin, tg.invdy, tg.ydivs, tg.ytop, yvals, ncols, interp);
             ctab_base = cc.base;
             pc += 1;
         } else if (code == M_SPIKE) {
@@ -262,9 +262,9 @@ __device__ __forceinline__ bool chan_compartment(const DevView &v, const ChanEnv
                         G x;
                         int pw = p;
                         if (p > 0) {
-                            x = ((G)(*st) * ((G)2.0 - X) + Y) / X;
+                            x = div_rn((G)(*st) * ((G)2.0 - X) + Y, X);
                         } else {
-                            x = Y / X;
+                            x = div_rn(Y, X);
                             pw = -p;
                         }
                         *st = (double)x;
@@ -979,6 +979,7 @@ __device__ __forceinline__ bool bracket_hit(const double *vals, int row, double 
 __device__ __forceinline__ void cursor_at(VCursor &c, int row, const double *vals, int ncols)
 {
     c.row = row;
+    c.rowd = (double)row;
     c.lo = vals[row];
     c.hi = vals[row + 1];
     c.base = row * ncols;

@@ -70,7 +70,7 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
     (void)neuron;
     (void)active;
     (void)c1;
-    const df vmd = d2df(Vm);
+    const df vmd = d2df_volt(Vm);
     df sumg = df_make(0.f, 0.f), ichan = sumg;
     double Im = 0.0;
     for (;;) {
@@ -130,9 +130,9 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
             pc += 4;
         } else if (code == M_END) {
             const df tbyc = ld_df(&N.P[(pc[1]) * STR]);
-            const df dv = df_mul(ichan, tbyc);
-            R = df2d(df_add(vmd, dv));
-            D = df2d(df_add(df_mul(sumg, tbyc), ld_df(&N.P[(pc[2]) * STR])));
+            const df dv = df_mul_un(ichan, tbyc);
+            R = df2d_row(df_add(vmd, dv));
+            D = df2d_row(df_add(ld_df(&N.P[(pc[2]) * STR]), df_mul_un(sumg, tbyc)));
             if (GIV) N.G[(pc[3]) * STR] = Im;
             pc += 4;
             break;
@@ -226,7 +226,7 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
                     df x;
                     int pw = p;
                     if (p > 0) {
-                        x = df_div(df_add(df_mul(ld_df(st), df_add_f(df_neg(X), 2.0f)), Y), X);
+                        x = df_div(df_add(df_mul_un(ld_df(st), df_add_f(df_neg(X), 2.0f)), Y), X);
                     } else {
                         x = df_div(Y, X);
                         pw = -p;
@@ -270,7 +270,7 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
                 } else if (k == M_ADDCURR) {
                     const int g = pc[1];
                     sumg = df_add(sumg, Gk);
-                    ichan = df_add(ichan, df_mul(Ek, Gk));
+                    ichan = df_add(ichan, df_mul_un(Ek, Gk));
                     const double gk = df2d(Gk), ek = df2d(Ek);
                     Ik = gk * (ek - Vm);
                     if (GIV) {
@@ -390,7 +390,7 @@ k_steps_mixed(DevView v, int tile0, int tile1, int smax, int nsteps, long long s
         } else {
         for (int s = 0; s < S; ++s) {
             const int p = par[s * LANES];
-            const double ri = rcp_newton(Dcol[s * LANES]);
+            const double ri = rcp_seed(Dcol[s * LANES]);
             Dcol[s * LANES] = ri;   // the row's diagonal is final here; keep only its reciprocal
             if (p >= 0) {
                 const double temp = Aw[s * LANES] * ri;
@@ -421,7 +421,7 @@ k_steps_mixed(DevView v, int tile0, int tile1, int smax, int nsteps, long long s
 
 // Stack elimination of the mixed form (see k_stack in gbh_kernels.cuh): the
 // same row order and per-lane stacks; the diagonal's reciprocal is formed
-// once per row (rcp_newton) and kept in the column for back substitution.
+// once per row (rcp_seed) and kept in the column for back substitution.
 //
 // SPLIT: two warps per tile. After a launch's first step the second warp
 // runs the channel phase of the rows above the static ones (kSplitRows at
@@ -572,7 +572,7 @@ k_stack_mixed(DevView v, int tile0, int tile1, int cap, int nsteps, long long st
                 D -= cd;
                 R -= cr;
             }
-            const double ri = rcp_newton(D);
+            const double ri = rcp_seed(D);
             col[s * LANES] = make_double2(R, ri);
             double temp = 0.0;
             if (f & FL_PARENT) {
@@ -932,7 +932,7 @@ k_wide_mixed(DevView v, int tile0, int tile1, int smax, int nsteps, long long st
                     d = fma(-B[c], temp, d);
                     r = fma(-Rs[c], temp, r);
                 }
-                Ds[s] = rcp_newton(d);
+                Ds[s] = rcp_seed(d);
                 Rs[s] = r;
             }
             __syncthreads();
