@@ -85,6 +85,7 @@ struct Launch {
     bool stack = false;   // stack elimination (smax = shared doubles per lane)
     bool split = false;   // stack: some tile's rows above its static ones go to a second warp
     int level = -1;       // level elimination: kernel index (tile0..tile1 are groups, smax the shared bytes)
+    int rows = -1;        // row-parallel step: kernel index (likewise)
 };
 
 // Element idx of a block of rows starting at row `base`: lane-interleaved
@@ -177,6 +178,15 @@ struct gbh_engine {
     DBuf<double2> d_lkt, d_lcy;
     DBuf<double> d_lc, d_ld, d_lpd;
     DBuf<unsigned> d_lgen;
+    // row-parallel steps (gbh_rows.cuh): the plan that uses them, timed against
+    // `launches` by the autotuner (empty: none)
+    std::vector<JitKernel> rw_kern;
+    std::vector<Launch> rows_launches;
+    DBuf<RowGroup> d_rgroups;
+    DBuf<int2> d_rchunks, d_rwork, d_rlink;
+    DBuf<int4> d_ritems;
+    DBuf<int> d_rmap, d_rprev, d_rpos;
+    DBuf<double> d_rA, d_rB, d_rC;
     int steps_per_launch = 1;
     bool has_network = false;
     bool givals_enabled = false;
@@ -963,6 +973,203 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
     return GBH_OK;
 }
 
+// ---- row-parallel steps (gbh_rows.cuh) ----
+// Batches whose lane-mapped tiles are fewer than this may run row-parallel
+// (the autotuner times it): eight tiles an SM. Beyond, the lanes of the SMs are
+// full either way and the barriers between levels only cost.
+constexpr int64_t kRowsTiles = 8 * 152;
+constexpr size_t kRowsKernels = 8;
+
+bool rows_type(const TileType &tt, const std::vector<int> &prog, RowsProg &rp)
+{
+    if (tt.wide || tt.nslots < 4 || tt.sym || tt.nitot) return false;
+    if (rows_smem(tt.nslots, tt.nslots) > (size_t)kLevelSmemMax || tt.nslots > 0xffff) return false;
+    rp = rows_prog(tt, prog);
+    return rp.ok;
+}
+
+// Groups, kernels and launches of the types that can run row-parallel; their
+// TileType::rows is set. Leaves `out` empty when there are none.
+int rows_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const std::vector<int> &prog_pool,
+              const std::vector<TableGeom> &tg, std::vector<Launch> &out)
+{
+    const Decoded &dec = e->dec;
+    const bool mixed = e->opt.precision == GBH_PREC_MIXED;
+    std::map<std::string, int> kern;
+    std::vector<std::string> srcs;
+    std::vector<RowsProg> prog(e->types.size());
+    int64_t cells = 0, tiles = 0;
+    for (size_t ti = 0; ti < e->types.size(); ++ti)
+        if (!e->types[ti].level && !e->types[ti].wide) tiles += ((int64_t)members[ti].size() + LANES - 1) / LANES;
+    if (tiles > kRowsTiles) return GBH_OK;
+    for (size_t ti = 0; ti < e->types.size(); ++ti) {
+        TileType &tt = e->types[ti];
+        if (tt.level || !rows_type(tt, prog_pool, prog[ti])) continue;
+        auto it = kern.find(prog[ti].key);
+        if (it == kern.end()) {
+            if (kern.size() >= kRowsKernels) continue;
+            const std::string src = jit_rows_source(prog[ti], tt, tg[tt.table_set], mixed);
+            if (src.empty()) continue;
+            it = kern.emplace(prog[ti].key, (int)kern.size()).first;
+            srcs.push_back(src);
+        }
+        tt.rows = 1 + it->second;
+        cells += (int64_t)members[ti].size();
+    }
+    if (srcs.empty()) return GBH_OK;
+    int major = 10, minor = 3;
+    cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, e->opt.device);
+    cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, e->opt.device);
+    e->rw_kern.resize(srcs.size());
+    std::vector<int> ok(srcs.size(), 0);
+    std::vector<std::string> logs(srcs.size());
+    std::vector<std::thread> th;
+    for (size_t c = 0; c < srcs.size(); ++c)
+        th.emplace_back([&, c]() {
+            cudaSetDevice(e->opt.device);
+            ok[c] = jit_compile(srcs[c], !mixed, major, minor, &e->rw_kern[c], &logs[c]) == 0 &&
+                    jit_allow_smem(e->rw_kern[c], kLevelSmemMax);
+        });
+    for (auto &x : th) x.join();
+    for (size_t c = 0; c < srcs.size(); ++c)
+        if (!ok[c]) {
+            if (e->jit_log.size() < 4000) e->jit_log += logs[c];
+            for (TileType &tt : e->types)
+                if (tt.rows == 1 + (int)c) tt.rows = 0;
+        }
+    const int per = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + kLevelGroups - 1) / kLevelGroups));
+    std::vector<RowGroup> groups;
+    std::vector<int2> chunks, work, link;
+    std::vector<int4> items;
+    std::vector<int> map, prev, pos;
+    std::vector<double> A, B, C;
+    std::vector<std::vector<int>> cells_of(e->tiles.size());
+    for (size_t i = 0; i < dec.neurons.size(); ++i) {
+        const int t = e->neuron_tile[i];
+        if (!e->types[e->tiles[t].type].rows) continue;
+        cells_of[t].resize(e->tiles[t].nlanes, -1);
+        cells_of[t][e->neuron_lane[i]] = (int)i;
+    }
+    struct Cand { RowGroup g; int warps, kern; size_t smem; };
+    std::vector<Cand> cand;
+    auto most_cells = [&](const TileType &tt) {   // (a chunk has at least 32 rows or ends a level)
+        const int S = tt.nslots;
+        int most = per;
+        while (most > 1 && rows_smem(most * S, most * S / LANES + S + 1) > (size_t)kLevelSmemMax / 2) --most;
+        return most;
+    };
+    int64_t ngroups = 0;
+    for (const Tile &tl : e->tiles)
+        if (e->types[tl.type].rows) {
+            const int most = most_cells(e->types[tl.type]);
+            ngroups += (tl.nlanes + most - 1) / most;
+        }
+    const bool crowded = ngroups > kLevelGroups;
+    for (size_t t = 0; t < e->tiles.size(); ++t) {
+        const Tile &tl = e->tiles[t];
+        const TileType &tt = e->types[tl.type];
+        if (!tt.rows) continue;
+        const RowsProg &rp = prog[tl.type];
+        const int S = tt.nslots, most = most_cells(tt);
+        const int ng = (tl.nlanes + most - 1) / most;
+        for (int q = 0, l0 = 0; q < ng; ++q) {
+            const int nl = (tl.nlanes - l0 + (ng - q) - 1) / (ng - q), n = nl * S;
+            RowGroup g{};
+            g.tile = (int)t;
+            g.lane0 = l0;
+            g.nlanes = nl;
+            g.n = n;
+            g.eoff = (int64_t)map.size();
+            g.choff = (int)chunks.size();
+            g.itoff = (int)items.size();
+            // level order: the roots, then the children of each row in turn
+            std::vector<std::vector<int>> kids((size_t)n);
+            std::vector<int> order, start(1, 0), at(n), gpar(n), gkid(n, 0), gnk(n, 0);
+            std::vector<const Neuron *> cl;
+            for (int l = 0; l < nl; ++l) cl.push_back(&dec.neurons[cells_of[t][l0 + l]]);
+            for (int l = 0; l < nl; ++l)
+                for (int s = 0; s < S; ++s) {
+                    const int p = cl[l]->parent[s];
+                    if (p >= 0) kids[(size_t)p * nl + l].push_back(s);
+                    else {
+                        gpar[order.size()] = n;
+                        order.push_back(s * nl + l);
+                    }
+                }
+            while ((int)order.size() > start.back()) {
+                const int e0 = start.back(), e1 = (int)order.size();
+                start.push_back(e1);
+                for (int x = e0; x < e1; ++x) {
+                    gkid[x] = (int)order.size();
+                    gnk[x] = (int)kids[order[x]].size();
+                    for (int s : kids[order[x]]) {
+                        gpar[order.size()] = x;
+                        order.push_back(s * nl + order[x] % nl);
+                    }
+                }
+            }
+            for (int x = 0; x < n; ++x) at[order[x]] = x;
+            // a warp for every 32 rows, unless more blocks than SMs have to share them
+            const int warps = std::min(crowded ? 8 : 16, (n + LANES - 1) / LANES), nt = warps * LANES;
+            for (size_t d = 0; d + 1 < start.size(); ++d)
+                for (int a = start[d]; a < start[d + 1]; a += nt) {
+                    const int m = std::min(nt, start[d + 1] - a);
+                    chunks.push_back(make_int2(a, m | (a == start[d] ? RW_FIRST : 0) |
+                                                      (a + m == start[d + 1] ? RW_LAST : 0)));
+                }
+            g.nch = (int)chunks.size() - g.choff;
+            for (int x : order) {
+                const int s = x / nl, l = x % nl;
+                map.push_back(s * LANES + l0 + l);
+                A.push_back(cl[l]->A[s]);
+                B.push_back(cl[l]->B[s]);
+                C.push_back(cl[l]->parent[s] >= 0 ? cl[l]->C[s] : 0.0);
+                prev.push_back(rp.prev[s] >= 0 ? at[rp.prev[s] * nl + l] : rp.prev[s]);
+            }
+            for (int x = 0; x < n; ++x) link.push_back(make_int2(gkid[x] | gnk[x] << 16, gpar[x]));
+            pos.insert(pos.end(), at.begin(), at.end());
+            // work by class, the longest programs first (they start first)
+            std::vector<int> by(rp.cls.size());
+            for (size_t c = 0; c < by.size(); ++c) by[c] = (int)c;
+            std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return rp.cls[a].size() > rp.cls[b].size(); });
+            int done = 0;
+            for (int c : by) {
+                const int w0 = done;
+                for (int s = 0; s < S; ++s)
+                    if (rp.of[s] == c)
+                        for (int l = 0; l < nl; ++l) {
+                            work.push_back(make_int2(at[s * nl + l], rp.f0[s] * LANES + l0 + l));
+                            ++done;
+                        }
+                for (int a = w0; a < done; a += LANES)
+                    items.push_back(make_int4(c, a, std::min(LANES, done - a), 0));
+            }
+            g.nitems = (int)items.size() - g.itoff;
+            cand.push_back({g, warps, tt.rows - 1, rows_smem(n, g.nch)});
+            l0 += nl;
+        }
+    }
+    if (cand.empty()) return GBH_OK;
+    std::stable_sort(cand.begin(), cand.end(), [](const Cand &a, const Cand &b) {
+        return a.kern != b.kern ? a.kern < b.kern : a.warps != b.warps ? a.warps > b.warps : a.g.n > b.g.n;
+    });
+    for (size_t a = 0; a < cand.size();) {
+        size_t b = a, smem = 0;
+        for (; b < cand.size() && cand[b].kern == cand[a].kern && cand[b].warps == cand[a].warps; ++b)
+            smem = std::max(smem, cand[b].smem);
+        Launch L{(int)a, (int)b, (int)smem, cand[a].warps};
+        L.rows = cand[a].kern;
+        out.push_back(L);
+        a = b;
+    }
+    for (const Cand &c : cand) groups.push_back(c.g);
+    if (e->d_rgroups.upload(groups) || e->d_rchunks.upload(chunks) || e->d_rwork.upload(work) ||
+        e->d_ritems.upload(items) || e->d_rmap.upload(map) || e->d_rlink.upload(link) || e->d_rprev.upload(prev) || e->d_rpos.upload(pos) || e->d_rA.upload(A) ||
+        e->d_rB.upload(B) || e->d_rC.upload(C))
+        return GBH_ERR_CUDA;
+    return GBH_OK;
+}
+
 int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn, const gbh_remote_synapses *remote,
                  gbh_error *err)
 {
@@ -1458,6 +1665,13 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
             return fail_err(err, GBH_ERR_CUDA, "upload of the tile types failed");
     }
 
+    // ---- row-parallel steps of small batches, for the autotuner ----
+    std::vector<Launch> rplan;
+    if (!e->has_network && e->opt.jit == 0 && e->opt.steps_per_launch == 0 && jit_available(nullptr)) {
+        const int rcw = rows_plan(e, members, prog_pool, tg, rplan);
+        if (rcw) return fail_err(err, rcw, "%s", g_last_error);
+    }
+
     // ---- specialised kernels (one per tile type with enough tiles) ----
     std::vector<int> type_t0(e->types.size(), -1), type_t1(e->types.size(), -1);
     for (size_t ti = 0; ti < e->tiles.size(); ++ti) {
@@ -1559,10 +1773,10 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         }
     }
     // ---- launch plan: specialised types alone, the rest bucketed by slot count ----
-    // (skip_level: the level-eliminated tiles are launched by groups, below)
-    auto plan = [&](std::vector<Launch> &out, bool skip_level) {
+    // (skip_level, skip_rows: those tiles are launched by groups instead)
+    auto plan = [&](std::vector<Launch> &out, bool skip_level, bool skip_rows) {
         auto typ = [&](size_t t) -> const TileType & { return e->types[e->tiles[t].type]; };
-        auto lev = [&](size_t t) { return skip_level && typ(t).level; };
+        auto lev = [&](size_t t) { return (skip_level && typ(t).level) || (skip_rows && typ(t).rows); };
         size_t t0 = 0;
         while (t0 < e->tiles.size()) {
             const int ty0 = e->tiles[t0].type;
@@ -1622,12 +1836,19 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         }
         return (int)GBH_OK;
     };
-    if (!lplan.groups.empty()) {
-        const int rcg = plan(e->giv_launches, false);
+    const bool lvl = !lplan.groups.empty();
+    if (lvl || !rplan.empty()) {   // a step with givals runs the interpreting kernels
+        const int rcg = plan(e->giv_launches, false, false);
         if (rcg) return rcg;
-        e->launches = lplan.launches;
     }
-    return plan(e->launches, !lplan.groups.empty());
+    if (!rplan.empty()) {
+        e->rows_launches = lplan.launches;
+        e->rows_launches.insert(e->rows_launches.end(), rplan.begin(), rplan.end());
+        const int rcr = plan(e->rows_launches, lvl, true);
+        if (rcr) return rcr;
+    }
+    e->launches = lplan.launches;
+    return plan(e->launches, lvl, false);
 }
 
 DevView view_of(gbh_engine *e)
@@ -1719,6 +1940,28 @@ int launch_one(gbh_engine *e, const DevView &v, const Launch &L, int k, long lon
                                                 step, (size_t)L.smax, st);
         if (je != cudaSuccess) {
             set_last("level elimination launch failed: %s", cudaGetErrorString(je));
+            return GBH_ERR_CUDA;
+        }
+        e->stats.launches++;
+        return GBH_OK;
+    }
+    if (L.rows >= 0) {
+        RowView rv{};
+        rv.groups = e->d_rgroups.p;
+        rv.chunks = e->d_rchunks.p;
+        rv.items = e->d_ritems.p;
+        rv.work = e->d_rwork.p;
+        rv.map = e->d_rmap.p;
+        rv.link = e->d_rlink.p;
+        rv.prev = e->d_rprev.p;
+        rv.pos = e->d_rpos.p;
+        rv.A = e->d_rA.p;
+        rv.B = e->d_rB.p;
+        rv.C = e->d_rC.p;
+        const cudaError_t je = jit_rows_launch(e->rw_kern[L.rows], v, rv, L.tile0, L.tile1 - L.tile0, L.warps, k, step,
+                                               (size_t)L.smax, st);
+        if (je != cudaSuccess) {
+            set_last("row-parallel launch failed: %s", cudaGetErrorString(je));
             return GBH_ERR_CUDA;
         }
         e->stats.launches++;
@@ -1950,7 +2193,7 @@ int autotune_trials(gbh_engine *e)
     if (e->has_network) spls = {1};
     else spls = {16, 64, 256};
     const int nvar = e->jit_var.empty() ? 1 : (int)e->jit_var[0].size();
-    if ((int)spls.size() * nvar <= 1) {
+    if ((int)spls.size() * nvar <= 1 && e->rows_launches.empty()) {
         e->steps_per_launch = spls[0];
         return GBH_OK;
     }
@@ -1988,36 +2231,63 @@ int autotune_trials(gbh_engine *e)
     };
     double best = 1e300;
     int best_v = 0, best_s = spls[0];
-    for (int vi = 0; vi < nvar; ++vi) {
+    // time per step of the plan and variant in use, from the saved state
+    auto timed = [&](int spl, double &per) {
+        e->steps_per_launch = spl;
+        const int steps = std::max(2 * spl, 128);
+        int rc_t = run_steps(e, 8, e->stream);   // warm caches and clocks
+        CK(cudaEventRecord(e->ev0, e->stream));
+        if (rc_t == GBH_OK) rc_t = run_steps(e, steps, e->stream);
+        CK(cudaEventRecord(e->ev1, e->stream));
+        CK(cudaEventSynchronize(e->ev1));
+        float ms = 0.f;
+        CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
+        // a variant that cannot launch here (resources) never wins
+        per = rc_t == GBH_OK ? ms / steps : 1e300;
+        if (rc_t != GBH_OK) cudaGetLastError();
+        return restore();
+    };
+    auto use_variant = [&](int vi) {
         for (size_t k = 0; k < e->jits.size(); ++k) e->jits[k] = e->jit_var[k][vi];
         e->jit_choice = vi;   // launch_one sizes the shared memory of the variant in use
-        for (int spl : spls) {
-            e->steps_per_launch = spl;
-            const int steps = std::max(2 * spl, 128);
-            int rc_t = run_steps(e, 8, e->stream);   // warm caches and clocks
-            CK(cudaEventRecord(e->ev0, e->stream));
-            if (rc_t == GBH_OK) rc_t = run_steps(e, steps, e->stream);
-            CK(cudaEventRecord(e->ev1, e->stream));
-            CK(cudaEventSynchronize(e->ev1));
-            float ms = 0.f;
-            CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
-            // a variant that cannot launch here (resources) never wins
-            const double per = rc_t == GBH_OK ? ms / steps : 1e300;
-            if (rc_t != GBH_OK) cudaGetLastError();
-            if (getenv("GBH_VERBOSE") && !e->jit_minb.empty())
-                fprintf(stderr, "gbhsolve: trial %d warps x min blocks %d, form %d, %d steps/launch: %.2f us/step\n",
-                        e->jit_warps[vi], e->jit_minb[vi], e->jit_compact[vi] ? 1 : e->jit_smemrows[vi] ? 2 : 0, spl,
-                        per * 1e3);
-            if (per < best) { best = per; best_v = vi; best_s = spl; }
-            if (restore()) return GBH_ERR_CUDA;
-        }
+    };
+    // every variant at the middle launch length, then the row-parallel plan of
+    // a small batch, then the other launch lengths of the fastest: the length
+    // moves a step by a few per cent, the same way in every variant
+    const int mid = spls[spls.size() / 2];
+    bool use_rows = false;
+    for (int vi = 0; vi < nvar; ++vi) {
+        use_variant(vi);
+        double per;
+        if (timed(mid, per)) return GBH_ERR_CUDA;
+        if (getenv("GBH_VERBOSE") && !e->jit_minb.empty())
+            fprintf(stderr, "gbhsolve: trial %d warps x min blocks %d, form %d, %d steps/launch: %.2f us/step\n",
+                    e->jit_warps[vi], e->jit_minb[vi], e->jit_compact[vi] ? 1 : e->jit_smemrows[vi] ? 2 : 0, mid,
+                    per * 1e3);
+        if (per < best) { best = per; best_v = vi; best_s = mid; }
+    }
+    use_variant(best_v);
+    if (!e->rows_launches.empty()) {
+        e->launches.swap(e->rows_launches);
+        double per;
+        if (timed(mid, per)) return GBH_ERR_CUDA;
+        if (getenv("GBH_VERBOSE"))
+            fprintf(stderr, "gbhsolve: trial row-parallel, %d steps/launch: %.2f us/step\n", mid, per * 1e3);
+        use_rows = per < best;
+        if (use_rows) best = per;
+        else e->launches.swap(e->rows_launches);
+    }
+    for (int spl : spls) {
+        if (spl == mid) continue;
+        double per;
+        if (timed(spl, per)) return GBH_ERR_CUDA;
+        if (getenv("GBH_VERBOSE")) fprintf(stderr, "gbhsolve: trial %d steps/launch: %.2f us/step\n", spl, per * 1e3);
+        if (per < best) { best = per; best_s = spl; }
     }
     // networks: the cooperative multi-step launch against the best per-step plan
     bool any_wide = false;
     for (const TileType &tt : e->types) any_wide = any_wide || tt.wide;
     if (e->has_network && e->nremote == 0 && e->d_gbar.p && !any_wide && !e->spike_pre) {
-        for (size_t k = 0; k < e->jits.size(); ++k) e->jits[k] = e->jit_var[k][best_v];
-        e->jit_choice = best_v;
         e->steps_per_launch = best_s;
         int coop_k = 0;
         for (int K : {16, 64}) {
@@ -2058,8 +2328,6 @@ int autotune_trials(gbh_engine *e)
     if (e->d_spiked.p)   // trial spikes
         CK(cudaMemsetAsync(e->d_spiked.p, 0, e->d_spiked.n * sizeof(unsigned), e->stream));
     if (e->rows_itot) CK(cudaMemsetAsync(e->d_IT.p, 0, e->d_IT.n * sizeof(double), e->stream));   // trial itotal sums
-    for (size_t k = 0; k < e->jits.size(); ++k) e->jits[k] = e->jit_var[k][best_v];
-    e->jit_choice = best_v;
     e->steps_per_launch = best_s;
     e->step = 0;
     e->stats.launches = 0;
@@ -2558,7 +2826,7 @@ int gbh_run_io(gbh_engine *e, const double *host_in, double *host_out, int nstep
     // a block of steps runs as multi-step launches
     bool fused = !e->has_network && !e->givals_enabled && !e->net_coop && (n_in == 0 || e->fuse_in) &&
                  !e->launches.empty();
-    for (const Launch &L : e->launches) fused = fused && L.jit >= 0 && !L.wide;
+    for (const Launch &L : e->launches) fused = fused && (L.jit >= 0 || L.rows >= 0) && !L.wide;
     const unsigned grid = (unsigned)((nio + 255) / 256);
     int last = 0;
     for (int s0 = 0, j = 0; s0 < nsteps; s0 += B, ++j) {
@@ -2734,10 +3002,12 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
                         const gbh_options *opt, gbh_error *err, gbh_engine *&made, const Decoded *pre = nullptr);
 
 // Do all neurons that could run wide (32 compartments and more) run the
-// level elimination when lane-mapped (level_type)?
+// level elimination when lane-mapped (level_type), or, in a small batch whose
+// steps per launch are autotuned, row-parallel (rows_type)?
 bool level_everywhere(const gbh_engine *e)
 {
     if (e->has_network || e->opt.jit != 0 || !jit_available(nullptr)) return false;
+    const bool small = e->opt.steps_per_launch == 0 && (int64_t)e->dec.neurons.size() <= kRowsTiles;
     struct Seen { const Neuron *first; bool uniform; };
     std::map<std::string, Seen> types;
     std::vector<int> fl;
@@ -2757,7 +3027,8 @@ bool level_everywhere(const gbh_engine *e)
         tt.stack = !tt.sym;
         tt.nstatic = static_rows(slot_field_ranges(prog, tt), tt.nslots);
         LevelProg lp;
-        if (!level_type(tt, prog, N.parent, kv.second.uniform, lp)) return false;
+        RowsProg rp;
+        if (!level_type(tt, prog, N.parent, kv.second.uniform, lp) && !(small && rows_type(tt, prog, rp))) return false;
     }
     return true;
 }
@@ -2784,7 +3055,7 @@ int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses
     for (int w : {32, 64, 128})
         if (w <= maxrows) cand.push_back(w);
     if (cand.empty()) return -1;   // nothing large enough to run wide
-    if (level_everywhere(e)) return -1;   // no trial: the level elimination beats every mapping it tries
+    if (level_everywhere(e)) return -1;   // no trial: these beat every mapping it tries
     cand.push_back(-1);
     int best = cand[0];
     double best_ms = 1e300;
@@ -2889,8 +3160,8 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
             e->d_vm_at.release();
         }
     }
-    if (e->launches.size() > 1) {
-        const int ns = (int)std::min<size_t>(e->launches.size(), 8);
+    if (std::max(e->launches.size(), e->rows_launches.size()) > 1) {
+        const int ns = (int)std::min<size_t>(std::max(e->launches.size(), e->rows_launches.size()), 8);
         e->side.resize(ns);
         e->ev_join.resize(ns);
         for (int i = 0; i < ns; ++i) {
@@ -2944,7 +3215,7 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
     if (getenv("GBH_VERBOSE"))
         for (const Launch &L : e->launches)
             fprintf(stderr, "gbhsolve: launch group tiles [%d, %d) smax %d %s\n", L.tile0, L.tile1, L.smax,
-                    L.jit >= 0 ? "specialised" : "interpreted");
+                    L.jit >= 0 ? "specialised" : L.level >= 0 ? "level elimination" : L.rows >= 0 ? "row-parallel" : "interpreted");
     if (getenv("GBH_VERBOSE") && !e->jit_log.empty())
         fprintf(stderr, "gbhsolve: specialised kernels: %d; compiler log:\n%.4000s\n", e->jit_compiled,
                 e->jit_log.c_str());
@@ -3668,6 +3939,10 @@ void gbh_destroy(gbh_engine *e)
     for (auto &vars : e->jit_var)
         for (JitKernel &k : vars) jit_release(k);
     for (JitKernel &k : e->lv_kern) jit_release(k);
+    for (JitKernel &k : e->rw_kern) jit_release(k);
+    e->d_rgroups.release(); e->d_rchunks.release(); e->d_rwork.release(); e->d_ritems.release(); e->d_rmap.release();
+    e->d_rlink.release(); e->d_rprev.release(); e->d_rpos.release();
+    e->d_rA.release(); e->d_rB.release(); e->d_rC.release();
     e->d_lgroups.release(); e->d_lchunks.release(); e->d_lmap.release(); e->d_lkid.release(); e->d_lnkid.release(); e->d_lpar.release();
     e->d_ltopkid.release(); e->d_lkt.release(); e->d_lcy.release(); e->d_lc.release(); e->d_ld.release(); e->d_lpd.release();
     e->d_lgen.release();

@@ -136,6 +136,7 @@ struct TileType {
                      // (FL_SLOT_*), so the sweeps index the stack without a running top
     int level;       // stack: 1 + index of the level-elimination kernel its tiles run (gbh_level.cuh), 0 none
     int lv_f0;       // level: the first field row of the rows above the static ones
+    int rows;        // 1 + index of the row-parallel kernel its tiles may run (gbh_rows.cuh), 0 none
 };
 
 // Per-row flags of the stack elimination (DevView::ltop, topo rows, one word

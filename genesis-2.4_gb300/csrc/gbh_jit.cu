@@ -517,6 +517,10 @@ bool emit_ca_pools(std::ostream &t, const int *pp)
 // Level-elimination blocks: at most 8 sweeping warps and the one of the top
 // rows; the residency sets the register budget (see jit_level_source).
 constexpr int kLevelThreads = 9 * LANES, kLevelBlocks = 2;
+// Row-parallel blocks: at most 16 warps, so 128 registers a thread.
+constexpr int kRowsThreads = 16 * LANES;
+// A field row of another compartment in a row program's class: absolute.
+constexpr int kForeignField = 1 << 20;
 
 }  // namespace
 
@@ -838,38 +842,44 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
     return t.str();
 }
 
+namespace {
+
+// Operands that are field rows (bit i: operand i) and the givals row (-1
+// none) of the ops a step without givals may hold.
+bool op_roles(int code, int &fields, int &giv)
+{
+    fields = 0;
+    giv = -1;
+    switch (code) {
+    case M_BEGIN: fields = 0x7; giv = 3; return true;
+    case M_NEWVOLT: case M_NEWCONC1: case M_FLUX: case M_DO_TABGHK: case M_CONCVAL: case M_NEWCONC2: return true;
+    case M_DOMAIN: case M_SCALE_FLUX: case M_SAME_GHK: case M_CHAN_G: case M_SPIKE: fields = 0x1; return true;
+    case M_ELMMPUMP: fields = 0x7; giv = 3; return true;
+    case M_GHK: fields = 0x7; return true;
+    case M_NERNST: case M_CHAN: fields = 0x3; return true;
+    case M_END: fields = 0x3; giv = 2; return true;
+    case M_GATE: fields = 0x8; return true;
+    case M_SYN: fields = 0x39; return true;
+    case M_MGBLOCK: fields = 0x7; giv = 3; return true;
+    case M_ADDCURR: giv = 0; return true;
+    default: return false;
+    }
+}
+
+}  // namespace
+
 LevelProg level_prog(const TileType &tt, const std::vector<int> &prog)
 {
     LevelProg lp;
     lp.ntop = tt.nslots - tt.nstatic;
     if (tt.nstatic <= 0 || lp.ntop <= 0 || lp.ntop > kSplitRows || tt.has_cd || tt.nscratch || tt.sym || tt.nitot)
         return lp;
-    // operands that are field rows (bit i: operand i) and the givals row (-1
-    // none) of the ops a step without givals may hold
-    auto roles = [](int code, int &fields, int &giv) {
-        fields = 0;
-        giv = -1;
-        switch (code) {
-        case M_BEGIN: fields = 0x7; giv = 3; return true;
-        case M_NEWVOLT: case M_NEWCONC1: case M_FLUX: case M_DO_TABGHK: case M_CONCVAL: case M_NEWCONC2: return true;
-        case M_DOMAIN: case M_SCALE_FLUX: case M_SAME_GHK: case M_CHAN_G: case M_SPIKE: fields = 0x1; return true;
-        case M_ELMMPUMP: fields = 0x7; giv = 3; return true;
-        case M_GHK: fields = 0x7; return true;
-        case M_NERNST: case M_CHAN: fields = 0x3; return true;
-        case M_END: fields = 0x3; giv = 2; return true;
-        case M_GATE: fields = 0x8; return true;
-        case M_SYN: fields = 0x39; return true;
-        case M_MGBLOCK: fields = 0x7; giv = 3; return true;
-        case M_ADDCURR: giv = 0; return true;
-        default: return false;
-        }
-    };
     std::vector<size_t> fpos;
     size_t pc = (size_t)tt.prog_off + 9 * (size_t)tt.nstatic;   // a passive row's program is 9 ints
     for (int s = 0; s < lp.ntop;) {
         const int code = prog[pc], n = nops_of(code);
         int fields, giv;
-        if (n < 0 || !roles(code, fields, giv)) return lp;
+        if (n < 0 || !op_roles(code, fields, giv)) return lp;
         if (code == M_SYN && prog[pc + 1] >= 0) return lp;   // SYN3 draws are keyed by the field row
         const size_t base = lp.prog.size();
         for (int i = 0; i <= n; ++i) lp.prog.push_back(prog[pc + i]);
@@ -895,6 +905,191 @@ LevelProg level_prog(const TileType &tt, const std::vector<int> &prog)
     lp.key = k.str();
     lp.ok = true;
     return lp;
+}
+
+RowsProg rows_prog(const TileType &tt, const std::vector<int> &prog)
+{
+    RowsProg rp;
+    if (tt.has_cd || tt.nscratch || tt.sym || tt.nitot) return rp;
+    std::map<std::vector<int>, int> classes;
+    std::map<int, int> pool_of;   // a pool's flux is reset and summed by one compartment
+    size_t pc = tt.prog_off;
+    int last = -1, conc_rows = 0;
+    for (int s = 0; s < tt.nslots; ++s) {
+        // the compartment's own field rows run from Em/Rm to its diagonal term
+        size_t end = pc;
+        while (prog[end] != M_END) {
+            if (nops_of(prog[end]) < 0) return rp;
+            end += 1 + nops_of(prog[end]);
+        }
+        if (prog[pc] != M_BEGIN) return rp;
+        const int f0 = prog[pc + 1], f1 = prog[end + 2];
+        std::vector<int> p;
+        bool volt = false, conc = false, sel = false, ik = false;
+        for (;;) {
+            const int code = prog[pc], n = nops_of(code);
+            int fields, giv;
+            if (n < 0 || !op_roles(code, fields, giv)) return rp;
+            switch (code) {   // as wide_plan: nothing carried from another compartment but the voltage bracket
+            case M_DOMAIN: case M_NEWCONC2: case M_SAME_GHK: case M_DO_TABGHK: return rp;
+            case M_CONCVAL:
+                sel = true;
+                if (pool_of.emplace(prog[pc + 1], s).first->second != s) return rp;
+                break;
+            case M_NEWVOLT: if (volt) return rp; volt = true; break;
+            case M_NEWCONC1: if (!sel || conc) return rp; conc = true; break;
+            case M_ELMMPUMP: if (!sel) return rp; ik = true; break;
+            case M_GHK: case M_NERNST: if (!sel) return rp; break;
+            case M_FLUX: case M_SCALE_FLUX: if (!sel || !ik) return rp; break;
+            case M_GATE:
+                if (prog[pc + 1] != GK_1V && prog[pc + 1] != GK_1C) return rp;
+                if (prog[pc + 1] == GK_1V ? !volt : !conc) return rp;
+                break;
+            case M_SYN: if (prog[pc + 1] >= 0) return rp; break;   // SYN3 draws are keyed by the field row
+            case M_ADDCURR: ik = true; break;
+            default: break;
+            }
+            p.push_back(code);
+            for (int i = 0; i < n; ++i) {
+                int x = prog[pc + 1 + i];
+                if (i == giv) x = 0;
+                else if ((fields >> i & 1) && x >= 0) x = x >= f0 && x <= f1 ? x - f0 : kForeignField + x;
+                p.push_back(x);
+            }
+            pc += 1 + n;
+            if (code == M_END) break;
+        }
+        if (conc && ++conc_rows > 1) return rp;   // the conc bracket carried between compartments
+        auto it = classes.find(p);
+        if (it == classes.end()) {
+            if (rp.cls.size() >= 8) return rp;   // every class is code of its own
+            it = classes.emplace(p, (int)rp.cls.size()).first;
+            rp.cls.push_back(p);
+        }
+        rp.of.push_back(it->second);
+        rp.f0.push_back(f0);
+        rp.prev.push_back(volt ? last : -2);
+        if (volt) last = s;
+    }
+    for (const int *pp = prog.data() + tt.pool_off; pp[0] != 0; pp += 5) {
+        if (pp[0] != PO_CACONC) return rp;
+        rp.pool.insert(rp.pool.end(), pp, pp + 5);
+    }
+    rp.pool.push_back(0);
+    std::ostringstream k;
+    k << tt.crank << ' ' << tt.chanmode5 << ' ' << tt.interp << ' ' << tt.table_set;
+    for (const auto &c : rp.cls) {
+        k << " |";
+        for (int x : c) k << ' ' << x;
+    }
+    k << " ||";
+    for (int x : rp.pool) k << ' ' << x;
+    rp.key = k.str();
+    rp.ok = true;
+    return rp;
+}
+
+std::string jit_rows_source(const RowsProg &rp, const TileType &tt, const TableGeom &tg, bool mixed)
+{
+    Emit E;
+    E.mixed = mixed;
+    E.giv = false;
+    E.sidx = "0";
+    std::ostringstream &o = E.o;
+    const char *form = mixed ? "true" : "false", *crank = tt.crank ? "true" : "false";
+    const std::string axis = lit(tg.xmin) + ", " + lit(tg.invdx) + ", " + std::to_string(tg.xdivs) + ", " +
+                             std::to_string(tg.xtop) + "u";
+    const bool chain = !mixed && tg.ncols > 0;   // the voltage bracket is carried between compartments
+    if (tg.ncols == 0)
+        for (const std::vector<int> &c : rp.cls)
+            for (size_t at = 0; at < c.size(); at += 1 + nops_of(c[at]))
+                if (c[at] == M_NEWVOLT) return std::string();
+    o << "#include \"gbh_devfn.cuh\"\n#include \"gbh_rows.cuh\"\nusing namespace gbh;\n"
+      << "extern \"C\" __global__ void __launch_bounds__(" << kRowsThreads
+      << ") gbh_jit(DevView v, RowView L, int g0, int nsteps, long long step0)\n{\n"
+      << "  extern __shared__ double sm[];\n"
+      << "  const RowGroup g = L.groups[g0 + blockIdx.x];\n"
+      << "  { unsigned dsz; asm(\"mov.u32 %0, %%dynamic_smem_size;\" : \"=r\"(dsz));\n"
+      << "    if (dsz < rows_smem(g.n, g.nch)) { if (v.status && threadIdx.x == 0) atomicOr(v.status, ST_SMEM); return; } }\n"
+      << "  const Tile tl = v.tiles[g.tile]; const int S = v.types[tl.type].nslots; (void)S;\n"
+      << "  const RowSm q = rows_smem_of(sm, g);\n"
+      << "  const int tid = threadIdx.x, lane32 = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;\n"
+      << "  const long long sbase = v.step_dev ? *v.step_dev : 0;\n"
+      << "  const bool c5 = " << (tt.chanmode5 ? "true" : "false") << "; (void)c5;\n"
+      << "  const bool interp = " << (tt.interp ? "true" : "false") << "; (void)interp; const bool active = true; (void)active;\n"
+      << "  double *Vt = v.V + tl.vm * 32, *Pt = v.P + tl.fld * 32; const int *map = L.map + g.eoff;\n";
+    if (mixed) {
+        o << "  const float4 *tab = v.tabdf + " << tg.tab_off << "; (void)tab;\n"
+          << "  const df xnmin = df_make(" << litf(-tg.xmin_hi) << ", " << litf(-tg.xmin_lo) << "), xinv = df_make("
+          << litf(tg.invdx_hi) << ", " << litf(tg.invdx_lo) << "); (void)xnmin; (void)xinv;\n"
+          << "  const df ynmin = df_make(" << litf(-tg.ymin_hi) << ", " << litf(-tg.ymin_lo) << "), yinv = df_make("
+          << litf(tg.invdy_hi) << ", " << litf(tg.invdy_lo) << "); (void)ynmin; (void)yinv;\n";
+    } else {
+        o << "  const double *tab = v.tab64 + " << tg.tab_off << "; (void)tab;\n"
+          << "  const double2 *tabd = v.tabd + " << tg.tab_off << "; (void)tabd;\n"
+          << "  const double *xvals = v.xyvals + " << tg.xv_off << "; (void)xvals;\n"
+          << "  const double *yvals = v.xyvals + " << (tg.yv_off >= 0 ? tg.yv_off : tg.xv_off) << "; (void)yvals;\n";
+    }
+    o << "  rows_load(L, g, q, Vt);\n"
+      << "  for (int it = 0; it < nsteps; ++it) {\n"
+      << "    const long long step = sbase + step0 + it; (void)step;\n"
+      << "    if (v.io_in) {   // this step's inputs into the group's fields\n"
+      << "      const double *src = v.io_in + (step - v.io_step0) * v.io_nin;\n"
+      << "      for (int k = v.tin_start[g.tile] + tid; k < v.tin_start[g.tile + 1]; k += blockDim.x) {\n"
+      << "        const int at = v.tin_off[k], off = at & ~(1 << 30), l = off & 31; if (l < g.lane0 || l >= g.lane0 + g.nlanes) continue;\n"
+      << "        const double x = src[v.tin_idx[k]];\n"
+      << "        if (at & (1 << 30)) { const float hi = __double2float_rn(x); st_df(&Pt[off], df_make(hi, __double2float_rn(x - (double)hi))); }\n"
+      << "        else Pt[off] = x; }\n"
+      << "      __syncthreads(); }\n";
+    if (chain) o << "    rows_cursors(L, g, q, xvals, " << axis << ", S);\n";
+    o << "    for (int i = warp; i < g.nitems; i += nwarps) {\n"
+      << "      const int4 im = L.items[g.itoff + i];\n"
+      << "      if (lane32 >= im.z) continue;\n"
+      << "      const int2 wk = L.work[g.eoff + im.y + lane32]; const int e = wk.x, lane = wk.y & 31, f0 = wk.y >> 5; (void)f0;\n"
+      << "      double *Pw = Pt + wk.y; int *Iw = v.I + tl.ints * 32 + lane; (void)Iw;\n"
+      << "      double *Cw = v.C + tl.pools * 32 + lane, *Fw = v.F + tl.pools * 32 + lane; (void)Cw; (void)Fw;\n"
+      << "      const int64_t neuron = tl.first_neuron + lane; (void)neuron;\n"
+      << "      const double Vw[1] = {q.V[e]}; double R[1], D[1];\n";
+    if (mixed) {
+        o << "      DCursor vc, cc, c1; vc.row = vc.base = 0; vc.frac = df_make(0.f, 0.f); cc = vc; c1 = vc;\n"
+          << "      df Ek = df_make(0.f, 0.f), Gk = Ek, gmax = Ek; (void)gmax;\n";
+    } else {
+        o << "      VCursor vc, cc; rows_cursor(vc, " << (chain ? "q.in[e]" : "-1") << ", xvals, " << tg.ncols << "); rows_cursor(cc, -1, xvals, 0);\n"
+          << "      double save_frac = 0.0; int tab_base = 0, ctab_base = 0; (void)save_frac; (void)tab_base; (void)ctab_base;\n"
+          << "      double Ek = 0.0, Gk = 0.0, gmax = 0.0; (void)gmax;\n";
+    }
+    o << "      double GHK = 0.0, Ik = 0.0; int doGHK = 0, sel = 0; (void)GHK; (void)doGHK; (void)sel; (void)Ik;\n";
+    for (size_t c = 0; c < rp.cls.size(); ++c) {
+        E.fx.clear();   // field rows of other compartments: from the tile's first
+        const std::vector<int> &p = rp.cls[c];
+        for (size_t at = 0; at < p.size(); at += 1 + nops_of(p[at])) {
+            int fields, giv;
+            op_roles(p[at], fields, giv);
+            for (int i = 0; i < nops_of(p[at]); ++i)
+                if ((fields >> i & 1) && p[at + 1 + i] >= kForeignField)
+                    E.fx[p[at + 1 + i]] = std::to_string(p[at + 1 + i] - kForeignField) + " - f0";
+        }
+        o << "      " << (c ? "else " : "") << "if (im.x == " << c << ") {\n";
+        const int *pc = p.data();
+        if (!emit_slot(E, 0, pc, tg)) return std::string();
+        o << "      }\n";
+    }
+    o << "      q.R[e] = R[0]; q.D[e] = D[0];\n    }\n    __syncthreads();\n";
+    if (rp.pool[0] != 0) {   // the pools: one thread per neuron, from the last warp down
+        o << "    if ((int)blockDim.x - 1 - tid < g.nlanes) { const int lane = g.lane0 + (int)blockDim.x - 1 - tid; double *Pw = Pt + lane;\n"
+          << "      double *Cw = v.C + tl.pools * 32 + lane, *Fw = v.F + tl.pools * 32 + lane;\n";
+        emit_ca_pools(o, rp.pool.data());
+        o << "    }\n";
+    }
+    o << "    rows_eliminate<" << form << ", " << crank << ">(v, g, q);\n"
+      << "    if (v.io_out) {   // this step's outputs\n"
+      << "      for (int e = tid; e < g.n; e += blockDim.x) Vt[map[e]] = q.V[e];\n"
+      << "      __syncthreads(); double *dst = v.io_out + (step - v.io_step0) * v.io_nout;\n"
+      << "      for (int k = v.tout_start[g.tile] + tid; k < v.tout_start[g.tile + 1]; k += blockDim.x) {\n"
+      << "        const int off = v.tout_off[k], l = off & 31; if (l >= g.lane0 && l < g.lane0 + g.nlanes) dst[v.tout_idx[k]] = Vt[off]; } }\n"
+      << "  }\n"
+      << "  for (int e = tid; e < g.n; e += blockDim.x) Vt[map[e]] = q.V[e];\n}\n";
+    return o.str();
 }
 
 std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed, bool resident)
@@ -1005,11 +1200,11 @@ int jit_compile(const std::string &src, bool fp64_exact, int device_major, int d
 {
     if (!jit_available(log)) return -1;
     nvrtcProgram prog;
-    const char *hdr_src[] = {kSrc_gbh_internal_h, kSrc_gbh_df_cuh, kSrc_gbh_devfn_cuh, kSrc_gbh_level_cuh, "",
-                             kStdintStub};
-    const char *hdr_name[] = {"gbh_internal.h", "gbh_df.cuh", "gbh_devfn.cuh", "gbh_level.cuh", "cuda_runtime.h",
-                              "stdint.h"};
-    if (g_api.create(&prog, src.c_str(), "gbh_jit.cu", 6, hdr_src, hdr_name) != NVRTC_SUCCESS) {
+    const char *hdr_src[] = {kSrc_gbh_internal_h, kSrc_gbh_df_cuh, kSrc_gbh_devfn_cuh, kSrc_gbh_level_cuh,
+                             kSrc_gbh_rows_cuh, "", kStdintStub};
+    const char *hdr_name[] = {"gbh_internal.h", "gbh_df.cuh", "gbh_devfn.cuh", "gbh_level.cuh", "gbh_rows.cuh",
+                              "cuda_runtime.h", "stdint.h"};
+    if (g_api.create(&prog, src.c_str(), "gbh_jit.cu", 7, hdr_src, hdr_name) != NVRTC_SUCCESS) {
         if (log) *log = "nvrtcCreateProgram failed";
         return -1;
     }
@@ -1077,6 +1272,19 @@ cudaError_t jit_level_launch(const JitKernel &k, const DevView &v, const LevelVi
     void *args[] = {&vv, &ll, &g0, &nsteps, &step};
     const CUresult r = g_api.launch((CUfunction)k.fn, ngroups, 1, 1, (warps + 1) * LANES, 1, 1, (unsigned)smem,
                                     (CUstream)st, args, nullptr);
+    if (r == CUDA_SUCCESS) return cudaSuccess;
+    return r == CUDA_ERROR_LAUNCH_FAILED || r == CUDA_ERROR_ILLEGAL_ADDRESS ? cudaErrorLaunchFailure
+                                                                          : cudaErrorInvalidConfiguration;
+}
+
+cudaError_t jit_rows_launch(const JitKernel &k, const DevView &v, const RowView &rv, int g0, int ngroups, int warps,
+                            int nsteps, long long step, size_t smem, cudaStream_t st)
+{
+    DevView vv = v;
+    RowView rr = rv;
+    void *args[] = {&vv, &rr, &g0, &nsteps, &step};
+    const CUresult r = g_api.launch((CUfunction)k.fn, ngroups, 1, 1, warps * LANES, 1, 1, (unsigned)smem, (CUstream)st,
+                                    args, nullptr);
     if (r == CUDA_SUCCESS) return cudaSuccess;
     return r == CUDA_ERROR_LAUNCH_FAILED || r == CUDA_ERROR_ILLEGAL_ADDRESS ? cudaErrorLaunchFailure
                                                                           : cudaErrorInvalidConfiguration;

@@ -7,6 +7,7 @@
 
 #include "gbh_devfn.cuh"
 #include "gbh_level.cuh"
+#include "gbh_rows.cuh"
 
 namespace gbh {
 
@@ -45,6 +46,21 @@ LevelProg level_prog(const TileType &tt, const std::vector<int> &prog);
 std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed, bool resident);
 cudaError_t jit_level_launch(const JitKernel &k, const DevView &v, const LevelView &lv, int g0, int ngroups, int warps,
                              int nsteps, long long step, size_t smem, cudaStream_t st);
+// A type's compartments as the row-parallel kernel runs them (gbh_rows.cuh):
+// their programs, grouped into classes of equal ones (field rows relative to
+// the compartment's first). ok: the generator emits every op and no compartment
+// reads what another leaves but the table bracket.
+struct RowsProg {
+    bool ok = false;
+    std::vector<std::vector<int>> cls;   // one program per class
+    std::vector<int> of, f0, prev;       // per slot: class, first field row, previous slot with a voltage lookup (-1 none, -2 has none)
+    std::vector<int> pool;               // 0-terminated pool program
+    std::string key;
+};
+RowsProg rows_prog(const TileType &tt, const std::vector<int> &prog);
+std::string jit_rows_source(const RowsProg &rp, const TileType &tt, const TableGeom &tg, bool mixed);
+cudaError_t jit_rows_launch(const JitKernel &k, const DevView &v, const RowView &rv, int g0, int ngroups, int warps,
+                            int nsteps, long long step, size_t smem, cudaStream_t st);
 // Largest dynamic shared memory the kernel may be launched with.
 bool jit_allow_smem(const JitKernel &k, size_t smem);
 

@@ -44,7 +44,8 @@ def up_to_date() -> bool:
     return all(os.path.getmtime(s) <= t for s in _sources())
 
 
-JIT_HEADERS = ["gbh_internal.h", "gbh_df.cuh", "gbh_devfn.cuh", "gbh_level.cuh"]
+JIT_HEADERS = ["gbh_internal.h", "gbh_df.cuh", "gbh_devfn.cuh", "gbh_level.cuh",
+               "gbh_rows.cuh"]
 STDINT_STUB = ("typedef signed char int8_t; typedef short int16_t; typedef int int32_t; "
                "typedef long long int64_t; typedef unsigned char uint8_t; typedef unsigned short uint16_t; "
                "typedef unsigned int uint32_t; typedef unsigned long long uint64_t;")
