@@ -17,16 +17,16 @@ cudaError_t launch_adj_copy(const AdjView &v, int ntiles, int maxrows, int c, in
                             cudaStream_t st)
 {
     if (ntiles <= 0 || maxrows <= 0) return cudaSuccess;
-    const dim3 grid(ntiles, (maxrows + 31) / 32);
-    k_adj_copy<<<grid, LANES, 0, st>>>(v, c, dir, to_tape ? 1 : 0);
+    const dim3 grid(ntiles, (maxrows + ADJ_COPY_ROWS - 1) / ADJ_COPY_ROWS);
+    k_adj_copy<<<grid, dim3(LANES, ADJ_COPY_ROWS), 0, st>>>(v, c, dir, to_tape ? 1 : 0);
     return cudaGetLastError();
 }
 
 cudaError_t launch_adj_ck_to_tape(const AdjView &v, int ntiles, int maxrows, int c0, int nk, cudaStream_t st)
 {
     if (ntiles <= 0 || maxrows <= 0 || nk <= 0) return cudaSuccess;
-    const dim3 grid(ntiles, (maxrows + 31) / 32, nk);
-    k_adj_ck_to_tape<<<grid, LANES, 0, st>>>(v, c0);
+    const dim3 grid(ntiles, (maxrows + ADJ_COPY_ROWS - 1) / ADJ_COPY_ROWS, nk);
+    k_adj_ck_to_tape<<<grid, dim3(LANES, ADJ_COPY_ROWS), 0, st>>>(v, c0);
     return cudaGetLastError();
 }
 
@@ -40,19 +40,19 @@ cudaError_t launch_adj_linearize(const AdjView &v, int ntiles, int smax, int nk,
     return cudaGetLastError();
 }
 
-size_t adj_reverse_smem(int smax, int hmax)
+size_t adj_reverse_smem(int n, int nch, int nslots, int hmax)
 {
-    return ((size_t)2 * smax * LANES + (size_t)ADJ_REV_WARPS * LANES) * sizeof(double) + (size_t)smax * sizeof(AdjSlot) +
-           (size_t)hmax * sizeof(AdjChan);
+    return sizeof(double) * (6 * (size_t)n + 2) + sizeof(int2) * ((size_t)nch + n) + 2 * sizeof(int) * (size_t)n +
+           (size_t)nslots * sizeof(AdjSlot) + (size_t)hmax * sizeof(AdjChan);
 }
 
-cudaError_t launch_adj_reverse(const AdjView &v, int ntiles, int smax, int hmax, int nk, int step0, cudaStream_t st)
+cudaError_t launch_adj_reverse(const AdjView &v, const AdjPlan &pl, int ngroups, int warps, size_t smem, int hmax, int nk,
+                               int step0, cudaStream_t st)
 {
-    if (ntiles <= 0 || nk <= 0) return cudaSuccess;
-    const size_t smem = adj_reverse_smem(smax, hmax);
+    if (ngroups <= 0 || nk <= 0) return cudaSuccess;
     cudaError_t ce = smem_attr((const void *)k_adj_reverse, smem);
     if (ce != cudaSuccess) return ce;
-    k_adj_reverse<<<ntiles, ADJ_REV_WARPS * LANES, smem, st>>>(v, smax, hmax, nk, step0);
+    k_adj_reverse<<<ngroups, warps * LANES, smem, st>>>(v, pl, hmax, nk, step0);
     return cudaGetLastError();
 }
 

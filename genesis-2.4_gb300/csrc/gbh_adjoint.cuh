@@ -22,8 +22,7 @@
 //             of every channel, and per gate d prod/dx, dx'/dVm (table slope,
 //             zero where the lookup clamps or without interpolation) and
 //             dx'/dx (the trapezoid factor (2-B')/B', zero for instant gates);
-//   k_adj_reverse   (sequential over steps, one lane per neuron; the tree
-//             walk on one warp, the channel phase spread over four) the
+//   k_adj_reverse   (sequential over steps, a thread per compartment) the
 //             adjoint recurrence of Vm and the gate states:
 //               seed      Vm-bar += 2 (Vm after - target) at target rows
 //                         (Crank-Nicolson: Vm after = 2x - Vm before);
@@ -79,30 +78,28 @@ __device__ __forceinline__ bool locate_lin(VCursor &c, double v, const TableGeom
 }
 
 // ---------------------------------------------------------------- copies
-// grid (tiles, row chunks of 32), 32 threads: one lane each.
-__global__ void __launch_bounds__(32)
+// grid (tiles, row chunks of ADJ_COPY_ROWS), one warp a row. (One warp walking
+// 32 rows took 20 us for 24 tiles of 256 rows, a load's latency a row.)
+__global__ void __launch_bounds__(LANES * ADJ_COPY_ROWS)
 k_adj_copy(AdjView v, int c, int dir, int to_tape)
 {
     const int lane = threadIdx.x;
     const int t = blockIdx.x;
     const Tile tl = v.tiles[t];
     const AdjType at = v.atypes[tl.type];
-    const int rows = at.nslots + at.ngates;
-    const int r0 = blockIdx.y * 32;
-    const int r1 = min(rows, r0 + 32);
+    const int r = blockIdx.y * ADJ_COPY_ROWS + threadIdx.y;
+    if (r >= at.nslots + at.ngates) return;
     double *blk = to_tape ? adj_tape(v, c, t, lane)
                           : v.ckpt + ((int64_t)c * v.ck_stride + v.ck_off[t]) * LANES + lane;
-    for (int r = r0; r < r1; ++r) {
-        double *w = r < at.nslots ? v.V + (tl.vm + r) * LANES + lane
-                                  : v.P + (tl.fld + v.snap_field[at.snap_off + r - at.nslots]) * LANES + lane;
-        if (dir == 0) blk[r * LANES] = *w;
-        else *w = blk[r * LANES];
-    }
+    double *w = r < at.nslots ? v.V + (tl.vm + r) * LANES + lane
+                              : v.P + (tl.fld + v.snap_field[at.snap_off + r - at.nslots]) * LANES + lane;
+    if (dir == 0) blk[r * LANES] = *w;
+    else *w = blk[r * LANES];
 }
 
 // Checkpoint c0 + k -> tape step k (blockIdx.z = k): the snapshot rows of a
 // segment whose every step was kept by the forward pass.
-__global__ void __launch_bounds__(LANES)
+__global__ void __launch_bounds__(LANES * ADJ_COPY_ROWS)
 k_adj_ck_to_tape(AdjView v, int c0)
 {
     const int lane = threadIdx.x;
@@ -110,12 +107,10 @@ k_adj_ck_to_tape(AdjView v, int c0)
     const int k = blockIdx.z;
     const Tile tl = v.tiles[t];
     const AdjType at = v.atypes[tl.type];
-    const int rows = at.nslots + at.ngates;
-    const int r0 = blockIdx.y * 32;
-    const int r1 = min(rows, r0 + 32);
+    const int r = blockIdx.y * ADJ_COPY_ROWS + threadIdx.y;
+    if (r >= at.nslots + at.ngates) return;
     const double *src = v.ckpt + ((int64_t)(c0 + k) * v.ck_stride + v.ck_off[t]) * LANES + lane;
-    double *dst = adj_tape(v, k, t, lane);
-    for (int r = r0; r < r1; ++r) dst[r * LANES] = src[r * LANES];
+    adj_tape(v, k, t, lane)[r * LANES] = src[r * LANES];
 }
 
 // ---------------------------------------------------------------- linearisation
@@ -275,123 +270,158 @@ k_adj_linearize(AdjView v, int smax)
 }
 
 // ---------------------------------------------------------------- reverse
-// grid (tiles), ADJ_REV_WARPS warps per tile. Warp 0 runs the elimination's
-// reverse (a chain along the tree); the channel phase and the seeds of the
-// next step are split over the warps by slot (slot s to warp s mod W), so
-// the block keeps every FP64 unit of its SM busy. Shared memory: the D and R
-// adjoint columns (2 * smax * 32 doubles), per-warp loss partials
-// (W * 32 doubles) and the tile type's slot and channel plans.
-constexpr int ADJ_REV_WARPS = 4;
-
-__global__ void __launch_bounds__(ADJ_REV_WARPS * 32)
-k_adj_reverse(AdjView v, int smax, int hmax, int nk, int step0)
+// grid (groups), up to 16 warps: a block owns some neurons of a tile and gives
+// each of their compartments a thread. The elimination's reverse goes through
+// the tree depth by depth (back substitution reversed from the deepest rows
+// up, a row pulling its children's contributions in ascending row order;
+// forward elimination reversed from the root down), the channels' reverse and
+// the next step's seeds take all rows at once. With one neuron per lane and
+// the tree walked on one warp a step took 120 us for 24 tiles of 64
+// compartments on 24 SMs (3 FP64 instructions up and 8 down per row, 64 rows
+// in a row); with a thread per compartment it takes 22 us, bound by the
+// levels' barriers and the tape's loads. Shared memory: the adjoints of R and
+// D, what a parent takes from its children, the adjoint of Vm, the
+// coefficients and links of the group's rows, and the tile type's slot and
+// channel plans.
+__global__ void __launch_bounds__(ADJ_REV_THREADS)
+k_adj_reverse(AdjView v, AdjPlan pl, int hmax, int nk, int step0)
 {
     extern __shared__ double sm[];
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-    const int t = blockIdx.x;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const AdjGroup g = pl.groups[blockIdx.x];
+    const int t = g.tile, n = g.n;
     const Tile tl = v.tiles[t];
     const TileType ty = v.types[tl.type];
     const AdjType at = v.atypes[tl.type];
     const int S = at.nslots;
     const bool crank = ty.crank != 0;
     const AdjRows R = adj_rows(S, at.ngates, at.nchans);
-    const double *P = v.P + tl.fld * LANES + lane;
-    const int *par = v.parent + tl.topo * LANES + lane;
-    const double *Bw = v.B + tl.topo * LANES + lane;
-    const double *Cw = v.Cb + tl.topo * LANES + lane;
-    const int *tgt = v.tgt + tl.topo * LANES + lane;
-    double *Vb = v.Vbar + tl.vm * LANES + lane;
-    double *Xb = v.Xbar + v.xb_off[t] * LANES + lane;
-    double *loss = v.loss + (size_t)t * LANES + lane;
-    double *Db = sm + lane;
-    double *Rb = Db + (size_t)smax * LANES;
-    double *lpart = sm + (size_t)2 * smax * LANES;       // [warp][lane]
-    AdjSlot *slots = reinterpret_cast<AdjSlot *>(lpart + nw * LANES);
-    AdjChan *chans = reinterpret_cast<AdjChan *>(slots + smax);
-    for (int i = threadIdx.x; i < S; i += blockDim.x) slots[i] = v.slot_plan[at.slot_off + i];
-    for (int i = threadIdx.x; i < at.nchans && i < hmax; i += blockDim.x) chans[i] = v.chan_plan[at.chan_off + i];
+    double *Rb = sm, *Db = Rb + n + 1, *CR = Db + n + 1, *Vb = CR + n, *B = Vb + n, *C = B + n;
+    int2 *ch = reinterpret_cast<int2 *>(C + n), *link = ch + g.nch;
+    int *map = reinterpret_cast<int *>(link + n), *tgt = map + n;
+    AdjSlot *slots = reinterpret_cast<AdjSlot *>(tgt + n);
+    AdjChan *chans = reinterpret_cast<AdjChan *>(slots + S);
+    for (int i = tid; i < g.nch; i += nt) ch[i] = pl.chunks[g.choff + i];
+    for (int i = tid; i < n; i += nt) {
+        const int m = pl.map[g.eoff + i];
+        map[i] = m;
+        link[i] = pl.link[g.eoff + i];
+        B[i] = v.B[tl.topo * LANES + m];
+        C[i] = v.Cb[tl.topo * LANES + m];
+        tgt[i] = v.tgt[tl.topo * LANES + m];
+        Vb[i] = v.Vbar[tl.vm * LANES + m];
+    }
+    for (int i = tid; i < S; i += nt) slots[i] = v.slot_plan[at.slot_off + i];
+    for (int i = tid; i < at.nchans && i < hmax; i += nt) chans[i] = v.chan_plan[at.chan_off + i];
+    if (tid == 0) Rb[n] = Db[n] = 0.0;
+    __syncthreads();
+    auto tape = [&](int k) { return v.tape + ((int64_t)k * v.tp_stride + v.tp_off[t]) * LANES; };
 
-    // seed of step k at slot s: vb is the adjoint of Vm after step k
-    auto seed = [&](int k, int s, double vb) {
-        double l = 0.0;
-        const int j = tgt[s * LANES];
+    // seed of step k at row e: vb is the adjoint of Vm after step k; each
+    // row's squared errors are summed on their own, steps descending
+    auto seed = [&](int k, int e, double vb) {
+        const int j = tgt[e];
         if (j >= 0) {
-            const double *tp = adj_tape(v, k, t, lane);
-            const double x = __ldg(tp + (R.X + s) * LANES);
-            const double vnext = crank ? x + x - __ldg(tp + (R.V + s) * LANES) : x;
+            const double *tp = tape(k) + map[e];
+            const double x = __ldg(tp + R.X * LANES);
+            const double vnext = crank ? x + x - __ldg(tp + R.V * LANES) : x;
             const double diff = vnext - __ldg(v.trace + (size_t)(step0 + k) * v.ntargets + j);
-            l = diff * diff;
+            v.loss[tl.topo * LANES + map[e]] += diff * diff;
             vb += 2.0 * diff;
         }
-        Rb[s * LANES] = crank ? 2.0 * vb : vb;
-        Vb[s * LANES] = crank ? -vb : 0.0;
-        return l;
+        Rb[e] = crank ? 2.0 * vb : vb;
+        Vb[e] = crank ? -vb : 0.0;
     };
-
-    double lw = 0.0;
-    for (int s = warp; s < S; s += nw) lw += seed(nk - 1, s, Vb[s * LANES]);
-    lpart[warp * LANES + lane] = lw;
-    __syncthreads();
-    for (int k = nk - 1; k >= 0; --k) {
-        double *tp = adj_tape(v, k, t, lane);
-        if (warp == 0) {
-            // loss of step k, summed in warp order, steps descending
-            double l = 0.0;
-            for (int w = 0; w < nw; ++w) l += lpart[w * LANES + lane];
-            *loss += l;
-            // back substitution reversed
-#pragma unroll 4
-            for (int s = 0; s < S; ++s) {
-                const int p = __ldg(par + s * LANES);
-                const double rb = Rb[s * LANES] * __ldg(tp + (R.RD + s) * LANES);
-                Rb[s * LANES] = rb;
-                tp[(R.RBBS + s) * LANES] = rb;
-                if (p >= 0) Rb[p * LANES] -= __ldg(Cw + s * LANES) * rb;
-                Db[s * LANES] = -__ldg(tp + (R.X + s) * LANES) * rb;
-            }
-            // forward elimination reversed
-#pragma unroll 4
-            for (int s = S - 1; s >= 0; --s) {
-                const int p = __ldg(par + s * LANES);
-                if (p < 0) continue;
-                const double tt = __ldg(tp + (R.T + s) * LANES);
-                const double rd = __ldg(tp + (R.RD + s) * LANES);
-                const double tb = -__ldg(Bw + s * LANES) * Db[p * LANES] - __ldg(tp + (R.RP + s) * LANES) * Rb[p * LANES];
-                Rb[s * LANES] -= tt * Rb[p * LANES];
-                Db[s * LANES] -= tt * (tb * rd);
-            }
-        }
-        __syncthreads();
-        // channels reversed (adjoint of Vm and of the gate states), then the
-        // seed of step k-1
-        lw = 0.0;
-        for (int s = warp; s < S; s += nw) {
-            const AdjSlot sp = slots[s];
-            const double rb = Rb[s * LANES], db = Db[s * LANES];
-            tp[(R.RBF + s) * LANES] = rb;
-            tp[(R.DBF + s) * LANES] = db;
-            const double tbyc = __ldg(P + sp.f_tbyc * LANES);
-            const double Ibar = rb * tbyc, Sbar = db * tbyc;
-            double vbn = Vb[s * LANES] + rb;
+    // the tape rows of step k this thread's compartments will read, into L1
+    auto ahead = [&](int k) {
+        if (k < 0) return;
+        const double *tp = tape(k);
+        for (int e = tid; e < n; e += nt) {
+            const double *q = tp + map[e];
+            prefetch_l1(q + R.RD * LANES);
+            prefetch_l1(q + R.T * LANES);
+            prefetch_l1(q + R.RP * LANES);
+            prefetch_l1(q + R.X * LANES);
+            const AdjSlot sp = slots[map[e] / LANES];
+            const int lane = map[e] % LANES;
             for (int c = sp.ch0; c < sp.ch0 + sp.nch; ++c) {
-                const AdjChan ch = c < hmax ? chans[c] : v.chan_plan[at.chan_off + c];
-                const double Ek = ch.f_ek >= 0 ? __ldg(P + ch.f_ek * LANES) : 0.0;
-                const double w = (Sbar + Ibar * Ek) * __ldg(P + ch.f_gmax * LANES);
-#pragma unroll 2
-                for (int g = ch.g0; g < ch.g0 + ch.ng; ++g) {
-                    const double xhat = Xb[g * LANES] + w * __ldg(tp + (R.Q + g) * LANES);
-                    vbn += xhat * __ldg(tp + (R.DXDV + g) * LANES);
-                    Xb[g * LANES] = xhat * __ldg(tp + (R.DXDST + g) * LANES);
+                const AdjChan h = c < hmax ? chans[c] : v.chan_plan[at.chan_off + c];
+                for (int i = h.g0; i < h.g0 + h.ng; ++i) {
+                    prefetch_l1(tp + (R.Q + i) * LANES + lane);
+                    prefetch_l1(tp + (R.DXDV + i) * LANES + lane);
+                    prefetch_l1(tp + (R.DXDST + i) * LANES + lane);
                 }
             }
-            if (k > 0) lw += seed(k - 1, s, vbn);
-            else Vb[s * LANES] = vbn;
         }
-        lpart[warp * LANES + lane] = lw;
+    };
+    ahead(nk - 1);
+    for (int e = tid; e < n; e += nt) seed(nk - 1, e, Vb[e]);
+    __syncthreads();
+    for (int k = nk - 1; k >= 0; --k) {
+        double *tp = tape(k);
+        ahead(k - 1);
+        // back substitution reversed, children before their parents
+        for (int c = g.nch - 1; c >= 0; --c) {
+            const int2 m = ch[c];
+            if (tid < (m.y & ADJ_COUNT)) {
+                const int e = m.x + tid, k0 = link[e].x & 0xffff, nkid = link[e].x >> 16;
+                double *q = tp + map[e];
+                const double rd = __ldg(q + R.RD * LANES), x = __ldg(q + R.X * LANES);
+                double r = Rb[e];
+                for (int i = k0; i < k0 + nkid; ++i) r -= CR[i];
+                const double rb = r * rd;
+                Rb[e] = rb;
+                CR[e] = C[e] * rb;
+                Db[e] = -x * rb;
+                q[R.RBBS * LANES] = rb;
+            }
+            if (m.y & ADJ_FIRST) __syncthreads();
+        }
+        // forward elimination reversed, parents before their children
+        for (int c = 0; c < g.nch; ++c) {
+            const int2 m = ch[c];
+            if (tid < (m.y & ADJ_COUNT)) {
+                const int e = m.x + tid, p = link[e].y;
+                if (p < n) {
+                    const double *q = tp + map[e];
+                    const double tt = __ldg(q + R.T * LANES), rd = __ldg(q + R.RD * LANES);
+                    const double tb = -B[e] * Db[p] - __ldg(q + R.RP * LANES) * Rb[p];
+                    Rb[e] -= tt * Rb[p];
+                    Db[e] -= tt * (tb * rd);
+                }
+            }
+            if (m.y & ADJ_LAST) __syncthreads();
+        }
+        // channels reversed (adjoint of Vm and of the gate states), then the
+        // seed of step k-1
+        for (int e = tid; e < n; e += nt) {
+            const int mp = map[e], lane = mp % LANES;
+            const AdjSlot sp = slots[mp / LANES];
+            const double *P = v.P + tl.fld * LANES + lane;
+            double *Xb = v.Xbar + v.xb_off[t] * LANES + lane;
+            const double rb = Rb[e], db = Db[e];
+            tp[R.RBF * LANES + mp] = rb;
+            tp[R.DBF * LANES + mp] = db;
+            const double tbyc = __ldg(P + sp.f_tbyc * LANES);
+            const double Ibar = rb * tbyc, Sbar = db * tbyc;
+            double vbn = Vb[e] + rb;
+            for (int c = sp.ch0; c < sp.ch0 + sp.nch; ++c) {
+                const AdjChan h = c < hmax ? chans[c] : v.chan_plan[at.chan_off + c];
+                const double Ek = h.f_ek >= 0 ? __ldg(P + h.f_ek * LANES) : 0.0;
+                const double w = (Sbar + Ibar * Ek) * __ldg(P + h.f_gmax * LANES);
+#pragma unroll 2
+                for (int i = h.g0; i < h.g0 + h.ng; ++i) {
+                    const double xhat = Xb[i * LANES] + w * __ldg(tp + (R.Q + i) * LANES + lane);
+                    vbn += xhat * __ldg(tp + (R.DXDV + i) * LANES + lane);
+                    Xb[i * LANES] = xhat * __ldg(tp + (R.DXDST + i) * LANES + lane);
+                }
+            }
+            if (k > 0) seed(k - 1, e, vbn);
+            else Vb[e] = vbn;
+        }
         __syncthreads();
     }
+    for (int e = tid; e < n; e += nt) v.Vbar[tl.vm * LANES + map[e]] = Vb[e];
 }
 
 // ---------------------------------------------------------------- gradient sums

@@ -104,8 +104,24 @@ struct AdjView {
     const int *tgt;         // topo rows: trace column of the row or -1
     const double *trace;    // [step][ntargets]
     int ntargets;
-    double *loss;           // per tile lane
+    double *loss;           // topo rows: squared errors of the row
     int *status;
+};
+
+// Row order of the reverse sweep: a block's share of a tile, lanes [lane0,
+// lane0 + nlanes), their n rows by depth at elements eoff, in nch chunks (first
+// row, rows | ADJ_FIRST | ADJ_LAST of a level) of at most the block's threads.
+struct AdjGroup {
+    int tile, lane0, nlanes, n, nch, choff;
+    int64_t eoff;
+};
+constexpr int ADJ_FIRST = 1 << 30, ADJ_LAST = 1 << 29, ADJ_COUNT = (1 << 29) - 1;
+constexpr int ADJ_REV_THREADS = 512, ADJ_COPY_ROWS = 8;
+struct AdjPlan {
+    const AdjGroup *groups;
+    const int2 *chunks;
+    const int2 *link;   // first child | number of children << 16; parent (roots: n)
+    const int *map;     // row * 32 + lane
 };
 
 // Checkpoint / snapshot copies between the work state and a block of
@@ -122,9 +138,11 @@ cudaError_t launch_adj_ck_to_tape(const AdjView &v, int ntiles, int maxrows, int
 // its snapshot (parallel over steps and tiles) and fills the tape rows.
 cudaError_t launch_adj_linearize(const AdjView &v, int ntiles, int smax, int nk, cudaStream_t st);
 // Reverse sweep over tape steps nk-1 .. 0 (step0: trace row of step 0);
-// hmax: channels per neuron whose plan is cached in shared memory.
-size_t adj_reverse_smem(int smax, int hmax);
-cudaError_t launch_adj_reverse(const AdjView &v, int ntiles, int smax, int hmax, int nk, int step0, cudaStream_t st);
+// hmax: channels per neuron whose plan is cached in shared memory; smem: the
+// largest adj_reverse_smem of the groups, warps: of a block.
+size_t adj_reverse_smem(int n, int nch, int nslots, int hmax);
+cudaError_t launch_adj_reverse(const AdjView &v, const AdjPlan &pl, int ngroups, int warps, size_t smem, int hmax, int nk,
+                               int step0, cudaStream_t st);
 // Gradient sums of one segment's nk steps (parallel over tiles and slots).
 cudaError_t launch_adj_reduce(const AdjView &v, int ntiles, int smax, int nk, cudaStream_t st);
 

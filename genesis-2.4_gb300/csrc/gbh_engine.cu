@@ -239,6 +239,12 @@ struct gbh_engine {
     double *io_pend_host = nullptr;
     int io_pend_buf = 0;
     cudaStream_t io_pend_stream = nullptr;
+    // gbh_loss_gradient: the reverse sweep's row order, from the first call on
+    DBuf<AdjGroup> d_agroups;
+    DBuf<int2> d_achunks, d_alink;
+    DBuf<int> d_amap;
+    int adj_ngroups = 0, adj_warps = 0;
+    size_t adj_smem = 0;
     // gbh_get_state: Vm gathered into the descriptor's order
     DBuf<int64_t> d_vm_at;
     DBuf<double> d_vm_out;
@@ -980,6 +986,60 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
 constexpr int64_t kRowsTiles = 8 * 152;
 constexpr size_t kRowsKernels = 8;
 
+// Rows of some neurons of one type by depth: the roots, then the children of
+// each row in turn, so a row's children are consecutive and ascending.
+struct TreeOrder {
+    std::vector<int> order;          // row * neurons + neuron
+    std::vector<int> start;          // levels
+    std::vector<int> kid, nk, par;   // first child, children, parent (roots: the number of rows)
+    std::vector<int> at;             // place of row * neurons + neuron
+};
+
+TreeOrder tree_order(const std::vector<const Neuron *> &cl, int S)
+{
+    const int nl = (int)cl.size(), n = nl * S;
+    TreeOrder o;
+    std::vector<std::vector<int>> kids((size_t)n);
+    o.start.assign(1, 0);
+    o.kid.assign(n, 0);
+    o.nk.assign(n, 0);
+    o.par.assign(n, n);
+    o.at.assign(n, 0);
+    for (int l = 0; l < nl; ++l)
+        for (int s = 0; s < S; ++s) {
+            const int p = cl[l]->parent[s];
+            if (p >= 0) kids[(size_t)p * nl + l].push_back(s);
+            else o.order.push_back(s * nl + l);
+        }
+    while ((int)o.order.size() > o.start.back()) {
+        const int e0 = o.start.back(), e1 = (int)o.order.size();
+        o.start.push_back(e1);
+        for (int x = e0; x < e1; ++x) {
+            o.kid[x] = (int)o.order.size();
+            o.nk[x] = (int)kids[o.order[x]].size();
+            for (int s : kids[o.order[x]]) {
+                o.par[o.order.size()] = x;
+                o.order.push_back(s * nl + o.order[x] % nl);
+            }
+        }
+    }
+    for (int x = 0; x < n; ++x) o.at[o.order[x]] = x;
+    return o;
+}
+
+// The levels of a tree order in chunks of at most nt rows (RW_FIRST, RW_LAST).
+int tree_chunks(const TreeOrder &o, int nt, std::vector<int2> &chunks)
+{
+    const size_t c0 = chunks.size();
+    for (size_t d = 0; d + 1 < o.start.size(); ++d)
+        for (int a = o.start[d]; a < o.start[d + 1]; a += nt) {
+            const int m = std::min(nt, o.start[d + 1] - a);
+            chunks.push_back(make_int2(a, m | (a == o.start[d] ? RW_FIRST : 0) |
+                                              (a + m == o.start[d + 1] ? RW_LAST : 0)));
+        }
+    return (int)(chunks.size() - c0);
+}
+
 bool rows_type(const TileType &tt, const std::vector<int> &prog, RowsProg &rp)
 {
     if (tt.wide || tt.nslots < 4 || tt.sym || tt.nitot) return false;
@@ -1082,52 +1142,22 @@ int rows_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const
             g.eoff = (int64_t)map.size();
             g.choff = (int)chunks.size();
             g.itoff = (int)items.size();
-            // level order: the roots, then the children of each row in turn
-            std::vector<std::vector<int>> kids((size_t)n);
-            std::vector<int> order, start(1, 0), at(n), gpar(n), gkid(n, 0), gnk(n, 0);
             std::vector<const Neuron *> cl;
             for (int l = 0; l < nl; ++l) cl.push_back(&dec.neurons[cells_of[t][l0 + l]]);
-            for (int l = 0; l < nl; ++l)
-                for (int s = 0; s < S; ++s) {
-                    const int p = cl[l]->parent[s];
-                    if (p >= 0) kids[(size_t)p * nl + l].push_back(s);
-                    else {
-                        gpar[order.size()] = n;
-                        order.push_back(s * nl + l);
-                    }
-                }
-            while ((int)order.size() > start.back()) {
-                const int e0 = start.back(), e1 = (int)order.size();
-                start.push_back(e1);
-                for (int x = e0; x < e1; ++x) {
-                    gkid[x] = (int)order.size();
-                    gnk[x] = (int)kids[order[x]].size();
-                    for (int s : kids[order[x]]) {
-                        gpar[order.size()] = x;
-                        order.push_back(s * nl + order[x] % nl);
-                    }
-                }
-            }
-            for (int x = 0; x < n; ++x) at[order[x]] = x;
+            const TreeOrder o = tree_order(cl, S);
             // a warp for every 32 rows, unless more blocks than SMs have to share them
             const int warps = std::min(crowded ? 8 : 16, (n + LANES - 1) / LANES), nt = warps * LANES;
-            for (size_t d = 0; d + 1 < start.size(); ++d)
-                for (int a = start[d]; a < start[d + 1]; a += nt) {
-                    const int m = std::min(nt, start[d + 1] - a);
-                    chunks.push_back(make_int2(a, m | (a == start[d] ? RW_FIRST : 0) |
-                                                      (a + m == start[d + 1] ? RW_LAST : 0)));
-                }
-            g.nch = (int)chunks.size() - g.choff;
-            for (int x : order) {
+            g.nch = tree_chunks(o, nt, chunks);
+            for (int x : o.order) {
                 const int s = x / nl, l = x % nl;
                 map.push_back(s * LANES + l0 + l);
                 A.push_back(cl[l]->A[s]);
                 B.push_back(cl[l]->B[s]);
                 C.push_back(cl[l]->parent[s] >= 0 ? cl[l]->C[s] : 0.0);
-                prev.push_back(rp.prev[s] >= 0 ? at[rp.prev[s] * nl + l] : rp.prev[s]);
+                prev.push_back(rp.prev[s] >= 0 ? o.at[rp.prev[s] * nl + l] : rp.prev[s]);
             }
-            for (int x = 0; x < n; ++x) link.push_back(make_int2(gkid[x] | gnk[x] << 16, gpar[x]));
-            pos.insert(pos.end(), at.begin(), at.end());
+            for (int x = 0; x < n; ++x) link.push_back(make_int2(o.kid[x] | o.nk[x] << 16, o.par[x]));
+            pos.insert(pos.end(), o.at.begin(), o.at.end());
             // work by class, the longest programs first (they start first)
             std::vector<int> by(rp.cls.size());
             for (size_t c = 0; c < by.size(); ++c) by[c] = (int)c;
@@ -1138,7 +1168,7 @@ int rows_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const
                 for (int s = 0; s < S; ++s)
                     if (rp.of[s] == c)
                         for (int l = 0; l < nl; ++l) {
-                            work.push_back(make_int2(at[s * nl + l], rp.f0[s] * LANES + l0 + l));
+                            work.push_back(make_int2(o.at[s * nl + l], rp.f0[s] * LANES + l0 + l));
                             ++done;
                         }
                 for (int a = w0; a < done; a += LANES)
@@ -3488,6 +3518,65 @@ int gbh_get_stats(const gbh_engine *e, gbh_stats *st)
     return GBH_OK;
 }
 
+// The reverse sweep's groups and row order (AdjPlan), laid out at the first
+// gradient: groups for every SM, as many neurons each as that leaves and the
+// shared memory holds.
+static int adj_plan(gbh_engine *e, int hmax)
+{
+    if (e->adj_ngroups > 0) return GBH_OK;
+    const Decoded &dec = e->dec;
+    const int per = (int)std::min<size_t>(LANES, (dec.neurons.size() + kLevelGroups - 1) / kLevelGroups);
+    std::vector<std::vector<int>> cells_of(e->tiles.size());
+    for (size_t i = 0; i < dec.neurons.size(); ++i) {
+        const int t = e->neuron_tile[i];
+        cells_of[t].resize(e->tiles[t].nlanes, -1);
+        cells_of[t][e->neuron_lane[i]] = (int)i;
+    }
+    std::vector<AdjGroup> groups;
+    std::vector<int2> chunks, link;
+    std::vector<int> map;
+    int warps = 1;
+    size_t smem = 0;
+    for (size_t t = 0; t < e->tiles.size(); ++t) {
+        const Tile &tl = e->tiles[t];
+        const int S = e->types[tl.type].nslots;
+        auto need = [&](int cells) { return adj_reverse_smem(cells * S, cells * S / LANES + S + 1, S, hmax); };
+        int most = std::max(1, per);
+        while (most > 1 && need(most) > (size_t)kLevelSmemMax / 2) --most;
+        if (S > 0xffff || need(most) > (size_t)kLevelSmemMax)
+            return fail_err(nullptr, GBH_ERR_UNSUPPORTED,
+                            "gbh_loss_gradient: %d compartments per neuron exceed shared memory", S);
+        const int ng = (tl.nlanes + most - 1) / most;
+        for (int q = 0, l0 = 0; q < ng; ++q) {
+            const int nl = (tl.nlanes - l0 + (ng - q) - 1) / (ng - q);
+            std::vector<const Neuron *> cl;
+            for (int l = l0; l < l0 + nl; ++l) cl.push_back(&dec.neurons[cells_of[t][l]]);
+            const TreeOrder o = tree_order(cl, S);
+            const int w = std::min(ADJ_REV_THREADS / LANES, (nl * S + LANES - 1) / LANES);
+            AdjGroup g{(int)t, l0, nl, nl * S, 0, (int)chunks.size(), (int64_t)map.size()};
+            // (every block has the largest group's threads; chunks of this one's suffice)
+            g.nch = tree_chunks(o, w * LANES, chunks);
+            for (int x = 0; x < g.n; ++x) {
+                link.push_back(make_int2(o.kid[x] | o.nk[x] << 16, o.par[x]));
+                map.push_back(o.order[x] / nl * LANES + l0 + o.order[x] % nl);
+            }
+            groups.push_back(g);
+            warps = std::max(warps, w);
+            smem = std::max(smem, adj_reverse_smem(g.n, g.nch, S, hmax));
+            l0 += nl;
+        }
+    }
+    static_assert(RW_FIRST == ADJ_FIRST && RW_LAST == ADJ_LAST, "tree_chunks serves both");
+    if (e->d_agroups.upload(groups) || e->d_achunks.upload(chunks) || e->d_alink.upload(link) || e->d_amap.upload(map)) {
+        e->d_agroups.release(); e->d_achunks.release(); e->d_alink.release(); e->d_amap.release();
+        return GBH_ERR_CUDA;
+    }
+    e->adj_ngroups = (int)groups.size();
+    e->adj_warps = warps;
+    e->adj_smem = smem;
+    return GBH_OK;
+}
+
 int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh_loss_spec *spec,
                       double *loss, double *dchip, double *dravals, double *dvm0)
 {
@@ -3642,7 +3731,9 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
                         smax);
     int hmax = 0;   // channel plans cached in shared memory by the reverse kernel
     for (const AdjType &at : atypes) hmax = std::max(hmax, at.nchans);
-    while (hmax > 0 && adj_reverse_smem(smax, hmax) > 227 * 1024) hmax /= 2;
+    hmax = std::min(hmax, 1024);
+    const int rc_plan = adj_plan(e, hmax);
+    if (rc_plan) return rc_plan;
     // ---- device buffers (released on every return path) ----
     struct Bufs {
         DBuf<double> P, V, ck, tape, tape2, Vb, Xb, Gf, Gek, Ggm, GA, GB, GC, trace, loss;
@@ -3686,7 +3777,7 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
     if ((!keep && b.ck.alloc((size_t)nseg * ck_stride * L)) || b.P.alloc(nfld) || b.V.alloc(nvm) ||
         b.tape.alloc((size_t)K * tp_stride * L) || b.Vb.alloc(nvm) || b.Xb.alloc(xb_rows * L) ||
         b.Gf.alloc(nfld) || b.Gek.alloc(ch_rows * L) || b.Ggm.alloc(ch_rows * L) || b.GA.alloc(ntopo) ||
-        b.GB.alloc(ntopo) || b.GC.alloc(ntopo) || b.loss.alloc((size_t)ntiles * L) ||
+        b.GB.alloc(ntopo) || b.GC.alloc(ntopo) || b.loss.alloc(ntopo) ||
         b.trace.alloc(std::max<size_t>(1, (size_t)nsteps * spec->ntargets)))
         return GBH_ERR_CUDA;
     if (b.tgt.upload(tgt) || b.snap.upload(snap_field) || b.ck_off.upload(ck_off) || b.tp_off.upload(tp_off) ||
@@ -3708,7 +3799,7 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
     CK(cudaMemsetAsync(b.GA.p, 0, ntopo * sizeof(double), st));
     CK(cudaMemsetAsync(b.GB.p, 0, ntopo * sizeof(double), st));
     CK(cudaMemsetAsync(b.GC.p, 0, ntopo * sizeof(double), st));
-    CK(cudaMemsetAsync(b.loss.p, 0, (size_t)ntiles * L * sizeof(double), st));
+    CK(cudaMemsetAsync(b.loss.p, 0, ntopo * sizeof(double), st));
     AdjView v{};
     v.tiles = e->d_tiles.p;
     v.types = e->d_types.p;
@@ -3747,6 +3838,11 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
     v.ntargets = spec->ntargets;
     v.loss = b.loss.p;
     v.status = e->d_status.p;
+    AdjPlan pl;
+    pl.groups = e->d_agroups.p;
+    pl.chunks = e->d_achunks.p;
+    pl.link = e->d_alink.p;
+    pl.map = e->d_amap.p;
     // the engine's own FP64 step kernels advance the work copies
     DevView fv = view_of(e);
     fv.P = b.P.p;
@@ -3821,7 +3917,8 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
         CK(cudaEventRecord(b.ev_tape[buf], st));
         CK(cudaStreamWaitEvent(b.ast, b.ev_tape[buf], 0));
         if (!keep && ck_launch(launch_adj_linearize(w, ntiles, smax, nk, b.ast))) return GBH_ERR_CUDA;
-        if (ck_launch(launch_adj_reverse(w, ntiles, smax, hmax, nk, seg * K, b.ast))) return GBH_ERR_CUDA;
+        if (ck_launch(launch_adj_reverse(w, pl, e->adj_ngroups, e->adj_warps, e->adj_smem, hmax, nk, seg * K, b.ast)))
+            return GBH_ERR_CUDA;
         if (ck_launch(launch_adj_reduce(w, ntiles, smax, nk, b.ast))) return GBH_ERR_CUDA;
         CK(cudaEventRecord(b.ev_done[buf], b.ast));
     }
@@ -3845,7 +3942,7 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
     }
     // ---- gather ----
     std::vector<double> Vb(nvm), Xb(xb_rows * L), Gf(nfld), Gek(ch_rows * L), Ggm(ch_rows * L), GA(ntopo),
-        GB(ntopo), GC(ntopo), ls((size_t)ntiles * L);
+        GB(ntopo), GC(ntopo), ls(ntopo);
     auto down = [&](std::vector<double> &h, const DBuf<double> &d) {
         if (h.empty()) return GBH_OK;
         CK(cudaMemcpy(h.data(), d.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost));
@@ -3855,9 +3952,13 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
         down(GA, b.GA) || down(GB, b.GB) || down(GC, b.GC) || down(ls, b.loss))
         return GBH_ERR_CUDA;
     if (loss) {
-        double sum = 0.0;
+        double sum = 0.0;   // neuron by neuron, rows ascending
         for (int t = 0; t < ntiles; ++t)
-            for (int l = 0; l < e->tiles[t].nlanes; ++l) sum += ls[(size_t)t * L + l];
+            for (int l = 0; l < e->tiles[t].nlanes; ++l)
+                for (int s = 0; s < e->types[e->tiles[t].type].nslots; ++s) {
+                    const int64_t i = (e->tiles[t].topo + s) * L + l;
+                    if (tgt[i] >= 0) sum += ls[i];
+                }
         *loss = sum;
     }
     if (dchip) memset(dchip, 0, e->chip_start.back() * sizeof(double));
@@ -3913,6 +4014,7 @@ void gbh_destroy(gbh_engine *e)
     e->d_tout_start.release(); e->d_tout_off.release(); e->d_tout_idx.release();
     e->d_out_vals.release(); e->d_out_addr.release();
     e->d_vm_at.release(); e->d_vm_out.release();
+    e->d_agroups.release(); e->d_achunks.release(); e->d_alink.release(); e->d_amap.release();
     drop_graphs(e);
     if (e->cap_stream) cudaStreamDestroy(e->cap_stream);
     for (cudaStream_t x : {e->io_stream, e->io_out_stream})

@@ -243,6 +243,18 @@ def test_gradient_one_solver_many_trees(oracle, gpu_engine):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,ncomp,method", [(33, 5, model.BEULER), (2, 65, model.CRANK), (1, 2, model.CRANK),
+                                            (5, 32, model.BEULER)])
+def test_gradient_row_order_edges(oracle, gpu_engine, n, ncomp, method):
+    """The reverse sweep by depth: a second tile of one neuron, rows just past
+    a warp's, two rows, exactly a warp; every row a target in the last
+    neuron, over several segments (25 steps of 8)."""
+    _, _, hs = _trees(n, ncomp, seed=31 + n, method=method)
+    rows = [[h.ncompts - 1] for h in hs[:-1]] + [list(range(hs[-1].ncompts))]
+    _engine_vs_reference(oracle, gpu_engine, hs, rows, 25, checkpoint_every=8)
+
+
+@pytest.mark.gpu
 def test_checkpoint_interval_invariance_and_state(oracle, gpu_engine):
     trees, _, hs = _trees(40, 16, seed=25)
     nsteps = 600
