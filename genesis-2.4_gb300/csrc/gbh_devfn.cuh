@@ -125,24 +125,47 @@ __device__ __forceinline__ void prefetch_l1(const void *p)
 
 // One synaptic event, counted in the target synchan's ring slot for the step
 // it acts in; for a weighted synchan also its synapse's rank bit.
-__device__ __forceinline__ void put_event(unsigned *ring, int ring_len, unsigned *wmask, int64_t base, int delay,
-                                          int64_t mword, int mbit, long long step)
+// step % ring_len (the 64-bit remainder is a call of some 100 instructions)
+__device__ __forceinline__ int ring_phase(long long step, int ring_len)
 {
-    const int slot = (int)((step + delay) % ring_len);
+    return (unsigned long long)step >> 32 ? (int)(step % ring_len) : (int)((unsigned)step % (unsigned)ring_len);
+}
+
+// One event, `delay` steps (less than ring_len) after the step at `phase`.
+__device__ __forceinline__ void put_event(unsigned *ring, int ring_len, unsigned *wmask, int64_t base, int delay,
+                                          int64_t mword, int mbit, int phase)
+{
+    int slot = phase + delay;
+    if (slot >= ring_len) slot -= ring_len;
     atomicAdd(&ring[base + (int64_t)slot * LANES], 1u);
     if (mword >= 0) atomicOr(&wmask[mword + (int64_t)slot * (mbit >> 5)], 1u << (mbit & 31));
 }
 
-// h_dospike_event (hines_conn.c:44-58): an event on every synapse of the
-// neuron, counted as a spike.
-__device__ __forceinline__ void deliver_spike(const DevView &v, int64_t neuron, long long step)
+// h_dospike_event (hines_conn.c:44-58): an event on every synapse of each
+// neuron that fires, counted as a spike. The calling warp's lanes share the
+// synapses of one firing neuron after another: the events only count and set
+// bits, so their order does not matter, and a step waits for its slowest tile
+// (4,000 point neurons of 80 synapses: 10.7 -> 8.5 us a step).
+__device__ __forceinline__ void deliver_spikes(const DevView &v, bool fires, int64_t neuron, long long step)
 {
-    const int64_t e0 = v.syn_out_start[neuron], e1 = v.syn_out_start[neuron + 1];
-    for (int64_t e = e0; e < e1; ++e)
-        put_event(v.ring, v.ring_len, v.wmask, v.syn_out_base[e], v.syn_out_delay[e],
-                  v.syn_out_mword ? v.syn_out_mword[e] : -1, v.syn_out_mbit ? v.syn_out_mbit[e] : 0, step);
-    v.spikes[neuron] += 1ULL;
-    if (v.spiked) atomicOr(&v.spiked[neuron >> 5], 1u << (neuron & 31));
+    const unsigned with = __activemask();
+    unsigned left = __ballot_sync(with, fires);
+    if (!left) return;
+    if (fires) {
+        v.spikes[neuron] += 1ULL;
+        if (v.spiked) atomicOr(&v.spiked[neuron >> 5], 1u << (neuron & 31));
+    }
+    const int lane = (int)((threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & 31u);
+    const int rank = __popc(with & ((1u << lane) - 1u)), share = __popc(with);
+    const int phase = ring_phase(step, v.ring_len);
+    while (left) {
+        const int64_t n = __shfl_sync(with, (long long)neuron, __ffs(left) - 1);
+        left &= left - 1;
+        const int64_t e1 = v.syn_out_start[n + 1];
+        for (int64_t e = v.syn_out_start[n] + rank; e < e1; e += share)
+            put_event(v.ring, v.ring_len, v.wmask, v.syn_out_base[e], v.syn_out_delay[e],
+                      v.syn_out_mword ? v.syn_out_mword[e] : -1, v.syn_out_mbit ? v.syn_out_mbit[e] : 0, phase);
+    }
 }
 
 // SPIKE_OP (hines_chip.c:266-276): the refractory counter counts down every
@@ -152,10 +175,9 @@ __device__ __forceinline__ int spike_op(const DevView &v, double Vm, double thre
                                         bool active, int64_t neuron, long long step)
 {
     cnt -= 1;
-    if (Vm > thresh && cnt <= 0 && active) {
-        deliver_spike(v, neuron, step);
-        cnt = refract;
-    }
+    const bool fires = Vm > thresh && cnt <= 0 && active;
+    if (fires) cnt = refract;
+    deliver_spikes(v, fires, neuron, step);
     return cnt;
 }
 
@@ -177,7 +199,7 @@ __device__ __forceinline__ bool syn_due(const DevView &v, unsigned *cell, double
         for (unsigned q = 0; q < n; ++q) act += w_dt;
     } else {
         const SynW d = v.synw[(int64_t)(-w_dt) - 1];
-        unsigned *m = v.wmask + d.mbase + (int64_t)(step % v.ring_len) * d.nwords;
+        unsigned *m = v.wmask + d.mbase + (int64_t)ring_phase(step, v.ring_len) * d.nwords;
         const double *w = v.wval + d.wbase;
         for (int k = 0; k < d.nwords; ++k) {
             unsigned b = m[k];

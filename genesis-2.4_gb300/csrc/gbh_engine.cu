@@ -2458,8 +2458,9 @@ __global__ void k_deliver_remote(const unsigned char *bits, int n, const int64_t
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || !(bits[i >> 3] & (1u << (i & 7)))) return;
+    const int phase = ring_phase(step, ring_len);
     for (int64_t k = start[i]; k < start[i + 1]; ++k)
-        put_event(ring, ring_len, wmask, base[k], delay[k], mword ? mword[k] : -1, mbit ? mbit[k] : 0, step);
+        put_event(ring, ring_len, wmask, base[k], delay[k], mword ? mword[k] : -1, mbit ? mbit[k] : 0, phase);
 }
 
 // Spike detection of every neuron with a spike detector, before the step's

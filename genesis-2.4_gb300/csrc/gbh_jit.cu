@@ -378,7 +378,7 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                           << fx << "; if (syn3_uniform(key) <= " << E.P(ff) << ") *px += sl[3]; }\n";
                     o << "        double X = *px * sl[0];\n"
                       << "        unsigned *cell = v.ring + ((tl.syn + (int64_t)" << srow
-                      << " * v.ring_len + (int64_t)(step % v.ring_len)) * 32 + lane);\n"
+                      << " * v.ring_len + ring_phase(step, v.ring_len)) * 32 + lane);\n"
                       << "        { double act; if (syn_due(v, cell, " << E.P(fw) << ", step, act)) X += v.dt * act * sl[3]; }\n"
                       << "        *px = X; const double Y = X * sl[1] + *py * sl[2]; *py = Y;";
                     if (mx) o << " Gk = df_mul(Gk, d2df(Y)); }\n";

@@ -285,7 +285,7 @@ __device__ __forceinline__ bool chan_compartment(const DevView &v, const ChanEnv
                     }
                     double X = *px * sl[0];
                     unsigned *cell = N.ring + ((int64_t)pc[3] * v.ring_len +
-                                               (int64_t)(step % v.ring_len)) * LANES;
+                                               ring_phase(step, v.ring_len)) * LANES;
                     double act;
                     if (syn_due(v, cell, N.P[(pc[6]) * STR], step, act)) X += v.dt * act * sl[3];
                     *px = X;

@@ -245,7 +245,7 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
                         if (syn3_uniform(key) <= N.P[(pc[1]) * STR]) *px += sl[3];
                     }
                     double X = *px * sl[0];
-                    unsigned *cell = N.ring + ((int64_t)pc[3] * v.ring_len + (int64_t)(step % v.ring_len)) * LANES;
+                    unsigned *cell = N.ring + ((int64_t)pc[3] * v.ring_len + ring_phase(step, v.ring_len)) * LANES;
                     double act;
                     if (syn_due(v, cell, N.P[(pc[6]) * STR], step, act)) X += v.dt * act * sl[3];
                     *px = X;

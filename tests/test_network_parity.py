@@ -43,6 +43,25 @@ def test_network_spikes_and_vm_bitwise(oracle, gpu_engine, jit):
     np.testing.assert_array_equal(vm, np.concatenate([s.vm for s in solvers]))
 
 
+@pytest.mark.parametrize("n,p", [(65, 0.02), (33, 0.97), (40, 1.0)])
+@pytest.mark.parametrize("jit,K", [(True, 1), (False, 1), (True, -16), (False, -16)])
+def test_network_synchronous_spikes(oracle, gpu_engine, n, p, jit, K):
+    """Whole tiles fire in the same step (the same current into every cell),
+    with one synapse, about a warp's worth and more than a warp's per neuron:
+    the lanes share each other's synapses. Bit for bit, per-step and
+    cooperative launches, specialised and interpreted."""
+    hs, esyn, child = _network(n, p, seed=13, inject=np.full(n, 0.2e-9))
+    eng = gpu_engine.Engine(hs, synapses=esyn, jit=jit, steps_per_launch=K)
+    assert eng.stats().cooperative == (K < 0)
+    for m in (517, 300):
+        eng.run(m)
+    solvers, ref_spikes = _oracle_net(oracle, hs, esyn, child, 817)
+    assert ref_spikes.any()
+    np.testing.assert_array_equal(eng.spike_counts(), ref_spikes)
+    np.testing.assert_array_equal(eng.vm(), np.concatenate([s.vm for s in solvers]))
+    eng.close()
+
+
 def test_network_longer_delays(oracle, gpu_engine):
     rng = np.random.default_rng(4)
     n = 60
