@@ -1943,7 +1943,7 @@ int launch_one(gbh_engine *e, const DevView &v, const Launch &L, int k, long lon
         const bool cols = !L.uniform || e->jit_compact[e->jit_choice] || e->jit_smemrows[e->jit_choice];
         const int warps = e->jit_warps[e->jit_choice];
         const size_t smem = cols ? (size_t)warps * 2 * L.smax * LANES * sizeof(double) : 0;
-        const cudaError_t je = jit_launch(e->jits[L.jit], v, L.tile0, L.tile1, L.smax, warps, k, step, smem, st);
+        const cudaError_t je = jit_launch(e->jits[L.jit], v, L.tile0, L.tile1, L.smax, warps, k, step, smem, false, st);
         if (je != cudaSuccess) {
             set_last("specialised kernel launch failed: %s", cudaGetErrorString(je));
             return GBH_ERR_CUDA;
@@ -2139,8 +2139,15 @@ int run_graph(gbh_engine *e, int nsteps, cudaStream_t st)
     return GBH_OK;
 }
 
-// Networks: K steps per cooperative launch of the interpreting kernel over
-// every tile, a grid barrier between steps (events cross tiles).
+// Steps of a run from which a chosen cooperative plan is used: its launch and
+// the reset of the barrier's words cost more than they save below (4,000 point
+// neurons, us a run, per-step launches against cooperative: 4 steps 55.4 and
+// 56.4, 6 steps 73.1 and 72.4, 8 steps 90.9 and 89.3, 64 steps 580 and 528).
+constexpr int kCoopMin = 6;
+
+// Networks: K steps per cooperative launch over every tile, a grid barrier
+// between steps (events cross tiles): the specialised kernel where one serves
+// every tile, a warp per block, else the interpreting one.
 int run_coop(gbh_engine *e, int nsteps, cudaStream_t st)
 {
     DevView v = view_of(e);
@@ -2148,11 +2155,17 @@ int run_coop(gbh_engine *e, int nsteps, cudaStream_t st)
     const bool mixed = e->opt.precision == GBH_PREC_MIXED;
     int smax = 1;
     for (const TileType &tt : e->types) smax = std::max(smax, tt.nslots);
+    const int jit = e->launches.size() == 1 ? e->launches[0].jit : -1;
+    const bool cols = jit >= 0 && (!e->launches[0].uniform || e->jit_compact[e->jit_choice] ||
+                                   e->jit_smemrows[e->jit_choice]);
     for (int done = 0; done < nsteps;) {
         const int k = std::min(e->net_spl, nsteps - done);
         CK(cudaMemsetAsync(e->d_gbar.p, 0, 3 * sizeof(unsigned), st));
-        const cudaError_t ce = mixed ? launch_mixed_coop(v, (int)e->tiles.size(), smax, k, e->step, st)
-                                     : launch_fp64_coop(v, (int)e->tiles.size(), smax, k, e->step, st);
+        const cudaError_t ce =
+            jit >= 0 ? jit_launch(e->jits[jit], v, 0, (int)e->tiles.size(), smax, 1, k, e->step,
+                                  cols ? (size_t)2 * smax * LANES * sizeof(double) : 0, true, st)
+            : mixed ? launch_mixed_coop(v, (int)e->tiles.size(), smax, k, e->step, st)
+                    : launch_fp64_coop(v, (int)e->tiles.size(), smax, k, e->step, st);
         if (ce != cudaSuccess) {
             set_last("cooperative launch failed: %s", cudaGetErrorString(ce));
             return GBH_ERR_CUDA;
@@ -2182,7 +2195,8 @@ int run_steps(gbh_engine *e, int nsteps, cudaStream_t st)
         const int rci = stack_invalidate(e, st);
         if (rci) return rci;
     }
-    if (e->net_coop && !e->givals_enabled && e->nremote == 0) {
+    if (e->net_coop && !e->givals_enabled && e->nremote == 0 &&
+        (nsteps >= kCoopMin || e->opt.steps_per_launch < 0)) {
         e->dstep_valid = false;
         return run_coop(e, nsteps, st);
     }
@@ -2334,6 +2348,8 @@ int autotune_trials(gbh_engine *e)
             float ms = 0.f;
             if (rc_c == GBH_OK && se == cudaSuccess && cudaEventElapsedTime(&ms, e->ev0, e->ev1) == cudaSuccess) {
                 const double per = ms / steps;
+                if (getenv("GBH_VERBOSE"))
+                    fprintf(stderr, "gbhsolve: trial cooperative, %d steps/launch: %.2f us/step\n", K, per * 1e3);
                 if (per < best) { best = per; coop_k = K; }
             } else {
                 cudaGetLastError();   // e.g. too many tiles to be resident at once: keep per-step launches

@@ -52,6 +52,8 @@ struct Api {
     CUresult (*getfn)(CUfunction *, CUmodule, const char *) = nullptr;
     CUresult (*launch)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
                        CUstream, void **, void **) = nullptr;
+    CUresult (*launch_coop)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
+                            CUstream, void **) = nullptr;
     CUresult (*setattr)(CUfunction, CUfunction_attribute, int) = nullptr;
     CUresult (*unload)(CUmodule) = nullptr;
 };
@@ -94,7 +96,8 @@ void init_api()
               sym(h, "nvrtcGetCUBINSize", g_api.cubinsize) && sym(h, "nvrtcGetCUBIN", g_api.getcubin) &&
               sym(h, "nvrtcDestroyProgram", g_api.destroy);
     ok = ok && drv("cuModuleLoadData", g_api.load) && drv("cuModuleGetFunction", g_api.getfn) &&
-         drv("cuLaunchKernel", g_api.launch) && drv("cuFuncSetAttribute", g_api.setattr) &&
+         drv("cuLaunchKernel", g_api.launch) && drv("cuLaunchCooperativeKernel", g_api.launch_coop) &&
+         drv("cuFuncSetAttribute", g_api.setattr) &&
          drv("cuModuleUnload", g_api.unload);
     if (!ok) {
         g_api.why = "NVRTC or driver entry points missing";
@@ -838,6 +841,8 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
     t << "    if (v.io_out) {   // this step's outputs\n"
       << "      __syncwarp(); double *dst = v.io_out + (step - v.io_step0) * v.io_nout; const double *Vt = v.V + tl.vm * 32;\n"
       << "      for (int q = v.tout_start[t] + lane; q < v.tout_start[t + 1]; q += 32) dst[v.tout_idx[q]] = Vt[v.tout_off[q]]; }\n";
+    // networks, several steps in a cooperative launch: events cross tiles
+    if (tt.nsyn > 0 || tt.has_spike) t << "    if (v.gbar && !grid_sync(v.gbar, gridDim.x, v.status)) return;\n";
     t << "  }\n}\n";
     return t.str();
 }
@@ -1245,7 +1250,7 @@ int jit_compile(const std::string &src, bool fp64_exact, int device_major, int d
 }
 
 cudaError_t jit_launch(const JitKernel &k, const DevView &v, int tile0, int tile1, int smax, int warps, int nsteps,
-                       long long step, size_t smem, cudaStream_t st)
+                       long long step, size_t smem, bool coop, cudaStream_t st)
 {
     const int ntiles = tile1 - tile0;
     const int blocks = (ntiles + warps - 1) / warps;
@@ -1255,8 +1260,10 @@ cudaError_t jit_launch(const JitKernel &k, const DevView &v, int tile0, int tile
     }
     DevView vv = v;
     void *args[] = {&vv, &tile0, &tile1, &smax, &nsteps, &step};
-    const CUresult r = g_api.launch((CUfunction)k.fn, blocks, 1, 1, warps * LANES, 1, 1, (unsigned)smem,
-                                    (CUstream)st, args, nullptr);
+    const CUresult r =
+        coop ? g_api.launch_coop((CUfunction)k.fn, blocks, 1, 1, warps * LANES, 1, 1, (unsigned)smem, (CUstream)st, args)
+             : g_api.launch((CUfunction)k.fn, blocks, 1, 1, warps * LANES, 1, 1, (unsigned)smem, (CUstream)st, args,
+                            nullptr);
     if (r == CUDA_SUCCESS) return cudaSuccess;
     // a fault of earlier work stays a launch failure; a launch this device
     // refuses (resources, shared memory) is a configuration error

@@ -68,7 +68,7 @@ bool jit_available(std::string *why);
 int jit_compile(const std::string &src, bool fp64_exact, int device_major, int device_minor, JitKernel *out,
                 std::string *log);
 cudaError_t jit_launch(const JitKernel &k, const DevView &v, int tile0, int tile1, int smax, int warps, int nsteps,
-                       long long step, size_t smem, cudaStream_t st);
+                       long long step, size_t smem, bool coop, cudaStream_t st);
 void jit_release(JitKernel &k);
 
 }  // namespace gbh
