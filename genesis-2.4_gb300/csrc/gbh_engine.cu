@@ -1,5 +1,6 @@
 // gbh_engine.cu -- the GB300 hsolve engine: tile layout, device memory,
 // launches, and the C ABI declared in include/gbhsolve.h.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -2751,20 +2752,61 @@ int gbh_get_outputs_async(gbh_engine *e, double *host_values, void *stream)
     return GBH_OK;
 }
 
-// Issues the deferred output copy of the previous call together with this
-// call's input scatter (in_buf < 0: no input).
-static int io_between(gbh_engine *e, cudaStream_t st, int in_buf)
+// The device's view of n doubles of pinned host memory (all of it in one
+// allocation or registration), or null: what k_io reads and writes itself, in
+// place of two copies, three events and two waits of the host's a call. Up to
+// kIoDirect values: further on the copies' overlap with the steps is worth
+// more (us a call, staged and direct: 512 cells 17.7 and 12.3, 16,384 25.3 and
+// 13.6, 65,536 29.8 and 22.9; with 16 compartments each 32,768 27.3 and 24.3,
+// with 8 each 65,536 30.4 and 31.4).
+constexpr int64_t kIoDirect = 32768;
+
+static double *pinned_view(const double *p, int64_t n)
+{
+    using Fn = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const Fn query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 13000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<Fn>(f);
+    }();
+    if (!query || n <= 0 || n > kIoDirect) return nullptr;
+    unsigned type = 0, managed = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[] = {&type, &managed, &dev, &start, &size};
+    const CUdeviceptr at = (CUdeviceptr)(uintptr_t)p;
+    if (at % sizeof(double) || query(5, what, to, at) != CUDA_SUCCESS) return nullptr;
+    if (type != CU_MEMORYTYPE_HOST || managed || !dev || dev % sizeof(double)) return nullptr;
+    // the range is given by its address on the device
+    if (dev < start || dev + n * sizeof(double) > start + size) return nullptr;
+    return reinterpret_cast<double *>(dev);
+}
+
+// Issues the deferred outputs of the previous call together with this call's
+// input scatter (in_vals null: no input). Outputs into pinned memory are
+// written there by the gather; others go through the staging buffer.
+static int io_between(gbh_engine *e, cudaStream_t st, const double *in_vals)
 {
     const bool out = e->io_pend_host != nullptr;
-    const int n_tg = in_buf >= 0 ? e->n_tgt : 0;
+    const int n_tg = in_vals ? e->n_tgt : 0;
     const int n_out = out ? e->n_out : 0;
     const int n = std::max(n_tg, n_out);
     if (n == 0) return GBH_OK;
-    k_io<<<(n + 255) / 256, 256, 0, st>>>(e->d_V.p, e->d_out_addr.p, n_out, out ? e->d_io_out[e->io_pend_buf].p : nullptr,
-                                          in_buf >= 0 ? e->d_io_in[in_buf].p : nullptr, in_plan(e), e->d_P.p,
-                                          e->d_F.p);
+    double *direct = out ? pinned_view(e->io_pend_host, e->n_out) : nullptr;
+    k_io<<<(n + 255) / 256, 256, 0, st>>>(e->d_V.p, e->d_out_addr.p, n_out,
+                                          !out ? nullptr : direct ? direct : e->d_io_out[e->io_pend_buf].p, in_vals,
+                                          in_plan(e), e->d_P.p, e->d_F.p);
     CK(cudaGetLastError());
-    if (out) {
+    if (direct) {
+        CK(cudaEventRecord(e->io_out_copied[e->io_pend_buf], st));
+        e->io_pend_host = nullptr;
+    } else if (out) {
         const int pb = e->io_pend_buf;
         CK(cudaEventRecord(e->io_gathered[pb], st));
         CK(cudaStreamWaitEvent(e->io_out_stream, e->io_gathered[pb], 0));
@@ -2804,14 +2846,14 @@ int gbh_step_io(gbh_engine *e, const double *host_in, double *host_out, int nste
     const int b = (int)(e->io_calls & 1);
     // the buffers of the call before last are free once its output copy is done
     if (e->io_calls >= 2) CK(cudaEventSynchronize(e->io_out_copied[b]));
-    int in_buf = -1;
-    if (e->n_in && host_in) {
+    const double *in_vals = nullptr;
+    if (e->n_in && host_in && !(in_vals = pinned_view(host_in, e->n_in))) {
         CK(cudaMemcpyAsync(e->d_io_in[b].p, host_in, e->n_in * sizeof(double), cudaMemcpyHostToDevice, e->io_stream));
         CK(cudaEventRecord(e->io_in_copied[b], e->io_stream));
         CK(cudaStreamWaitEvent(st, e->io_in_copied[b], 0));
-        in_buf = b;
+        in_vals = e->d_io_in[b].p;
     }
-    int rc = io_between(e, st, in_buf);
+    int rc = io_between(e, st, in_vals);
     if (rc) return rc;
     if (nsteps > 0) {
         rc = run_steps(e, nsteps, st);
@@ -2949,7 +2991,7 @@ int gbh_io_sync(gbh_engine *e)
 {
     if (!e) return GBH_ERR_ARG;
     if (e->io_pend_host) {
-        const int rc = io_between(e, e->io_pend_stream, -1);
+        const int rc = io_between(e, e->io_pend_stream, nullptr);
         if (rc) return rc;
     }
     if (e->io_stream) CK(cudaStreamSynchronize(e->io_stream));

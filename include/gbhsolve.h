@@ -337,8 +337,10 @@ int gbh_get_outputs_async(gbh_engine *e, double *host_values, void *stream);
  * for overlap) are copied to the device on the engine's copy stream while
  * earlier work runs, scattered and stepped (nsteps steps) on `stream` (NULL
  * = the engine's stream), and the registered outputs are gathered and copied
- * to host_out on the copy stream while the next call's step runs. Device
- * staging is double-buffered: the buffers passed to a call may be reused,
+ * to host_out on the copy stream while the next call's step runs. Pinned
+ * buffers of up to 32,768 values are read and written by the scatter and
+ * gather kernel itself, without the copies. Device staging is
+ * double-buffered: the buffers passed to a call may be reused,
  * and its host_out is complete, once the second following call has
  * returned, or after gbh_io_sync. Either pointer may be NULL. Results equal
  * gbh_set_inputs_async + gbh_run_async + gbh_get_outputs_async. No

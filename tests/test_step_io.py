@@ -55,6 +55,42 @@ def test_step_io_matches_plain_calls(gpu_engine, pinned):
         e.close()
 
 
+@pytest.mark.parametrize("n", [1, 32767, 32768, 32769])
+def test_step_io_direct_buffers(gpu_engine, n):
+    """Pinned buffers either side of the size up to which the kernels read and
+    write them directly, at odd offsets into one allocation, input and output
+    of a call in the same buffer: equal to the staged form, and nothing around
+    the buffers is written."""
+    import torch
+    hs, _ = configs.cables_replicated(n, ncomp=2, seed=9)
+    slot = configs.inject_slot(hs[0])
+    soma = hs[0].ncompts - 1
+    inputs = np.random.default_rng(1).uniform(0.0, 0.6e-9, size=(7, n))
+    block = torch.full((3 * (n + 3),), 7.0, dtype=torch.float64, pin_memory=True).numpy()
+    pinned = [block[i * (n + 3) + 1:i * (n + 3) + 1 + n] for i in range(3)]
+    plain = [np.empty(n) for _ in range(3)]
+    got = []
+    for bufs in (pinned, plain):
+        e = gpu_engine.Engine(hs, steps_per_launch=1)
+        e.register_inputs(np.arange(n, dtype=np.int32), np.full(n, slot, dtype=np.int64))
+        e.register_outputs(np.arange(n, dtype=np.int32), np.full(n, soma, dtype=np.int32))
+        out = []
+        for k in range(7):
+            bufs[k % 3][:] = inputs[k]
+            e.step_io(bufs[k % 3], bufs[k % 3], 1)
+            if k >= 2:
+                out.append(bufs[(k - 2) % 3].copy())
+        e.io_sync()
+        got.append((np.array(out + [bufs[5 % 3].copy(), bufs[6 % 3].copy()]), e.vm()))
+        e.close()
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    np.testing.assert_array_equal(got[0][1], got[1][1])
+    rest = np.ones(len(block), dtype=bool)
+    for i in range(3):
+        rest[i * (n + 3) + 1:i * (n + 3) + 1 + n] = False
+    assert (block[rest] == 7.0).all()
+
+
 @pytest.mark.parametrize("block,pinned", [(0, True), (7, False), (1, True), (64, True)])
 def test_run_io_matches_plain_calls(gpu_engine, block, pinned):
     """gbh_run_io streams a whole run's per-step inputs and outputs in blocks
