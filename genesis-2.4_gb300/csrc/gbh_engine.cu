@@ -2276,31 +2276,45 @@ int autotune_trials(gbh_engine *e)
     };
     double best = 1e300;
     int best_v = 0, best_s = spls[0];
-    // time per step of the plan and variant in use, from the saved state
+    // time per step of the plan and variant in use, from the saved state; one
+    // whose first steps take twice the best so far is not timed further
     auto timed = [&](int spl, double &per) {
         e->steps_per_launch = spl;
-        const int steps = std::max(2 * spl, 128);
-        int rc_t = run_steps(e, 8, e->stream);   // warm caches and clocks
-        CK(cudaEventRecord(e->ev0, e->stream));
-        if (rc_t == GBH_OK) rc_t = run_steps(e, steps, e->stream);
-        CK(cudaEventRecord(e->ev1, e->stream));
-        CK(cudaEventSynchronize(e->ev1));
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
-        // a variant that cannot launch here (resources) never wins
-        per = rc_t == GBH_OK ? ms / steps : 1e300;
-        if (rc_t != GBH_OK) cudaGetLastError();
+        int rc_t = run_steps(e, 2, e->stream);   // warm caches and clocks
+        for (int steps : {8, std::max(2 * spl, 128)}) {
+            CK(cudaEventRecord(e->ev0, e->stream));
+            if (rc_t == GBH_OK) rc_t = run_steps(e, steps, e->stream);
+            CK(cudaEventRecord(e->ev1, e->stream));
+            CK(cudaEventSynchronize(e->ev1));
+            float ms = 0.f;
+            CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
+            // a variant that cannot launch here (resources) never wins
+            per = rc_t == GBH_OK ? ms / steps : 1e300;
+            if (rc_t != GBH_OK) cudaGetLastError();
+            if (per > 2.0 * best) break;
+        }
         return restore();
     };
     auto use_variant = [&](int vi) {
         for (size_t k = 0; k < e->jits.size(); ++k) e->jits[k] = e->jit_var[k][vi];
         e->jit_choice = vi;   // launch_one sizes the shared memory of the variant in use
     };
-    // every variant at the middle launch length, then the row-parallel plan of
-    // a small batch, then the other launch lengths of the fastest: the length
+    // the row-parallel plan of a small batch and every variant at the middle
+    // launch length, then the other launch lengths of the fastest: the length
     // moves a step by a few per cent, the same way in every variant
     const int mid = spls[spls.size() / 2];
     bool use_rows = false;
+    if (!e->rows_launches.empty()) {
+        e->launches.swap(e->rows_launches);
+        double per;
+        if (timed(mid, per)) return GBH_ERR_CUDA;
+        if (getenv("GBH_VERBOSE"))
+            fprintf(stderr, "gbhsolve: trial row-parallel, %d steps/launch: %.2f us/step\n", mid, per * 1e3);
+        e->launches.swap(e->rows_launches);
+        use_rows = per < best;
+        if (use_rows) best = per;
+        best_s = mid;
+    }
     for (int vi = 0; vi < nvar; ++vi) {
         use_variant(vi);
         double per;
@@ -2309,19 +2323,10 @@ int autotune_trials(gbh_engine *e)
             fprintf(stderr, "gbhsolve: trial %d warps x min blocks %d, form %d, %d steps/launch: %.2f us/step\n",
                     e->jit_warps[vi], e->jit_minb[vi], e->jit_compact[vi] ? 1 : e->jit_smemrows[vi] ? 2 : 0, mid,
                     per * 1e3);
-        if (per < best) { best = per; best_v = vi; best_s = mid; }
+        if (per < best) { best = per; best_v = vi; best_s = mid; use_rows = false; }
     }
     use_variant(best_v);
-    if (!e->rows_launches.empty()) {
-        e->launches.swap(e->rows_launches);
-        double per;
-        if (timed(mid, per)) return GBH_ERR_CUDA;
-        if (getenv("GBH_VERBOSE"))
-            fprintf(stderr, "gbhsolve: trial row-parallel, %d steps/launch: %.2f us/step\n", mid, per * 1e3);
-        use_rows = per < best;
-        if (use_rows) best = per;
-        else e->launches.swap(e->rows_launches);
-    }
+    if (use_rows) e->launches.swap(e->rows_launches);
     for (int spl : spls) {
         if (spl == mid) continue;
         double per;
