@@ -3755,19 +3755,25 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
     // ---- target rows ----
     std::vector<int> tgt(e->rows_topo * L, -1);
     {
-        std::unordered_map<int64_t, int> at;   // (solver, row) -> neuron
-        for (size_t i = 0; i < e->dec.neurons.size(); ++i) {
-            const Neuron &N = e->dec.neurons[i];
-            for (int s = 0; s < N.nrows; ++s) at[(int64_t)N.solver * (1LL << 32) + N.row0 + s] = (int)i;
-        }
+        // neurons by solver and first row: a target's is the last at or before it
+        const std::vector<Neuron> &ns = e->dec.neurons;
+        std::vector<int> by(ns.size());
+        for (size_t i = 0; i < by.size(); ++i) by[i] = (int)i;
+        auto before = [&](int x, int y) {
+            return ns[x].solver != ns[y].solver ? ns[x].solver < ns[y].solver : ns[x].row0 < ns[y].row0;
+        };
+        if (!std::is_sorted(by.begin(), by.end(), before)) std::sort(by.begin(), by.end(), before);
         for (int j = 0; j < spec->ntargets; ++j) {
-            auto it = at.find((int64_t)spec->solver[j] * (1LL << 32) + spec->row[j]);
-            if (it == at.end())
-                return fail_err(nullptr, GBH_ERR_ARG, "target %d: solver %d has no row %d", j, spec->solver[j],
-                                spec->row[j]);
-            const Neuron &N = e->dec.neurons[it->second];
-            const Tile &t = e->tiles[e->neuron_tile[it->second]];
-            int &cell = tgt[(t.topo + spec->row[j] - N.row0) * L + e->neuron_lane[it->second]];
+            const int sv = spec->solver[j], row = spec->row[j];
+            auto it = std::upper_bound(by.begin(), by.end(), j, [&](int, int y) {
+                return sv != ns[y].solver ? sv < ns[y].solver : row < ns[y].row0;
+            });
+            const int i = it == by.begin() ? -1 : *(it - 1);
+            if (i < 0 || ns[i].solver != sv || row >= ns[i].row0 + ns[i].nrows)
+                return fail_err(nullptr, GBH_ERR_ARG, "target %d: solver %d has no row %d", j, sv, row);
+            const Neuron &N = ns[i];
+            const Tile &t = e->tiles[e->neuron_tile[i]];
+            int &cell = tgt[(t.topo + row - N.row0) * L + e->neuron_lane[i]];
             if (cell >= 0) return fail_err(nullptr, GBH_ERR_ARG, "target %d repeats target %d", j, cell);
             cell = j;
         }
@@ -4028,36 +4034,66 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
     if (dchip) memset(dchip, 0, e->chip_start.back() * sizeof(double));
     if (dravals) memset(dravals, 0, e->rav_start.back() * sizeof(double));
     if (dvm0) memset(dvm0, 0, e->vm_start.back() * sizeof(double));
-    for (size_t i = 0; i < e->dec.neurons.size(); ++i) {
-        const Neuron &N = e->dec.neurons[i];
-        const int ti = e->neuron_tile[i];
-        const Tile &t = e->tiles[ti];
-        const AdjType &at = atypes[t.type];
-        const int l = e->neuron_lane[i];
-        if (dvm0)
-            for (int s = 0; s < N.nrows; ++s) dvm0[e->vm_start[N.solver] + N.row0 + s] = Vb[(t.vm + s) * L + l];
-        if (dchip) {
-            // field gradients: per-slot fields, per-channel Ek and gmax, initial gate states
-            std::vector<double> gfield(N.fsrc.size(), 0.0);
-            for (size_t f = 0; f < N.fsrc.size(); ++f) gfield[f] = Gf[(t.fld + f) * L + l];
-            for (int c = 0; c < at.nchans; ++c) {
-                const AdjChan &ch = chan_plan[at.chan_off + c];
-                if (ch.f_ek >= 0) gfield[ch.f_ek] += Gek[(ch_off[ti] + c) * L + l];
-                gfield[ch.f_gmax] += Ggm[(ch_off[ti] + c) * L + l];
-            }
-            for (int g = 0; g < at.ngates; ++g) gfield[snap_field[at.snap_off + g]] += Xb[(xb_off[ti] + g) * L + l];
-            for (size_t f = 0; f < N.fsrc.size(); ++f)
-                if (N.fsrc[f].kind == FS_CHIP) dchip[e->chip_start[N.solver] + N.fsrc[f].idx] += gfield[f];
-        }
-        if (dravals)
-            for (int s = 0; s < N.nrows; ++s) {
-                const double g[3] = {GA[(t.topo + s) * L + l], GB[(t.topo + s) * L + l], GC[(t.topo + s) * L + l]};
-                for (int q = 0; q < 3; ++q) {
-                    const int r = N.ridx[3 * s + q];
-                    if (r >= 0) dravals[e->rav_start[N.solver] + r] += g[q];
+    // neurons [i0, i1), gfield: room for a neuron's fields
+    auto gather = [&](size_t i0, size_t i1, double *gfield) {
+        for (size_t i = i0; i < i1; ++i) {
+            const Neuron &N = e->dec.neurons[i];
+            const int ti = e->neuron_tile[i];
+            const Tile &t = e->tiles[ti];
+            const AdjType &at = atypes[t.type];
+            const int l = e->neuron_lane[i];
+            if (dvm0)
+                for (int s = 0; s < N.nrows; ++s) dvm0[e->vm_start[N.solver] + N.row0 + s] = Vb[(t.vm + s) * L + l];
+            if (dchip) {
+                // field gradients: per-slot fields, per-channel Ek and gmax, initial gate states
+                for (size_t f = 0; f < N.fsrc.size(); ++f) gfield[f] = Gf[(t.fld + f) * L + l];
+                for (int c = 0; c < at.nchans; ++c) {
+                    const AdjChan &ch = chan_plan[at.chan_off + c];
+                    if (ch.f_ek >= 0) gfield[ch.f_ek] += Gek[(ch_off[ti] + c) * L + l];
+                    gfield[ch.f_gmax] += Ggm[(ch_off[ti] + c) * L + l];
                 }
+                for (int g = 0; g < at.ngates; ++g) gfield[snap_field[at.snap_off + g]] += Xb[(xb_off[ti] + g) * L + l];
+                for (size_t f = 0; f < N.fsrc.size(); ++f)
+                    if (N.fsrc[f].kind == FS_CHIP) dchip[e->chip_start[N.solver] + N.fsrc[f].idx] += gfield[f];
             }
+            if (dravals)
+                for (int s = 0; s < N.nrows; ++s) {
+                    const double g[3] = {GA[(t.topo + s) * L + l], GB[(t.topo + s) * L + l], GC[(t.topo + s) * L + l]};
+                    for (int q = 0; q < 3; ++q) {
+                        const int r = N.ridx[3 * s + q];
+                        if (r >= 0) dravals[e->rav_start[N.solver] + r] += g[q];
+                    }
+                }
+        }
+    };
+    // in ranges of whole solvers (neurons of one may share entries)
+    size_t fields = 0, nf = 1;
+    for (const Neuron &N : e->dec.neurons) {
+        fields += N.fsrc.size();
+        nf = std::max(nf, N.fsrc.size());
     }
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t parts = std::max<size_t>(1, std::min({hw, (size_t)8, fields / 65536}));
+    std::vector<double> gfield(parts * nf);
+    std::vector<size_t> cut(parts + 1, 0);
+    for (size_t q = 1; q < parts; ++q) {
+        cut[q] = std::max(cut[q - 1], e->dec.neurons.size() * q / parts);
+        while (cut[q] > 0 && cut[q] < e->dec.neurons.size() &&
+               e->dec.neurons[cut[q]].solver == e->dec.neurons[cut[q] - 1].solver)
+            ++cut[q];
+    }
+    cut[parts] = e->dec.neurons.size();
+    std::vector<std::thread> th;
+    th.reserve(parts);
+    for (size_t q = 1; q < parts; ++q) {
+        try {
+            th.emplace_back(gather, cut[q], cut[q + 1], gfield.data() + q * nf);
+        } catch (...) {   // no thread to be had
+            gather(cut[q], cut[q + 1], gfield.data() + q * nf);
+        }
+    }
+    gather(cut[0], cut[1], gfield.data());
+    for (auto &x : th) x.join();
     return GBH_OK;
 }
 
