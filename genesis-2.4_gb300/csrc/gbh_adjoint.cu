@@ -34,9 +34,10 @@ cudaError_t launch_adj_linearize(const AdjView &v, int ntiles, int smax, int nk,
 {
     if (ntiles <= 0 || nk <= 0) return cudaSuccess;
     const size_t smem = (size_t)2 * smax * LANES * sizeof(double);
-    cudaError_t ce = smem_attr((const void *)k_adj_linearize, smem);
+    cudaError_t ce = smem_attr((const void *)k_adj_eliminate, smem);
     if (ce != cudaSuccess) return ce;
-    k_adj_linearize<<<dim3(ntiles, nk), LANES, smem, st>>>(v, smax);
+    k_adj_linearize<<<dim3(ntiles, nk), LANES, 0, st>>>(v);
+    k_adj_eliminate<<<dim3(ntiles, nk), LANES, smem, st>>>(v, smax);
     return cudaGetLastError();
 }
 

@@ -15,13 +15,14 @@
 //   forward   the engine's own step kernel advances work copies of Vm and the
 //             gate states; k_adj_copy stores them every K steps (checkpoints)
 //             and, when a segment is recomputed, before every step (snapshot);
-//   k_adj_linearize   (parallel over steps) recomputes each step of a segment
-//             from its snapshot with the step's exact arithmetic and stores
-//             the local derivatives the reverse needs: 1/D', A/D', R' and x of
-//             every row, ichan and sumg of every compartment, the gate product
-//             of every channel, and per gate d prod/dx, dx'/dVm (table slope,
-//             zero where the lookup clamps or without interpolation) and
-//             dx'/dx (the trapezoid factor (2-B')/B', zero for instant gates);
+//   k_adj_linearize, k_adj_eliminate   (parallel over steps) recompute each
+//             step of a segment from its snapshot with the step's exact
+//             arithmetic and store the local derivatives the reverse needs:
+//             1/D', A/D', R' and x of every row, ichan and sumg of every
+//             compartment, the gate product of every channel, and per gate
+//             d prod/dx, dx'/dVm (table slope, zero where the lookup clamps or
+//             without interpolation) and dx'/dx (the trapezoid factor
+//             (2-B')/B', zero for instant gates);
 //   k_adj_reverse   (sequential over steps, a thread per compartment) the
 //             adjoint recurrence of Vm and the gate states:
 //               seed      Vm-bar += 2 (Vm after - target) at target rows
@@ -114,11 +115,21 @@ k_adj_ck_to_tape(AdjView v, int c0)
 }
 
 // ---------------------------------------------------------------- linearisation
-// grid (tiles, steps), 32 threads. Shared memory: 2 * smax * 32 doubles.
-__global__ void __launch_bounds__(32)
-k_adj_linearize(AdjView v, int smax)
+// a / b with y = rcp_rn(b) at hand
+__device__ __forceinline__ double div_of(double a, double b, double y)
 {
-    extern __shared__ double sm[];
+    return mid_range(a) && divisor_ok(b) ? div_by(a, b, y) : div_ieee(a, b);
+}
+
+// Channels: grid (tiles, steps), 32 threads; each row's diagonal and right-hand
+// side go to the tape's RD and RP rows. Apart from the elimination, whose two
+// shared-memory columns (32 KB a warp at 64 rows) leave 7 warps an SM: the
+// gates' loads, one behind another, want more in flight (24 tiles of 64 rows x
+// 100 steps: 2.40 ms in one kernel, 1.09 + 0.37 ms apart and with one
+// reciprocal a divisor; that alone 2.19).
+__global__ void __launch_bounds__(32)
+k_adj_linearize(AdjView v)
+{
     const int lane = threadIdx.x;
     const int t = blockIdx.x;
     const int k = blockIdx.y;
@@ -133,13 +144,7 @@ k_adj_linearize(AdjView v, int smax)
     const int S = at.nslots;
     const AdjRows R = adj_rows(S, at.ngates, at.nchans);
     const double *P = v.P + tl.fld * LANES + lane;
-    const int *par = v.parent + tl.topo * LANES + lane;
-    const double *Aw = v.A + tl.topo * LANES + lane;
-    const double *Bw = v.B + tl.topo * LANES + lane;
-    const double *Cw = v.Cb + tl.topo * LANES + lane;
     double *tp = adj_tape(v, k, t, lane);
-    double *Dc = sm + lane;
-    double *Rc = Dc + (size_t)smax * LANES;
 
     VCursor vc;
     if (ncols) { vc.lo = vc.hi = 0.0; } else { vc.lo = -1e20; vc.hi = 1e20; }
@@ -195,16 +200,10 @@ k_adj_linearize(AdjView v, int smax)
                 }
                 const int p = pc[3];
                 const double st = tp[(R.ST + gi) * LANES];
-                double x;
-                int pw = p;
-                if (p > 0) {
-                    x = (st * (2.0 - X) + Y) / X;
-                } else {
-                    x = Y / X;
-                    pw = -p;
-                }
+                const int pw = abs(p);
+                const double rX = rcp_rn(X);
+                const double x = div_of(p > 0 ? st * (2.0 - X) + Y : Y, X, rX);
                 Gk = gpow<double>(Gk, x, pw);
-                const double rX = 1.0 / X;
                 const double along = p > 0 ? st + x : x;   // -(dx'/dB') * B'
                 tp[(R.DXDV + gi) * LANES] = rX * dfdv * (sY - along * sX);
                 tp[(R.DXDST + gi) * LANES] = p > 0 ? (2.0 - X) * rX : 0.0;
@@ -234,8 +233,8 @@ k_adj_linearize(AdjView v, int smax)
                 pc += 2;
             } else if (code == M_END) {
                 const double tbyc = P[pc[1] * LANES];
-                Rc[s * LANES] = Vm + ichan * tbyc;
-                Dc[s * LANES] = sumg * tbyc + P[pc[2] * LANES];
+                tp[(R.RP + s) * LANES] = Vm + ichan * tbyc;
+                tp[(R.RD + s) * LANES] = sumg * tbyc + P[pc[2] * LANES];
                 tp[(R.ICH + s) * LANES] = ichan;
                 tp[(R.SG + s) * LANES] = sumg;
                 pc += 4;
@@ -246,14 +245,42 @@ k_adj_linearize(AdjView v, int smax)
             }
         }
     }
+}
+
+// Elimination: grid (tiles, steps), 32 threads. Shared memory: 2 * smax * 32
+// doubles.
+__global__ void __launch_bounds__(32)
+k_adj_eliminate(AdjView v, int smax)
+{
+    extern __shared__ double sm[];
+    const int lane = threadIdx.x;
+    const int t = blockIdx.x;
+    const int k = blockIdx.y;
+    const Tile tl = v.tiles[t];
+    const AdjType at = v.atypes[tl.type];
+    const int S = at.nslots;
+    const AdjRows R = adj_rows(S, at.ngates, at.nchans);
+    const int *par = v.parent + tl.topo * LANES + lane;
+    const double *Aw = v.A + tl.topo * LANES + lane;
+    const double *Bw = v.B + tl.topo * LANES + lane;
+    const double *Cw = v.Cb + tl.topo * LANES + lane;
+    double *tp = adj_tape(v, k, t, lane);
+    double *Dc = sm + lane;
+    double *Rc = Dc + (size_t)smax * LANES;
+#pragma unroll 4
+    for (int s = 0; s < S; ++s) {
+        Dc[s * LANES] = tp[(R.RD + s) * LANES];
+        Rc[s * LANES] = tp[(R.RP + s) * LANES];
+    }
     for (int s = 0; s < S; ++s) {
         const int p = par[s * LANES];
         const double d = Dc[s * LANES];
-        tp[(R.RD + s) * LANES] = 1.0 / d;
+        const double rd = rcp_rn(d);
+        tp[(R.RD + s) * LANES] = rd;
         tp[(R.RP + s) * LANES] = Rc[s * LANES];
         double temp = 0.0;
         if (p >= 0) {
-            temp = Aw[s * LANES] / d;
+            temp = div_of(Aw[s * LANES], d, rd);
             Dc[p * LANES] -= Bw[s * LANES] * temp;
             Rc[p * LANES] -= Rc[s * LANES] * temp;
         }
@@ -263,7 +290,7 @@ k_adj_linearize(AdjView v, int smax)
         const int p = par[s * LANES];
         double r = Rc[s * LANES];
         if (p >= 0) r -= Cw[s * LANES] * Rc[p * LANES];
-        r = r / Dc[s * LANES];
+        r = div_of(r, Dc[s * LANES], tp[(R.RD + s) * LANES]);
         Rc[s * LANES] = r;
         tp[(R.X + s) * LANES] = r;
     }

@@ -4002,8 +4002,8 @@ int gbh_loss_gradient(gbh_engine *e, int nsteps, int checkpoint_every, const gbh
     e->stats.grad_reverse_ms = ms_rev;
     e->stats.grad_kept_steps = keep ? 1 : 0;
     // forward step launches are counted by launch_one; add the copies
-    // (checkpoint saves and restores, snapshots) and three kernels per segment
-    e->stats.launches += (keep ? (int64_t)nsteps + nseg : 2 * (int64_t)nseg + nsteps) + 3 * (int64_t)nseg;
+    // (checkpoint saves and restores, snapshots) and four kernels per segment
+    e->stats.launches += (keep ? (int64_t)nsteps + nseg : 2 * (int64_t)nseg + nsteps) + 4 * (int64_t)nseg;
     int status = 0;
     CK(cudaMemcpy(&status, e->d_status.p, sizeof(int), cudaMemcpyDeviceToHost));
     if (status) {
