@@ -172,7 +172,11 @@ typedef struct gbh_options {
                             -- and let the autotuner pick; 1 = unrolled form
                             only; 2 = compact form only; 3 = unrolled form with
                             shared-memory rows only; -1 = interpret the
-                            programs                                          */
+                            programs. With 0 (no synapses), trees whose
+                            dendrites are passive are eliminated level by
+                            level over several warps, and for small batches
+                            with channels along the dendrites the autotuner
+                            also times a thread per compartment               */
     int wide_min;        /* neurons with at least this many compartments run
                             one per warp, compartments across its threads;
                             the other large neurons run 32 per warp, one per
@@ -206,11 +210,13 @@ typedef struct gbh_stats {
                                   0 unrolled, 1 compact (looped), 2 unrolled
                                   with its rows in shared memory              */
     int cooperative;           /* network steps run K per cooperative launch
-                                  with a grid barrier between steps           */
+                                  with a grid barrier between steps (an
+                                  autotuned choice: runs of 6 steps or more)  */
     int64_t wide_tiles;        /* tiles holding one neuron across a warp's
                                   threads (level-by-level elimination)        */
-    int64_t stack_tiles;       /* tiles of 32 large neurons, one per lane,
-                                  eliminated with per-lane stacks             */
+    int64_t stack_tiles;       /* tiles of 32 large neurons whose passive rows
+                                  keep their factors: eliminated with per-lane
+                                  stacks, or level by level over several warps */
     int64_t grad_kept_steps;   /* last gbh_loss_gradient: 1 if every step's
                                   state stayed in device memory (no segment
                                   recomputed), 0 if segments were recomputed
