@@ -718,7 +718,7 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
                 }
                 if (fast && kept) {
                 } else if (mixed) {
-                    el << " const double ri = rcp_seed(D[" << s << "]); D[" << s << "] = ri;";
+                    el << " const double ri = rcp_step(D[" << s << "]); D[" << s << "] = ri;";
                     if (par[s] >= 0) el << " T[" << s << "] = Aw[" << s * LANES << "] * ri;";
                 } else {
                     // FP64: one correctly rounded y = 1/D' per row; T = A/D' and the back
@@ -820,7 +820,7 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
     } else {
         t << "    for (int s = 0; s < " << S << "; ++s) { const int p = par[s * 32];\n";
         if (mixed)
-            t << "      const double ri = rcp_seed(Dc[s * 32]); Dc[s * 32] = ri;\n"
+            t << "      const double ri = rcp_step(Dc[s * 32]); Dc[s * 32] = ri;\n"
               << "      if (p >= 0) { const double temp = Aw[s * 32] * ri; Dc[p * 32] = fma(-Bw[s * 32], temp, Dc[p * 32]); Rc[p * 32] = fma(-Rc[s * 32], temp, Rc[p * 32]); } }\n";
         else
             t << "      if (p >= 0) { const double d = Dc[s * 32]; const double temp = Aw[s * 32] / d; Dc[p * 32] -= Bw[s * 32] * temp; Rc[p * 32] -= Rc[s * 32] * temp; } }\n";
@@ -1172,7 +1172,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
         o << "      level_top_kids<" << form << ", " << res << ">(L, g, q, " << s << ", lid, R" << S << ", D" << S << ");\n";
         for (int j = 0; j < s; ++j)   // top rows below this one, after the static rows: ascending row order
             o << "      if (tp[" << j << "] == " << s << ") { D" << S << " -= PD[" << j << "]; R" << S << " -= T[" << j << "]; }\n";
-        if (mixed) o << "      D" << S << " = rcp_seed(D" << S << ");\n";
+        if (mixed) o << "      D" << S << " = rcp_step(D" << S << ");\n";
         if (s < N - 1)   // T holds R T
             o << "      { const double temp = " << (mixed ? "Aw[" + r + "] * D" + S : "div_rn(Aw[" + r + "], D" + S + ")")
               << "; PD" << S << " = Bw[" << r << "] * temp; T" << S << " = R" << S << " * temp; }\n";

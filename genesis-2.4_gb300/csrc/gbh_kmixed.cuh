@@ -390,7 +390,7 @@ k_steps_mixed(DevView v, int tile0, int tile1, int smax, int nsteps, long long s
         } else {
         for (int s = 0; s < S; ++s) {
             const int p = par[s * LANES];
-            const double ri = rcp_seed(Dcol[s * LANES]);
+            const double ri = rcp_step(Dcol[s * LANES]);
             Dcol[s * LANES] = ri;   // the row's diagonal is final here; keep only its reciprocal
             if (p >= 0) {
                 const double temp = Aw[s * LANES] * ri;
@@ -572,7 +572,7 @@ k_stack_mixed(DevView v, int tile0, int tile1, int cap, int nsteps, long long st
                 D -= cd;
                 R -= cr;
             }
-            const double ri = rcp_seed(D);
+            const double ri = rcp_step(D);
             col[s * LANES] = make_double2(R, ri);
             double temp = 0.0;
             if (f & FL_PARENT) {
@@ -932,7 +932,7 @@ k_wide_mixed(DevView v, int tile0, int tile1, int smax, int nsteps, long long st
                     d = fma(-B[c], temp, d);
                     r = fma(-Rs[c], temp, r);
                 }
-                Ds[s] = rcp_seed(d);
+                Ds[s] = rcp_step(d);
                 Rs[s] = r;
             }
             __syncthreads();

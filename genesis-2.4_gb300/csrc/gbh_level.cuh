@@ -281,7 +281,7 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
                 else D = 0.0 * P[ps[4] * LANES + l] + P[ps[5] * LANES + l];
                 const int k0 = kid[e] & 0xffff, nk = L.nkid[g.eoff + e];
                 for (int k = 0; k < nk; ++k) D -= PR[k0 + k];
-                const double y = MIXED ? rcp_seed(D) : 1.0 / D;   // FP64: correctly rounded
+                const double y = MIXED ? rcp_step(D) : 1.0 / D;   // FP64: correctly rounded
                 const double T = MIXED ? A[r] * y : A[r] / D;
                 const double b = B[r] * T;
                 PR[e] = b;

@@ -186,7 +186,7 @@ __device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup 
                 D -= q.PD[k];
                 R -= q.PR[k];
             }
-            const double y = MIXED ? rcp_seed(D) : rcp_rn(D);
+            const double y = MIXED ? rcp_step(D) : rcp_rn(D);
             const double T = MIXED ? a * y : div_by(a, D, y);
             q.PD[e] = b * T;
             q.PR[e] = R * T;

@@ -37,7 +37,7 @@ __device__ bool differ(double a, double b)
     return a != a ? b == b : __double_as_longlong(a) != __double_as_longlong(b);
 }
 
-enum { DIV, RCP, SPECIAL, KEY, ROW, SEED, DF, VOLT, N };
+enum { DIV, RCP, SPECIAL, KEY, ROW, SEED, STEP, DF, VOLT, N };
 
 __global__ void k_check(unsigned long long *bad, int rounds, uint64_t seed, const double *special, int nspecial)
 {
@@ -74,6 +74,8 @@ __global__ void k_check(unsigned long long *bad, int rounds, uint64_t seed, cons
         const double r0 = (double)rcp_approx(__double2float_rz(m1)), r1 = fma(r0, fma(-m1, r0, 1.0), r0);
         const double e = fabs(rcp_seed(m1) / r1 - 1.0) * 0x1p53 + (rcp_seed(y) * m1 / ay * (y < 0 ? -1 : 1) < 0 ? 1e9 : 0);
         if (e > (double)b[SEED]) b[SEED] = (unsigned long long)ceil(e);
+        const double es = fabs(rcp_step(m1) / r1 - 1.0) * 0x1p53 + (rcp_step(y) * m1 / ay * (y < 0 ? -1 : 1) < 0 ? 1e9 : 0);
+        if (es > (double)b[STEP]) b[STEP] = (unsigned long long)ceil(es);
         const double v = pick(s, 100);
         float hi = (float)v, lo = (float)(v - (double)hi);
         if (i & 1) {   // a significand that ends in hi, lo far below or taken off a power of two
@@ -81,14 +83,13 @@ __global__ void k_check(unsigned long long *bad, int rounds, uint64_t seed, cons
         }
         const double exact = (double)hi + (double)lo;
         const double er = fabs((df2d(df_make(hi, lo)) - exact) / exact) * 0x1p53;
-        const df w = d2df_volt(v);
-        const double ew = fabs(((double)w.hi + (double)w.lo - v) / v) * 0x1p53;
-        if (fabs(v) > 0x1p-70 && ew > (double)b[VOLT]) b[VOLT] = (unsigned long long)ceil(ew);
+        const df w = d2df_volt(v), u = d2df(v);
+        b[VOLT] += fabs(v) > 0x1p-70 && (w.hi != u.hi || w.lo != u.lo);
         b[SPECIAL] += isfinite(p) ? 0 : !(fabs((double)d2df_volt(p).hi) > 1e38);
         if (er > (double)b[DF]) b[DF] = (unsigned long long)ceil(er);
     }
     for (int j = 0; j < N; ++j)
-        if (j == SEED || j == DF || j == VOLT) atomicMax(&bad[j], b[j]);
+        if (j == SEED || j == STEP || j == DF) atomicMax(&bad[j], b[j]);
         else atomicAdd(&bad[j], b[j]);
 }
 
@@ -105,7 +106,7 @@ int main()
     const int blocks = 152 * 4, threads = 128, rounds = 400;
     k_check<<<blocks, threads>>>(bad, rounds, 42, dsp, (int)(sizeof(sp) / sizeof(sp[0])));
     if (cudaMemcpy(h, bad, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return 3;
-    const char *name[N] = {"div", "rcp", "special", "key", "row", "seed", "df", "volt"};
+    const char *name[N] = {"div", "rcp", "special", "key", "row", "seed", "step", "df", "volt"};
     for (int j = 0; j < N; ++j) printf("%s %llu\n", name[j], h[j]);
     return 0;
 }
