@@ -198,13 +198,12 @@ __device__ __forceinline__ double f2d_raw(float f)
 }
 __device__ __forceinline__ double df2d_row(df x) { return f2d_raw(x.hi) + f2d_raw(x.lo); }
 
-// Reciprocal of a normal double to about 2^-44, one Newton step without FP64
-// instructions: the significand m in [1,2) as a float pair, a float seed r
-// (MUFU), its residual e = 1 - m r on FP32 multiply-adds (below 2^-22, so it
-// and r e are off by 2^-46), and r + r e assembled on the integer pipe, r e in
-// units of 2^-53. Valid for 2^-1021 < |b| < 2^1021. (With the e^2 term, good
-// to 2^-45.5, the mixed form's error on 100,000 16-compartment cables over 500
-// steps is 2.6e-10 instead of 3.0e-10 relative: no more than the rest of it.)
+// Reciprocal of a normal double to about 2^-44, the seed of the FP64 corrections
+// below: one Newton step without FP64 instructions, the significand m in [1,2)
+// as a float pair, a float seed r (MUFU), its residual e = 1 - m r on FP32
+// multiply-adds (below 2^-22, so it and r e are off by 2^-46), and r + r e
+// assembled on the integer pipe, r e in units of 2^-53. Valid for
+// 2^-1021 < |b| < 2^1021.
 __device__ __forceinline__ double rcp_seed(double b)
 {
     const uint32_t hi = (uint32_t)__double2hiint(b), lo = (uint32_t)__double2loint(b);
@@ -222,7 +221,7 @@ __device__ __forceinline__ double rcp_seed(double b)
 // The same with the step's products kept to 2^-47: the mixed form's reciprocal.
 // (FP64's first-order step to its last bits: with the seed's rounding a neuron
 // at its threshold among 100,000 16-compartment cables left the trace of the
-// FP64 step by 3e-8 over 500 steps, with this 1e-8; 28.0 -> 28.6 us a step.)
+// FP64 step by 3e-8 over 500 steps, with this 1e-8; 28.0 -> 28.4 us a step.)
 __device__ __forceinline__ double rcp_step(double b)
 {
     const uint32_t hi = (uint32_t)__double2hiint(b), lo = (uint32_t)__double2loint(b);
