@@ -55,4 +55,19 @@ struct Decoded {
 // *err filled (solver, row, opcode, position, message).
 int decode_batch(const gbh_batch_desc *d, Decoded &out, gbh_error *err);
 
+// Levels of the rows below `nstatic` of one neuron (parent: per row, -1 the
+// root's): the most of them on one path towards the root. Children have lower
+// rows than their parents.
+inline int static_levels(const std::vector<int> &parent, int nstatic)
+{
+    std::vector<int> depth(nstatic, 0);
+    int levels = 0;
+    for (int s = nstatic - 1; s >= 0; --s) {
+        const int p = parent[s];   // -1: without channels the root is passive too
+        depth[s] = p >= 0 && p < nstatic ? depth[p] + 1 : 1;
+        if (depth[s] > levels) levels = depth[s];
+    }
+    return levels;
+}
+
 }  // namespace gbh

@@ -734,15 +734,7 @@ bool level_type(const TileType &tt, const std::vector<int> &prog, const std::vec
                 LevelProg &lp)
 {
     if (!tt.stack) return false;
-    if (uniform && tt.nslots <= kJitMaxSlots) {
-        std::vector<int> depth(tt.nslots, 0);
-        int levels = 0;
-        for (int s = tt.nstatic - 1; s >= 0; --s) {   // children have lower rows than their parents
-            depth[s] = parent[s] < tt.nstatic ? depth[parent[s]] + 1 : 1;
-            levels = std::max(levels, depth[s]);
-        }
-        if (tt.nstatic < 2 * levels) return false;
-    }
+    if (uniform && tt.nslots <= kJitMaxSlots && tt.nstatic < 2 * static_levels(parent, tt.nstatic)) return false;
     // one neuron's rows must fit a block (constants in global memory)
     if (level_smem(kSplitRows, tt.nstatic, tt.nstatic + 1, tt.crank != 0, false, false) > (size_t)kLevelSmemMax)
         return false;
