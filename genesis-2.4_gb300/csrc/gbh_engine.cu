@@ -2205,6 +2205,25 @@ int run_steps(gbh_engine *e, int nsteps, cudaStream_t st)
 
 }  // namespace
 
+// The engine's device made current for a launch on the default stream, which
+// belongs to the current device; the caller's is current again afterwards.
+struct OnDevice {
+    int was = -1;
+    cudaError_t rc;
+    explicit OnDevice(int dev)
+    {
+        rc = cudaGetDevice(&was);
+        if (rc == cudaSuccess && was == dev) was = -1;
+        else if (rc == cudaSuccess) rc = cudaSetDevice(dev);
+    }
+    ~OnDevice()
+    {
+        if (was >= 0) cudaSetDevice(was);
+    }
+    OnDevice(const OnDevice &) = delete;
+    OnDevice &operator=(const OnDevice &) = delete;
+};
+
 int autotune_trials(gbh_engine *e);
 
 // Autotuner: times trial steps for every (kernel variant, steps per launch)
@@ -3365,11 +3384,14 @@ int gbh_run(gbh_engine *e, int nsteps)
 // of 16 compartments: copying every state block and walking the neurons on
 // the host took 8 ms, more than 200 steps. On the default stream, as the
 // other copies of gbh_get_state: it waits for the caller's blocking streams.
+// That stream is the current device's, whatever engine the call names.
 static int get_vm(gbh_engine *e, double *vm)
 {
     const int64_t n = e->vm_start.back();
     if (n == 0) return GBH_OK;
     if (e->d_vm_at.p) {
+        const OnDevice on(e->opt.device);
+        CK(on.rc);
         k_gather_vm<<<(unsigned)((n + 255) / 256), 256>>>(e->d_V.p, e->d_vm_at.p, n, e->d_vm_out.p);
         CK(cudaGetLastError());
         CK(cudaMemcpy(vm, e->d_vm_out.p, n * sizeof(double), cudaMemcpyDeviceToHost));
