@@ -3602,6 +3602,8 @@ int gbh_get_stats(const gbh_engine *e, gbh_stats *st)
 static int adj_plan(gbh_engine *e, int hmax)
 {
     if (e->adj_ngroups > 0) return GBH_OK;
+    const OnDevice on(e->opt.device);   // kept for later calls, whatever device is current in this one
+    CK(on.rc);
     const Decoded &dec = e->dec;
     const int per = (int)std::min<size_t>(LANES, (dec.neurons.size() + kLevelGroups - 1) / kLevelGroups);
     std::vector<std::vector<int>> cells_of(e->tiles.size());

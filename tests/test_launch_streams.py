@@ -30,3 +30,13 @@ def test_launches_name_a_stream_or_a_device(name):
         args = _split(m.group(1))
         function = text[text.rfind("\n}\n", 0, m.start()):m.start()]
         assert len(args) == 4 and args[3] not in ("0", "nullptr") or "OnDevice on(" in function, m.group(0)
+
+
+def test_buffers_kept_by_a_later_call_are_the_engines_devices():
+    """Outside gbh_create, whose device is current throughout, allocations go to
+    the caller's current device; the reverse sweep's plan outlives its call."""
+    text = open(os.path.join(build.CSRC, "gbh_engine.cu")).read()
+    start = text.index("static int adj_plan(")
+    body = text[start:text.index("\n}\n", start)]
+    assert ".upload(" in body
+    assert body.index("OnDevice on(e->opt.device)") < body.index(".upload(")
