@@ -2271,6 +2271,7 @@ int autotune_trials(gbh_engine *e)
     rc |= keep(e->d_RV.p, e->d_RV.n * sizeof(double));
     rc |= keep(e->d_I.p, e->d_I.n * sizeof(int));
     rc |= keep(e->d_ring.p, e->d_ring.n * sizeof(unsigned));
+    rc |= keep(e->d_wmask.p, e->d_wmask.n * sizeof(unsigned));   // the bits of the events d_ring counts
     rc |= keep(e->d_spikes.p, e->d_spikes.n * sizeof(unsigned long long));
     if (rc) {
         for (Save &s : saves) cudaFree(s.dst);
