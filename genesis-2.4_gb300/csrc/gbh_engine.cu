@@ -2240,6 +2240,9 @@ int autotune(gbh_engine *e)
     // the trials' kernels kept the static rows' factors with their own
     // arithmetic: the chosen kernels keep theirs at their first launch
     if (rc_t == GBH_OK && stack_invalidate(e, e->stream)) return GBH_ERR_CUDA;
+    // nothing orders the clears of the trials' spikes and sums and the new
+    // generation before a first step on a stream of the caller's
+    CK(cudaStreamSynchronize(e->stream));
     return rc_t;
 }
 
@@ -2387,7 +2390,7 @@ int autotune_trials(gbh_engine *e)
             e->net_spl = coop_k;
         }
     }
-    CK(cudaStreamSynchronize(e->stream));
+    CK(cudaStreamSynchronize(e->stream));   // (the copies back, before their sources go)
     for (Save &s : saves) cudaFree(s.dst);
     if (e->d_spiked.p)   // trial spikes
         CK(cudaMemsetAsync(e->d_spiked.p, 0, e->d_spiked.n * sizeof(unsigned), e->stream));
