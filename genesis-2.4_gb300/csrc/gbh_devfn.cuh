@@ -505,7 +505,7 @@ __device__ __forceinline__ void st_df(double *p, df x)
 __device__ __forceinline__ df interp_df(const float4 *tab, int e, df fr)
 {
     const float4 t = __ldg(tab + e);
-    return df_add(df_make(t.x, t.y), df_mul_un(df_make(t.z, t.w), fr));
+    return df_add(df_make(t.x, t.y), df_mul(df_make(t.z, t.w), fr));
 }
 
 __device__ __forceinline__ df val_df(const float4 *tab, int e)

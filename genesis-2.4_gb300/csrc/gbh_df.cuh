@@ -68,16 +68,6 @@ __device__ __forceinline__ df df_mul(df x, df y)
     return fast_two_sum(p.hi, p.lo);
 }
 
-// A product left as it comes, |lo| up to some 2^-22 |hi|: for an operand of
-// df_add, whose first step takes any pair of leading parts.
-__device__ __forceinline__ df df_mul_un(df x, df y)
-{
-    df p = two_prod(x.hi, y.hi);
-    p.lo = __fmaf_rn(x.hi, y.lo, p.lo);
-    p.lo = __fmaf_rn(x.lo, y.hi, p.lo);
-    return p;
-}
-
 __device__ __forceinline__ df df_mul_f(df x, float y)
 {
     df p = two_prod(x.hi, y);
@@ -166,23 +156,24 @@ __device__ __forceinline__ df d2df_volt(double d)
 }
 
 // df -> double on the integer pipe: lo's significand, shifted to hi's unit in
-// the last place (truncated there, below 2^-52 of hi), is added to or taken
-// from hi's bits. No FP64 instruction: the FP64 unit takes one warp
-// instruction per 19 clocks of an SM, an addition as much as a multiply-add.
-// Needs |lo| < 2^-22 |hi| (any normalised df); hi zero or below the float
-// normal range gives a signed zero.
+// the last place and rounded there to nearest even, is added to or taken from
+// hi's bits: the FP64 sum of the two (a denormal part counts as zero). No FP64
+// instruction: the FP64 unit takes one warp instruction per 19 clocks of an SM,
+// an addition as much as a multiply-add. Needs |lo| below hi's unit in the
+// last place (any df but an unfinished one).
 __device__ __forceinline__ double df2d(df x)
 {
     const uint32_t uh = __float_as_uint(x.hi), ul = __float_as_uint(x.lo);
     const uint32_t eh = (uh >> 23) & 0xffu, el = (ul >> 23) & 0xffu;
     const uint32_t sign = uh & 0x80000000u;
     const uint32_t h = ((uh & 0x7fffffffu) >> 3) + 0x38000000u, l = uh << 29;
-    // lo in units of 2^-52 of hi's binade: its 24 bits, 29 places up and eh - el down
-    const uint32_t sh = eh - max(el, 1u) - 22u;
-    uint32_t m = sh > 31u ? 0u : (((ul & 0x7fffffu) | (el ? 0x800000u : 0u)) << 7) >> sh;
     const bool minus = (int)(uh ^ ul) < 0;
-    // just below a power of two the unit is half as large
-    if (minus && (uh & 0x7fffffu) == 0u) m <<= 1;
+    // lo in units of 2^-52 of hi's binade, half of that where the difference
+    // falls below hi's power of two: its 24 bits, 7 places up and sh down
+    const uint32_t sh = eh - el - 22u - (minus && (uh & 0x7fffffu) == 0u ? 1u : 0u);
+    const uint32_t a = ((ul << 7) & 0x3fffff80u) | 0x40000000u;
+    uint32_t m = 0u;
+    if (el && sh < 32u) m = (a + (1u << (sh - 1u)) - 1u + ((a >> sh) & 1u)) >> sh;
     const uint64_t mag = ((uint64_t)h << 32) | l;
     const uint64_t r = minus ? mag - m : mag + m;
     return __hiloint2double(eh == 0u ? (int)sign : (int)((uint32_t)(r >> 32) | sign), eh == 0u ? 0 : (int)(uint32_t)r);
@@ -218,21 +209,23 @@ __device__ __forceinline__ double rcp_seed(double b)
     return __hiloint2double((int)yh, (int)(uint32_t)y);
 }
 
-// The same with the step's products kept to 2^-47: the mixed form's reciprocal.
-// (FP64's first-order step to its last bits: with the seed's rounding a neuron
-// at its threshold among 100,000 16-compartment cables left the trace of the
-// FP64 step by 3e-8 over 500 steps, with this 1e-8; 28.0 -> 28.4 us a step.)
+// The mixed form's reciprocal: one Newton step r + r e in FP64's own precision,
+// fma(r, fma(-b, r, 1), r) to its last place, without an FP64 instruction. The
+// residual e = 1 - m r of the significand m (53 bits) and the seed r (24 bits)
+// is exact in 76 fraction bits and below 2^-21, so 64-bit integer arithmetic
+// modulo 1 holds it; r e is rounded to r's last place. (With e in FP32 pairs
+// the reciprocal was good to 2^-43.8 instead of this step's 2^-44.)
 __device__ __forceinline__ double rcp_step(double b)
 {
     const uint32_t hi = (uint32_t)__double2hiint(b), lo = (uint32_t)__double2loint(b);
-    const float mh = __uint_as_float(0x3f800000u | (__funnelshift_l(lo, hi, 3) & 0x7fffffu));
-    const float ml = (float)(lo & 0x1fffffffu) * 0x1p-52f;
-    const float r = rcp_approx(mh);
-    const float e1 = __fmaf_rn(-mh, r, 1.0f), e = __fmaf_rn(-ml, r, e1), p = r * e;
-    const float q = __fmaf_rn(r, __fmaf_rn(-ml, r, e1 - e), __fmaf_rn(r, e, -p));
-    const int c = __float2int_rn(p * 0x1p53f) + __float2int_rn(q * 0x1p53f);
-    const uint32_t ru = __float_as_uint(r);
-    const uint64_t y = (((uint64_t)((ru >> 3) + 0x38000000u) << 32) | (ru << 29)) + (uint64_t)(int64_t)c;
+    const float r = rcp_approx(__uint_as_float(0x3f800000u | (__funnelshift_l(lo, hi, 3) & 0x7fffffu)));
+    const uint32_t ru = __float_as_uint(r), R = ru - 0x3e800000u;   // r in [1/2, 1], times 2^24
+    const uint64_t p = (uint64_t)R * lo + ((uint64_t)(R * ((hi & 0xfffffu) | 0x100000u)) << 32);
+    const int64_t e = -(int64_t)p;                                  // times 2^76
+    const int32_t eh = (int32_t)(e >> 24);
+    const uint32_t rl = __umulhi(R, (uint32_t)e << 8);              // r times e's last 24 bits
+    const int64_t c = ((int64_t)(int32_t)R * eh + (int64_t)(rl + (1u << 22))) >> 23;
+    const uint64_t y = (((uint64_t)((ru >> 3) + 0x38000000u) << 32) | (ru << 29)) + (uint64_t)c;
     const uint32_t yh = ((uint32_t)(y >> 32) + 0x3ff00000u - (hi & 0x7ff00000u)) | (hi & 0x80000000u);
     return __hiloint2double((int)yh, (int)(uint32_t)y);
 }

@@ -250,9 +250,9 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
             break;
         case M_END:
             if (mx) {
-                o << "      { const df tbyc = " << E.ldr(a[0]) << "; const df dv = df_mul_un(ichan, tbyc);\n"
+                o << "      { const df tbyc = " << E.ldr(a[0]) << "; const df dv = df_mul(ichan, tbyc);\n"
                   << "        R[" << E.S(s) << "] = df2d_row(df_add(vmd, dv));\n"
-                  << "        D[" << E.S(s) << "] = df2d_row(df_add(" << E.ldr(a[1]) << ", df_mul_un(sumg, tbyc))); }\n";
+                  << "        D[" << E.S(s) << "] = df2d_row(df_add(" << E.ldr(a[1]) << ", df_mul(sumg, tbyc))); }\n";
             } else {
                 o << "      { const double tbyc = " << E.Pr(a[0]) << "; R[" << E.S(s) << "] = Vm + ichan * tbyc; D[" << E.S(s)
                   << "] = sumg * tbyc + " << E.Pr(a[1]) << "; }\n";
@@ -334,7 +334,7 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                         }
                         o << "        double *st = " << E.pP(fs) << ";\n";
                         if (p > 0)
-                            o << "        const df x = df_div(df_add(df_mul_un(ld_df(st), df_add_f(df_neg(X), 2.0f)), Y), X);\n";
+                            o << "        const df x = df_div(df_add(df_mul(ld_df(st), df_add_f(df_neg(X), 2.0f)), Y), X);\n";
                         else
                             o << "        const df x = df_div(Y, X);\n";
                         o << "        st_df(st, x); Gk = dpow(Gk, x, " << (p > 0 ? p : -p) << ");\n      }\n";
@@ -412,7 +412,7 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                     const bool first = !summed;   // (0 + Gk is Gk)
                     summed = true;
                     if (mx) {
-                        o << "      { sumg = " << (first ? "Gk" : "df_add(sumg, Gk)") << "; ichan = df_add(ichan, df_mul_un(Ek, Gk)); const double gk = df2d(Gk), ek = df2d(Ek); Ik = gk * (ek - Vm);";
+                        o << "      { sumg = " << (first ? "Gk" : "df_add(sumg, Gk)") << "; ichan = df_add(ichan, df_mul(Ek, Gk)); const double gk = df2d(Gk), ek = df2d(Ek); Ik = gk * (ek - Vm);";
                         if (giv)
                             o << " { const double gm = c5 ? df2d(gmax) : 1.0; " << E.G(g) << " = gk / gm; " << E.G(g + 1)
                               << " = Ik / gm; " << E.G(g + 2) << " = ek; }";

@@ -130,9 +130,9 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
             pc += 4;
         } else if (code == M_END) {
             const df tbyc = ld_df(&N.P[(pc[1]) * STR]);
-            const df dv = df_mul_un(ichan, tbyc);
+            const df dv = df_mul(ichan, tbyc);
             R = df2d_row(df_add(vmd, dv));
-            D = df2d_row(df_add(ld_df(&N.P[(pc[2]) * STR]), df_mul_un(sumg, tbyc)));
+            D = df2d_row(df_add(ld_df(&N.P[(pc[2]) * STR]), df_mul(sumg, tbyc)));
             if (GIV) N.G[(pc[3]) * STR] = Im;
             pc += 4;
             break;
@@ -226,7 +226,7 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
                     df x;
                     int pw = p;
                     if (p > 0) {
-                        x = df_div(df_add(df_mul_un(ld_df(st), df_add_f(df_neg(X), 2.0f)), Y), X);
+                        x = df_div(df_add(df_mul(ld_df(st), df_add_f(df_neg(X), 2.0f)), Y), X);
                     } else {
                         x = df_div(Y, X);
                         pw = -p;
@@ -270,7 +270,7 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
                 } else if (k == M_ADDCURR) {
                     const int g = pc[1];
                     sumg = df_add(sumg, Gk);
-                    ichan = df_add(ichan, df_mul_un(Ek, Gk));
+                    ichan = df_add(ichan, df_mul(Ek, Gk));
                     const double gk = df2d(Gk), ek = df2d(Ek);
                     Ik = gk * (ek - Vm);
                     if (GIV) {
@@ -421,7 +421,7 @@ k_steps_mixed(DevView v, int tile0, int tile1, int smax, int nsteps, long long s
 
 // Stack elimination of the mixed form (see k_stack in gbh_kernels.cuh): the
 // same row order and per-lane stacks; the diagonal's reciprocal is formed
-// once per row (rcp_seed) and kept in the column for back substitution.
+// once per row (rcp_step) and kept in the column for back substitution.
 //
 // SPLIT: two warps per tile. After a launch's first step the second warp
 // runs the channel phase of the rows above the static ones (kSplitRows at
