@@ -115,7 +115,7 @@ k_adj_ck_to_tape(AdjView v, int c0)
 }
 
 // ---------------------------------------------------------------- linearisation
-// a / b with y = rcp_rn(b) at hand
+// a / b with y = rcp_exact(b) at hand
 __device__ __forceinline__ double div_of(double a, double b, double y)
 {
     return mid_range(a) && divisor_ok(b) ? div_by(a, b, y) : div_ieee(a, b);
@@ -201,7 +201,7 @@ k_adj_linearize(AdjView v)
                 const int p = pc[3];
                 const double st = tp[(R.ST + gi) * LANES];
                 const int pw = abs(p);
-                const double rX = rcp_rn(X);
+                const double rX = rcp_exact(X);
                 const double x = div_of(p > 0 ? st * (2.0 - X) + Y : Y, X, rX);
                 Gk = gpow<double>(Gk, x, pw);
                 const double along = p > 0 ? st + x : x;   // -(dx'/dB') * B'
@@ -275,7 +275,7 @@ k_adj_eliminate(AdjView v, int smax)
     for (int s = 0; s < S; ++s) {
         const int p = par[s * LANES];
         const double d = Dc[s * LANES];
-        const double rd = rcp_rn(d);
+        const double rd = rcp_exact(d);
         tp[(R.RD + s) * LANES] = rd;
         tp[(R.RP + s) * LANES] = Rc[s * LANES];
         double temp = 0.0;

@@ -254,12 +254,25 @@ __device__ __noinline__ static double div_ieee(double a, double b) { return a / 
 // seed good to 2^-44. Before its rounding the step is off by 2^-88, so the
 // result is the correctly rounded one unless 1/b lies within 2^-88 of the
 // middle between two doubles (of the other divisors one in 2^34; there it may
-// be the neighbour). 2 FP64 instructions against the division's 5.5.
+// be the neighbour: for quotients through div_by, see rcp_exact). 2 FP64
+// instructions against the division's 5.5.
 __device__ __forceinline__ double rcp_rn(double b)
 {
     if (!divisor_ok(b)) return div_ieee(1.0, b);
     const double y = rcp_seed(b);
     return fma(y, fma(-b, y, 1.0), y);
+}
+
+// RN(1 / b) without exception, for a reciprocal that is a result of its own:
+// the step once more. From the result or its neighbour e = 1 - b z is exact and
+// below 2^-53, so before its rounding the step is off by e^2 < 2^-106 of it;
+// and 1/b is 2^-106 of itself or more from the middle between two doubles (b's
+// 53 bits times the middle's 54 differ from 2^106). 4 FP64 instructions.
+__device__ __forceinline__ double rcp_exact(double b)
+{
+    if (!divisor_ok(b)) return div_ieee(1.0, b);
+    const double y = rcp_seed(b), z = fma(y, fma(-b, y, 1.0), y);
+    return fma(z, fma(-b, z, 1.0), z);
 }
 
 // RN(a / b) from y = rcp_rn(b) by Markstein's correction (P. Markstein, IBM
