@@ -976,6 +976,7 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
 // Batches whose lane-mapped tiles are fewer than this may run row-parallel
 // (the autotuner times it): eight tiles an SM. Beyond, the lanes of the SMs are
 // full either way and the barriers between levels only cost.
+constexpr int kJitRows = 4;   // gbh_options.jit: the row-parallel plan, untimed
 constexpr int64_t kRowsTiles = 8 * 152;
 constexpr size_t kRowsKernels = 8;
 
@@ -1688,9 +1689,10 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
             return fail_err(err, GBH_ERR_CUDA, "upload of the tile types failed");
     }
 
-    // ---- row-parallel steps of small batches, for the autotuner ----
+    // ---- row-parallel steps of small batches, for the autotuner or alone ----
     std::vector<Launch> rplan;
-    if (!e->has_network && e->opt.jit == 0 && e->opt.steps_per_launch == 0 && jit_available(nullptr)) {
+    const bool rows_only = e->opt.jit == kJitRows;   // the plan without a trial
+    if (!e->has_network && (rows_only || (e->opt.jit == 0 && e->opt.steps_per_launch == 0)) && jit_available(nullptr)) {
         const int rcw = rows_plan(e, members, prog_pool, tg, rplan);
         if (rcw) return fail_err(err, rcw, "%s", g_last_error);
     }
@@ -1712,7 +1714,7 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         std::vector<int> cand;
         for (int ti : torder)
             if (type_t0[ti] >= 0 && !e->types[ti].wide && !e->types[ti].sym && !e->types[ti].nitot &&
-                !e->types[ti].level && e->types[ti].nslots <= kJitMaxSlots)
+                !e->types[ti].level && !(rows_only && e->types[ti].rows) && e->types[ti].nslots <= kJitMaxSlots)
                 cand.push_back(ti);
         std::stable_sort(cand.begin(), cand.end(), [&](int a, int b) {
             return (type_t1[a] - type_t0[a]) > (type_t1[b] - type_t0[b]);
@@ -1730,7 +1732,8 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         e->jit_compact.clear();
         e->jit_smemrows.clear();
         e->jit_warps.clear();
-        const int form = e->opt.jit;   // 0 autotuned, 1 unrolled, 2 compact, 3 unrolled with shared rows
+        // 0 autotuned, 1 unrolled, 2 compact, 3 unrolled with shared rows
+        const int form = rows_only ? 1 : e->opt.jit;
         if (e->opt.steps_per_launch > 0 || form > 0) {
             const bool unrolled = form == 0 || form == 1;
             e->jit_minb.push_back(unrolled ? 24 : 6);
@@ -1865,10 +1868,11 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         if (rcg) return rcg;
     }
     if (!rplan.empty()) {
-        e->rows_launches = lplan.launches;
-        e->rows_launches.insert(e->rows_launches.end(), rplan.begin(), rplan.end());
-        const int rcr = plan(e->rows_launches, lvl, true);
-        if (rcr) return rcr;
+        std::vector<Launch> &out = rows_only ? e->launches : e->rows_launches;
+        out = lplan.launches;
+        out.insert(out.end(), rplan.begin(), rplan.end());
+        const int rcr = plan(out, lvl, true);
+        if (rcr || rows_only) return rcr;
     }
     e->launches = lplan.launches;
     return plan(e->launches, lvl, false);
@@ -3115,8 +3119,9 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
 // steps per launch are autotuned, row-parallel (rows_type)?
 bool level_everywhere(const gbh_engine *e)
 {
-    if (e->has_network || e->opt.jit != 0 || !jit_available(nullptr)) return false;
-    const bool small = e->opt.steps_per_launch == 0 && (int64_t)e->dec.neurons.size() <= kRowsTiles;
+    if (e->has_network || (e->opt.jit != 0 && e->opt.jit != kJitRows) || !jit_available(nullptr)) return false;
+    const bool small = (e->opt.steps_per_launch == 0 || e->opt.jit == kJitRows) &&
+                       (int64_t)e->dec.neurons.size() <= kRowsTiles;
     struct Seen { const Neuron *first; bool uniform; };
     std::map<std::string, Seen> types;
     std::vector<int> fl;
@@ -3137,7 +3142,9 @@ bool level_everywhere(const gbh_engine *e)
         tt.nstatic = static_rows(slot_field_ranges(prog, tt), tt.nslots);
         LevelProg lp;
         RowsProg rp;
-        if (!level_type(tt, prog, N.parent, kv.second.uniform, lp) && !(small && rows_type(tt, prog, rp))) return false;
+        if (!(e->opt.jit == 0 && level_type(tt, prog, N.parent, kv.second.uniform, lp)) &&
+            !(small && rows_type(tt, prog, rp)))
+            return false;
     }
     return true;
 }

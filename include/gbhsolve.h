@@ -171,7 +171,9 @@ typedef struct gbh_options {
                             and compact (runs of identical compartments looped)
                             -- and let the autotuner pick; 1 = unrolled form
                             only; 2 = compact form only; 3 = unrolled form with
-                            shared-memory rows only; -1 = interpret the
+                            shared-memory rows only; 4 = a thread per
+                            compartment wherever the batch allows it (below),
+                            without a trial, else as 1; -1 = interpret the
                             programs. With 0 (no synapses), trees whose
                             dendrites are passive are eliminated level by
                             level over several warps, and for small batches
