@@ -109,6 +109,13 @@ __device__ __forceinline__ void finite_check(const DevView &v, double x, bool ac
     if (!(fabs(x) <= 1.0e30) && active && v.status) atomicOr(v.status, ST_NONFINITE);
 }
 
+// The same on x's high word, without FP64 instructions, where every row is
+// checked.
+__device__ __forceinline__ void finite_row(const DevView &v, double x)
+{
+    if (((unsigned)__double2hiint(x) & 0x7fffffffu) >= 0x46293e59u && v.status) atomicOr(v.status, ST_NONFINITE);
+}
+
 // Named barrier `id` (1-15; 0 is __syncthreads') over `n` threads, a
 // multiple of 32: warps that do different work in a step meet here from
 // different places in the code.

@@ -1186,7 +1186,10 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
         o << (mixed ? " r = r * D" + S : " r = div_rn(r, D" + S + ")") << "; U[" << r << "] = r;";
         if (tt.crank) o << " Vw[" << r << "] = " << (mixed ? "fma(2.0, r, -Vw[" + r + "]);" : "r + r - Vw[" + r + "];");
         else o << " Vw[" << r << "] = r;";
-        if (s == N - 1) o << " finite_check(v, r, active);";   // the root: a NaN anywhere below it reaches it
+        // the root: a NaN of the static rows, which stay in FP64, reaches it; the mixed form's channel rows lose theirs
+        // to a value near 2^128
+        if (mixed) o << " finite_row(v, r);";
+        else if (s == N - 1) o << " finite_check(v, r, active);";
         o << " }\n";
     }
     o << "    }\n    __syncwarp();\n    bar_named(LB_TOP, blockDim.x);\n  }\n}\n";

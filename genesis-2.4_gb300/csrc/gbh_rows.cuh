@@ -223,7 +223,10 @@ __device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup 
                 r = div_by(r, D, y);
             }
             q.R[e] = r;
-            if (p == g.n) finite_check(v, r, true);   // the root: a NaN anywhere in the tree reaches it
+            // every row: the mixed form turns a lost Vm into a value near 2^128
+            // (finite_check), which the couplings on the way to the root take
+            // below its bound in a long tree
+            finite_row(v, r);
         }
         if (c + 1 < g.nch) back(c + 1);
         if (last) __syncthreads();
