@@ -803,6 +803,14 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
 {
     const Decoded &dec = e->dec;
     const bool mixed = e->opt.precision == GBH_PREC_MIXED;
+    // shared memory of a group of n neurons (a chunk has at least 32 rows or
+    // ends a level); does one neuron's block hold its constants too?
+    auto need = [&](const TileType &tt, int nt_top, int n, bool res) {
+        return level_smem(nt_top, n * tt.nstatic, n * tt.nstatic / LANES + tt.nstatic + 1, tt.crank != 0, mixed, res);
+    };
+    auto resident = [&](const TileType &tt, int nt_top) {
+        return need(tt, nt_top, 1, true) <= (size_t)kLevelSmemMax;
+    };
     // ---- eligible types and their kernels ----
     std::map<std::string, int> kern;
     std::vector<std::string> srcs;
@@ -821,12 +829,14 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
             if (src.empty()) continue;
             it = kern.emplace(lp.key, (int)kern.size()).first;
             srcs.push_back(src);   // kernel 2k: constants resident in shared memory, 2k + 1: streamed
-            srcs.push_back(jit_level_source(lp, tt, tg[tt.table_set], mixed, false));
+            srcs.emplace_back();
         }
         tt.level = 1 + it->second;
         tt.lv_f0 = lp.f0;
         ntop[ti] = lp.ntop;
-        cells += (int64_t)members[ti].size();
+        std::string &streamed = srcs[2 * it->second + 1];
+        if (streamed.empty() && !resident(tt, lp.ntop))
+            streamed = jit_level_source(lp, tt, tg[tt.table_set], mixed, false);
     }
     if (srcs.empty()) return GBH_OK;
     int major = 10, minor = 3;
@@ -837,33 +847,30 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
     std::vector<std::string> logs(srcs.size());
     std::vector<std::thread> th;
     for (size_t c = 0; c < srcs.size(); ++c)
-        th.emplace_back([&, c]() {
-            cudaSetDevice(e->opt.device);
-            ok[c] = jit_compile(srcs[c], !mixed, major, minor, &e->lv_kern[c], &logs[c]) == 0 &&
-                    jit_allow_smem(e->lv_kern[c], kLevelSmemMax);
-        });
+        if (!srcs[c].empty())
+            th.emplace_back([&, c]() {
+                cudaSetDevice(e->opt.device);
+                ok[c] = jit_compile(srcs[c], !mixed, major, minor, &e->lv_kern[c], &logs[c]) == 0 &&
+                        jit_allow_smem(e->lv_kern[c], kLevelSmemMax);
+            });
     for (auto &x : th) x.join();
     for (size_t c = 0; c < srcs.size(); ++c)
-        if (!ok[c]) {   // these types keep the stack elimination
-            if (e->jit_log.size() < 4000) e->jit_log += logs[c];
-            for (TileType &tt : e->types)
-                if (tt.level == 1 + (int)c / 2) tt.level = 0;
-        }
+        if (!ok[c] && e->jit_log.size() < 4000) e->jit_log += logs[c];
+    for (size_t k = 0; k < kern.size(); ++k) e->jit_compiled += ok[2 * k] || ok[2 * k + 1];
+    for (size_t ti = 0; ti < e->types.size(); ++ti) {
+        TileType &tt = e->types[ti];
+        if (!tt.level) continue;
+        if (ok[2 * (tt.level - 1) + (resident(tt, ntop[ti]) ? 0 : 1)]) cells += (int64_t)members[ti].size();
+        else tt.level = 0;   // keeps the stack elimination
+    }
     // ---- groups: enough of them for every SM, as many neurons each as that
     // leaves (the top rows' warp issues for 32 neurons what it issues for one) ----
     const int per_cells = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + kLevelGroups - 1) / kLevelGroups));
-    // neurons of a type that go into one group: their rows fit the shared
-    // memory (a chunk has at least 32 rows or ends a level); resident: so do
-    // their constants
+    // neurons of a type that go into one group
     auto most_cells = [&](const TileType &tt, int nt_top, bool &res) {
-        auto need = [&](int n) {
-            return level_smem(nt_top, n * tt.nstatic, n * tt.nstatic / LANES + tt.nstatic + 1, tt.crank != 0, mixed,
-                              res);
-        };
-        res = true;
-        res = need(1) <= (size_t)kLevelSmemMax;
+        res = resident(tt, nt_top);
         int fit = per_cells;
-        while (fit > 1 && need(fit) > (size_t)kLevelSmemGroup) --fit;
+        while (fit > 1 && need(tt, nt_top, fit, res) > (size_t)kLevelSmemGroup) --fit;
         return fit;
     };
     // sweeping warps: as many as a level has rows for, on average; twice that
@@ -1085,12 +1092,14 @@ int rows_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const
                     jit_allow_smem(e->rw_kern[c], kLevelSmemMax);
         });
     for (auto &x : th) x.join();
-    for (size_t c = 0; c < srcs.size(); ++c)
+    for (size_t c = 0; c < srcs.size(); ++c) {
+        e->jit_compiled += ok[c];
         if (!ok[c]) {
             if (e->jit_log.size() < 4000) e->jit_log += logs[c];
             for (TileType &tt : e->types)
                 if (tt.rows == 1 + (int)c) tt.rows = 0;
         }
+    }
     const int per = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + kLevelGroups - 1) / kLevelGroups));
     std::vector<RowGroup> groups;
     std::vector<int2> chunks, work, link;
@@ -3323,7 +3332,7 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
     e->stats.warps_per_block = e->launches.empty() ? 0 : e->launches[0].warps;
     if (!e->launches.empty() && e->launches[0].jit >= 0 && !e->jit_warps.empty())
         e->stats.warps_per_block = e->jit_warps[e->jit_choice];
-    e->stats.jit_kernels = e->jit_compiled + (int)e->lv_kern.size();
+    e->stats.jit_kernels = e->jit_compiled;
     e->stats.jit_min_blocks = e->jit_minb.empty() ? 0 : e->jit_minb[e->jit_choice];
     e->stats.jit_compact = e->jit_compact.empty() ? 0
                            : e->jit_compact[e->jit_choice] ? 1
