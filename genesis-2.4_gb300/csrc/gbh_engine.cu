@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "gbh_decode.h"
+#include "gbh_parallel.h"
 #include "gbh_kernels.cuh"
 #include "gbh_df.cuh"
 #include "gbh_jit.h"
@@ -845,15 +846,11 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
     e->lv_kern.resize(srcs.size());
     std::vector<int> ok(srcs.size(), 0);
     std::vector<std::string> logs(srcs.size());
-    std::vector<std::thread> th;
-    for (size_t c = 0; c < srcs.size(); ++c)
-        if (!srcs[c].empty())
-            th.emplace_back([&, c]() {
-                cudaSetDevice(e->opt.device);
-                ok[c] = jit_compile(srcs[c], !mixed, major, minor, &e->lv_kern[c], &logs[c]) == 0 &&
-                        jit_allow_smem(e->lv_kern[c], kLevelSmemMax);
-            });
-    for (auto &x : th) x.join();
+    in_threads(srcs.size(), [&](size_t c) { return !srcs[c].empty(); }, [&](size_t c) {
+        cudaSetDevice(e->opt.device);
+        ok[c] = jit_compile(srcs[c], !mixed, major, minor, &e->lv_kern[c], &logs[c]) == 0 &&
+                jit_allow_smem(e->lv_kern[c], kLevelSmemMax);
+    });
     for (size_t c = 0; c < srcs.size(); ++c)
         if (!ok[c] && e->jit_log.size() < 4000) e->jit_log += logs[c];
     for (size_t k = 0; k < kern.size(); ++k) e->jit_compiled += ok[2 * k] || ok[2 * k + 1];
@@ -1084,14 +1081,11 @@ int rows_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const
     e->rw_kern.resize(srcs.size());
     std::vector<int> ok(srcs.size(), 0);
     std::vector<std::string> logs(srcs.size());
-    std::vector<std::thread> th;
-    for (size_t c = 0; c < srcs.size(); ++c)
-        th.emplace_back([&, c]() {
-            cudaSetDevice(e->opt.device);
-            ok[c] = jit_compile(srcs[c], !mixed, major, minor, &e->rw_kern[c], &logs[c]) == 0 &&
-                    jit_allow_smem(e->rw_kern[c], kLevelSmemMax);
-        });
-    for (auto &x : th) x.join();
+    in_threads(srcs.size(), [](size_t) { return true; }, [&](size_t c) {
+        cudaSetDevice(e->opt.device);
+        ok[c] = jit_compile(srcs[c], !mixed, major, minor, &e->rw_kern[c], &logs[c]) == 0 &&
+                jit_allow_smem(e->rw_kern[c], kLevelSmemMax);
+    });
     for (size_t c = 0; c < srcs.size(); ++c) {
         e->jit_compiled += ok[c];
         if (!ok[c]) {
@@ -1781,14 +1775,10 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         std::vector<JitKernel> ks(srcs.size());
         std::vector<int> ok(srcs.size(), 0);
         std::vector<std::string> logs(srcs.size());
-        std::vector<std::thread> th;
-        for (size_t c = 0; c < srcs.size(); ++c)
-            th.emplace_back([&, c]() {
-                cudaSetDevice(dev);
-                if (!srcs[c].empty())
-                    ok[c] = jit_compile(srcs[c], !mixed, major, minor, &ks[c], &logs[c]) == 0;
-            });
-        for (auto &x : th) x.join();
+        in_threads(srcs.size(), [&](size_t c) { return !srcs[c].empty(); }, [&](size_t c) {
+            cudaSetDevice(dev);
+            ok[c] = jit_compile(srcs[c], !mixed, major, minor, &ks[c], &logs[c]) == 0;
+        });
         for (size_t c = 0; c < cand.size(); ++c) {
             bool all = true;
             for (int vi = 0; vi < nvar; ++vi) all = all && ok[c * nvar + vi];
