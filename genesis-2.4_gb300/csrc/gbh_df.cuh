@@ -157,10 +157,10 @@ __device__ __forceinline__ df d2df_volt(double d)
 
 // df -> double on the integer pipe: lo's significand, shifted to hi's unit in
 // the last place and rounded there to nearest even, is added to or taken from
-// hi's bits: the FP64 sum of the two (a denormal part counts as zero). No FP64
-// instruction: the FP64 unit takes one warp instruction per 19 clocks of an SM,
-// an addition as much as a multiply-add. Needs |lo| below hi's unit in the
-// last place (any df but an unfinished one).
+// hi's bits: the FP64 sum of the two (hi below the float normal range gives a
+// signed zero). No FP64 instruction: the FP64 unit takes one warp instruction
+// per 19 clocks of an SM, an addition as much as a multiply-add. Needs |lo|
+// below hi's unit in the last place (any df but an unfinished one).
 __device__ __forceinline__ double df2d(df x)
 {
     const uint32_t uh = __float_as_uint(x.hi), ul = __float_as_uint(x.lo);
@@ -170,10 +170,9 @@ __device__ __forceinline__ double df2d(df x)
     const bool minus = (int)(uh ^ ul) < 0;
     // lo in units of 2^-52 of hi's binade, half of that where the difference
     // falls below hi's power of two: its 24 bits, 7 places up and sh down
-    const uint32_t sh = eh - el - 22u - (minus && (uh & 0x7fffffu) == 0u ? 1u : 0u);
-    const uint32_t a = ((ul << 7) & 0x3fffff80u) | 0x40000000u;
-    uint32_t m = 0u;
-    if (el && sh < 32u) m = (a + (1u << (sh - 1u)) - 1u + ((a >> sh) & 1u)) >> sh;
+    const uint32_t sh = eh - max(el, 1u) - 22u - (minus && (uh & 0x7fffffu) == 0u ? 1u : 0u);
+    const uint32_t a = ((ul & 0x7fffffu) | (el ? 0x800000u : 0u)) << 7;
+    const uint32_t m = sh < 32u ? (a + (1u << (sh - 1u)) - 1u + ((a >> sh) & 1u)) >> sh : 0u;
     const uint64_t mag = ((uint64_t)h << 32) | l;
     const uint64_t r = minus ? mag - m : mag + m;
     return __hiloint2double(eh == 0u ? (int)sign : (int)((uint32_t)(r >> 32) | sign), eh == 0u ? 0 : (int)(uint32_t)r);

@@ -21,11 +21,6 @@ __device__ uint64_t rnd(uint64_t &s)
     return z ^ (z >> 31);
 }
 
-__device__ double widen(float f)   // denormals count as zero
-{
-    return fabsf(f) < 0x1p-126f ? 0.0 : (double)f;
-}
-
 enum { STEP, CONVERT, STEP64, STEP_INT, N };
 
 __global__ void k_check(unsigned long long *bad, int rounds, uint64_t seed)
@@ -71,7 +66,7 @@ __global__ void k_check(unsigned long long *bad, int rounds, uint64_t seed)
         }
         if (hi < 0.0f ? lo > 0.0f : lo < 0.0f)   // taken off a power of two: half a unit below it
             if ((__float_as_uint(hi) & 0x7fffffu) == 0u) lo *= 0.5f;
-        const double a = df2d(df_make(hi, lo)), c = widen(hi) + widen(lo);
+        const double a = df2d(df_make(hi, lo)), c = (double)hi + (double)lo;
         b[CONVERT] += __double_as_longlong(a) != __double_as_longlong(c);
     }
     for (int j = 0; j < N; ++j)
