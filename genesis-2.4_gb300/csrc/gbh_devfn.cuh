@@ -100,17 +100,19 @@ struct DevView {
 
 // A neuron whose Vm is no longer finite: a NaN or infinity anywhere in its
 // tree reaches every row through the elimination within the step, so one
-// row per neuron per step is checked (after back substitution). The mixed
-// form's exact float<->double conversions run on the integer pipe and turn a
-// NaN or infinity into a finite value near 2^128, so any |Vm| above 1e30 --
-// no voltage in any unit system -- counts as lost as well.
+// row per neuron per step is checked (after back substitution). |Vm| above
+// 1e30 -- no voltage in any unit system -- counts as lost as well.
 __device__ __forceinline__ void finite_check(const DevView &v, double x, bool active)
 {
     if (!(fabs(x) <= 1.0e30) && active && v.status) atomicOr(v.status, ST_NONFINITE);
 }
 
-// The same on x's high word, without FP64 instructions, where every row is
-// checked.
+// The mixed form loses a NaN or infinity on the way: its float<->double
+// conversions run on the integer pipe and make it a finite value near 2^128,
+// in a row's diagonal (through the gates' tables) as in its right-hand side,
+// whose quotient looks like any voltage. So every row's diagonal is checked
+// where it is formed, and a solution that other rows' couplings would take
+// below the bound, on the high word of x: no FP64 instruction.
 __device__ __forceinline__ void finite_row(const DevView &v, double x)
 {
     if (((unsigned)__double2hiint(x) & 0x7fffffffu) >= 0x46293e59u && v.status) atomicOr(v.status, ST_NONFINITE);

@@ -252,7 +252,8 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
             if (mx) {
                 o << "      { const df tbyc = " << E.ldr(a[0]) << "; const df dv = df_mul(ichan, tbyc);\n"
                   << "        R[" << E.S(s) << "] = df2d_row(df_add(vmd, dv));\n"
-                  << "        D[" << E.S(s) << "] = df2d_row(df_add(" << E.ldr(a[1]) << ", df_mul(sumg, tbyc))); }\n";
+                  << "        D[" << E.S(s) << "] = df2d_row(df_add(" << E.ldr(a[1]) << ", df_mul(sumg, tbyc)));\n"
+                  << "        if (active) finite_row(v, D[" << E.S(s) << "]); }\n";
             } else {
                 o << "      { const double tbyc = " << E.Pr(a[0]) << "; R[" << E.S(s) << "] = Vm + ichan * tbyc; D[" << E.S(s)
                   << "] = sumg * tbyc + " << E.Pr(a[1]) << "; }\n";
@@ -1186,10 +1187,9 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
         o << (mixed ? " r = r * D" + S : " r = div_rn(r, D" + S + ")") << "; U[" << r << "] = r;";
         if (tt.crank) o << " Vw[" << r << "] = " << (mixed ? "fma(2.0, r, -Vw[" + r + "]);" : "r + r - Vw[" + r + "];");
         else o << " Vw[" << r << "] = r;";
-        // the root: a NaN of the static rows, which stay in FP64, reaches it; the mixed form's channel rows lose theirs
-        // to a value near 2^128
-        if (mixed) o << " finite_row(v, r);";
-        else if (s == N - 1) o << " finite_check(v, r, active);";
+        // the root: a NaN of the static rows, which stay in FP64, reaches it; the mixed form's rows with channels are
+        // checked where they lose theirs (M_END)
+        if (s == N - 1) o << " finite_check(v, r, active);";
         o << " }\n";
     }
     o << "    }\n    __syncwarp();\n    bar_named(LB_TOP, blockDim.x);\n  }\n}\n";

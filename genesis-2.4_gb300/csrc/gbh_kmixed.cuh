@@ -68,7 +68,6 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
     const int64_t neuron = N.neuron;
     const bool active = N.active;
     (void)neuron;
-    (void)active;
     (void)c1;
     const df vmd = d2df_volt(Vm);
     df sumg = df_make(0.f, 0.f), ichan = sumg;
@@ -133,6 +132,7 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
             const df dv = df_mul(ichan, tbyc);
             R = df2d_row(df_add(vmd, dv));
             D = df2d_row(df_add(ld_df(&N.P[(pc[2]) * STR]), df_mul(sumg, tbyc)));
+            if (active) finite_row(v, D);
             if (GIV) N.G[(pc[3]) * STR] = Im;
             pc += 4;
             break;

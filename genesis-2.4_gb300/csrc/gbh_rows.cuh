@@ -223,9 +223,8 @@ __device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup 
                 r = div_by(r, D, y);
             }
             q.R[e] = r;
-            // every row: the mixed form turns a lost Vm into a value near 2^128
-            // (finite_check), which the couplings on the way to the root take
-            // below its bound in a long tree
+            // every row: without a channel to show in the diagonal, a Vm the mixed
+            // form has lost (finite_row) shows in its own solution alone
             finite_row(v, r);
         }
         if (c + 1 < g.nch) back(c + 1);

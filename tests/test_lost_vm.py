@@ -37,3 +37,13 @@ def test_level_tree(gpu_engine, prec, row):
     eng = gpu_engine.Engine(hs, precision=p, steps_per_launch=16)
     assert eng.stats().stack_tiles == eng.stats().tiles
     _lose(eng, 60 * 2 + {"leaf": 0, "top": 56, "root": 59}[row], np.nan)
+
+
+@pytest.mark.parametrize("kw", [dict(jit=False, wide_min=-1), dict(jit=1, wide_min=-1), dict(jit=2, wide_min=-1),
+                                dict(jit=False, wide_min=32)])
+@pytest.mark.parametrize("row", [0, 20, 39])
+def test_mixed_channel_rows(gpu_engine, kw, row):
+    """Rows with channels under the other mappings: lane-mapped interpreted,
+    specialised and compact, and one neuron per block."""
+    hs = [model.build(configs.cables(1, ncomp=40, gk_dend=36.0)[0]) for _ in range(40)]
+    _lose(gpu_engine.Engine(hs, precision=gpu_engine.PREC_MIXED, steps_per_launch=10, **kw), 40 * 33 + row, np.nan)
