@@ -253,7 +253,7 @@ bool emit_slot(Emit &E, int s, const int *&pc, const TableGeom &tg)
                 o << "      { const df tbyc = " << E.ldr(a[0]) << "; const df dv = df_mul(ichan, tbyc);\n"
                   << "        R[" << E.S(s) << "] = df2d_row(df_add(vmd, dv));\n"
                   << "        D[" << E.S(s) << "] = df2d_row(df_add(" << E.ldr(a[1]) << ", df_mul(sumg, tbyc)));\n"
-                  << "        if (active) finite_row(v, D[" << E.S(s) << "]); }\n";
+                  << "        see_row(lost, D[" << E.S(s) << "]); }\n";
             } else {
                 o << "      { const double tbyc = " << E.Pr(a[0]) << "; R[" << E.S(s) << "] = Vm + ichan * tbyc; D[" << E.S(s)
                   << "] = sumg * tbyc + " << E.Pr(a[1]) << "; }\n";
@@ -580,6 +580,7 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
     E.stream = uniform_parent && !cols;
     o << "  const " << (E.stream ? "RoStream" : "RoRow")
       << "<double> Aw{v.A + tl.topo * 32 + lane}, Bw{v.B + tl.topo * 32 + lane}, Cbw{v.Cb + tl.topo * 32 + lane};\n";
+    if (mixed) o << "  unsigned lost = 0u;\n";
     o << "  for (int it = 0; it < nsteps; ++it) {\n"
       << "    const long long step = sbase + step0 + it; (void)step;\n"
       << "    if (v.io_in) {   // this step's inputs into the tile's fields, then visible to every lane\n"
@@ -844,7 +845,7 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
       << "      for (int q = v.tout_start[t] + lane; q < v.tout_start[t + 1]; q += 32) dst[v.tout_idx[q]] = Vt[v.tout_off[q]]; }\n";
     // networks, several steps in a cooperative launch: events cross tiles
     if (tt.nsyn > 0 || tt.has_spike) t << "    if (v.gbar && !grid_sync(v.gbar, gridDim.x, v.status)) return;\n";
-    t << "  }\n}\n";
+    t << "  }\n" << (mixed ? "  lost_rows(v, lost, active);\n" : "") << "}\n";
     return t.str();
 }
 
@@ -1036,7 +1037,7 @@ std::string jit_rows_source(const RowsProg &rp, const TileType &tt, const TableG
           << "  const double *xvals = v.xyvals + " << tg.xv_off << "; (void)xvals;\n"
           << "  const double *yvals = v.xyvals + " << (tg.yv_off >= 0 ? tg.yv_off : tg.xv_off) << "; (void)yvals;\n";
     }
-    o << "  rows_load(L, g, q, Vt);\n"
+    o << "  rows_load(L, g, q, Vt);\n  unsigned lost = 0u;\n"
       << "  for (int it = 0; it < nsteps; ++it) {\n"
       << "    const long long step = sbase + step0 + it; (void)step;\n"
       << "    if (v.io_in) {   // this step's inputs into the group's fields\n"
@@ -1087,14 +1088,14 @@ std::string jit_rows_source(const RowsProg &rp, const TileType &tt, const TableG
         emit_ca_pools(o, rp.pool.data());
         o << "    }\n";
     }
-    o << "    rows_eliminate<" << form << ", " << crank << ">(v, g, q);\n"
+    o << "    rows_eliminate<" << form << ", " << crank << ">(v, g, q, lost);\n"
       << "    if (v.io_out) {   // this step's outputs\n"
       << "      for (int e = tid; e < g.n; e += blockDim.x) Vt[map[e]] = q.V[e];\n"
       << "      __syncthreads(); double *dst = v.io_out + (step - v.io_step0) * v.io_nout;\n"
       << "      for (int k = v.tout_start[g.tile] + tid; k < v.tout_start[g.tile + 1]; k += blockDim.x) {\n"
       << "        const int off = v.tout_off[k], l = off & 31; if (l >= g.lane0 && l < g.lane0 + g.nlanes) dst[v.tout_idx[k]] = Vt[off]; } }\n"
       << "  }\n"
-      << "  for (int e = tid; e < g.n; e += blockDim.x) Vt[map[e]] = q.V[e];\n}\n";
+      << "  for (int e = tid; e < g.n; e += blockDim.x) Vt[map[e]] = q.V[e];\n  lost_rows(v, lost, true);\n}\n";
     return o.str();
 }
 
@@ -1147,7 +1148,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
           << "  const double *yvals = v.xyvals + " << (tg.yv_off >= 0 ? tg.yv_off : tg.xv_off) << "; (void)yvals;\n";
     }
     o << "  const LevelSm q = level_smem_of<" << form << ", " << crank << ", " << N << ", " << res
-      << ">(sm, g);\n  double *U = q.U + lid;\n"
+      << ">(sm, g);\n  double *U = q.U + lid;\n  unsigned lost = 0u; (void)lost;\n"
       << "  for (int it = 0; it < nsteps; ++it) {\n"
       << "    const long long step = sbase + step0 + it; (void)step;\n"
       << "    double D[" << N << "], R[" << N << "], T[" << N << "], PD[" << N << "]; (void)T; (void)PD;\n"
@@ -1192,7 +1193,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
         if (s == N - 1) o << " finite_check(v, r, active);";
         o << " }\n";
     }
-    o << "    }\n    __syncwarp();\n    bar_named(LB_TOP, blockDim.x);\n  }\n}\n";
+    o << "    }\n    __syncwarp();\n    bar_named(LB_TOP, blockDim.x);\n  }\n  lost_rows(v, lost, active);\n}\n";
     return o.str();
 }
 

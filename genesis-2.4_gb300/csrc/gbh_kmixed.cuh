@@ -132,7 +132,9 @@ __device__ __forceinline__ bool chan_compartment_df(const DevView &v, const Chan
             const df dv = df_mul(ichan, tbyc);
             R = df2d_row(df_add(vmd, dv));
             D = df2d_row(df_add(ld_df(&N.P[(pc[2]) * STR]), df_mul(sumg, tbyc)));
-            if (active) finite_row(v, D);
+            unsigned lost = 0u;
+            see_row(lost, D);
+            lost_rows(v, lost, active);
             if (GIV) N.G[(pc[3]) * STR] = Im;
             pc += 4;
             break;

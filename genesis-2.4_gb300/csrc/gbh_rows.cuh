@@ -160,7 +160,7 @@ __device__ __forceinline__ void rows_cursors(const RowView &L, const RowGroup &g
 // backward -- and whatever does not wait for the level before is read ahead of
 // its barrier.
 template <bool MIXED, bool CRANK>
-__device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup &g, const RowSm &q)
+__device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup &g, const RowSm &q, unsigned &lost)
 {
     const int tid = threadIdx.x;
     int2 m = q.ch[g.nch - 1];
@@ -223,9 +223,9 @@ __device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup 
                 r = div_by(r, D, y);
             }
             q.R[e] = r;
-            // every row: without a channel to show in the diagonal, a Vm the mixed
-            // form has lost (finite_row) shows in its own solution alone
-            finite_row(v, r);
+            // FP64: the root, which a NaN anywhere in the tree reaches
+            if (MIXED) see_row(lost, r);
+            else if (p == g.n) finite_check(v, r, true);
         }
         if (c + 1 < g.nch) back(c + 1);
         if (last) __syncthreads();
