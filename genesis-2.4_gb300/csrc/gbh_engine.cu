@@ -189,6 +189,7 @@ struct gbh_engine {
     DBuf<int4> d_ritems;
     DBuf<int> d_rmap, d_rprev, d_rpos;
     DBuf<double> d_rA, d_rB, d_rC;
+    int nsm = 152;           // the device's SMs (GB300's where the query fails)
     int steps_per_launch = 1;
     bool has_network = false;
     bool givals_enabled = false;
@@ -473,9 +474,9 @@ constexpr int kStackCapMax = 200 * 1024 / (LANES * (int)sizeof(double)) - 2 * kS
 // Level elimination: most shared memory a block may take, and what groups of
 // several neurons are kept to (three blocks an SM: 16,384 random trees of
 // 8-256 compartments, mixed, 23.4 us a step; 110 KB 24.0, 224 KB 26.1, 40 KB
-// 25.4); groups wanted (one an SM; 2,000 trees, FP64: 12.1 us a step, 14.0
-// with two); distinct programs compiled.
-constexpr int kLevelSmemMax = 224 * 1024, kLevelSmemGroup = 72 * 1024, kLevelGroups = 152;
+// 25.4); distinct programs compiled. Groups are wanted one an SM (2,000 trees,
+// FP64, on 152 SMs: 12.1 us a step, 14.0 with two).
+constexpr int kLevelSmemMax = 224 * 1024, kLevelSmemGroup = 72 * 1024;
 constexpr size_t kLevelKernels = 8;
 
 // Largest types specialised whole: the looped forms keep 2 x nslots x 32 rows
@@ -862,7 +863,7 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
     }
     // ---- groups: enough of them for every SM, as many neurons each as that
     // leaves (the top rows' warp issues for 32 neurons what it issues for one) ----
-    const int per_cells = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + kLevelGroups - 1) / kLevelGroups));
+    const int per_cells = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + e->nsm - 1) / e->nsm));
     // neurons of a type that go into one group
     auto most_cells = [&](const TileType &tt, int nt_top, bool &res) {
         res = resident(tt, nt_top);
@@ -883,7 +884,7 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
             ngroups += (tl.nlanes + most - 1) / most;
         }
     }
-    const int spread = ngroups <= 2 * kLevelGroups ? 2 : 1;
+    const int spread = ngroups <= 2 * e->nsm ? 2 : 1;
     struct Cand { LevelGroup g; int warps, bucket; size_t smem; };
     std::vector<Cand> cand;
     LevelPools P;
@@ -981,7 +982,7 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
 // (the autotuner times it): eight tiles an SM. Beyond, the lanes of the SMs are
 // full either way and the barriers between levels only cost.
 constexpr int kJitRows = 4;   // gbh_options.jit: the row-parallel plan, untimed
-constexpr int64_t kRowsTiles = 8 * 152;
+constexpr int64_t kRowsTilesPerSm = 8;
 constexpr size_t kRowsKernels = 8;
 
 // Rows of some neurons of one type by depth: the roots, then the children of
@@ -1059,7 +1060,7 @@ int rows_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const
     int64_t cells = 0, tiles = 0;
     for (size_t ti = 0; ti < e->types.size(); ++ti)
         if (!e->types[ti].level && !e->types[ti].wide) tiles += ((int64_t)members[ti].size() + LANES - 1) / LANES;
-    if (tiles > kRowsTiles) return GBH_OK;
+    if (tiles > kRowsTilesPerSm * e->nsm) return GBH_OK;
     for (size_t ti = 0; ti < e->types.size(); ++ti) {
         TileType &tt = e->types[ti];
         if (tt.level || !rows_type(tt, prog_pool, prog[ti])) continue;
@@ -1094,7 +1095,7 @@ int rows_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const
                 if (tt.rows == 1 + (int)c) tt.rows = 0;
         }
     }
-    const int per = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + kLevelGroups - 1) / kLevelGroups));
+    const int per = (int)std::min<int64_t>(LANES, std::max<int64_t>(1, (cells + e->nsm - 1) / e->nsm));
     std::vector<RowGroup> groups;
     std::vector<int2> chunks, work, link;
     std::vector<int4> items;
@@ -1121,7 +1122,7 @@ int rows_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const
             const int most = most_cells(e->types[tl.type]);
             ngroups += (tl.nlanes + most - 1) / most;
         }
-    const bool crowded = ngroups > kLevelGroups;
+    const bool crowded = ngroups > e->nsm;
     for (size_t t = 0; t < e->tiles.size(); ++t) {
         const Tile &tl = e->tiles[t];
         const TileType &tt = e->types[tl.type];
@@ -3120,7 +3121,7 @@ bool level_everywhere(const gbh_engine *e)
 {
     if (e->has_network || (e->opt.jit != 0 && e->opt.jit != kJitRows) || !jit_available(nullptr)) return false;
     const bool small = (e->opt.steps_per_launch == 0 || e->opt.jit == kJitRows) &&
-                       (int64_t)e->dec.neurons.size() <= kRowsTiles;
+                       (int64_t)e->dec.neurons.size() <= kRowsTilesPerSm * e->nsm;
     struct Seen { const Neuron *first; bool uniform; };
     std::map<std::string, Seen> types;
     std::vector<int> fl;
@@ -3231,6 +3232,9 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
         delete e;
         return nullptr;
     }
+    int nsm = 0;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->opt.device) == cudaSuccess && nsm > 0)
+        e->nsm = nsm;
     int rc = GBH_OK;
     if (pre) e->dec = *pre;   // a trial engine over a batch already decoded
     else rc = decode_batch(desc, e->dec, err);
@@ -3615,7 +3619,7 @@ static int adj_plan(gbh_engine *e, int hmax)
     const OnDevice on(e->opt.device);   // kept for later calls, whatever device is current in this one
     CK(on.rc);
     const Decoded &dec = e->dec;
-    const int per = (int)std::min<size_t>(LANES, (dec.neurons.size() + kLevelGroups - 1) / kLevelGroups);
+    const int per = (int)std::min<size_t>(LANES, (dec.neurons.size() + e->nsm - 1) / e->nsm);
     std::vector<std::vector<int>> cells_of(e->tiles.size());
     for (size_t i = 0; i < dec.neurons.size(); ++i) {
         const int t = e->neuron_tile[i];
