@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <set>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -171,7 +172,11 @@ struct gbh_engine {
     int64_t rows_fld = 0, rows_int = 0, rows_pool = 0, rows_giv = 0, rows_vm = 0, rows_topo = 0,
             rows_syn = 0, rows_scr = 0, rows_rav = 0, rows_itot = 0;
     std::vector<Launch> launches;
-    std::vector<Launch> giv_launches;   // the plan of a step that records givals, where it differs
+    // every tile lane-mapped or wide, where `launches` has others: the plan of a
+    // step that records givals, and of single steps where it is the faster one
+    std::vector<Launch> lane_launches;
+    bool single_lane = false;
+    std::vector<Launch> level_launches;   // the level plan, timed against `launches` (empty: not timed)
     // level elimination (gbh_level.cuh)
     std::vector<JitKernel> lv_kern;
     DBuf<LevelGroup> d_lgroups;
@@ -189,6 +194,7 @@ struct gbh_engine {
     DBuf<int4> d_ritems;
     DBuf<int> d_rmap, d_rprev, d_rpos;
     DBuf<double> d_rA, d_rB, d_rC;
+    bool trial = false;      // built to time a mapping (choose_mapping)
     int nsm = 152;           // the device's SMs (GB300's where the query fails)
     int steps_per_launch = 1;
     bool has_network = false;
@@ -730,8 +736,8 @@ void wide_schedule(const std::vector<int> &parent, std::vector<int> &out)
 // ---- level elimination (gbh_level.cuh) ----
 // Is a type of neurons with passive dendrites swept level by level? Not when
 // its neurons share one tree of little branching (fewer than two rows a
-// level, as in a cable): the specialised kernel then keeps the rows in
-// registers and needs neither barriers nor indices. parent: any neuron's.
+// level, as in a cable) that the specialised kernel keeps in registers: it
+// then needs neither barriers nor indices. parent: any neuron's.
 bool level_type(const TileType &tt, const std::vector<int> &prog, const std::vector<int> &parent, bool uniform,
                 LevelProg &lp)
 {
@@ -744,6 +750,25 @@ bool level_type(const TileType &tt, const std::vector<int> &prog, const std::vec
     lp = level_prog(tt, prog);
     return lp.ok;
 }
+
+// Do these neurons' trees branch: two passive rows a level or more, on
+// average? Level elimination then beats the stack kernels whatever their
+// number. In an unbranched cable a level is one row: the block waits at a
+// barrier for it, and it is only the faster while the blocks have the SMs to
+// themselves (200 compartments, FP64, us a step, levels and stack: 600 neurons
+// 91 and 114, 1,200 186 and 114, 5,000 225 and 116).
+template <class At> bool branched(size_t n, int nstatic, At parent_of)
+{
+    int64_t levels = 0;
+    for (size_t i = 0; i < n; ++i) levels += static_levels(parent_of(i), nstatic);
+    return (int64_t)n * nstatic >= 2 * levels;
+}
+
+// Populations of one small tree from this many tiles an SM on keep the lanes
+// of the specialised kernels full: which of the two is faster is timed (20,000
+// trees, FP64, us a step, levels and lanes: 16 compartments 17.3 and 11.8, 64
+// compartments 36 and 55).
+constexpr int64_t kLevelTimedTilesPerSm = 2;
 
 struct LevelPlan {
     std::vector<LevelGroup> groups;
@@ -800,8 +825,9 @@ void level_order(const std::vector<const Neuron *> &cells, int nst, int ntop, st
     }
 }
 
+// timed: per type, the level plan is not certain to be the faster one.
 int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, const std::vector<int> &prog_pool,
-               const std::vector<TableGeom> &tg, LevelPlan &out)
+               const std::vector<TableGeom> &tg, LevelPlan &out, std::vector<char> &timed)
 {
     const Decoded &dec = e->dec;
     const bool mixed = e->opt.precision == GBH_PREC_MIXED;
@@ -824,6 +850,14 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
         for (int i : members[ti]) uni = uni && dec.neurons[i].parent == dec.neurons[members[ti][0]].parent;
         LevelProg lp;
         if (!level_type(tt, prog_pool, dec.neurons[members[ti][0]].parent, uni, lp)) continue;
+        const int64_t count = (int64_t)members[ti].size();
+        const bool branches = branched(members[ti].size(), tt.nstatic, [&](size_t i) -> const std::vector<int> & {
+            return dec.neurons[members[ti][i]].parent;
+        });
+        // (a trial engine is what times it)
+        if (!branches && e->opt.steps_per_launch != 0 && count > e->nsm && !e->trial) continue;
+        timed[ti] = !branches || (uni && tt.nslots <= kJitMaxSlots &&
+                                  (count + LANES - 1) / LANES > kLevelTimedTilesPerSm * e->nsm);
         auto it = kern.find(lp.key);
         if (it == kern.end()) {
             if (kern.size() >= kLevelKernels) continue;
@@ -1046,6 +1080,13 @@ bool rows_type(const TileType &tt, const std::vector<int> &prog, RowsProg &rp)
     rp = rows_prog(tt, prog);
     return rp.ok;
 }
+
+// Is a row-parallel type certain to be faster so than lane-mapped: channels on
+// most of its rows, and enough of them? (us a step, rows and the best
+// specialised form, 1 to 1,216 neurons: cables of 32 compartments 33 and
+// 51-62, mixed 24 and 30; trees of 32 13-16 and 90-122, mixed 9-11 and 40-44;
+// longer ones more. 300 mixed cables of 23 compartments 17.4 and 15.2.)
+bool rows_surely(const TileType &tt) { return tt.nslots >= 32 && 4 * tt.nstatic <= tt.nslots; }
 
 // Groups, kernels and launches of the types that can run row-parallel; their
 // TileType::rows is set. Leaves `out` empty when there are none.
@@ -1684,8 +1725,9 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
 
     // ---- level elimination of the trees with passive dendrites ----
     LevelPlan lplan;
+    std::vector<char> timed(e->types.size(), 0);
     if (!e->has_network && e->opt.jit == 0 && jit_available(nullptr)) {
-        const int rcl = level_plan(e, members, prog_pool, tg, lplan);
+        const int rcl = level_plan(e, members, prog_pool, tg, lplan, timed);
         if (rcl) return fail_err(err, rcl, "%s", g_last_error);
         // the types' level flags
         if (!lplan.groups.empty() && cudaMemcpy(e->d_types.p, e->types.data(), e->types.size() * sizeof(TileType),
@@ -1716,10 +1758,12 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
     if (jit_on) {
         // types in tile order, largest first
         std::vector<int> cand;
-        for (int ti : torder)
-            if (type_t0[ti] >= 0 && !e->types[ti].wide && !e->types[ti].sym && !e->types[ti].nitot &&
-                !e->types[ti].level && !(rows_only && e->types[ti].rows) && e->types[ti].nslots <= kJitMaxSlots)
+        for (int ti : torder) {
+            const TileType &tt = e->types[ti];
+            if (type_t0[ti] >= 0 && !tt.wide && !tt.sym && !tt.nitot && !(tt.level && !timed[ti]) &&
+                !(rows_only && tt.rows) && !(tt.rows && rows_surely(tt)) && tt.nslots <= kJitMaxSlots)
                 cand.push_back(ti);
+        }
         std::stable_sort(cand.begin(), cand.end(), [&](int a, int b) {
             return (type_t1[a] - type_t0[a]) > (type_t1[b] - type_t0[b]);
         });
@@ -1863,8 +1907,8 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         return (int)GBH_OK;
     };
     const bool lvl = !lplan.groups.empty();
-    if (lvl || !rplan.empty()) {   // a step with givals runs the interpreting kernels
-        const int rcg = plan(e->giv_launches, false, false);
+    if (lvl || !rplan.empty()) {
+        const int rcg = plan(e->lane_launches, false, false);
         if (rcg) return rcg;
     }
     if (!rplan.empty()) {
@@ -1874,8 +1918,14 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
         const int rcr = plan(out, lvl, true);
         if (rcr || rows_only) return rcr;
     }
-    e->launches = lplan.launches;
-    return plan(e->launches, lvl, false);
+    bool time_level = false;
+    for (size_t ti = 0; ti < e->types.size(); ++ti) time_level = time_level || (e->types[ti].level && timed[ti]);
+    time_level = time_level && e->opt.steps_per_launch == 0;
+    std::vector<Launch> &out = time_level ? e->level_launches : e->launches;
+    out = lplan.launches;
+    const int rcl = plan(out, lvl, false);
+    if (time_level) e->launches = e->lane_launches;
+    return rcl;
 }
 
 DevView view_of(gbh_engine *e)
@@ -2022,7 +2072,10 @@ int issue_steps(gbh_engine *e, const DevView &v, int nsteps, long long step0, bo
                 int64_t *kernels)
 {
     const bool mixed = e->opt.precision == GBH_PREC_MIXED;
-    const int nl = (int)e->launches.size();
+    // (per-step inputs and outputs inside the launches: the plan they were asked for)
+    const std::vector<Launch> &plan = nsteps == 1 && e->single_lane && !v.io_in && !v.io_out ? e->lane_launches
+                                                                                              : e->launches;
+    const int nl = (int)plan.size();
     const int ns = (int)e->side.size();
     const int plain = giv_last ? nsteps - 1 : nsteps;
     auto spikes = [&](long long step, cudaStream_t s) {   // spike detection before the step
@@ -2035,7 +2088,7 @@ int issue_steps(gbh_engine *e, const DevView &v, int nsteps, long long step0, bo
         for (int done = 0; done < plain;) {
             const int k = e->spike_pre ? 1 : std::min(e->steps_per_launch, plain - done);
             if (spikes(step0 + done, st)) return GBH_ERR_CUDA;
-            for (const Launch &L : e->launches) {
+            for (const Launch &L : plan) {
                 const int rc = launch_one(e, v, L, k, step0 + done, mixed, false, st);
                 if (rc) return rc;
                 if (kernels) ++*kernels;
@@ -2050,7 +2103,7 @@ int issue_steps(gbh_engine *e, const DevView &v, int nsteps, long long step0, bo
             CK(cudaEventRecord(e->ev_fork, st));
             for (int i = 0; i < ns; ++i) CK(cudaStreamWaitEvent(e->side[i], e->ev_fork, 0));
             for (int li = 0; li < nl; ++li) {
-                const Launch &L = e->launches[li];
+                const Launch &L = plan[li];
                 cudaStream_t s = e->side[li % ns];
                 for (int d = 0; d < n;) {
                     const int k = std::min(e->steps_per_launch, n - d);
@@ -2068,7 +2121,7 @@ int issue_steps(gbh_engine *e, const DevView &v, int nsteps, long long step0, bo
     }
     if (giv_last && nsteps > 0) {
         if (spikes(step0 + nsteps - 1, st)) return GBH_ERR_CUDA;
-        for (const Launch &L : e->giv_launches.empty() ? e->launches : e->giv_launches) {
+        for (const Launch &L : e->lane_launches.empty() ? e->launches : e->lane_launches) {
             const int rc = launch_one(e, v, L, 1, step0 + nsteps - 1, mixed, true, st);
             if (rc) return rc;
             if (kernels) ++*kernels;
@@ -2256,7 +2309,7 @@ int autotune_trials(gbh_engine *e)
     if (e->has_network) spls = {1};
     else spls = {16, 64, 256};
     const int nvar = e->jit_var.empty() ? 1 : (int)e->jit_var[0].size();
-    if ((int)spls.size() * nvar <= 1 && e->rows_launches.empty()) {
+    if ((int)spls.size() * nvar <= 1 && e->rows_launches.empty() && e->level_launches.empty()) {
         e->steps_per_launch = spls[0];
         return GBH_OK;
     }
@@ -2296,8 +2349,8 @@ int autotune_trials(gbh_engine *e)
     double best = 1e300;
     int best_v = 0, best_s = spls[0];
     // time per step of the plan and variant in use, from the saved state; one
-    // whose first steps take twice the best so far is not timed further
-    auto timed = [&](int spl, double &per) {
+    // whose first steps take twice `limit` is not timed further
+    auto timed = [&](int spl, double limit, double &per) {
         e->steps_per_launch = spl;
         int rc_t = run_steps(e, 2, e->stream);   // warm caches and clocks
         for (int steps : {8, std::max(2 * spl, 128)}) {
@@ -2310,7 +2363,7 @@ int autotune_trials(gbh_engine *e)
             // a variant that cannot launch here (resources) never wins
             per = rc_t == GBH_OK ? ms / steps : 1e300;
             if (rc_t != GBH_OK) cudaGetLastError();
-            if (per > 2.0 * best) break;
+            if (per > 2.0 * limit) break;
         }
         return restore();
     };
@@ -2318,38 +2371,41 @@ int autotune_trials(gbh_engine *e)
         for (size_t k = 0; k < e->jits.size(); ++k) e->jits[k] = e->jit_var[k][vi];
         e->jit_choice = vi;   // launch_one sizes the shared memory of the variant in use
     };
-    // the row-parallel plan of a small batch and every variant at the middle
-    // launch length, then the other launch lengths of the fastest: the length
-    // moves a step by a few per cent, the same way in every variant
+    // the row-parallel plan of a small batch, the level plan where it is not
+    // certain to win, and every variant at the middle launch length, then the
+    // other launch lengths of the fastest: the length moves a step by a few per
+    // cent, the same way in every variant
     const int mid = spls[spls.size() / 2];
-    bool use_rows = false;
-    if (!e->rows_launches.empty()) {
-        e->launches.swap(e->rows_launches);
+    std::vector<Launch> *use = nullptr;   // the plan to put in place of `launches`
+    const std::pair<std::vector<Launch> *, const char *> plans[] = {{&e->rows_launches, "row-parallel"},
+                                                                    {&e->level_launches, "level elimination"}};
+    for (const auto &pl : plans) {
+        if (pl.first->empty()) continue;
+        e->launches.swap(*pl.first);
         double per;
-        if (timed(mid, per)) return GBH_ERR_CUDA;
+        if (timed(mid, best, per)) return GBH_ERR_CUDA;
         if (getenv("GBH_VERBOSE"))
-            fprintf(stderr, "gbhsolve: trial row-parallel, %d steps/launch: %.2f us/step\n", mid, per * 1e3);
-        e->launches.swap(e->rows_launches);
-        use_rows = per < best;
-        if (use_rows) best = per;
+            fprintf(stderr, "gbhsolve: trial %s, %d steps/launch: %.2f us/step\n", pl.second, mid, per * 1e3);
+        e->launches.swap(*pl.first);
+        if (per < best) { best = per; use = pl.first; }
         best_s = mid;
     }
     for (int vi = 0; vi < nvar; ++vi) {
         use_variant(vi);
         double per;
-        if (timed(mid, per)) return GBH_ERR_CUDA;
-        if (getenv("GBH_VERBOSE") && !e->jit_minb.empty())
+        if (timed(mid, best, per)) return GBH_ERR_CUDA;
+        if (getenv("GBH_VERBOSE") && !e->jit_var.empty())
             fprintf(stderr, "gbhsolve: trial %d warps x min blocks %d, form %d, %d steps/launch: %.2f us/step\n",
                     e->jit_warps[vi], e->jit_minb[vi], e->jit_compact[vi] ? 1 : e->jit_smemrows[vi] ? 2 : 0, mid,
                     per * 1e3);
-        if (per < best) { best = per; best_v = vi; best_s = mid; use_rows = false; }
+        if (per < best) { best = per; best_v = vi; best_s = mid; use = nullptr; }
     }
     use_variant(best_v);
-    if (use_rows) e->launches.swap(e->rows_launches);
+    if (use) e->launches.swap(*use);
     for (int spl : spls) {
         if (spl == mid) continue;
         double per;
-        if (timed(spl, per)) return GBH_ERR_CUDA;
+        if (timed(spl, best, per)) return GBH_ERR_CUDA;
         if (getenv("GBH_VERBOSE")) fprintf(stderr, "gbhsolve: trial %d steps/launch: %.2f us/step\n", spl, per * 1e3);
         if (per < best) { best = per; best_s = spl; }
     }
@@ -3114,39 +3170,81 @@ namespace {
 gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, const gbh_remote_synapses *remote,
                         const gbh_options *opt, gbh_error *err, gbh_engine *&made, const Decoded *pre = nullptr);
 
-// Do all neurons that could run wide (32 compartments and more) run the
-// level elimination when lane-mapped (level_type), or, in a small batch whose
-// steps per launch are autotuned, row-parallel (rows_type)?
-bool level_everywhere(const gbh_engine *e)
+// What the level and row-parallel kernels serve of a batch's neurons that could
+// run wide (32 compartments and more) when they are lane-mapped instead.
+struct Served {
+    bool surely = false;             // all of them, and faster than any mapping a trial looks at
+    bool level = false, rows = false;   // some
+};
+
+Served kernels_serve(const gbh_engine *e)
 {
-    if (e->has_network || (e->opt.jit != 0 && e->opt.jit != kJitRows) || !jit_available(nullptr)) return false;
+    Served sv;
+    if (e->has_network || (e->opt.jit != 0 && e->opt.jit != kJitRows) || !jit_available(nullptr)) return sv;
     const bool small = (e->opt.steps_per_launch == 0 || e->opt.jit == kJitRows) &&
                        (int64_t)e->dec.neurons.size() <= kRowsTilesPerSm * e->nsm;
-    struct Seen { const Neuron *first; bool uniform; };
-    std::map<std::string, Seen> types;
-    std::vector<int> fl;
+    std::map<std::string, int> index;
+    std::vector<std::vector<const Neuron *>> types;   // in the order build_layout meets them
     for (const Neuron &N : e->dec.neurons) {
-        if (N.nrows < 32) continue;
-        int cap = 0;
-        if (!stack_plan(N.parent, fl, cap) || cap > kStackCapMax) return false;
-        auto it = types.emplace(N.key, Seen{&N, true}).first;
-        it->second.uniform = it->second.uniform && N.parent == it->second.first->parent;
+        const auto it = index.emplace(N.key, (int)types.size());
+        if (it.second) types.emplace_back();
+        types[it.first->second].push_back(&N);
     }
-    for (const auto &kv : types) {
-        const Neuron &N = *kv.second.first;
+    std::set<std::string> level_keys, rows_keys;
+    int64_t cells = 0;
+    for (const auto &m : types) cells += (int64_t)m.size();
+    const int per = (int)std::min<int64_t>(LANES, (cells + e->nsm - 1) / e->nsm);
+    size_t rows_bytes = 0;   // of all row-parallel blocks
+    bool surely = true;
+    std::vector<int> fl;
+    for (const auto &m : types) {
+        const Neuron &N = *m[0];
+        if (N.nrows < kStackMin) continue;
         TileType tt = tile_type_of(N);
         std::vector<int> prog = N.prog;
         tt.pool_off = (int)prog.size();
         prog.insert(prog.end(), N.pool_prog.begin(), N.pool_prog.end());
+        bool uniform = true;
         tt.stack = !tt.sym;
+        for (const Neuron *x : m) {
+            int cap = 0;
+            if (uniform && x->parent != N.parent) uniform = false;
+            if (tt.stack && (!uniform || x == &N) && (!stack_plan(x->parent, fl, cap) || cap > kStackCapMax)) tt.stack = 0;
+        }
         tt.nstatic = static_rows(slot_field_ranges(prog, tt), tt.nslots);
+        // only so many programs get a kernel (level_plan, rows_plan)
         LevelProg lp;
         RowsProg rp;
-        if (!(e->opt.jit == 0 && level_type(tt, prog, N.parent, kv.second.uniform, lp)) &&
-            !(small && rows_type(tt, prog, rp)))
-            return false;
+        bool level = e->opt.jit == 0 && level_type(tt, prog, N.parent, uniform, lp);
+        if (level && !level_keys.count(lp.key)) {
+            level = level_keys.size() < kLevelKernels;
+            if (level) level_keys.insert(lp.key);
+        }
+        bool rows = !level && small && rows_type(tt, prog, rp);
+        if (rows && !rows_keys.count(rp.key)) {
+            rows = rows_keys.size() < kRowsKernels;
+            if (rows) rows_keys.insert(rp.key);
+        }
+        if (rows) {
+            int most = per;
+            while (most > 1 && rows_smem(most * tt.nslots, most * tt.nslots / LANES + tt.nslots + 1) >
+                                   (size_t)kLevelSmemMax / 2)
+                --most;
+            rows_bytes += (m.size() + most - 1) / most * rows_smem(most * tt.nslots, tt.nslots);
+        }
+        if (N.nrows < 32) continue;
+        sv.level = sv.level || level;
+        sv.rows = sv.rows || rows;
+        surely = surely &&
+                 ((level && branched(m.size(), tt.nstatic, [&](size_t i) -> const std::vector<int> & {
+                       return m[i]->parent;
+                   })) ||
+                  (rows && (e->opt.jit == kJitRows || rows_surely(tt))));
     }
-    return true;
+    // row-parallel blocks that do not all fit at once take turns, which a trial has to weigh
+    // (1,200 mixed cables of 400 compartments 583 us a step, 430 with the stack elimination; 800 295 and 411)
+    sv.surely = surely && (e->opt.jit == kJitRows || rows_bytes <= (size_t)e->nsm * kLevelSmemMax);
+    return sv;
 }
 
 // The neuron-to-warp mapping, chosen by trial (gbh_options.wide_min 0): for
@@ -3160,7 +3258,9 @@ bool level_everywhere(const gbh_engine *e)
 // specialised kernels pay on this batch: they run beside the stack or wide
 // launches and can slow the longest of them down (50,000 random trees: the
 // 24 specialised kernels of the small neurons made the step 15-30 % slower).
-// `no_jit` is set when the chosen mapping ran faster interpreted.
+// `no_jit` is set when the chosen mapping ran faster interpreted. The level and
+// row-parallel kernels, which go with lane-mapped neurons, are timed likewise,
+// unless they are certain to win (kernels_serve).
 int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses *syn,
                    const gbh_remote_synapses *remote, bool &no_jit)
 {
@@ -3171,7 +3271,8 @@ int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses
     for (int w : {32, 64, 128})
         if (w <= maxrows) cand.push_back(w);
     if (cand.empty()) return -1;   // nothing large enough to run wide
-    if (level_everywhere(e)) return -1;   // no trial: these beat every mapping it tries
+    const Served sv = kernels_serve(e);
+    if (sv.surely) return -1;   // no trial
     cand.push_back(-1);
     int best = cand[0];
     double best_ms = 1e300;
@@ -3210,7 +3311,22 @@ int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses
             best = w;
         }
     }
-    if (e->opt.jit == 0 && best_ms < 1e300) no_jit = trial(best, 0) > best_ms;
+    if (e->opt.jit != 0 || best_ms == 1e300) return best;
+    // the kernels generated for the batch: with the chosen mapping, and those
+    // that need the lane mapping against it
+    no_jit = true;
+    auto against = [&](int w, int jit) {
+        const double ms = trial(w, jit);
+        if (ms <= best_ms) {
+            best_ms = ms;
+            best = w;
+            no_jit = false;
+        }
+    };
+    const int interpreted = best;
+    against(interpreted, 0);
+    if (sv.level && interpreted != -1) against(-1, 0);
+    if (sv.rows) against(-1, kJitRows);
     return best;
 }
 
@@ -3236,6 +3352,7 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->opt.device) == cudaSuccess && nsm > 0)
         e->nsm = nsm;
     int rc = GBH_OK;
+    e->trial = pre != nullptr;
     if (pre) e->dec = *pre;   // a trial engine over a batch already decoded
     else rc = decode_batch(desc, e->dec, err);
     if (rc) {
@@ -3279,8 +3396,9 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
             e->d_vm_at.release();
         }
     }
-    if (std::max(e->launches.size(), e->rows_launches.size()) > 1) {
-        const int ns = (int)std::min<size_t>(std::max(e->launches.size(), e->rows_launches.size()), 8);
+    const size_t groups = std::max({e->launches.size(), e->rows_launches.size(), e->level_launches.size()});
+    if (groups > 1) {
+        const int ns = (int)std::min<size_t>(groups, 8);
         e->side.resize(ns);
         e->ev_join.resize(ns);
         for (int i = 0; i < ns; ++i) {
@@ -3319,7 +3437,10 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
         if (L.wide) e->stats.wide_tiles += L.tile1 - L.tile0;
         if (L.stack) e->stats.stack_tiles += L.tile1 - L.tile0;
     }
-    for (const Tile &t : e->tiles) e->stats.stack_tiles += e->types[t.type].level ? 1 : 0;
+    bool level = false;
+    for (const Launch &L : e->launches) level = level || L.level >= 0;
+    if (level)
+        for (const Tile &t : e->tiles) e->stats.stack_tiles += e->types[t.type].level ? 1 : 0;
     e->stats.precision = e->opt.precision;
     e->stats.steps_per_launch = e->net_coop ? e->net_spl : e->steps_per_launch;
     e->stats.cooperative = e->net_coop ? 1 : 0;
