@@ -2353,7 +2353,7 @@ int autotune_trials(gbh_engine *e)
     auto timed = [&](int spl, double limit, double &per) {
         e->steps_per_launch = spl;
         int rc_t = run_steps(e, 2, e->stream);   // warm caches and clocks
-        for (int steps : {8, std::max(2 * spl, 128)}) {
+        for (int steps : {8, spl == 1 && !e->has_network ? 24 : std::max(2 * spl, 128)}) {
             CK(cudaEventRecord(e->ev0, e->stream));
             if (rc_t == GBH_OK) rc_t = run_steps(e, steps, e->stream);
             CK(cudaEventRecord(e->ev1, e->stream));
@@ -2408,6 +2408,22 @@ int autotune_trials(gbh_engine *e)
         if (timed(spl, best, per)) return GBH_ERR_CUDA;
         if (getenv("GBH_VERBOSE")) fprintf(stderr, "gbhsolve: trial %d steps/launch: %.2f us/step\n", spl, per * 1e3);
         if (per < best) { best = per; best_s = spl; }
+    }
+    // single steps: a level launch reads its rows' constants first, which only
+    // pays over several steps where the batch is large (20,000 trees of 96
+    // compartments, us for one step: levels 127, lanes 102)
+    bool level = false;
+    for (const Launch &L : e->launches) level = level || L.level >= 0;
+    if (level) {
+        double by_level, by_lane;
+        if (timed(1, 1e300, by_level)) return GBH_ERR_CUDA;
+        e->launches.swap(e->lane_launches);
+        if (timed(1, by_level, by_lane)) return GBH_ERR_CUDA;
+        e->launches.swap(e->lane_launches);
+        e->single_lane = by_lane < by_level;
+        if (getenv("GBH_VERBOSE"))
+            fprintf(stderr, "gbhsolve: trial single steps: level elimination %.2f us/step, lanes %.2f\n",
+                    by_level * 1e3, by_lane * 1e3);
     }
     // networks: the cooperative multi-step launch against the best per-step plan
     bool any_wide = false;
