@@ -8,6 +8,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <set>
 #include <string>
@@ -185,6 +186,12 @@ struct gbh_engine {
     DBuf<double2> d_lkt, d_lcy;
     DBuf<double> d_lc, d_ld, d_lpd;
     DBuf<unsigned> d_lgen;
+    // element of static row * 32 + lane within its group, per tile (empty: not
+    // level), and for the registered per-step inputs and outputs of the tiles
+    std::vector<std::vector<int>> lv_place;
+    DBuf<int> d_ltin, d_ltout;
+    DBuf<int2> d_lio;
+    std::vector<int2> lio;
     // row-parallel steps (gbh_rows.cuh): the plan that uses them, timed against
     // `launches` by the autotuner (empty: none)
     std::vector<JitKernel> rw_kern;
@@ -922,6 +929,7 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
     struct Cand { LevelGroup g; int warps, bucket; size_t smem; };
     std::vector<Cand> cand;
     LevelPools P;
+    e->lv_place.resize(e->tiles.size());
     std::vector<std::vector<int>> cells_of(e->tiles.size());
     for (size_t i = 0; i < dec.neurons.size(); ++i) {
         const int t = e->neuron_tile[i];
@@ -963,6 +971,9 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
                                                         (a + n == start[d + 1] ? LV_LAST : 0)));
                 }
             g.nch = (int)P.chunks.size() - g.choff;
+            std::vector<int> &place = e->lv_place[t];
+            place.resize((size_t)nst * LANES, -1);
+            for (size_t k = 0; k < order.size(); ++k) place[order[k] + l0] = (int)k;
             for (int x : order) {
                 const int row = x / LANES, l = x % LANES;
                 P.map.push_back(row * LANES + l0 + l);
@@ -2013,6 +2024,9 @@ int launch_one(gbh_engine *e, const DevView &v, const Launch &L, int k, long lon
         lv.d = e->d_ld.p;
         lv.pd = e->d_lpd.p;
         lv.gen = e->d_lgen.p;
+        lv.tin = e->d_ltin.p;
+        lv.tout = e->d_ltout.p;
+        lv.io = e->d_lio.p;
         const cudaError_t je = jit_level_launch(e->lv_kern[L.level], v, lv, L.tile0, L.tile1 - L.tile0, L.warps, k,
                                                 step, (size_t)L.smax, st);
         if (je != cudaSuccess) {
@@ -2640,6 +2654,32 @@ int upload_tile_lists(gbh_engine *e, std::vector<std::vector<std::pair<int, int>
     return GBH_OK;
 }
 
+// Per-step inputs or outputs of the level tiles: the element of each entry of
+// `per_tile` whose row is passive (-1: the others', which the top rows' warp
+// sees to), and whether a tile has any.
+static int upload_level_lists(gbh_engine *e, const std::vector<std::vector<std::pair<int, int>>> &per_tile,
+                              const std::function<int(size_t, int)> &row_of, bool inputs, DBuf<int> &elem)
+{
+    if (e->lv_place.empty()) return GBH_OK;
+    e->lio.resize(per_tile.size(), make_int2(0, 0));
+    std::vector<int> el;
+    for (size_t t = 0; t < per_tile.size(); ++t) {
+        const std::vector<int> &place = e->lv_place[t];
+        int any = 0;
+        for (const auto &x : per_tile[t]) {
+            const int off = x.first & ~(1 << 30), row = place.empty() ? -1 : row_of(t, off / LANES);
+            const size_t at = (size_t)row * LANES + off % LANES;
+            el.push_back(row >= 0 && at < place.size() ? place[at] : -1);
+            any |= el.back() >= 0;
+        }
+        (inputs ? e->lio[t].x : e->lio[t].y) = any;
+    }
+    if (el.empty()) el.push_back(-1);
+    elem.release();
+    e->d_lio.release();
+    return elem.upload(el) || e->d_lio.upload(e->lio) ? GBH_ERR_CUDA : GBH_OK;
+}
+
 InPlan in_plan(const gbh_engine *e)
 {
     InPlan pl;
@@ -2780,6 +2820,23 @@ int gbh_register_inputs_typed(gbh_engine *e, int n, const int *solver, const int
     if (e->fuse_in) {
         for (auto &kv : last) per_tile[kv.first.first].push_back({kv.first.second, kv.second});
         if (upload_tile_lists(e, per_tile, e->d_tin_start, e->d_tin_off, e->d_tin_idx)) return GBH_ERR_CUDA;
+        std::vector<std::vector<int>> slot(e->types.size());   // per type: the row whose inject a field is
+        for (size_t q = 0; q < e->dec.neurons.size(); ++q) {
+            const Neuron &N = e->dec.neurons[q];
+            std::vector<int> &sl = slot[e->tiles[e->neuron_tile[q]].type];
+            if (!sl.empty() || e->lv_place.empty()) continue;
+            sl.assign(std::max<size_t>(N.fsrc.size(), 1), -1);
+            int row = 0;
+            for (size_t pc = 0; pc < N.prog.size() && row < N.nrows;) {
+                const int code = N.prog[pc], m = micro_operands(code);
+                if (m < 0) break;
+                if (code == M_BEGIN) sl[N.prog[pc + 2]] = row;
+                if (code == M_END) ++row;
+                pc += 1 + m;
+            }
+        }
+        if (upload_level_lists(e, per_tile, [&](size_t t, int f) { return slot[e->tiles[t].type][f]; }, true, e->d_ltin))
+            return GBH_ERR_CUDA;
     }
     return GBH_OK;
 }
@@ -2833,7 +2890,7 @@ int gbh_register_outputs(gbh_engine *e, int n, const int *solver, const int *row
         }
     }
     if (upload_tile_lists(e, per_tile, e->d_tout_start, e->d_tout_off, e->d_tout_idx)) return GBH_ERR_CUDA;
-    return GBH_OK;
+    return upload_level_lists(e, per_tile, [](size_t, int row) { return row; }, false, e->d_ltout);
 }
 
 int gbh_get_outputs_async(gbh_engine *e, double *host_values, void *stream)
@@ -3006,12 +3063,12 @@ int gbh_run_io(gbh_engine *e, const double *host_in, double *host_out, int nstep
     }
     const int nio = std::max(n_in ? e->n_tgt : 0, n_out);
     const InPlan plan = in_plan(e);
-    // every launch group specialised (lane tiles), no synapses: the step
+    // every launch group a generated kernel's (lane tiles), no synapses: the step
     // kernels apply each step's inputs and gather its outputs themselves, and
     // a block of steps runs as multi-step launches
     bool fused = !e->has_network && !e->givals_enabled && !e->net_coop && (n_in == 0 || e->fuse_in) &&
                  !e->launches.empty();
-    for (const Launch &L : e->launches) fused = fused && (L.jit >= 0 || L.rows >= 0) && !L.wide;
+    for (const Launch &L : e->launches) fused = fused && (L.jit >= 0 || L.rows >= 0 || L.level >= 0) && !L.wide;
     const unsigned grid = (unsigned)((nio + 255) / 256);
     int last = 0;
     for (int s0 = 0, j = 0; s0 < nsteps; s0 += B, ++j) {
@@ -4314,7 +4371,7 @@ void gbh_destroy(gbh_engine *e)
     e->d_rA.release(); e->d_rB.release(); e->d_rC.release();
     e->d_lgroups.release(); e->d_lchunks.release(); e->d_lmap.release(); e->d_lkid.release(); e->d_lnkid.release(); e->d_lpar.release();
     e->d_ltopkid.release(); e->d_lkt.release(); e->d_lcy.release(); e->d_lc.release(); e->d_ld.release(); e->d_lpd.release();
-    e->d_lgen.release();
+    e->d_lgen.release(); e->d_ltin.release(); e->d_ltout.release(); e->d_lio.release();
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
     if (e->stream) cudaStreamDestroy(e->stream);

@@ -69,6 +69,8 @@ struct LevelView {
     double *d;           // D' (FP64 form)
     double *pd;          // B T: what the row takes from its parent's diagonal
     unsigned *gen;       // per group: the fields' generation its factors were kept at (DevView::sgen)
+    const int *tin, *tout;   // per-step inputs and outputs (DevView::tin_*, tout_*): element of a static row, -1 others
+    const int2 *io;      // per tile: any input (x) or output (y) of a static row
 };
 
 // Shared memory of a group's block, in the order level_smem_of lays it out:
@@ -112,10 +114,62 @@ __device__ __forceinline__ LevelSm level_smem_of(double *sm, const LevelGroup &g
     return q;
 }
 
+// A static row's rhs term from its fields, as its channel program forms it
+// (m: row * 32 + lane of the tile).
+template <bool MIXED> __device__ __forceinline__ double level_kterm(const double *P, const int *pf, int m)
+{
+    const int *ps = pf + 6 * (m / LANES);
+    const int l = m % LANES;
+    if (MIXED)
+        return df2d(df_mul(df_add(ld_df(&P[ps[2] * LANES + l]), ld_df(&P[ps[3] * LANES + l])),
+                           ld_df(&P[ps[4] * LANES + l])));
+    return (P[ps[2] * LANES + l] + P[ps[3] * LANES + l]) * P[ps[4] * LANES + l];
+}
+
+// A step's inputs into the fields of a group (lanes [lane0, lane0 + nlanes) of
+// the tile) by `nt` threads: of its static rows, whose rhs terms in kt follow,
+// or, kt null, of the rows above them. Out of line, as level_out: within the
+// steps they took 10 to 20 registers more.
+template <bool MIXED>
+__device__ __noinline__ void level_in(const DevView &v, const LevelView &L, int tile, int lane0, int nlanes,
+                                      int64_t eoff, long long step, int tid, int nt, double2 *kt)
+{
+    const Tile &tl = v.tiles[tile];
+    const double *src = v.io_in + (step - v.io_step0) * v.io_nin;
+    double *P = v.P + tl.fld * LANES;
+    for (int k = v.tin_start[tile] + tid; k < v.tin_start[tile + 1]; k += nt) {
+        const int at = v.tin_off[k], off = at & ~(1 << 30), l = off & (LANES - 1), e = L.tin[k];
+        if ((e < 0) != (kt == nullptr) || l < lane0 || l >= lane0 + nlanes) continue;
+        const double x = src[v.tin_idx[k]];
+        if (at & (1 << 30)) {
+            const float hi = __double2float_rn(x);
+            st_df(&P[off], df_make(hi, __double2float_rn(x - (double)hi)));
+        } else {
+            P[off] = x;
+        }
+        if (kt) kt[e].x = level_kterm<MIXED>(P, v.prog + v.types[tl.type].pf_off, L.map[eoff + e]);
+    }
+}
+
+// A step's outputs of a group: of its static rows from their solutions X, or, X
+// null, of the rows above them, whose warp has stored their Vm.
+__device__ __noinline__ static void level_out(const DevView &v, const LevelView &L, int tile, int lane0, int nlanes,
+                                              long long step, int tid, int nt, const double *X)
+{
+    double *dst = v.io_out + (step - v.io_step0) * v.io_nout;
+    const double *V = v.V + v.tiles[tile].vm * LANES;
+    for (int k = v.tout_start[tile] + tid; k < v.tout_start[tile + 1]; k += nt) {
+        const int off = v.tout_off[k], l = off & (LANES - 1), e = L.tout[k];
+        if ((e < 0) != (X == nullptr) || l < lane0 || l >= lane0 + nlanes) continue;
+        dst[v.tout_idx[k]] = X ? X[e] : V[off];
+    }
+}
+
 // What the sweeping warps of a block do in a launch (sm: level_smem bytes).
 // MANY: a row may have more than two static children.
 template <bool MIXED, bool CRANK, int NTOP, bool RES, bool MANY>
-__device__ __forceinline__ void level_steps(const LevelView &L, const LevelGroup &g, const LevelSm &q, int nsteps)
+__device__ __forceinline__ void level_steps(const DevView &v, const LevelView &L, const LevelGroup &g,
+                                            const LevelSm &q, int nsteps, long long step0)
 {
     const int tid = threadIdx.x, nt = blockDim.x - LANES, nth = blockDim.x;
     double *const U = q.U, *const X = q.X, *const PR = q.PR, *const O = q.O;
@@ -138,7 +192,13 @@ __device__ __forceinline__ void level_steps(const LevelView &L, const LevelGroup
     // what does not wait for the level before is read and formed meanwhile:
     // the next level's constants, its Vm + K forward and, mixed, R / D'
     // backward, and the descriptors two chunks ahead.
+    const bool put = v.io_in && L.io[g.tile].x, take = v.io_out && L.io[g.tile].y;
     for (int it = 0; it < nsteps; ++it) {
+        if (put) {
+            level_in<MIXED>(v, L, g.tile, g.lane0, g.nlanes, g.eoff, step0 + it, tid, nt, RES ? q.kt : L.kt + g.eoff);
+            if (!RES) __threadfence_block();
+            sync();
+        }
         int2 m = ch[nch - 1], mn = ch[nch - 2];
         int e = element(m), k = kid[e];
         double T = kt[e].y, own = O[e] + kt[e].x;
@@ -235,12 +295,17 @@ __device__ __forceinline__ void level_steps(const LevelView &L, const LevelGroup
             m = mn;
             mn = m2;
         }
+        if (take) {   // before the next step's sweep
+            level_out(v, L, g.tile, g.lane0, g.nlanes, step0 + it, tid, nt, O);
+            sync();
+        }
     }
 }
 
 template <bool MIXED, bool CRANK, int NTOP, bool RES>
 __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L, const LevelGroup &g, const Tile &tl,
-                                            const TileType &ty, double *sm, int nsteps, bool full, bool refresh)
+                                            const TileType &ty, double *sm, int nsteps, long long step0, bool full,
+                                            bool refresh)
 {
     const int tid = threadIdx.x, nt = blockDim.x - LANES;
     const LevelSm q = level_smem_of<MIXED, CRANK, NTOP, RES>(sm, g);
@@ -256,17 +321,8 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
     for (int e = tid; e < g.n; e += nt) O[e] = V[map[e]];
     if (tid < LV_SPARE) X[g.n + tid] = O[g.n + tid] = PR[g.n + tid] = 0.0;
     bar_named(LB_SWEEP, nt);
-    // a row's rhs term from its fields, as its channel program forms it
     const int *pf = v.prog + ty.pf_off;
     const double *P = v.P + tl.fld * LANES;
-    auto kterm = [&](int m) {
-        const int *ps = pf + 6 * (m / LANES);
-        const int l = m % LANES;
-        if (MIXED)
-            return df2d(df_mul(df_add(ld_df(&P[ps[2] * LANES + l]), ld_df(&P[ps[3] * LANES + l])),
-                               ld_df(&P[ps[4] * LANES + l])));
-        return (P[ps[2] * LANES + l] + P[ps[3] * LANES + l]) * P[ps[4] * LANES + l];
-    };
     if (full) {
         // the factors from the fields: the diagonals' elimination, level by
         // level; PR holds B T meanwhile
@@ -286,14 +342,14 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
                 const double b = B[r] * T;
                 PR[e] = b;
                 pd[e] = b;
-                kt[e] = make_double2(kterm(r), T);
+                kt[e] = make_double2(level_kterm<MIXED>(P, pf, r), T);
                 cy[e] = make_double2(MIXED ? L.c[g.eoff + e] * y : L.c[g.eoff + e], y);
                 if (!MIXED) dd[e] = D;
             }
             if (m.y & LV_FIRST) bar_named(LB_SWEEP, nt);
         }
     } else if (refresh) {   // inputs on the rhs fields: their terms once per launch
-        for (int e = tid; e < g.n; e += nt) kt[e].x = kterm(map[e]);
+        for (int e = tid; e < g.n; e += nt) kt[e].x = level_kterm<MIXED>(P, pf, map[e]);
     }
     if (full || refresh) {
         __threadfence_block();
@@ -308,8 +364,8 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
             q.par[e] = par[e];
         }
     bar_named(LB_SWEEP, nt);
-    if (g.many) level_steps<MIXED, CRANK, NTOP, RES, true>(L, g, q, nsteps);
-    else level_steps<MIXED, CRANK, NTOP, RES, false>(L, g, q, nsteps);
+    if (g.many) level_steps<MIXED, CRANK, NTOP, RES, true>(v, L, g, q, nsteps, step0);
+    else level_steps<MIXED, CRANK, NTOP, RES, false>(v, L, g, q, nsteps, step0);
     bar_named(LB_SWEEP, nt);
     for (int e = tid; e < g.n; e += nt) V[map[e]] = O[e];
 }
