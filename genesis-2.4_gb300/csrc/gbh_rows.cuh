@@ -223,15 +223,14 @@ __device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup 
                 r = div_by(r, D, y);
             }
             q.R[e] = r;
-            // FP64: the root, which a NaN anywhere in the tree reaches
-            if (MIXED) see_row(lost, r);
-            else if (p == g.n) finite_check(v, r, true);
+            if (p == g.n) finite_check(v, r, true);   // the root: a NaN anywhere in the tree reaches it
         }
         if (c + 1 < g.nch) back(c + 1);
         if (last) __syncthreads();
     }
     for (int i = tid; i < g.n; i += blockDim.x) {
         const double r = q.R[i], old = q.V[i];
+        if (MIXED) see_row(lost, r);   // (what the mixed form makes of a NaN may not)
         q.V[i] = CRANK ? (MIXED ? fma(2.0, r, -old) : r + r - old) : r;
     }
     __syncthreads();
