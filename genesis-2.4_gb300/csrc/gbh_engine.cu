@@ -88,7 +88,7 @@ struct Launch {
     bool wide = false;    // one neuron per block (wide tiles)
     bool stack = false;   // stack elimination (smax = shared doubles per lane)
     bool split = false;   // stack: some tile's rows above its static ones go to a second warp
-    int level = -1;       // level elimination: kernel index (tile0..tile1 are groups, smax the shared bytes)
+    int level = -1;       // level elimination: lv_kern's index / 2 (tile0..tile1 are groups, smax the shared bytes)
     int rows = -1;        // row-parallel step: kernel index (likewise)
 };
 
@@ -179,7 +179,7 @@ struct gbh_engine {
     bool single_lane = false;
     std::vector<Launch> level_launches;   // the level plan, timed against `launches` (empty: not timed)
     // level elimination (gbh_level.cuh)
-    std::vector<JitKernel> lv_kern;
+    std::vector<JitKernel> lv_kern;   // four of a program: constants resident or streamed (+2), per-step I/O (+1)
     DBuf<LevelGroup> d_lgroups;
     DBuf<int2> d_lchunks;
     DBuf<int> d_lmap, d_lkid, d_lnkid, d_lpar, d_ltopkid;
@@ -201,7 +201,7 @@ struct gbh_engine {
     DBuf<int4> d_ritems;
     DBuf<int> d_rmap, d_rprev, d_rpos;
     DBuf<double> d_rA, d_rB, d_rC;
-    bool trial = false;      // built to time a mapping (choose_mapping)
+    bool trial = false, trial_rows = false;   // built to time a mapping (Trial)
     int nsm = 152;           // the device's SMs (GB300's where the query fails)
     int steps_per_launch = 1;
     bool has_network = false;
@@ -771,11 +771,13 @@ template <class At> bool branched(size_t n, int nstatic, At parent_of)
     return (int64_t)n * nstatic >= 2 * levels;
 }
 
-// Populations of one small tree from this many tiles an SM on keep the lanes
-// of the specialised kernels full: which of the two is faster is timed (20,000
-// trees, FP64, us a step, levels and lanes: 16 compartments 17.3 and 11.8, 64
-// compartments 36 and 55).
+// Populations of one tree of few compartments, from this many tiles an SM on,
+// keep the lanes of the specialised kernels full: which of the two is faster is
+// timed (20,000 trees, FP64, us a step, levels and lanes: 16 compartments 17.3
+// and 11.8, 32 compartments 23.0 and 20.9; of 64 36 and 55, and the specialised
+// forms of such trees take seconds to compile).
 constexpr int64_t kLevelTimedTilesPerSm = 2;
+constexpr int kLevelTimedSlots = 32;
 
 struct LevelPlan {
     std::vector<LevelGroup> groups;
@@ -863,23 +865,23 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
         });
         // (a trial engine is what times it)
         if (!branches && e->opt.steps_per_launch != 0 && count > e->nsm && !e->trial) continue;
-        timed[ti] = !branches || (uni && tt.nslots <= kJitMaxSlots &&
+        timed[ti] = !branches || (uni && tt.nslots <= kLevelTimedSlots &&
                                   (count + LANES - 1) / LANES > kLevelTimedTilesPerSm * e->nsm);
         auto it = kern.find(lp.key);
         if (it == kern.end()) {
             if (kern.size() >= kLevelKernels) continue;
-            const std::string src = jit_level_source(lp, tt, tg[tt.table_set], mixed, true);
-            if (src.empty()) continue;
+            if (jit_level_source(lp, tt, tg[tt.table_set], mixed, true, false).empty()) continue;
             it = kern.emplace(lp.key, (int)kern.size()).first;
-            srcs.push_back(src);   // kernel 2k: constants resident in shared memory, 2k + 1: streamed
-            srcs.emplace_back();
+            srcs.resize(4 * kern.size());   // (lv_kern)
         }
         tt.level = 1 + it->second;
         tt.lv_f0 = lp.f0;
         ntop[ti] = lp.ntop;
-        std::string &streamed = srcs[2 * it->second + 1];
-        if (streamed.empty() && !resident(tt, lp.ntop))
-            streamed = jit_level_source(lp, tt, tg[tt.table_set], mixed, false);
+        const bool res = resident(tt, lp.ntop);
+        for (int io = 0; io < 2; ++io) {
+            std::string &src = srcs[4 * it->second + (res ? 0 : 2) + io];
+            if (src.empty()) src = jit_level_source(lp, tt, tg[tt.table_set], mixed, res, io != 0);
+        }
     }
     if (srcs.empty()) return GBH_OK;
     int major = 10, minor = 3;
@@ -895,11 +897,12 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
     });
     for (size_t c = 0; c < srcs.size(); ++c)
         if (!ok[c] && e->jit_log.size() < 4000) e->jit_log += logs[c];
-    for (size_t k = 0; k < kern.size(); ++k) e->jit_compiled += ok[2 * k] || ok[2 * k + 1];
+    for (size_t k = 0; k < kern.size(); ++k) e->jit_compiled += ok[4 * k] || ok[4 * k + 2];
     for (size_t ti = 0; ti < e->types.size(); ++ti) {
         TileType &tt = e->types[ti];
         if (!tt.level) continue;
-        if (ok[2 * (tt.level - 1) + (resident(tt, ntop[ti]) ? 0 : 1)]) cells += (int64_t)members[ti].size();
+        const int k = 4 * (tt.level - 1) + (resident(tt, ntop[ti]) ? 0 : 2);
+        if (ok[k] && ok[k + 1]) cells += (int64_t)members[ti].size();
         else tt.level = 0;   // keeps the stack elimination
     }
     // ---- groups: enough of them for every SM, as many neurons each as that
@@ -1748,7 +1751,7 @@ int build_layout(gbh_engine *e, const gbh_batch_desc *d, const gbh_synapses *syn
 
     // ---- row-parallel steps of small batches, for the autotuner or alone ----
     std::vector<Launch> rplan;
-    const bool rows_only = e->opt.jit == kJitRows;   // the plan without a trial
+    const bool rows_only = e->opt.jit == kJitRows || e->trial_rows;   // the plan without being timed
     if (!e->has_network && (rows_only || (e->opt.jit == 0 && e->opt.steps_per_launch == 0)) && jit_available(nullptr)) {
         const int rcw = rows_plan(e, members, prog_pool, tg, rplan);
         if (rcw) return fail_err(err, rcw, "%s", g_last_error);
@@ -2027,7 +2030,7 @@ int launch_one(gbh_engine *e, const DevView &v, const Launch &L, int k, long lon
         lv.tin = e->d_ltin.p;
         lv.tout = e->d_ltout.p;
         lv.io = e->d_lio.p;
-        const cudaError_t je = jit_level_launch(e->lv_kern[L.level], v, lv, L.tile0, L.tile1 - L.tile0, L.warps, k,
+        const cudaError_t je = jit_level_launch(e->lv_kern[2 * L.level + (v.io_in || v.io_out)], v, lv, L.tile0, L.tile1 - L.tile0, L.warps, k,
                                                 step, (size_t)L.smax, st);
         if (je != cudaSuccess) {
             set_last("level elimination launch failed: %s", cudaGetErrorString(je));
@@ -3201,7 +3204,7 @@ int64_t gbh_jit_source(const gbh_batch_desc *desc, int precision, int type_index
     if (compact == 3 || compact == 4) {
         const LevelProg lp = level_prog(types[type_index], prog_pool);
         if (lp.ok) src = jit_level_source(lp, types[type_index], tg[types[type_index].table_set],
-                                          precision == GBH_PREC_MIXED, compact == 3);
+                                          precision == GBH_PREC_MIXED, compact == 3, false);
     } else {
         src = jit_source(types[type_index], prog_pool, tg[types[type_index].table_set], precision == GBH_PREC_MIXED,
                          false, uniform[type_index] ? &parents[type_index] : nullptr, 6, compact == 1, compact == 2);
@@ -3240,8 +3243,15 @@ gbh_engine *gbh_create(const gbh_batch_desc *desc, const gbh_synapses *syn, cons
 
 namespace {
 
+// An engine that only times a mapping: over a batch already decoded; rows: with
+// the row-parallel plan, which is otherwise left to the autotuner.
+struct Trial {
+    const Decoded *dec;
+    bool rows;
+};
+
 gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, const gbh_remote_synapses *remote,
-                        const gbh_options *opt, gbh_error *err, gbh_engine *&made, const Decoded *pre = nullptr);
+                        const gbh_options *opt, gbh_error *err, gbh_engine *&made, const Trial *trial = nullptr);
 
 // What the level and row-parallel kernels serve of a batch's neurons that could
 // run wide (32 compartments and more) when they are lane-mapped instead.
@@ -3350,7 +3360,7 @@ int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses
     int best = cand[0];
     double best_ms = 1e300;
     // one trial: 32 steps after 16 on an engine built with the mapping w
-    auto trial = [&](int w, int jit) {
+    auto trial = [&](int w, int jit, bool rows = false) {
         gbh_options o = e->opt;
         o.wide_min = w;
         o.jit = jit;
@@ -3359,7 +3369,8 @@ int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses
         gbh_error te{};
         gbh_engine *made = nullptr, *t = nullptr;
         try {
-            t = create_dist(desc, syn, remote, &o, &te, made, &e->dec);
+            const Trial tr{&e->dec, rows};
+            t = create_dist(desc, syn, remote, &o, &te, made, &tr);
         } catch (const std::exception &) {
             if (made) gbh_destroy(made);
             t = nullptr;
@@ -3371,8 +3382,8 @@ int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses
             if (gbh_run(t, 32) == GBH_OK) ms = t->stats.device_ms - ms0;
         }
         if (getenv("GBH_VERBOSE"))
-            fprintf(stderr, "gbhsolve: mapping trial wide_min %d%s: %.2f us/step (%lld wide, %lld stack tiles)\n", w,
-                    jit < 0 ? "" : " specialised", ms / 32 * 1e3, (long long)t->stats.wide_tiles,
+            fprintf(stderr, "gbhsolve: mapping trial wide_min %d%s%s: %.2f us/step (%lld wide, %lld stack tiles)\n", w,
+                    jit < 0 ? "" : " specialised", rows ? " row-parallel" : "", ms / 32 * 1e3, (long long)t->stats.wide_tiles,
                     (long long)t->stats.stack_tiles);
         gbh_destroy(t);
         return ms;
@@ -3388,8 +3399,8 @@ int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses
     // the kernels generated for the batch: with the chosen mapping, and those
     // that need the lane mapping against it
     no_jit = true;
-    auto against = [&](int w, int jit) {
-        const double ms = trial(w, jit);
+    auto against = [&](int w, bool rows) {
+        const double ms = trial(w, 0, rows);
         if (ms <= best_ms) {
             best_ms = ms;
             best = w;
@@ -3397,14 +3408,14 @@ int choose_mapping(gbh_engine *e, const gbh_batch_desc *desc, const gbh_synapses
         }
     };
     const int interpreted = best;
-    against(interpreted, 0);
-    if (sv.level && interpreted != -1) against(-1, 0);
-    if (sv.rows) against(-1, kJitRows);
+    against(interpreted, false);
+    if (sv.level && interpreted != -1) against(-1, false);
+    if (sv.rows) against(-1, true);
     return best;
 }
 
 gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, const gbh_remote_synapses *remote,
-                        const gbh_options *opt, gbh_error *err, gbh_engine *&made, const Decoded *pre)
+                        const gbh_options *opt, gbh_error *err, gbh_engine *&made, const Trial *trial)
 {
     memset(err, 0, sizeof(*err));
     if (!desc) {
@@ -3425,15 +3436,16 @@ gbh_engine *create_dist(const gbh_batch_desc *desc, const gbh_synapses *syn, con
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->opt.device) == cudaSuccess && nsm > 0)
         e->nsm = nsm;
     int rc = GBH_OK;
-    e->trial = pre != nullptr;
-    if (pre) e->dec = *pre;   // a trial engine over a batch already decoded
+    e->trial = trial != nullptr;
+    e->trial_rows = trial && trial->rows;
+    if (trial) e->dec = *trial->dec;
     else rc = decode_batch(desc, e->dec, err);
     if (rc) {
         set_last("%s", err->message);
         delete e;
         return nullptr;
     }
-    if (!pre && e->opt.wide_min == 0) {
+    if (!trial && e->opt.wide_min == 0) {
         bool no_jit = false;
         e->opt.wide_min = choose_mapping(e, desc, syn, remote, no_jit);
         if (no_jit) e->opt.jit = -1;

@@ -1099,7 +1099,8 @@ std::string jit_rows_source(const RowsProg &rp, const TileType &tt, const TableG
     return o.str();
 }
 
-std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed, bool resident)
+std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed, bool resident,
+                             bool io)
 {
     Emit E;
     E.mixed = mixed;
@@ -1110,8 +1111,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
                *res = resident ? "true" : "false";
     o << "#include \"gbh_devfn.cuh\"\n#include \"gbh_level.cuh\"\nusing namespace gbh;\n"
       << "extern \"C\" __global__ void __launch_bounds__(" << kLevelThreads << ", " << kLevelBlocks
-      << ") gbh_jit(const __grid_constant__ DevView v, const __grid_constant__ LevelView L, int g0, int nsteps, "
-      << "long long step0)\n{\n"
+      << ") gbh_jit(DevView v, LevelView L, int g0, int nsteps, long long step0)\n{\n"
       << "  extern __shared__ double sm[];\n"
       << "  const LevelGroup g = L.groups[g0 + blockIdx.x];\n"
       << "  { unsigned dsz; asm(\"mov.u32 %0, %%dynamic_smem_size;\" : \"=r\"(dsz));\n"
@@ -1121,7 +1121,7 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
       << "  const unsigned sgen = v.sgen ? *v.sgen : 0u;\n"
       << "  if (threadIdx.x < blockDim.x - 32) {\n"
       << "    const bool full = !v.sgen || L.gen[g0 + blockIdx.x] != sgen, refresh = *v.kref != 0;\n"
-      << "    level_sweep<" << form << ", " << crank << ", " << N << ", " << res << ">(v, L, g, tl, ty, sm, nsteps, (v.step_dev ? *v.step_dev : 0) + step0, full, refresh);\n"
+      << "    level_sweep<" << form << ", " << crank << ", " << N << ", " << res << (io ? ", true" : "") << ">(v, L, g, tl, ty, sm, nsteps, (v.step_dev ? *v.step_dev : 0) + step0, full, refresh);\n"
       << "    if (full && v.sgen && threadIdx.x == 0) L.gen[g0 + blockIdx.x] = sgen;\n    return;\n  }\n"
       << "  const int lid = threadIdx.x & 31; const bool active = lid < g.nlanes; const int lane = g.lane0 + (active ? lid : 0);\n"
       << "  const long long sbase = v.step_dev ? *v.step_dev : 0;\n"
@@ -1152,7 +1152,9 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
       << ">(sm, g);\n  double *U = q.U + lid;\n  unsigned lost = 0u; (void)lost;\n"
       << "  for (int it = 0; it < nsteps; ++it) {\n"
       << "    const long long step = sbase + step0 + it; (void)step;\n"
-      << "    if (v.io_in) { level_in<" << form << ">(v, L, g.tile, g.lane0, g.nlanes, g.eoff, step, lid, 32, nullptr); __syncwarp(); }\n"
+      << (io ? std::string("    if (v.io_in) { level_in<") + form +
+                   ">(v, L, g.tile, g.lane0, g.nlanes, g.eoff, step, lid, 32, nullptr); __syncwarp(); }\n"
+             : std::string())
       << "    double D[" << N << "], R[" << N << "], T[" << N << "], PD[" << N << "]; (void)T; (void)PD;\n"
       << "    if (active) {\n";
     if (mixed) {
@@ -1196,7 +1198,8 @@ std::string jit_level_source(const LevelProg &lp, const TileType &tt, const Tabl
         o << " }\n";
     }
     o << "    }\n    __syncwarp();\n    bar_named(LB_TOP, blockDim.x);\n"
-      << "    if (v.io_out) level_out(v, L, g.tile, g.lane0, g.nlanes, step, lid, 32, nullptr);\n  }\n  lost_rows(v, lost, active);\n}\n";
+      << (io ? "    if (v.io_out) level_out(v, L, g.tile, g.lane0, g.nlanes, step, lid, 32, nullptr);\n" : "")
+      << "  }\n  lost_rows(v, lost, active);\n}\n";
     return o.str();
 }
 

@@ -42,8 +42,10 @@ struct LevelProg {
 };
 LevelProg level_prog(const TileType &tt, const std::vector<int> &prog);
 // Source of the level-elimination kernel (entry gbh_jit) for one such program.
-// resident: the block keeps its rows' constants in shared memory.
-std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed, bool resident);
+// resident: the block keeps its rows' constants in shared memory; io: with
+// per-step inputs and outputs.
+std::string jit_level_source(const LevelProg &lp, const TileType &tt, const TableGeom &tg, bool mixed, bool resident,
+                             bool io);
 cudaError_t jit_level_launch(const JitKernel &k, const DevView &v, const LevelView &lv, int g0, int ngroups, int warps,
                              int nsteps, long long step, size_t smem, cudaStream_t st);
 // A type's compartments as the row-parallel kernel runs them (gbh_rows.cuh):

@@ -128,10 +128,9 @@ template <bool MIXED> __device__ __forceinline__ double level_kterm(const double
 
 // A step's inputs into the fields of a group (lanes [lane0, lane0 + nlanes) of
 // the tile) by `nt` threads: of its static rows, whose rhs terms in kt follow,
-// or, kt null, of the rows above them. Out of line, as level_out: within the
-// steps they took 10 to 20 registers more.
+// or, kt null, of the rows above them.
 template <bool MIXED>
-__device__ __noinline__ void level_in(const DevView &v, const LevelView &L, int tile, int lane0, int nlanes,
+__device__ __forceinline__ void level_in(const DevView &v, const LevelView &L, int tile, int lane0, int nlanes,
                                       int64_t eoff, long long step, int tid, int nt, double2 *kt)
 {
     const Tile &tl = v.tiles[tile];
@@ -153,7 +152,7 @@ __device__ __noinline__ void level_in(const DevView &v, const LevelView &L, int 
 
 // A step's outputs of a group: of its static rows from their solutions X, or, X
 // null, of the rows above them, whose warp has stored their Vm.
-__device__ __noinline__ static void level_out(const DevView &v, const LevelView &L, int tile, int lane0, int nlanes,
+__device__ __forceinline__ void level_out(const DevView &v, const LevelView &L, int tile, int lane0, int nlanes,
                                               long long step, int tid, int nt, const double *X)
 {
     double *dst = v.io_out + (step - v.io_step0) * v.io_nout;
@@ -166,8 +165,10 @@ __device__ __noinline__ static void level_out(const DevView &v, const LevelView 
 }
 
 // What the sweeping warps of a block do in a launch (sm: level_smem bytes).
-// MANY: a row may have more than two static children.
-template <bool MIXED, bool CRANK, int NTOP, bool RES, bool MANY>
+// MANY: a row may have more than two static children. IO: per-step inputs and
+// outputs, in a kernel of their own: with them the others' steps took up to
+// 12 % longer (10 to 20 registers more a thread).
+template <bool MIXED, bool CRANK, int NTOP, bool RES, bool IO, bool MANY>
 __device__ __forceinline__ void level_steps(const DevView &v, const LevelView &L, const LevelGroup &g,
                                             const LevelSm &q, int nsteps, long long step0)
 {
@@ -192,7 +193,7 @@ __device__ __forceinline__ void level_steps(const DevView &v, const LevelView &L
     // what does not wait for the level before is read and formed meanwhile:
     // the next level's constants, its Vm + K forward and, mixed, R / D'
     // backward, and the descriptors two chunks ahead.
-    const bool put = v.io_in && L.io[g.tile].x, take = v.io_out && L.io[g.tile].y;
+    const bool put = IO && v.io_in && L.io[g.tile].x, take = IO && v.io_out && L.io[g.tile].y;
     for (int it = 0; it < nsteps; ++it) {
         if (put) {
             level_in<MIXED>(v, L, g.tile, g.lane0, g.nlanes, g.eoff, step0 + it, tid, nt, RES ? q.kt : L.kt + g.eoff);
@@ -302,7 +303,7 @@ __device__ __forceinline__ void level_steps(const DevView &v, const LevelView &L
     }
 }
 
-template <bool MIXED, bool CRANK, int NTOP, bool RES>
+template <bool MIXED, bool CRANK, int NTOP, bool RES, bool IO = false>
 __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L, const LevelGroup &g, const Tile &tl,
                                             const TileType &ty, double *sm, int nsteps, long long step0, bool full,
                                             bool refresh)
@@ -364,8 +365,8 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
             q.par[e] = par[e];
         }
     bar_named(LB_SWEEP, nt);
-    if (g.many) level_steps<MIXED, CRANK, NTOP, RES, true>(v, L, g, q, nsteps, step0);
-    else level_steps<MIXED, CRANK, NTOP, RES, false>(v, L, g, q, nsteps, step0);
+    if (g.many) level_steps<MIXED, CRANK, NTOP, RES, IO, true>(v, L, g, q, nsteps, step0);
+    else level_steps<MIXED, CRANK, NTOP, RES, IO, false>(v, L, g, q, nsteps, step0);
     bar_named(LB_SWEEP, nt);
     for (int e = tid; e < g.n; e += nt) V[map[e]] = O[e];
 }
