@@ -878,7 +878,7 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
         tt.lv_f0 = lp.f0;
         ntop[ti] = lp.ntop;
         const bool res = resident(tt, lp.ntop);
-        for (int io = 0; io < 2; ++io) {
+        for (int io = 0; io < (e->trial ? 1 : 2); ++io) {
             std::string &src = srcs[4 * it->second + (res ? 0 : 2) + io];
             if (src.empty()) src = jit_level_source(lp, tt, tg[tt.table_set], mixed, res, io != 0);
         }
@@ -902,7 +902,7 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
         TileType &tt = e->types[ti];
         if (!tt.level) continue;
         const int k = 4 * (tt.level - 1) + (resident(tt, ntop[ti]) ? 0 : 2);
-        if (ok[k] && ok[k + 1]) cells += (int64_t)members[ti].size();
+        if (ok[k] && (e->trial || ok[k + 1])) cells += (int64_t)members[ti].size();
         else tt.level = 0;   // keeps the stack elimination
     }
     // ---- groups: enough of them for every SM, as many neurons each as that
@@ -2427,11 +2427,12 @@ int autotune_trials(gbh_engine *e)
         if (per < best) { best = per; best_s = spl; }
     }
     // single steps: a level launch reads its rows' constants first, which only
-    // pays over several steps where the batch is large (20,000 trees of 96
-    // compartments, us for one step: levels 127, lanes 102)
-    bool level = false;
-    for (const Launch &L : e->launches) level = level || L.level >= 0;
-    if (level) {
+    // pays over several steps where the SMs have several blocks to run (20,000
+    // trees of 96 compartments, us for one step: levels 127, lanes 102)
+    int level_groups = 0;
+    for (const Launch &L : e->launches)
+        if (L.level >= 0) level_groups += L.tile1 - L.tile0;
+    if (level_groups > e->nsm) {
         double by_level, by_lane;
         if (timed(1, 1e300, by_level)) return GBH_ERR_CUDA;
         e->launches.swap(e->lane_launches);
