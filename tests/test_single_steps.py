@@ -40,7 +40,7 @@ def test_alternating_run_lengths(oracle, gpu_engine, monkeypatch, capfd, batch):
     monkeypatch.setenv("GBH_VERBOSE", "1")
     eng = gpu_engine.Engine(hs, wide_min=-1)
     err = capfd.readouterr().err
-    if "level elimination\n" in err:
+    if "level elimination\n" in err and batch != "few":       # (a few blocks have the SMs to themselves: not timed)
         assert re.search(r"trial single steps: level elimination [\d.]+ us/step, lanes [\d.]+", err), err
     idx = sorted(set(range(0, len(hs), max(1, len(hs) // 7))) | {len(hs) - 1})
     refs = {i: oracle.Solver(hs[i]) for i in idx}
