@@ -390,7 +390,7 @@ k_adj_reverse(AdjView v, AdjPlan pl, int hmax, int nk, int step0)
         // back substitution reversed, children before their parents
         for (int c = g.nch - 1; c >= 0; --c) {
             const int2 m = ch[c];
-            if (tid < (m.y & ADJ_COUNT)) {
+            if (tid < (m.y & CHUNK_COUNT)) {
                 const int e = m.x + tid, k0 = link[e].x & 0xffff, nkid = link[e].x >> 16;
                 double *q = tp + map[e];
                 const double rd = __ldg(q + R.RD * LANES), x = __ldg(q + R.X * LANES);
@@ -402,12 +402,12 @@ k_adj_reverse(AdjView v, AdjPlan pl, int hmax, int nk, int step0)
                 Db[e] = -x * rb;
                 q[R.RBBS * LANES] = rb;
             }
-            if (m.y & ADJ_FIRST) __syncthreads();
+            if (m.y & CHUNK_FIRST) __syncthreads();
         }
         // forward elimination reversed, parents before their children
         for (int c = 0; c < g.nch; ++c) {
             const int2 m = ch[c];
-            if (tid < (m.y & ADJ_COUNT)) {
+            if (tid < (m.y & CHUNK_COUNT)) {
                 const int e = m.x + tid, p = link[e].y;
                 if (p < n) {
                     const double *q = tp + map[e];
@@ -417,7 +417,7 @@ k_adj_reverse(AdjView v, AdjPlan pl, int hmax, int nk, int step0)
                     Db[e] -= tt * (tb * rd);
                 }
             }
-            if (m.y & ADJ_LAST) __syncthreads();
+            if (m.y & CHUNK_LAST) __syncthreads();
         }
         // channels reversed (adjoint of Vm and of the gate states), then the
         // seed of step k-1

@@ -110,12 +110,11 @@ struct AdjView {
 
 // Row order of the reverse sweep: a block's share of a tile, lanes [lane0,
 // lane0 + nlanes), their n rows by depth at elements eoff, in nch chunks (first
-// row, rows | ADJ_FIRST | ADJ_LAST of a level) of at most the block's threads.
+// row, rows | CHUNK_FIRST | CHUNK_LAST of a level) of at most the block's threads.
 struct AdjGroup {
     int tile, lane0, nlanes, n, nch, choff;
     int64_t eoff;
 };
-constexpr int ADJ_FIRST = 1 << 30, ADJ_LAST = 1 << 29, ADJ_COUNT = (1 << 29) - 1;
 constexpr int ADJ_REV_THREADS = 512, ADJ_COPY_ROWS = 8;
 struct AdjPlan {
     const AdjGroup *groups;

@@ -139,15 +139,15 @@ __device__ __forceinline__ void prefetch_l1(const void *p)
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
-// One synaptic event, counted in the target synchan's ring slot for the step
-// it acts in; for a weighted synchan also its synapse's rank bit.
 // step % ring_len (the 64-bit remainder is a call of some 100 instructions)
 __device__ __forceinline__ int ring_phase(long long step, int ring_len)
 {
     return (unsigned long long)step >> 32 ? (int)(step % ring_len) : (int)((unsigned)step % (unsigned)ring_len);
 }
 
-// One event, `delay` steps (less than ring_len) after the step at `phase`.
+// One synaptic event, counted in the target synchan's ring slot for the step
+// it acts in, `delay` steps (less than ring_len) after the step at `phase`; for
+// a weighted synchan also its synapse's rank bit.
 __device__ __forceinline__ void put_event(unsigned *ring, int ring_len, unsigned *wmask, int64_t base, int delay,
                                           int64_t mword, int mbit, int phase)
 {

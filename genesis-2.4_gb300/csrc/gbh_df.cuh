@@ -95,18 +95,6 @@ __device__ __forceinline__ df df_div(df x, df y)
 }
 
 // ---- exact conversions on the integer pipe --------------------------------
-// float -> double (normal floats and zero; denormals flush to signed zero)
-__device__ __forceinline__ double f2d_bits(float f)
-{
-    const uint32_t u = __float_as_uint(f);
-    const uint32_t sign = u & 0x80000000u;
-    const uint32_t e = (u >> 23) & 0xffu;
-    const uint32_t m = u & 0x7fffffu;
-    const uint32_t hi = (e == 0u) ? sign : (sign | ((e + 896u) << 20) | (m >> 3));
-    const uint32_t lo = (e == 0u) ? 0u : (m << 29);
-    return __hiloint2double((int)hi, (int)lo);
-}
-
 // double -> float truncated toward zero (exact when the double already has at
 // most 24 significant bits; values below the float normal range flush to 0)
 __device__ __forceinline__ float d2f_trunc_bits(double d)

@@ -315,23 +315,6 @@ int micro_operands(int code)
     }
 }
 
-// Which operands of a micro-op are field rows (bit i: operand i).
-int field_operands(int code)
-{
-    switch (code) {
-    case M_BEGIN: return 0x7;
-    case M_DOMAIN: case M_SCALE_FLUX: case M_SAME_GHK: case M_CHAN_G: return 0x1;
-    case M_SPIKE: return 0x1;
-    case M_ELMMPUMP: return 0x7;
-    case M_GHK: return 0x7;
-    case M_NERNST: case M_CHAN: case M_END: case M_ITLEAK: return 0x3;
-    case M_GATE: return 0x8;
-    case M_SYN: return 0x39;
-    case M_MGBLOCK: return 0x7;
-    default: return 0;
-    }
-}
-
 // Per slot of a type's program, 6 ints for the stack kernels: the first and
 // last field row it reads (rows are allocated in program order, so a slot's
 // fields are mostly one contiguous range; prefetched a few rows ahead), and
@@ -970,8 +953,8 @@ int level_plan(gbh_engine *e, const std::vector<std::vector<int>> &members, cons
             for (int d = 0; d < nlev; ++d)
                 for (int a = start[d]; a < start[d + 1]; a += nt) {
                     const int n = std::min(nt, start[d + 1] - a);
-                    P.chunks.push_back(make_int2(a, n | (a == start[d] ? LV_FIRST : 0) |
-                                                        (a + n == start[d + 1] ? LV_LAST : 0)));
+                    P.chunks.push_back(make_int2(a, n | (a == start[d] ? CHUNK_FIRST : 0) |
+                                                        (a + n == start[d + 1] ? CHUNK_LAST : 0)));
                 }
             g.nch = (int)P.chunks.size() - g.choff;
             std::vector<int> &place = e->lv_place[t];
@@ -1074,15 +1057,15 @@ TreeOrder tree_order(const std::vector<const Neuron *> &cl, int S)
     return o;
 }
 
-// The levels of a tree order in chunks of at most nt rows (RW_FIRST, RW_LAST).
+// The levels of a tree order in chunks of at most nt rows (CHUNK_FIRST, CHUNK_LAST).
 int tree_chunks(const TreeOrder &o, int nt, std::vector<int2> &chunks)
 {
     const size_t c0 = chunks.size();
     for (size_t d = 0; d + 1 < o.start.size(); ++d)
         for (int a = o.start[d]; a < o.start[d + 1]; a += nt) {
             const int m = std::min(nt, o.start[d + 1] - a);
-            chunks.push_back(make_int2(a, m | (a == o.start[d] ? RW_FIRST : 0) |
-                                              (a + m == o.start[d + 1] ? RW_LAST : 0)));
+            chunks.push_back(make_int2(a, m | (a == o.start[d] ? CHUNK_FIRST : 0) |
+                                              (a + m == o.start[d + 1] ? CHUNK_LAST : 0)));
         }
     return (int)(chunks.size() - c0);
 }
@@ -3867,7 +3850,6 @@ static int adj_plan(gbh_engine *e, int hmax)
             l0 += nl;
         }
     }
-    static_assert(RW_FIRST == ADJ_FIRST && RW_LAST == ADJ_LAST, "tree_chunks serves both");
     if (e->d_agroups.upload(groups) || e->d_achunks.upload(chunks) || e->d_alink.upload(link) || e->d_amap.upload(map)) {
         e->d_agroups.release(); e->d_achunks.release(); e->d_alink.release(); e->d_amap.release();
         return GBH_ERR_CUDA;

@@ -150,6 +150,11 @@ struct TileType {
 // stack tile computes in shared memory while the first sweeps the static rows
 constexpr int kSplitRows = 8;
 
+// Chunks of rows of a tree taken depth by depth (first row, rows | flags): the
+// first and the last one of a level. A sweep from the leaves (descending) ends
+// a level at its first chunk, one from the root (ascending) at its last.
+constexpr int CHUNK_FIRST = 1 << 30, CHUNK_LAST = 1 << 29, CHUNK_COUNT = (1 << 29) - 1;
+
 enum StackFlag {
     FL_NPOP = 0xff,          // stack entries to apply: children other than the last
     FL_CARRY_IN = 1 << 8,    // the previous row is this row's last child

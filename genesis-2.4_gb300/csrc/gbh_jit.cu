@@ -850,26 +850,34 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
     return t.str();
 }
 
+int field_operands(int code)
+{
+    switch (code) {
+    case M_BEGIN: case M_ELMMPUMP: case M_GHK: case M_MGBLOCK: return 0x7;
+    case M_DOMAIN: case M_SCALE_FLUX: case M_SAME_GHK: case M_CHAN_G: case M_SPIKE: return 0x1;
+    case M_NERNST: case M_CHAN: case M_END: case M_ITLEAK: return 0x3;
+    case M_GATE: return 0x8;
+    case M_SYN: return 0x39;
+    default: return 0;
+    }
+}
+
 namespace {
 
-// Operands that are field rows (bit i: operand i) and the givals row (-1
-// none) of the ops a step without givals may hold.
+// Field operands and the givals operand (-1 none) of the ops the level and
+// row-parallel kernels may hold.
 bool op_roles(int code, int &fields, int &giv)
 {
-    fields = 0;
+    fields = field_operands(code);
     giv = -1;
     switch (code) {
-    case M_BEGIN: fields = 0x7; giv = 3; return true;
-    case M_NEWVOLT: case M_NEWCONC1: case M_FLUX: case M_DO_TABGHK: case M_CONCVAL: case M_NEWCONC2: return true;
-    case M_DOMAIN: case M_SCALE_FLUX: case M_SAME_GHK: case M_CHAN_G: case M_SPIKE: fields = 0x1; return true;
-    case M_ELMMPUMP: fields = 0x7; giv = 3; return true;
-    case M_GHK: fields = 0x7; return true;
-    case M_NERNST: case M_CHAN: fields = 0x3; return true;
-    case M_END: fields = 0x3; giv = 2; return true;
-    case M_GATE: fields = 0x8; return true;
-    case M_SYN: fields = 0x39; return true;
-    case M_MGBLOCK: fields = 0x7; giv = 3; return true;
+    case M_BEGIN: case M_ELMMPUMP: case M_MGBLOCK: giv = 3; return true;
+    case M_END: giv = 2; return true;
     case M_ADDCURR: giv = 0; return true;
+    case M_NEWVOLT: case M_NEWCONC1: case M_FLUX: case M_DO_TABGHK: case M_CONCVAL: case M_NEWCONC2: case M_DOMAIN:
+    case M_SCALE_FLUX: case M_SAME_GHK: case M_CHAN_G: case M_SPIKE: case M_GHK: case M_NERNST: case M_CHAN:
+    case M_GATE: case M_SYN:
+        return true;
     default: return false;
     }
 }

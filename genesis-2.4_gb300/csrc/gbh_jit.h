@@ -29,6 +29,9 @@ std::string jit_source(const TileType &tt, const std::vector<int> &prog, const T
                        const std::vector<int> *uniform_parent, int min_blocks = 4, bool compact = false,
                        bool smem_rows = false, int warps = 4);
 
+// Which operands of a micro-op are field rows (bit i: operand i).
+int field_operands(int code);
+
 // The rows above a type's static ones as the level-elimination kernel runs
 // them (gbh_level.cuh): their programs and the pool program with field rows
 // relative to `f0`, so that types which differ only in their dendrites share

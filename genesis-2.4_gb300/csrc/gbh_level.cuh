@@ -32,7 +32,7 @@ namespace gbh {
 // A block's share of a tile: lanes [lane0, lane0 + nlanes), their n static
 // rows at elements eoff of the level-ordered arrays (LV_SPARE more behind
 // them), in nch chunks of at most blockDim - 32 rows (first row, rows |
-// LV_FIRST | LV_LAST; LV_GUARD empty ones before and behind them).
+// CHUNK_FIRST | CHUNK_LAST; LV_GUARD empty ones before and behind them).
 struct LevelGroup {
     int tile, lane0, nlanes, n, nch, choff;
     int kidoff;      // the top rows' static children: topkid[kidoff + s * 32 + lane]
@@ -40,9 +40,6 @@ struct LevelGroup {
     int64_t eoff;
 };
 
-// First and last chunk of a level: the forward sweep (descending) ends a
-// level at its first chunk, the backward one (ascending) at its last.
-constexpr int LV_FIRST = 1 << 30, LV_LAST = 1 << 29, LV_COUNT = (1 << 29) - 1;
 // The sweeps read the descriptors two chunks ahead.
 constexpr int LV_GUARD = 2;
 // Spare elements behind a group's rows: a zero (what a row without children
@@ -182,8 +179,8 @@ __device__ __forceinline__ void level_steps(const DevView &v, const LevelView &L
     // mixed: a parent subtracts R T in one multiply-add, T from its child's
     // constants; FP64: the child leaves R T in PR
     const double *const pulled = MIXED ? X : PR;
-    auto element = [&](int2 m) { return tid < (m.y & LV_COUNT) ? m.x + tid : spare; };
-    auto busy = [&](int2 m) { return (tid & ~(LANES - 1)) < (m.y & LV_COUNT); };   // a warp with rows
+    auto element = [&](int2 m) { return tid < (m.y & CHUNK_COUNT) ? m.x + tid : spare; };
+    auto busy = [&](int2 m) { return (tid & ~(LANES - 1)) < (m.y & CHUNK_COUNT); };   // a warp with rows
     auto sync = [&]() {
         if (nt == LANES) __syncwarp();
         else bar_named(LB_SWEEP, nt);
@@ -236,7 +233,7 @@ __device__ __forceinline__ void level_steps(const DevView &v, const LevelView &L
                 ownn = O[en] + a.x;
                 Tn = a.y;
             }
-            if (m.y & LV_FIRST) sync();
+            if (m.y & CHUNK_FIRST) sync();
             k = kn;
             T = Tn;
             own = ownn;
@@ -286,7 +283,7 @@ __device__ __forceinline__ void level_steps(const DevView &v, const LevelView &L
                 if (!MIXED) Dn = dd[en];
                 if (CRANK) oldn = O[en];
             }
-            if (m.y & LV_LAST) sync();
+            if (m.y & CHUNK_LAST) sync();
             a = an;
             D = Dn;
             own = on;
@@ -330,7 +327,7 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
         const double *A = v.A + tl.topo * LANES, *B = v.B + tl.topo * LANES;
         for (int c = nch - 1; c >= 0; --c) {
             const int2 m = ch[c];
-            if (tid < (m.y & LV_COUNT)) {
+            if (tid < (m.y & CHUNK_COUNT)) {
                 const int e = m.x + tid, r = map[e], l = r % LANES;
                 const int *ps = pf + 6 * (r / LANES);
                 double D;
@@ -347,7 +344,7 @@ __device__ __forceinline__ void level_sweep(const DevView &v, const LevelView &L
                 cy[e] = make_double2(MIXED ? L.c[g.eoff + e] * y : L.c[g.eoff + e], y);
                 if (!MIXED) dd[e] = D;
             }
-            if (m.y & LV_FIRST) bar_named(LB_SWEEP, nt);
+            if (m.y & CHUNK_FIRST) bar_named(LB_SWEEP, nt);
         }
     } else if (refresh) {   // inputs on the rhs fields: their terms once per launch
         for (int e = tid; e < g.n; e += nt) kt[e].x = level_kterm<MIXED>(P, pf, map[e]);

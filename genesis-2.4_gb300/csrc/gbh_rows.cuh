@@ -21,14 +21,12 @@ namespace gbh {
 
 // A block's share of a tile: lanes [lane0, lane0 + nlanes), their n rows at
 // elements eoff of the level-ordered arrays, nch chunks of at most blockDim
-// rows (first, rows | RW_LAST at the last of a level), nitems runs of up to 32
+// rows (first, rows | CHUNK_LAST at the last of a level), nitems runs of up to 32
 // rows of one program class.
 struct RowGroup {
     int tile, lane0, nlanes, n, nch, choff, nitems, itoff;
     int64_t eoff;
 };
-
-constexpr int RW_FIRST = 1 << 30, RW_LAST = 1 << 29, RW_COUNT = (1 << 29) - 1;
 
 struct RowView {
     const RowGroup *groups;
@@ -164,11 +162,11 @@ __device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup 
 {
     const int tid = threadIdx.x;
     int2 m = q.ch[g.nch - 1];
-    int e = tid < (m.y & RW_COUNT) ? m.x + tid : -1, lk = 0;
+    int e = tid < (m.y & CHUNK_COUNT) ? m.x + tid : -1, lk = 0;
     double a = 0.0, b = 0.0, D = 0.0, R = 0.0;
     auto own = [&](int c) {   // the row of chunk c this thread takes
         m = q.ch[c];
-        e = tid < (m.y & RW_COUNT) ? m.x + tid : -1;
+        e = tid < (m.y & CHUNK_COUNT) ? m.x + tid : -1;
         if (e >= 0) {
             lk = q.link[e].x;
             a = q.A[e];
@@ -179,7 +177,7 @@ __device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup 
     };
     own(g.nch - 1);
     for (int c = g.nch - 1; c >= 0; --c) {
-        const int first = m.y & RW_FIRST;
+        const int first = m.y & CHUNK_FIRST;
         if (e >= 0) {
             const int k0 = lk & 0xffff, nk = lk >> 16;
             for (int k = k0; k < k0 + nk; ++k) {
@@ -201,7 +199,7 @@ __device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup 
     double cc = 0.0, y = 0.0;
     auto back = [&](int c) {
         m = q.ch[c];
-        e = tid < (m.y & RW_COUNT) ? m.x + tid : -1;
+        e = tid < (m.y & CHUNK_COUNT) ? m.x + tid : -1;
         if (e >= 0) {
             p = q.link[e].y;
             cc = q.C[e];
@@ -212,7 +210,7 @@ __device__ __forceinline__ void rows_eliminate(const DevView &v, const RowGroup 
     };
     back(0);
     for (int c = 0; c < g.nch; ++c) {
-        const int last = m.y & RW_LAST;
+        const int last = m.y & CHUNK_LAST;
         if (e >= 0) {
             const double xp = q.R[p];
             double r;
