@@ -3302,7 +3302,8 @@ Served kernels_serve(const gbh_engine *e)
         if (N.nrows < 32) continue;
         sv.level = sv.level || level;
         sv.rows = sv.rows || rows;
-        surely = surely &&
+        // (without a stack plan the lane-mapped kernels, which steps with givals run, may not hold the neuron)
+        surely = surely && tt.stack &&
                  ((level && branched(m.size(), tt.nstatic, [&](size_t i) -> const std::vector<int> & {
                        return m[i]->parent;
                    })) ||

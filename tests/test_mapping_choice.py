@@ -87,3 +87,16 @@ def test_channels_everywhere_compile_no_lane_kernels(oracle, gpu_engine, monkeyp
     assert eng.stats().jit_kernels == 1, err
     assert "mapping trial" not in err and "form 0" not in err, err
     _check(eng, oracle, hs)
+
+
+@pytest.mark.parametrize("active", [True, False])
+def test_many_dendrites_on_one_soma(oracle, gpu_engine, monkeypatch, capfd, active):
+    """450 dendrites on the soma are more than a lane's elimination stack holds
+    and than its shared-memory columns do: only some mappings take the neuron."""
+    m = configs.cables(1, ncomp=451, gk_dend=36.0 if active else 0.0, per_neuron_solvers=True)[0]
+    for c in m.compartments[1:]:
+        c.parent = 0
+    hs = [model.build(m) for _ in range(3)]
+    eng, err = _create(gpu_engine, monkeypatch, capfd, hs)
+    assert "mapping trial wide_min 32" in err, err
+    _check(eng, oracle, hs, 20)
