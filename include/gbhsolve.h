@@ -176,9 +176,11 @@ typedef struct gbh_options {
                             without a trial, else as 1; -1 = interpret the
                             programs. With 0 (no synapses), trees whose
                             dendrites are passive are eliminated level by
-                            level over several warps, and for small batches
-                            with channels along the dendrites the autotuner
-                            also times a thread per compartment               */
+                            level over several warps, and small batches with
+                            channels along the dendrites run a thread per
+                            compartment; where either may be the slower, or
+                            there are more than eight programs of a kind, it
+                            is timed against the other mappings               */
     int wide_min;        /* neurons with at least this many compartments run
                             one per warp, compartments across its threads;
                             the other large neurons run 32 per warp, one per
@@ -187,7 +189,8 @@ typedef struct gbh_options {
                             an interpreted engine per candidate times a few
                             steps; with jit 0 the chosen mapping is also timed
                             specialised, and specialisation is turned off
-                            when it is slower); < 0 = never
+                            when it is slower; no trial where the kernels
+                            under jit are certain to win); < 0 = never
                             (gbh_loss_gradient needs it)                      */
 } gbh_options;
 
@@ -364,11 +367,14 @@ int gbh_io_sync(gbh_engine *e);
  * rows of the registered outputs (row k after step k). Each block of `block`
  * steps (0 = 16) is copied host->device in one transfer on a copy stream
  * while the previous block steps, and its outputs device->host in one
- * transfer while the next block steps; between two steps one kernel gathers
- * the outputs and scatters the next inputs. Staging is double-buffered on
+ * transfer while the next block steps; the step kernels apply the inputs and
+ * gather the outputs themselves where they can, else one kernel does between
+ * two steps. Staging is double-buffered on
  * the device (2 x block x (n_in + n_out) doubles). Either pointer may be
  * NULL. Returns when host_out is complete. Results equal nsteps rounds of
- * gbh_set_inputs_async + gbh_run_async(1) + gbh_get_outputs_async. Host
+ * gbh_set_inputs_async + gbh_run_async(1) + gbh_get_outputs_async (in the
+ * mixed form to rounding: large batches of trees with passive dendrites may
+ * take another kernel for single steps than for runs of several). Host
  * buffers should be pinned for the copies to overlap. Serves h_in_msgs /
  * h_out_msgs-style stimulus and recording for a whole run (the reference
  * runs both on the host every step, hines_msgs.c:351-486).
