@@ -2193,7 +2193,8 @@ int run_graph(gbh_engine *e, int nsteps, cudaStream_t st)
 // the reset of the barrier's words cost more than they save below (4,000 point
 // neurons, us a run, per-step launches against cooperative: 4 steps 55.4 and
 // 56.4, 6 steps 73.1 and 72.4, 8 steps 90.9 and 89.3, 64 steps 580 and 528).
-constexpr int kCoopMin = 6;
+// Replayed from a graph the per-step launches cost less: 8 steps 76.8 and 82.
+constexpr int kCoopMin = 6, kCoopMinGraph = 16;
 
 // Networks: K steps per cooperative launch over every tile, a grid barrier
 // between steps (events cross tiles): the specialised kernel where one serves
@@ -2246,7 +2247,7 @@ int run_steps(gbh_engine *e, int nsteps, cudaStream_t st)
         if (rci) return rci;
     }
     if (e->net_coop && !e->givals_enabled && e->nremote == 0 &&
-        (nsteps >= kCoopMin || e->opt.steps_per_launch < 0)) {
+        (nsteps >= (e->opt.use_graph ? kCoopMinGraph : kCoopMin) || e->opt.steps_per_launch < 0)) {
         e->dstep_valid = false;
         return run_coop(e, nsteps, st);
     }
@@ -2281,7 +2282,7 @@ struct OnDevice {
     OnDevice &operator=(const OnDevice &) = delete;
 };
 
-int autotune_trials(gbh_engine *e);
+int autotune_trials(gbh_engine *e, bool graphs);
 
 // Autotuner: times trial steps for every (kernel variant, steps per launch)
 // candidate on the live engine, saving the mutable state first and restoring
@@ -2290,7 +2291,7 @@ int autotune(gbh_engine *e)
 {
     const int use_graph = e->opt.use_graph;
     e->opt.use_graph = 0;   // trials time plain launches; graphs are captured afterwards
-    const int rc_t = autotune_trials(e);
+    const int rc_t = autotune_trials(e, use_graph != 0);
     e->opt.use_graph = use_graph;
     drop_graphs(e);
     e->dstep_valid = false;
@@ -2303,7 +2304,8 @@ int autotune(gbh_engine *e)
     return rc_t;
 }
 
-int autotune_trials(gbh_engine *e)
+// graphs: runs of the chosen plan are captured and replayed.
+int autotune_trials(gbh_engine *e, bool graphs)
 {
     std::vector<int> spls;
     if (e->has_network) spls = {1};
@@ -2432,6 +2434,24 @@ int autotune_trials(gbh_engine *e)
     if (e->has_network && e->nremote == 0 && e->d_gbar.p && !any_wide && !e->spike_pre) {
         e->steps_per_launch = best_s;
         int coop_k = 0;
+        if (graphs) {   // against the replay of a captured run (10 neurons, mixed, us a step: 4.0, launches 6.2, cooperative 4.8)
+            const int steps = 128;
+            e->opt.use_graph = 1;
+            int rc_g = run_steps(e, steps, e->stream);   // captures
+            CK(cudaEventRecord(e->ev0, e->stream));
+            if (rc_g == GBH_OK) rc_g = run_steps(e, steps, e->stream);
+            CK(cudaEventRecord(e->ev1, e->stream));
+            CK(cudaEventSynchronize(e->ev1));
+            e->opt.use_graph = 0;
+            e->dstep_valid = false;
+            float ms = 0.f;
+            CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
+            if (rc_g == GBH_OK) best = std::min(best, (double)ms / steps);
+            else cudaGetLastError();
+            if (getenv("GBH_VERBOSE"))
+                fprintf(stderr, "gbhsolve: trial graph replay: %.2f us/step\n", ms / steps * 1e3);
+            if (restore()) return GBH_ERR_CUDA;
+        }
         for (int K : {16, 64}) {
             e->net_coop = true;
             e->net_spl = K;
@@ -3590,11 +3610,14 @@ int gbh_run(gbh_engine *e, int nsteps)
 // the host took 8 ms, more than 200 steps. On the default stream, as the
 // other copies of gbh_get_state: it waits for the caller's blocking streams.
 // That stream is the current device's, whatever engine the call names.
+constexpr int64_t kVmByHost = 64;
+
 static int get_vm(gbh_engine *e, double *vm)
 {
     const int64_t n = e->vm_start.back();
     if (n == 0) return GBH_OK;
-    if (e->d_vm_at.p) {
+    // (a few rows are walked here sooner than a kernel is launched)
+    if (e->d_vm_at.p && n > kVmByHost) {
         const OnDevice on(e->opt.device);
         CK(on.rc);
         k_gather_vm<<<(unsigned)((n + 255) / 256), 256>>>(e->d_V.p, e->d_vm_at.p, n, e->d_vm_out.p);
